@@ -151,8 +151,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                    const DecodeArgs a, uint32_t* error_word) {
   using Cfg = DecodeCfg<BT>;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* tiles = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
+  unsigned char* tiles = align_tiles(smem_raw);
   const int S = a.splits, stages = a.stages;
   float* aux = reinterpret_cast<float*>(tiles + (size_t)stages * Cfg::kStageBytes);
   float* s_recv = aux;  // [S - 1][slice][128]

@@ -55,8 +55,7 @@ gemm_persistent_pair(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const uint32_t r = cluster_ctarank();
   const int pair = cta >> 1, npairs = ncta >> 1;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* tiles = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
+  unsigned char* tiles = align_tiles(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + kStages * Cfg::kStageBytes);
   uint64_t* full = bars;                         // used in the leader only
   uint64_t* empty = bars + kStages;              // one in each CTA

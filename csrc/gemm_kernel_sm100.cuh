@@ -106,8 +106,7 @@ gemm_persistent(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   constexpr int kStages = Cfg::kStages;
   extern __shared__ unsigned char smem_raw[];
   // tiles need 1024-byte alignment for the 128-byte swizzle
-  unsigned char* tiles = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
+  unsigned char* tiles = align_tiles(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + kStages * Cfg::kStageBytes);
   uint64_t* full = bars;
   uint64_t* empty = bars + kStages;
