@@ -623,23 +623,25 @@ sm100::DecodePush Communicator::fused_norm_push_target(int rows, int hidden, int
   return p;
 }
 
-void Communicator::moe_dispatch(int dtype, const MoeArgs* args, const Tuning& t, cudaStream_t stream) {
+LaunchCfg Communicator::moe_cfg(const Tuning& t, cudaStream_t stream) const {
   LaunchCfg cfg;
   cfg.threads = t.threads > 0 ? t.threads : 256;
   cfg.stream = stream;
-  cfg.emu_world = emu_ ? world_ : 0;
-  const int cap = emu_ ? std::max(1, 128 / world_) : 64;  // every block polls blocks * world flags
+  cfg.emu_world = emu_ && world_ > 1 ? world_ : 0;
+  cfg.pdl = world_ == 1;
+  // every block polls blocks * world flags of its peers; a world of one has none and takes what the GPU holds
+  const int cap = world_ == 1 ? 3 * 148 : (emu_ ? std::max(1, 128 / world_) : 64);
   cfg.blocks = std::min(cap, t.blocks > 0 ? t.blocks : cap);
+  return cfg;
+}
+
+void Communicator::moe_dispatch(int dtype, const MoeArgs* args, const Tuning& t, cudaStream_t stream) {
+  const LaunchCfg cfg = moe_cfg(t, stream);
   ckrt(launch_moe_dispatch(dtype, ctx_, args, cfg), "moe_dispatch");
 }
 
 void Communicator::moe_combine(int dtype, const MoeArgs* args, const Tuning& t, cudaStream_t stream) {
-  LaunchCfg cfg;
-  cfg.threads = t.threads > 0 ? t.threads : 256;
-  cfg.stream = stream;
-  cfg.emu_world = emu_ ? world_ : 0;
-  const int cap = emu_ ? std::max(1, 128 / world_) : 64;
-  cfg.blocks = std::min(cap, t.blocks > 0 ? t.blocks : cap);
+  const LaunchCfg cfg = moe_cfg(t, stream);
   ckrt(launch_moe_combine(dtype, ctx_, args, cfg), "moe_combine");
 }
 

@@ -99,6 +99,7 @@ class Communicator {
   sm100::DecodePush fused_norm_push_target(int rows, int hidden, int elem_size, int view = 0);
 
   // MoE expert-parallel row exchange; args: views() entries (see MoeArgs).
+  LaunchCfg moe_cfg(const Tuning& t, cudaStream_t stream) const;
   void moe_dispatch(int dtype, const MoeArgs* args, const Tuning& t, cudaStream_t stream);
   void moe_combine(int dtype, const MoeArgs* args, const Tuning& t, cudaStream_t stream);
 

@@ -77,17 +77,22 @@ def build_routing_torch(topk_ids: torch.Tensor, experts: int):
             send_off.to(torch.int32).contiguous(), counts)
 
 
-def placement_device(counts_all: torch.Tensor):
-    """`placement` on the device: counts_all [W, E] int32 (CUDA) -> dst_base [W, E] int32 (stays on
-    the device for the dispatch kernel), and - the one host round trip of the layer, because the
-    expert GEMMs are launched with host-side shapes - rows_per_rank and per-rank expert ranges."""
+def _placement(counts_all: torch.Tensor):
+    """placement_device with the ranges of all experts as a device tensor [E, 2] as well."""
     W, E = counts_all.shape
     dst_base, rows, ranges = ops.moe_placement(counts_all.contiguous())
     host = torch.cat([rows, ranges.reshape(-1)]).cpu().tolist()
     rows_per_rank, flat = host[:W], host[W:]
     epr = E // W
     expert_ranges = [[(flat[2 * (d * epr + le)], flat[2 * (d * epr + le) + 1]) for le in range(epr)] for d in range(W)]
-    return dst_base, rows_per_rank, expert_ranges
+    return dst_base, rows_per_rank, expert_ranges, ranges
+
+
+def placement_device(counts_all: torch.Tensor):
+    """`placement` on the device: counts_all [W, E] int32 (CUDA) -> dst_base [W, E] int32 (stays on
+    the device for the dispatch kernel), and - the one host round trip of the layer, for the capacity
+    check - rows_per_rank and per-rank expert ranges."""
+    return _placement(counts_all)[:3]
 
 
 def placement(counts_all: torch.Tensor, world: int):
@@ -143,13 +148,22 @@ class MoeEPLayer:
         for r in self.ranks:
             g.manual_seed(seed * 7919 + 1)
             self.router.append((torch.randn(cfg.experts, cfg.hidden, device=dev, generator=g) * cfg.init_std).to(dt))
-            w13, w2 = [], []
+            # one tensor per kind and rank, the experts' matrices are views of it: the grouped GEMMs address
+            # all of them through one descriptor
+            w13 = torch.empty(self.epr, 2 * cfg.ffn, cfg.hidden, dtype=dt, device=dev)
+            w2 = torch.empty(self.epr, cfg.hidden, cfg.ffn, dtype=dt, device=dev)
             for le in range(self.epr):
                 g.manual_seed(seed * 7919 + 100 + r * self.epr + le)
-                w13.append((torch.randn(2 * cfg.ffn, cfg.hidden, device=dev, generator=g) * cfg.init_std).to(dt))
-                w2.append((torch.randn(cfg.hidden, cfg.ffn, device=dev, generator=g) * cfg.init_std).to(dt))
-            self.w13.append(w13)
-            self.w2.append(w2)
+                w13[le] = torch.randn(2 * cfg.ffn, cfg.hidden, device=dev, generator=g) * cfg.init_std
+                w2[le] = torch.randn(cfg.hidden, cfg.ffn, device=dev, generator=g) * cfg.init_std
+            self.w13.append(list(w13))
+            self.w2.append(list(w2))
+        # Rows one expert can receive: a token picks it at most once.  Up to 256 the streamed GEMM reads every
+        # expert's weights once; more rows make the experts tensor-core work for the tiled one.
+        self.expert_rows = min(self.world * tokens, self.cap_rows)
+        self.workspace = None
+        if backend == "penny" and use_own_gemm and 0 < self.expert_rows <= 256:
+            self.workspace = torch.zeros(ops.gemm_stream_workspace_bytes(self.expert_rows), dtype=torch.uint8, device=dev)
 
     def _as_views(self, t) -> List[torch.Tensor]:
         return list(t) if isinstance(t, (list, tuple)) else [t]
@@ -163,6 +177,34 @@ class MoeEPLayer:
         else:
             torch.matmul(a, w.t(), out=out)
         return out
+
+    @staticmethod
+    def _stack(mats: List[torch.Tensor]) -> torch.Tensor:
+        """[experts * rows, K] over the experts' matrices: the tensor they are views of, or a copy when a
+        caller has put other tensors into the list."""
+        m = mats[0]
+        step = m.numel() * m.element_size()
+        if all(t.data_ptr() == m.data_ptr() + i * step and t.is_contiguous() for i, t in enumerate(mats)):
+            return m.as_strided((len(mats) * m.shape[0], m.shape[1]), (m.shape[1], 1))
+        return torch.cat(mats)
+
+    def _experts_grouped(self, v: int, rows: torch.Tensor, ranges: torch.Tensor):
+        """SwiGLU FFN of this rank's local experts over its received rows in two launches; `ranges`
+        [local experts, 2] stays on the device."""
+        cfg = self.cfg
+        act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
+        y = torch.empty_like(rows)
+        w13, w2 = self._stack(self.w13[v]), self._stack(self.w2[v])
+        if self.workspace is not None:
+            ops.gemm_stream(rows, w13, act, self.workspace, 1, cfg.ffn, ranges, self.expert_rows)
+            ops.gemm_stream(act, w2, y, self.workspace, 0, 64, ranges, self.expert_rows)
+        else:
+            # 256-row tiles of CTA pairs, or 128-row ones where the average expert would leave half of those
+            # empty (the weights are read once per row tile either way)
+            block_n = 512 if self.world * self.tokens * cfg.topk > 160 * cfg.experts else 256
+            ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
+            ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n)
+        return y
 
     def _experts(self, v: int, rows: torch.Tensor, ranges):
         """SwiGLU FFN of this rank's local experts over its received rows."""
@@ -186,15 +228,18 @@ class MoeEPLayer:
             ids.append(i)
             gates.append(g)
             tables.append(build_routing(i, cfg.experts))
-            self.counts_buf[v].view(torch.int32).copy_(tables[v][3].to(torch.int32))
+        if self.world == 1 and self.backend == "penny" and self.use_own_gemm and ids[0].numel() <= self.cap_rows:
+            return self._forward_one_rank(xs[0], ids[0], gates[0], tables[0])
         # every rank learns how many rows each rank sends to each expert
         if self.world > 1:
+            for v in range(len(xs)):
+                self.counts_buf[v].view(torch.int32).copy_(tables[v][3].to(torch.int32))
             gathered = comm.all_gather(self.counts_buf if comm.emulated else self.counts_buf[0])
             gathered = self._as_views(gathered)
             counts_dev = gathered[0].view(torch.int32).view(self.world, cfg.experts)
         else:
             counts_dev = tables[0][3].to(torch.int32).view(1, cfg.experts)
-        dst_base, rows_per_rank, expert_ranges = placement_device(counts_dev)
+        dst_base, rows_per_rank, expert_ranges, ranges_dev = _placement(counts_dev)
         if max(rows_per_rank) > self.cap_rows:
             raise RuntimeError(f"MoE capacity exceeded: {max(rows_per_rank)} rows > {self.cap_rows}")
         dst_base_dev = [dst_base[r].contiguous() for r in self.ranks]
@@ -206,7 +251,11 @@ class MoeEPLayer:
                               cfg.experts)
             ys = []
             for v, r in enumerate(self.ranks):
-                ys.append(self._experts(v, self.recv[v][:rows_per_rank[r]], expert_ranges[r]))
+                rows = self.recv[v][:rows_per_rank[r]]
+                if self.use_own_gemm and rows.shape[0] > 0:
+                    ys.append(self._experts_grouped(v, rows, ranges_dev[r * self.epr:(r + 1) * self.epr]))
+                else:
+                    ys.append(self._experts(v, rows, expert_ranges[r]))
             outs = [torch.empty_like(xv) for xv in xs]
             comm.moe_combine(L(ys), L(outs), L([i.reshape(-1).contiguous() for i in ids]),
                              L([g.reshape(-1).contiguous() for g in gates]), L(self.meta), L(self.dst_row_of_pair),
@@ -214,6 +263,19 @@ class MoeEPLayer:
                              else rows_per_rank[self.ranks[0]], cfg.experts)
             return outs if comm.emulated else outs[0]
         return self._forward_nccl(xs[0], ids[0], gates[0], tables[0], counts_all, rows_per_rank, expert_ranges)
+
+    def _forward_one_rank(self, x, ids, gates, table):
+        """A world of one: the rows received are the pairs in sorted order, so their placement is the sender's
+        table, no capacity can be exceeded and nothing has to come back to the host between the kernels."""
+        cfg, comm = self.cfg, self.comm
+        order, expert_sorted, borders, _ = table
+        comm.moe_dispatch(x, order, expert_sorted, borders, borders[:cfg.experts], self.dst_row_of_pair[0],
+                          self.recv[0], self.meta[0], cfg.topk, cfg.experts)
+        y = self._experts_grouped(0, self.recv[0][:ids.numel()], borders)
+        out = torch.empty_like(x)
+        comm.moe_combine(y, out, ids.reshape(-1), gates.reshape(-1), self.meta[0], self.dst_row_of_pair[0], self.comb[0],
+                         0, cfg.experts)
+        return [out] if comm.emulated else out
 
     def _forward_nccl(self, x, ids, gates, table, counts_all, rows_per_rank, expert_ranges):
         """Baseline: the same layer with NCCL all_to_all_single for both exchanges."""
