@@ -15,6 +15,7 @@
 
 #include "decode_attn_common.cuh"
 #include "decode_kernels.h"
+#include "pdl.h"
 
 #include <stdio.h>
 
@@ -78,6 +79,89 @@ __global__ void k_rope_rows(__nv_bfloat16* __restrict__ qkv, int Hq, int Hkv, in
   const float a = bf2f(x[i]), bb = bf2f(x[i + half]);
   x[i] = __float2bfloat16_rn(a * c - bb * s);
   x[i + half] = __float2bfloat16_rn(bb * c + a * s);
+}
+
+// The same with 16-byte accesses, for head sizes that are whole vectors per half and aligned rows: one block
+// per token, whose half x (sin, cos) are computed once in shared memory and reused by all heads.  Bound by
+// one read and one write of q and k: 40 heads x 4096 tokens (84 MB) 44 -> 15 us against the kernel above,
+// which computes a power, a sine and a cosine for every two 2-byte elements.
+__global__ void __launch_bounds__(320) k_rope_rows_vec(__nv_bfloat16* __restrict__ qkv, int Hq, int Hkv, int D, int pos0,
+                                                       float theta) {
+  extern __shared__ float s_cs[];  // [half] cosines, [half] sines
+  const int half = D / 2, t = blockIdx.x;
+  pdl_launch_dependents();
+  const float lt = log2f(theta);
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf((float)(pos0 + t) * exp2f(-2.0f * (float)i / (float)D * lt), &sn, &cs);
+    s_cs[i] = cs;
+    s_cs[half + i] = sn;
+  }
+  pdl_wait();
+  __syncthreads();
+  const int per_head = half / 8;
+  __nv_bfloat16* row = qkv + (size_t)t * (Hq + 2 * Hkv) * D;
+  for (int idx = threadIdx.x; idx < (Hq + Hkv) * per_head; idx += blockDim.x) {
+    const int h = idx / per_head, i = (idx - h * per_head) * 8;
+    uint4* pa = reinterpret_cast<uint4*>(row + h * D + i);
+    uint4* pb = reinterpret_cast<uint4*>(row + h * D + half + i);
+    const uint4 va = *pa, vb = *pb;
+    const __nv_bfloat162* xa = reinterpret_cast<const __nv_bfloat162*>(&va);
+    const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&vb);
+    uint4 oa, ob;
+    uint32_t* ya = reinterpret_cast<uint32_t*>(&oa);
+    uint32_t* yb = reinterpret_cast<uint32_t*>(&ob);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float c0 = s_cs[i + 2 * k], c1 = s_cs[i + 2 * k + 1], s0 = s_cs[half + i + 2 * k],
+                  s1 = s_cs[half + i + 2 * k + 1];
+      const float a0 = bf2f(xa[k].x), a1 = bf2f(xa[k].y), b0 = bf2f(xb[k].x), b1 = bf2f(xb[k].y);
+      ya[k] = pack2(a0 * c0 - b0 * s0, a1 * c1 - b1 * s1);
+      yb[k] = pack2(b0 * c0 + a0 * s0, b1 * c1 + a1 * s1);
+    }
+    *pa = oa;
+    *pb = ob;
+  }
+}
+
+// Start of a stack whose norms ride in the GEMM epilogues: row `index[r]` (or r) of src becomes residual row r,
+// its product with the first norm's weight the first linear's input, and its sum of squares what that
+// linear scales its rows by.  One block per row.
+__global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restrict__ src, const long long* __restrict__ index,
+                                                   const __nv_bfloat16* __restrict__ norm_w,
+                                                   __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out,
+                                                   float* __restrict__ sumsq, int H) {
+  __shared__ float s_part[16];
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t r = blockIdx.x;
+  const uint4* in = reinterpret_cast<const uint4*>(src + (index != nullptr ? (size_t)index[r] : r) * H);
+  const uint4* w = reinterpret_cast<const uint4*>(norm_w);
+  float ss = 0.f;
+  for (int v = threadIdx.x; v < H / 8; v += blockDim.x) {
+    const uint4 x = in[v], n = w[v];
+    const __nv_bfloat162* xe = reinterpret_cast<const __nv_bfloat162*>(&x);
+    const __nv_bfloat162* ne = reinterpret_cast<const __nv_bfloat162*>(&n);
+    uint4 o;
+    uint32_t* oe = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float a = bf2f(xe[k].x), b = bf2f(xe[k].y);
+      ss += a * a + b * b;
+      oe[k] = pack2(a * bf2f(ne[k].x), b * bf2f(ne[k].y));
+    }
+    reinterpret_cast<uint4*>(residual + r * H)[v] = x;
+    reinterpret_cast<uint4*>(out + r * H)[v] = o;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int i = 0; i < (int)blockDim.x / 32; ++i) t += s_part[i];
+    sumsq[r] = t;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -451,9 +535,23 @@ cudaError_t launch_rope_append(void* qkv, void* kcache, void* vcache, const int*
 cudaError_t launch_rope_rows(void* qkv, int T, int Hq, int Hkv, int D, int pos0, float theta,
                              cudaStream_t stream) {
   if (D % 2 != 0 || D / 2 > 256 || T <= 0) return cudaErrorInvalidValue;
+  if (D % 16 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 15u) == 0) {
+    const int items = (Hq + Hkv) * (D / 16), threads = std::min(320, (items + 31) / 32 * 32);
+    return launch_kernel_ex(k_rope_rows_vec, dim3((unsigned)T), dim3((unsigned)threads), (size_t)D * sizeof(float), stream,
+                            true, 1, (__nv_bfloat16*)qkv, Hq, Hkv, D, pos0, theta);
+  }
   dim3 grid(T, (Hq + Hkv + 3) / 4), block(D / 2, 4);
   k_rope_rows<<<grid, block, 0, stream>>>((__nv_bfloat16*)qkv, Hq, Hkv, D, pos0, theta);
   return cudaGetLastError();
+}
+
+cudaError_t launch_norm_prep(const void* src, const long long* index, const void* norm_w, void* residual, void* out,
+                             float* sumsq, int rows, int H, cudaStream_t stream) {
+  if (rows < 1 || H < 8 || H % 8 != 0) return cudaErrorInvalidValue;
+  const int threads = std::min(512, (H / 8 + 31) / 32 * 32);
+  return launch_kernel_ex(k_norm_prep, dim3((unsigned)rows), dim3((unsigned)threads), 0, stream, true, 1,
+                          (const __nv_bfloat16*)src, index, (const __nv_bfloat16*)norm_w, (__nv_bfloat16*)residual,
+                          (__nv_bfloat16*)out, sumsq, H);
 }
 
 size_t decode_attn_workspace_bytes(int B, int Hq, int splits) {

@@ -98,6 +98,14 @@ class LlamaSPPrefill:
         self.gathered = e(tokens, H) if backend == "nccl" and not self.cpu else None
         self.full = e(tokens, H) if backend == "nccl" and not self.cpu else None
         self.scale = 1.0 / math.sqrt(D)
+        # one rank: nothing to gather or scatter, so the linears are plain GEMMs whose epilogues take the
+        # residual add, silu * mul and the norms (see _forward_local)
+        self.local = backend == "penny" and world == 1 and not self.cpu and (2 * self.F) % 128 == 0
+        if self.local:
+            self.sumsq = [torch.empty(n, tokens, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
+            self.workspace = None
+            if tokens <= 256:
+                self.workspace = torch.zeros(ops.gemm_stream_workspace_bytes(tokens), dtype=torch.uint8, device=self.dev)
         # kernels of this library per forward: per layer 2 norms, RoPE, silu*mul and (penny) 4 fused GEMMs
         self.kernels_per_forward = self.L * (4 + (4 if backend == "penny" else 0))
 
@@ -162,17 +170,49 @@ class LlamaSPPrefill:
         k = self.qkv[:, self.Hq * D:(self.Hq + self.Hkv) * D].view(T, self.Hkv, D).permute(1, 0, 2).unsqueeze(0)
         v = self.qkv[:, (self.Hq + self.Hkv) * D:].view(T, self.Hkv, D).permute(1, 0, 2).unsqueeze(0)
         o = F_.scaled_dot_product_attention(q, k, v, is_causal=True, scale=self.scale, enable_gqa=True)
-        self.attn.view(T, self.Hq, D).copy_(o[0].permute(1, 0, 2))
+        o = o[0].permute(1, 0, 2)
+        if o.is_contiguous():  # the library returned token-major rows: they are the linear's input as they are
+            return o.reshape(T, self.Hq * D)
+        self.attn.view(T, self.Hq, D).copy_(o)
+        return self.attn
 
     # ------------------------------------------------------------------ forward
+    def _gemm(self, x, w, out, epi=0, sumsq=None, residual=None, norm_w=None, sumsq_out=None):
+        """One linear with its epilogue: up to 256 tokens it is a read of the weights (streamed GEMM), above
+        that tensor-core work (tiled GEMM)."""
+        if self.workspace is not None and not (epi == 2 and norm_w is None):
+            ops.gemm_stream(x, w, out, self.workspace, epi, w.shape[0] // 2 if epi == 1 else 64, sumsq=sumsq,
+                            eps=self.cfg.eps, residual=residual, norm_w=norm_w, sumsq_out=sumsq_out)
+        else:
+            ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
+                          sumsq_out=sumsq_out)
+
+    def _forward_local(self, x: torch.Tensor) -> torch.Tensor:
+        """One rank.  h holds the residual stream times the next norm's weight, sumsq its sums of squares; the
+        linear that reads h scales its output rows by 1 / rms, so a norm costs no pass of its own."""
+        res, h, ss = torch.empty_like(x), self.h, self.sumsq[0]
+        ops.norm_prep(x, None, self.layers[0]["norm1"], res, h, ss)
+        for li, l in enumerate(self.layers):
+            self._gemm(h, l["wqkv"], self.qkv, sumsq=ss)
+            attn = self._attention()
+            ss = self.sumsq[1]
+            self._gemm(attn, l["wo"], h, 2, residual=res, norm_w=l["norm2"], sumsq_out=ss)
+            self._gemm(h, l["wgu"], self.act, 1, sumsq=ss)
+            if li + 1 < len(self.layers):
+                self._gemm(self.act, l["wd"], h, 2, residual=res, norm_w=self.layers[li + 1]["norm1"], sumsq_out=ss)
+            else:
+                self._gemm(self.act, l["wd"], h, 2, residual=res)
+        return res
+
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
         """x_shard: this rank's [T / world, hidden] rows of the residual stream; returns the same rows after all layers."""
+        if self.local and x_shard.is_contiguous() and x_shard.data_ptr() % 16 == 0:
+            return self._forward_local(x_shard)
         res = x_shard.clone()
         self._add_rmsnorm(res, None, self.layers[0]["norm1"], self.h, None)
         for li, l in enumerate(self.layers):
             self._col(self.h, l["wqkv"], self.qkv)
-            self._attention()
-            self._row(self.attn, l["wo"], self.part)
+            self._row(self._attention(), l["wo"], self.part)
             self._add_rmsnorm(self.part, res, l["norm2"], self.h, res)          # res += o_proj; h = norm(res)
             self._col(self.h, l["wgu"], self.gu)
             self._silu_mul()

@@ -166,3 +166,21 @@ def test_tile_groups(counts, block_n):
         y = x[s:t].float() @ w[e * 2 * F:(e + 1) * 2 * F].float().t()
         want[s:t] = torch.nn.functional.silu(y[:, :F]) * y[:, F:]
     _close(out, want)
+
+
+@pytest.mark.parametrize("tokens", [128, 384])  # streamed and tiled linears
+def test_prefill_one_rank_matches_fp32(tokens):
+    from penny_b200.models.llama_sp import LlamaSPPrefill
+    from penny_b200.models.llama_tp import LlamaConfig
+    from penny_b200.parallel.comm import Communicator
+    cfg, layers = LlamaConfig.tiny(), 2
+    x = torch.randn(tokens, cfg.hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).bfloat16()
+    want = LlamaSPPrefill.reference_forward(cfg, x, layers, seed=1)
+    comm = Communicator.emulated(1, heap_bytes=64 << 20)
+    try:
+        m = LlamaSPPrefill(cfg, comm=comm, tokens=tokens, layers=layers, seed=1)
+        for _ in range(2):
+            got = m.forward(x).float()
+            assert ((got - want).norm() / want.norm()).item() < 1.5e-2
+    finally:
+        comm.close()
