@@ -132,15 +132,18 @@ void bind_gemm(py::module_& m) {
       g.scale_width = g.K;
     }
     if (epi == 2) {
-      TORCH_CHECK(residual.has_value() && norm_w.has_value() && sumsq_out.has_value(), "gemm_stream: residual epilogue operands");
-      TORCH_CHECK(bf16(*residual) && residual->sizes() == out.sizes() && residual->stride(0) == out.stride(0) &&
-                      bf16(*norm_w) && norm_w->numel() == g.w_rows && sumsq_out->is_cuda() &&
-                      sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
-                      sumsq_out->numel() == (int64_t)(g.w_rows / 128) * g.rows,
-                  "gemm_stream: residual like out, norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
+      TORCH_CHECK(residual.has_value() && bf16(*residual) && residual->sizes() == out.sizes() &&
+                      residual->stride(0) == out.stride(0) && norm_w.has_value() == sumsq_out.has_value(),
+                  "gemm_stream: residual like out; norm_w and sumsq_out together");
       g.residual = residual->data_ptr();
-      g.norm_w = norm_w->data_ptr();
-      g.sumsq_out = sumsq_out->data_ptr<float>();
+      if (norm_w.has_value()) {
+        TORCH_CHECK(bf16(*norm_w) && norm_w->numel() == g.w_rows && sumsq_out->is_cuda() &&
+                        sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
+                        sumsq_out->numel() == (int64_t)(g.w_rows / 128) * g.rows,
+                    "gemm_stream: norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
+        g.norm_w = norm_w->data_ptr();
+        g.sumsq_out = sumsq_out->data_ptr<float>();
+      }
     }
     TORCH_CHECK(workspace.is_cuda() && workspace.is_contiguous(), "gemm_stream: CUDA workspace");
     g.workspace = workspace.data_ptr();
@@ -160,7 +163,8 @@ void bind_gemm(py::module_& m) {
   // weight before its up rows; ranges: as gemm_stream, of a and out; b [groups * rows, K].
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
-                        c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl) {
+                        c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
+                        int64_t cluster) {
     auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
     TORCH_CHECK(bf16(a) && bf16(b) && bf16(out) && a.dim() == 2 && b.dim() == 2 && out.dim() == 2,
                 "gemm_tile: 2-D bf16 CUDA tensors with contiguous rows");
@@ -211,13 +215,15 @@ void bind_gemm(py::module_& m) {
     }
     g.block_n = (int)block_n;
     g.pdl = pdl;
+    g.cluster = (int)cluster;
     const at::cuda::OptionalCUDAGuard guard(a.device());
     const cudaError_t rc =
         penny::sm100::launch_gemm_tile(g, penny_gemm_error_word(), at::cuda::getCurrentCUDAStream().stream());
     TORCH_CHECK(rc == cudaSuccess, "gemm_tile: ", cudaGetErrorString(rc));
   }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epi") = 0, py::arg("ranges") = py::none(),
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
-     py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = true);
+     py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = true,
+     py::arg("cluster") = 0);
   m.def("gemm_stream_workspace_bytes", [](int64_t rows) {
     return (int64_t)penny::sm100::stream_workspace_bytes((int)rows, penny::sm100::stream_max_pairs());
   }, py::arg("rows"), "bytes of gemm_stream's workspace for up to `rows` rows per group; zero it once");

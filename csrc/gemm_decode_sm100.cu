@@ -116,30 +116,6 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, const float
                "f"(v.w)
                : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait for the peers' partials (they were written by other SMs, hence
-// the cluster-scope acquire).
-__device__ __forceinline__ bool mbar_wait_cluster_abortable(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const unsigned long long t0 = gtime_ns();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((i & 255u) == 0u) {
-      if (*abort_flag) return false;
-      if (gtime_ns() - t0 > kWaitNs) return false;
-    }
-  }
-}
 // One [128 x 64] box of W into L2 only (no shared memory, no barrier).
 __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
@@ -352,7 +328,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       // my rows of the peers' partials (gate/up pairing: every quarter)
       for (int w = 0; w < 4; ++w) {
         if (!silu && w != q) continue;
-        if (!mbar_wait_cluster_abortable(&recv_bar[w], 0u, s_abort)) ok = false;
+        if (!mbar_wait_cluster(&recv_bar[w], 0u, s_abort)) ok = false;
       }
       if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
       ok = __all_sync(0xffffffffu, ok);

@@ -93,33 +93,6 @@ __device__ __forceinline__ void tma_load_2d_pair_once(void* smem_dst, const CUte
       "l"(m), "r"(bar_cluster_addr), "r"(x), "r"(y), "l"(policy)
       : "memory");
 }
-// 16 bytes into another CTA's shared memory, counted on a barrier there: no separate arrival has to wait
-// for the stores.
-__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(addr),
-               "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait for something other CTAs of the cluster wrote.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const unsigned long long t0 = gtime_ns();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((i & 255u) == 0u && (*abort_flag || gtime_ns() - t0 > kWaitNs)) return false;
-  }
-}
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
@@ -240,7 +213,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t bar = full0 + (uint32_t)stage * 8u;
         const int y = s_group[gs] * a.w_rows + (2 * t + (int)r) * a.y_step;
         tma_load_2d_pair_once(sw, &map_w, bar, kb * kBlockK, y, policy);
-        tma_load_2d_pair_once(sw + kStWBytes / 2, &map_w, bar, kb * kBlockK, y + a.up_offset, policy);
+        if (a.up_offset != kBlockM / 2)  // gate and up rows are not neighbours: boxes of 64 rows
+          tma_load_2d_pair_once(sw + kStWBytes / 2, &map_w, bar, kb * kBlockK, y + a.up_offset, policy);
       };
       auto load_x = [&](int stage, int row0, int n_half, int kb) {
         unsigned char* sx = tiles + (size_t)stage * stage_bytes + kStWBytes;
@@ -408,6 +382,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       };
       bool last = true;
       if (p0 != p1) {
+        // where the other pairs have all been here already (a tile that ends one pair's range and began
+        // another's) nobody needs this part: no write, no fence
+        if (tid == 0) {
+          unsigned* cnt = a.counters + (tile * 4 + (int)r * 2 + h);
+          const int only_me = (int)*reinterpret_cast<volatile unsigned*>(cnt) == p1 - p0;
+          if (only_me) *cnt = 0u;
+          s_last[h] = only_me;
+        }
+        named_bar_sync(1 + h, 128);
+        last = s_last[h] != 0;
+        if (last) __threadfence();
+      }
+      if (!last) {
+        named_bar_sync(1 + h, 128);  // s_last has been read
         float4* dst = part(pair);
 #pragma unroll 1
         for (int c = 0; c < ncol; c += kStChunk) {
@@ -543,7 +531,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
               float ss = 0.f;
               if (live && col < a.n_out) {
                 const uint4 res = *reinterpret_cast<const uint4*>(a.residual + off);
-                const uint4 nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + col));
+                const uint4 nw = a.norm_w != nullptr ? __ldg(reinterpret_cast<const uint4*>(a.norm_w + col)) : uint4{};
                 const uint32_t rw[4] = {res.x, res.y, res.z, res.w}, ww[4] = {nw.x, nw.y, nw.z, nw.w};
                 float zw[8];
 #pragma unroll
@@ -555,12 +543,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                   zw[2 * k + 1] = o[2 * k + 1] * bf16_hi(ww[k]);
                 }
                 *reinterpret_cast<uint4*>(a.residual + off) = pack8(o);
-                *reinterpret_cast<uint4*>(a.out + off) = pack8(zw);
+                if (a.norm_w != nullptr) *reinterpret_cast<uint4*>(a.out + off) = pack8(zw);
               }
               // the 16 lanes of a row of x
 #pragma unroll
               for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-              if (g == 0 && live) a.sumsq_out[(size_t)blk * a.rows + xr] = ss;
+              if (g == 0 && live && a.norm_w != nullptr) a.sumsq_out[(size_t)blk * a.rows + xr] = ss;
             } else if (live) {
               __nv_bfloat16* dst = a.out + off;
               if (col + 8 <= a.n_out && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
@@ -640,8 +628,8 @@ cudaError_t launch_gemm_stream(const StreamGemm& g, uint32_t* error_word, cudaSt
   a.sumsq_out = g.sumsq_out;
   if ((long long)groups * a.tiles * 4 > kStreamCounters) return cudaErrorInvalidValue;
   if (g.epi == STREAM_EPI_RESIDUAL &&
-      (g.groups > 0 || g.w_rows % 128 != 0 || g.ldo % 8 != 0 || g.residual == nullptr || g.norm_w == nullptr ||
-       g.sumsq_out == nullptr ||
+      (g.groups > 0 || g.w_rows % 128 != 0 || g.ldo % 8 != 0 || g.residual == nullptr ||
+       (g.norm_w != nullptr && g.sumsq_out == nullptr) ||
        ((reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.residual) | reinterpret_cast<uintptr_t>(g.norm_w)) & 15u) != 0))
     return cudaErrorInvalidValue;
   if (g.groups > 0 && (g.ranges == nullptr || g.scale_sumsq != nullptr)) return cudaErrorInvalidValue;
@@ -652,29 +640,43 @@ cudaError_t launch_gemm_stream(const StreamGemm& g, uint32_t* error_word, cudaSt
   if (g.workspace == nullptr || (reinterpret_cast<uintptr_t>(g.workspace) & 15u) != 0 ||
       g.workspace_bytes < stream_workspace_bytes(g.rows, pairs))
     return cudaErrorInvalidValue;
-  a.cl = g.cluster > 0 ? g.cluster : stream_cluster(g.groups > 0 ? 0 : a.tiles, a.num_kb, max_pairs);
-  if (a.cl > kStMaxCluster || (a.cl > 1 && (g.groups > 0 || a.num_kb < a.cl))) return cudaErrorInvalidValue;
-  const int grid = 2 * (a.cl > 1 ? a.tiles * a.cl : pairs);
-  a.counters = reinterpret_cast<unsigned*>(g.workspace);
-  a.parts = reinterpret_cast<float*>(a.counters + kStreamCounters);
-  CUtensorMap mw, mx;
-  cudaError_t rc = make_tile_map(&mw, g.w, (uint64_t)groups * g.w_rows, (uint64_t)g.K, (uint64_t)g.ldw, kBlockM / 2);
-  if (rc != cudaSuccess) return rc;
-  rc = make_tile_map(&mx, g.x, (uint64_t)g.x_rows, (uint64_t)g.K, (uint64_t)g.ldx, (uint32_t)a.xbox);
-  if (rc != cudaSuccess) return rc;
   // Ring: up to 128 rows it stays within half of the shared memory, so that the next kernel of a chain
   // sets up and fills its own ring beside this one; above that one kernel has the SM.
   const int stage_bytes = kStWBytes + a.bt / 2 * (kBlockK * 2);
   const size_t budget = (size_t)(g.smem_kb > 0 ? std::min(g.smem_kb, 216) : (a.bt <= 128 ? 108 : 200)) << 10;
   // Without an area of its own the ring has to hold what the peers of a cluster send.
-  const int peer_bytes = (a.cl - 1) * ((a.bt / kStChunk + a.cl - 1) / a.cl) * kStChunk * kBlockM * 4;
-  a.own_recv = peer_bytes <= 24 << 10;
-  const size_t fixed = kStEpiBytes + 1024 + (a.own_recv ? peer_bytes : 0);
-  int stages = 2;
-  while (!a.own_recv && stages * stage_bytes < peer_bytes) ++stages;
-  while (stages < kStMaxStages && fixed + (size_t)(stages + 1) * stage_bytes <= budget) ++stages;
-  a.stages = stages;
-  const size_t smem = fixed + (size_t)stages * stage_bytes;
+  auto plan_ring = [&](int cl) {
+    const int peer_bytes = (cl - 1) * ((a.bt / kStChunk + cl - 1) / cl) * kStChunk * kBlockM * 4;
+    a.own_recv = peer_bytes <= 24 << 10;
+    const size_t fixed = kStEpiBytes + 1024 + (a.own_recv ? peer_bytes : 0);
+    a.stages = 2;
+    while (!a.own_recv && a.stages * stage_bytes < peer_bytes) ++a.stages;
+    while (a.stages < kStMaxStages && fixed + (size_t)(a.stages + 1) * stage_bytes <= budget) ++a.stages;
+    return fixed + (size_t)a.stages * stage_bytes;
+  };
+  a.cl = g.cluster;
+  if (g.cluster == 0) {
+    int held[kStMaxCluster + 1] = {};
+    const void* fn = reinterpret_cast<const void*>(gemm_stream_kernel<STREAM_EPI_PLAIN>);
+    if (kernel_setup(fn, 220 << 10).rc == cudaSuccess)
+      for (int c = 2; c <= kStMaxCluster && g.groups == 0; ++c) {
+        const size_t bytes = plan_ring(c);
+        // (the query counts one CTA per SM; where two fit, twice as many clusters run together)
+        held[c] = max_clusters(fn, 2 * c, kStThreads, bytes) * (bytes + 3072 <= ((size_t)228 << 10) / 2 ? 2 : 1);
+      }
+    a.cl = stream_cluster(a.tiles, a.num_kb, held);
+  }
+  if (a.cl < 1 || a.cl > kStMaxCluster || (a.cl > 1 && (g.groups > 0 || a.num_kb < a.cl))) return cudaErrorInvalidValue;
+  const size_t smem = plan_ring(a.cl);
+  const int grid = 2 * (a.cl > 1 ? a.tiles * a.cl : pairs);
+  a.counters = reinterpret_cast<unsigned*>(g.workspace);
+  a.parts = reinterpret_cast<float*>(a.counters + kStreamCounters);
+  CUtensorMap mw, mx;
+  cudaError_t rc = make_tile_map(&mw, g.w, (uint64_t)groups * g.w_rows, (uint64_t)g.K, (uint64_t)g.ldw,
+                                 a.up_offset != kBlockM / 2 ? kBlockM / 2 : kBlockM);
+  if (rc != cudaSuccess) return rc;
+  rc = make_tile_map(&mx, g.x, (uint64_t)g.x_rows, (uint64_t)g.K, (uint64_t)g.ldx, (uint32_t)a.xbox);
+  if (rc != cudaSuccess) return rc;
   switch (g.epi) {
     case STREAM_EPI_PLAIN: return launch_epi<STREAM_EPI_PLAIN>(mw, mx, a, grid, smem, g.pdl, error_word, stream);
     case STREAM_EPI_SILU: return launch_epi<STREAM_EPI_SILU>(mw, mx, a, grid, smem, g.pdl, error_word, stream);

@@ -39,7 +39,7 @@ struct StreamGemm {
   float eps;
   // RESIDUAL epilogue
   void* residual;      // [rows, w_rows], ldo
-  const void* norm_w;  // [w_rows]
+  const void* norm_w;  // [w_rows]; null: only the residual add
   float* sumsq_out;    // [w_rows / 128][rows]
   void* workspace;     // stream_workspace_bytes(rows, 74 or more pairs), zeroed once
   size_t workspace_bytes;

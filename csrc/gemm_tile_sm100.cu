@@ -15,6 +15,8 @@ template <bool PAIR, int BN, int EPI>
 cudaError_t launch_tile(const TileGemm& g, TileArgs a, int sms, uint32_t* error_word, cudaStream_t stream) {
   using Cfg = TileCfg<PAIR, BN>;
   constexpr bool kSilu = EPI == TILE_EPI_SILU;
+  constexpr int kPasses = (kSilu ? BN / 2 : BN) / 64;
+  a.cl = 1;
   a.tiles_n = (a.n_out + (kSilu ? BN / 2 : BN) - 1) / (kSilu ? BN / 2 : BN);
   a.band = std::max(1, 2048 / Cfg::kRows);
   CUtensorMap ma, mb;
@@ -31,13 +33,46 @@ cudaError_t launch_tile(const TileGemm& g, TileArgs a, int sms, uint32_t* error_
   // grouped: the tile count is only known on the device
   const long long tiles = (long long)((g.M + Cfg::kRows - 1) / Cfg::kRows) * a.tiles_n;
   const int slots = PAIR ? ks.pairs : sms;
-  const int workers = g.groups > 0 ? slots : (int)std::min<long long>(slots, tiles);
+  if constexpr (PAIR) {
+    a.cl = std::min({std::max(1, g.cluster), kTileMaxCluster, kPasses / (EPI == TILE_EPI_RESIDUAL ? 2 : 1)});
+    if (a.cl > 1 && (g.groups > 0 || a.num_kb < a.cl)) return cudaErrorInvalidValue;
+  }
+  // (a cluster that splits its tiles works on one: its exchange areas are used once)
+  const int workers = a.cl > 1 ? (int)tiles : (g.groups > 0 ? slots : (int)std::min<long long>(slots, tiles));
   if constexpr (PAIR)
-    return launch_kernel_ex(gemm_tile_pair<BN, EPI>, dim3((unsigned)(2 * workers)), dim3(kTileThreads), Cfg::kSmemBytes,
-                            stream, g.pdl, 1, ma, mb, a, error_word);
+    return launch_kernel_ex(gemm_tile_pair<BN, EPI>, dim3((unsigned)(2 * workers * a.cl)), dim3(kTileThreads),
+                            Cfg::kSmemBytes, stream, g.pdl, 2 * a.cl, ma, mb, a, error_word);
   else
     return launch_kernel_ex(gemm_tile_single<BN, EPI>, dim3((unsigned)workers), dim3(kTileThreads), Cfg::kSmemBytes,
                             stream, g.pdl, 1, ma, mb, a, error_word);
+}
+
+// Tile and cluster by rounds times the time of a K step.  Steps measured on B200, one 4096-long K (us per
+// step, all operands through the 64 B / clk that an SM takes in): 128 x 128 0.32, 128 x 192 0.36, 128 x 256
+// 0.40, 256 x 256 on a pair 0.36; the exchange of a cluster's sums takes about as long as 11 steps.
+void choose_tile(TileGemm& g, int sms, int pairs) {
+  const long long m128 = (g.M + 127) / 128, m256 = (g.M + 255) / 256;
+  const int num_kb = (g.K + kBlockK - 1) / kBlockK;
+  double best = 0;
+  auto offer = [&](int block_n, int cluster, long long tiles, int slots, double steps) {
+    const double cost = (double)((tiles + slots - 1) / slots) * steps;
+    if (g.block_n == 0 || cost < best) best = cost, g.block_n = block_n, g.cluster = cluster;
+  };
+  auto clusters = [&](int c) {
+    return max_clusters(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>), 2 * c, kTileThreads,
+                        TileCfg<true, 256>::kSmemBytes);
+  };
+  auto cols = [&](int bn) { return (long long)((g.b_rows + bn - 1) / bn); };
+  offer(128, 1, m128 * cols(128), sms, 0.32 * num_kb);
+  if (g.epi == TILE_EPI_PLAIN) offer(192, 1, m128 * cols(192), sms, 0.36 * num_kb);
+  offer(256, 1, m128 * cols(256), sms, 0.40 * num_kb);
+  if (pairs > 0 && pair_kernel_enabled()) {
+    const long long tiles = m256 * cols(256);
+    offer(512, 1, tiles, pairs, 0.36 * num_kb);
+    const int most = g.epi == TILE_EPI_PLAIN ? kTileMaxCluster : 2;
+    for (int c = 2; c <= most && g.groups == 0; ++c)
+      if (tiles <= clusters(c) && num_kb >= 4 * c) offer(512, c, tiles, pairs, 0.36 * ((num_kb + c - 1) / c + 11));
+  }
 }
 
 template <int EPI>
@@ -86,17 +121,16 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   a.residual = reinterpret_cast<__nv_bfloat16*>(g.residual);
   a.norm_w = reinterpret_cast<const __nv_bfloat16*>(g.norm_w);
   a.sumsq_out = g.sumsq_out;
-  int block_n = g.block_n;
-  if (block_n == 0) {
+  TileGemm c = g;
+  if (g.block_n == 0) {
     const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>),
                                         TileCfg<true, 256>::kSmemBytes, kTileThreads);
-    block_n = choose_block_n(g.M, g.b_rows, g.K, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
-    if (block_n == 192 && g.epi != TILE_EPI_PLAIN) block_n = 256;
+    choose_tile(c, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
   }
   switch (g.epi) {
-    case TILE_EPI_PLAIN: return launch_tile_n<TILE_EPI_PLAIN>(g, a, block_n, sms, error_word, stream);
-    case TILE_EPI_SILU: return launch_tile_n<TILE_EPI_SILU>(g, a, block_n, sms, error_word, stream);
-    case TILE_EPI_RESIDUAL: return launch_tile_n<TILE_EPI_RESIDUAL>(g, a, block_n, sms, error_word, stream);
+    case TILE_EPI_PLAIN: return launch_tile_n<TILE_EPI_PLAIN>(c, a, c.block_n, sms, error_word, stream);
+    case TILE_EPI_SILU: return launch_tile_n<TILE_EPI_SILU>(c, a, c.block_n, sms, error_word, stream);
+    case TILE_EPI_RESIDUAL: return launch_tile_n<TILE_EPI_RESIDUAL>(c, a, c.block_n, sms, error_word, stream);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -9,8 +9,11 @@
 //              step into a ring (128-byte swizzle, no multicast)
 //   warp 1     MMA issuer (the pair's leader): two accumulators in TMEM, so the
 //              epilogue of a tile runs under the next tile's MMAs
-//   warps 2-5  epilogue: TMEM -> registers (thread = row) -> swizzled staging rows ->
-//              128-byte row segments
+//   warps 2-9  epilogue: TMEM -> registers (thread = row) -> swizzled staging rows ->
+//              128-byte row segments; two warps per lane quarter share the columns
+// Few tiles with a long K (o_proj and down of a few hundred tokens): the pairs of a
+// cluster split the K steps of a tile and exchange their fp32 sums through each
+// other's shared memory, every CTA finishing a part of the columns.
 // SILU: a b tile is BN / 2 gate rows and the BN / 2 up rows of the same features, so
 // both halves of a product are columns of one accumulator and only the activation
 // is written.  RESIDUAL: the output is added to the residual stream, which is kept
@@ -23,18 +26,21 @@
 #include "gemm_kernel_sm100.cuh"
 #include "gemm_tile_sm100.h"
 #include "pdl.h"
+#include "stream_gemm_plan.h"
 
 namespace penny {
 namespace sm100 {
 
-constexpr int kTileThreads = 192;
+constexpr int kTileThreads = 320;
 constexpr int kTileMaxGroups = 256;
+constexpr int kTileMaxCluster = 4;  // pairs
 
 struct TileArgs {
   __nv_bfloat16* out;
   int ldo, M, n_out;     // n_out: columns of out
   int num_kb, tiles_n, band;
   int groups, b_rows;
+  int cl;                // pairs per cluster; above 1 a cluster splits the K steps of every tile
   const int* ranges;
   int range_stride;
   const float* scale_sumsq;
@@ -52,9 +58,9 @@ struct TileCfg {
   static constexpr int kABytes = kBlockM * kBlockK * 2;
   static constexpr int kBBytes = kBRows * kBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = (200 << 10) / kStageBytes < 8 ? (200 << 10) / kStageBytes : 8;
+  static constexpr int kStages = (192 << 10) / kStageBytes < 8 ? (192 << 10) / kStageBytes : 8;
   static constexpr int kTmemCols = BN == 192 ? 512 : 2 * BN;
-  static constexpr int kEpiBytes = 4 * 32 * kStageRowBytes;
+  static constexpr int kEpiBytes = 8 * 32 * kStageRowBytes;
   static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024;
 };
 
@@ -72,6 +78,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   constexpr int kNOut = kSilu ? BN / 2 : BN;  // output columns of a tile
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t s_bars[2 * kStages + 4];
+  __shared__ uint64_t s_peer_ready[kTileMaxCluster], s_recv;
   __shared__ short s_group[kTileMaxGroups];
   __shared__ uint32_t s_tmem;
   __shared__ int s_active, s_tiles;
@@ -86,9 +93,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t r = PAIR ? cluster_ctarank() : 0u;
-  const int worker = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;
-  const int workers = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+  const uint32_t crank = PAIR ? cluster_ctarank() : 0u, r = crank & 1u, lead = crank & ~1u;
+  const int cl = PAIR ? a.cl : 1, cs = (int)(crank >> 1);  // this pair's K range in a cluster that shares a tile
+  const int worker = PAIR ? ((int)blockIdx.x >> 1) / cl : (int)blockIdx.x;
+  const int workers = PAIR ? ((int)gridDim.x >> 1) / cl : (int)gridDim.x;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&full[i], 1);
@@ -96,8 +104,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], PAIR ? 8 : 4);
+      mbar_init(&tmem_empty[i], PAIR ? 16 : 8);  // eight epilogue warps in each CTA
     }
+    for (int i = 0; i < kTileMaxCluster; ++i) mbar_init(&s_peer_ready[i], 1);
+    mbar_init(&s_recv, 1);
     s_abort = 0;
     s_active = 1;
     s_group[0] = 0;
@@ -111,7 +121,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     if (PAIR) tmem_alloc_pair(&s_tmem, Cfg::kTmemCols);
     else tmem_alloc(&s_tmem, Cfg::kTmemCols);
   }
-  pdl_wait();
+  if (a.groups > 0) pdl_wait();  // the row ranges come from the kernel before this one
   if (a.groups > 0 && warp == 0) {
     int n = 0, tot = 0;
     for (int g0 = 0; g0 < a.groups; g0 += 32) {
@@ -138,9 +148,11 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   const uint32_t tmem_base = s_tmem;
   const int num_tiles = s_tiles, active = s_active;
 
+  const int kb0 = stream_begin(a.num_kb, cl, PAIR ? cs : 0), kb1 = stream_begin(a.num_kb, cl, PAIR ? cs + 1 : 1);
   auto fail = [&](uint32_t code) {
     s_abort = 1;
-    if (PAIR) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(&s_abort)), r ^ 1u), 1u);
+    for (uint32_t c = 0; PAIR && c < 2u * (uint32_t)cl; ++c)
+      if (c != crank) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(&s_abort)), c), 1u);
     atomicCAS(error_word, 0u, code);
   };
   auto open_group = [&](TileCursor& c) {
@@ -179,32 +191,48 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      // b (weights) does not depend on the predecessor: its share of the first ring is requested before the
+      // wait, the rows of a after it
+      int ahead = 0;
       TileCursor cur;
       start(cur);
+      auto b_row = [&](int n_blk) {
+        const int b0 = s_group[cur.g] * a.b_rows + n_blk * kNOut;
+        if (!PAIR) return b0;
+        return kSilu ? b0 + (int)r * (a.b_rows / 2) : b0 + (int)r * (BN / 2);
+      };
+      auto load_b = [&](int stage, int kb, int by) {
+        unsigned char* sb = tiles + stage * Cfg::kStageBytes + Cfg::kABytes;
+        if (PAIR) {
+          if (r == 0) mbar_expect_tx(&full[stage], 2u * Cfg::kStageBytes);
+          tma_load_2d_pair(sb, &map_b, map_to_cta(smem_u32(&full[stage]), lead), kb * kBlockK, by);
+        } else {
+          mbar_expect_tx(&full[stage], Cfg::kStageBytes);
+          tma_load_2d(sb, &map_b, &full[stage], kb * kBlockK, by);
+          if (kSilu) tma_load_2d(sb + Cfg::kBBytes / 2, &map_b, &full[stage], kb * kBlockK, by + a.b_rows / 2);
+        }
+      };
+      if (a.groups == 0 && worker < num_tiles) {
+        int row, n_blk;
+        locate(cur, worker, row, n_blk);
+        ahead = min(kStages, kb1 - kb0);
+        for (int i = 0; i < ahead; ++i) load_b(i, kb0 + i, b_row(n_blk));
+      }
+      pdl_wait();
       for (int tile = worker; ok && tile < num_tiles && !s_abort; tile += workers) {
         int row, n_blk;
         locate(cur, tile, row, n_blk);
-        const int b0 = s_group[cur.g] * a.b_rows;
-        int by = b0 + (PAIR && !kSilu ? n_blk * BN + (int)r * (BN / 2) : n_blk * kNOut);
-        if (PAIR && kSilu) by += (int)r * (a.b_rows / 2);
-        for (int kb = 0; kb < a.num_kb; ++kb) {
+        const int by = b_row(n_blk);
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_abortable(&empty[stage], phase ^ 1u, abort_flag)) {
             ok = false;
             break;
           }
           unsigned char* sa = tiles + stage * Cfg::kStageBytes;
-          if (PAIR) {
-            const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0u);
-            if (r == 0) mbar_expect_tx(&full[stage], 2u * Cfg::kStageBytes);
-            tma_load_2d_pair(sa, &map_a, bar, kb * kBlockK, row);
-            tma_load_2d_pair(sa + Cfg::kABytes, &map_b, bar, kb * kBlockK, by);
-          } else {
-            mbar_expect_tx(&full[stage], Cfg::kStageBytes);
-            tma_load_2d(sa, &map_a, &full[stage], kb * kBlockK, row);
-            tma_load_2d(sa + Cfg::kABytes, &map_b, &full[stage], kb * kBlockK, by);
-            if (kSilu)
-              tma_load_2d(sa + Cfg::kABytes + Cfg::kBBytes / 2, &map_b, &full[stage], kb * kBlockK, by + a.b_rows / 2);
-          }
+          if (ahead > 0) --ahead;
+          else load_b(stage, kb, by);
+          if (PAIR) tma_load_2d_pair(sa, &map_a, map_to_cta(smem_u32(&full[stage]), lead), kb * kBlockK, row);
+          else tma_load_2d(sa, &map_a, &full[stage], kb * kBlockK, row);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -233,7 +261,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
         bool ok = mbar_wait_abortable(&tmem_empty[ab], (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag);
         tc_fence_after_sync();
         const uint32_t d = tmem_base + (uint32_t)(ab * BN);
-        for (int kb = 0; ok && kb < a.num_kb; ++kb) {
+        for (int kb = kb0; ok && kb < kb1; ++kb) {
           if (!mbar_wait_abortable(&full[stage], phase, abort_flag)) {
             ok = false;
             break;
@@ -243,10 +271,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + Cfg::kABytes);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k) {
-            if (PAIR) umma_bf16_pair(d, advance_desc_k(da, k), advance_desc_k(db, k), idesc, (kb | k) != 0);
-            else umma_bf16(d, advance_desc_k(da, k), advance_desc_k(db, k), idesc, (kb | k) != 0);
+            if (PAIR) umma_bf16_pair(d, advance_desc_k(da, k), advance_desc_k(db, k), idesc, kb != kb0 || k != 0);
+            else umma_bf16(d, advance_desc_k(da, k), advance_desc_k(db, k), idesc, kb != kb0 || k != 0);
           }
-          if (PAIR) umma_commit_pair(&empty[stage], (uint16_t)3);
+          if (PAIR) umma_commit_pair(&empty[stage], (uint16_t)(3u << lead));
           else umma_commit(&empty[stage]);
           if (++stage == kStages) {
             stage = 0;
@@ -257,16 +285,25 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           fail(GEMM_ERR_MMA_WAIT);
           break;
         }
-        if (PAIR) umma_commit_pair(&tmem_full[ab], (uint16_t)3);
+        if (PAIR) umma_commit_pair(&tmem_full[ab], (uint16_t)(3u << lead));
         else umma_commit(&tmem_full[ab]);
       }
     }
   } else {
     // ---------------------------------------------- epilogue (this CTA's 128 rows)
-    const int q = warp & 3;
+    const int q = warp & 3, h = (warp - 2) >> 2;  // TMEM lane quarter; which of the two warps of it
     unsigned char* stg = epi_stage + (warp - 2) * (32 * kStageRowBytes);
+    // 64-column passes of this warp (the residual's sums of squares want both passes of 128 columns).  In a
+    // cluster CTA cs finishes passes [cs * per, + per) of its rows.
+    constexpr int kPasses = kNOut / 64;
+    constexpr int kGrain = EPI == TILE_EPI_RESIDUAL ? 2 : 1;
+    const int per = (kPasses / kGrain + cl - 1) / cl * kGrain;
+    const int own0 = min(kPasses, cs * per), own1 = min(kPasses, own0 + per);
+    const int half = (((own1 - own0) / kGrain + 1) / 2) * kGrain;
+    const int c_begin = own0 + h * half, c_end = min(own1, c_begin + half);
     TileCursor cur;
     start(cur);
+    pdl_wait();
     int it = 0;
     for (int tile = worker; tile < num_tiles; tile += workers, ++it) {
       int row, n_blk;
@@ -279,7 +316,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
         float s = 0.f;
         const int rr = min(row + lane, a.M - 1);
 #pragma unroll 8
-        for (int p = 0; p < a.scale_parts; ++p) s += __ldg(a.scale_sumsq + (size_t)p * a.M + rr);
+        for (int p = 0; p < a.scale_parts; ++p) s += __ldcg(a.scale_sumsq + (size_t)p * a.M + rr);
         scale = rsqrtf(s * a.inv_width + a.eps);
       }
       bool ok = !s_abort && mbar_wait_abortable(&tmem_full[ab], ((uint32_t)it >> 1) & 1u, abort_flag);
@@ -287,42 +324,97 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after_sync();
       const uint32_t tacc = tmem_base + (uint32_t)(ab * BN) + ((uint32_t)(q * 32) << 16);
+      // Cluster: every CTA hands its peers (same rows, other K ranges) the columns they finish, as
+      // [peer][per passes][accumulator columns of a pass / 4][128 rows] float4 in the ring of a CTA that has
+      // said that its MMAs are complete (a cluster works on one tile).
+      constexpr int kAcc = kSilu ? 128 : 64;  // accumulator columns of a pass
+      float4* s_in = reinterpret_cast<float4*>(tiles) + q * 32 + lane;
+      if constexpr (PAIR) if (cl > 1) {
+        if (threadIdx.x == 64)
+          mbar_expect_tx(&s_recv, (uint32_t)((own1 - own0) * (cl - 1) * kAcc * kBlockM * 4));
+        if (warp == 2 && lane < cl && lane != cs)
+          mbar_arrive_cluster(map_to_cta(smem_u32(&s_peer_ready[cs]), 2u * (uint32_t)lane + r));
+        for (int d = 1; d < cl && ok; ++d) {
+          const int dst = (cs + d) % cl;  // everybody starts with another peer
+          ok = mbar_wait_cluster(&s_peer_ready[dst], 0u, abort_flag);
+          const uint32_t bar = map_to_cta(smem_u32(&s_recv), 2u * (uint32_t)dst + r);
+          const uint32_t remote = map_to_cta(smem_u32(s_in), 2u * (uint32_t)dst + r) +
+                                  (uint32_t)((cs - (cs > dst ? 1 : 0)) * per * kAcc * kBlockM * 4);
+          for (int c = dst * per; ok && c < min(kPasses, (dst + 1) * per); ++c)
+#pragma unroll 1
+            for (int k = h * (kAcc / 2); k < (h + 1) * (kAcc / 2); k += 32) {
+              uint32_t x[32];
+              tmem_ld_32x32(tacc + (k < 64 ? c * 64 + k : BN / 2 + c * 64 + k - 64), x);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                st_async_v4(remote + (uint32_t)((((c - dst * per) * kAcc + k) / 4 + j) * kBlockM * 16), bar, x[4 * j],
+                            x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+            }
+        }
+        if (own1 > own0) ok = ok && mbar_wait_cluster(&s_recv, 0u, abort_flag);
+        if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
+        if (!__all_sync(0xffffffffu, ok)) break;
+      }
+      // 32 accumulator columns of pass c of the finished tile: k in [0, kAcc)
+      auto load32 = [&](int c, int k, uint32_t (&x)[32]) {
+        tmem_ld_32x32(tacc + (k < 64 ? c * 64 + k : BN / 2 + c * 64 + k - 64), x);
+        tmem_ld_wait();
+        if (!PAIR || cl == 1) return;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        for (int p = 0; p < cl; ++p) {  // in K order, this CTA's own part in its place
+          if (p == cs) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(x[j]);
+          } else {
+            const float4* src = s_in + (((p - (p > cs ? 1 : 0)) * per + c - own0) * kAcc + k) / 4 * kBlockM;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float4 y = src[j * kBlockM];
+              v[4 * j] += y.x;
+              v[4 * j + 1] += y.y;
+              v[4 * j + 2] += y.z;
+              v[4 * j + 3] += y.w;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(v[j]);
+      };
       float ss[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) ss[i] = 0.f;
 #pragma unroll 1
-      for (int c = 0; c < kNOut / 64; ++c) {
+      for (int c = c_begin; c < c_end; ++c) {
         // 64 output columns of this warp's 32 rows
-        uint4 v[8];
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t x[32];
-          tmem_ld_32x32(tacc + c * 64 + hf * 32, x);
+          load32(c, hf * 32, x);
           if (kSilu) {
-            uint32_t u[32];
-            tmem_ld_32x32(tacc + BN / 2 + c * 64 + hf * 32, u);
-            tmem_ld_wait();
+            uint32_t up[32];
+            load32(c, 64 + hf * 32, up);
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-              const float gv = __uint_as_float(x[j]) * scale, uv = __uint_as_float(u[j]) * scale;
+              const float gv = __uint_as_float(x[j]) * scale, uv = __uint_as_float(up[j]) * scale;
               x[j] = __float_as_uint(__fdividef(gv, 1.f + __expf(-gv)) * uv);
             }
           } else {
-            tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(__uint_as_float(x[j]) * scale);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            v[hf * 4 + j].x = pack_bf16x2(x[8 * j], x[8 * j + 1]);
-            v[hf * 4 + j].y = pack_bf16x2(x[8 * j + 2], x[8 * j + 3]);
-            v[hf * 4 + j].z = pack_bf16x2(x[8 * j + 4], x[8 * j + 5]);
-            v[hf * 4 + j].w = pack_bf16x2(x[8 * j + 6], x[8 * j + 7]);
+            uint4 v;
+            v.x = pack_bf16x2(x[8 * j], x[8 * j + 1]);
+            v.y = pack_bf16x2(x[8 * j + 2], x[8 * j + 3]);
+            v.z = pack_bf16x2(x[8 * j + 4], x[8 * j + 5]);
+            v.w = pack_bf16x2(x[8 * j + 6], x[8 * j + 7]);
+            *reinterpret_cast<uint4*>(stg + lane * kStageRowBytes + (((hf * 4 + j) ^ (lane & 7)) << 4)) = v;
           }
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(stg + lane * kStageRowBytes + ((j ^ (lane & 7)) << 4)) = v[j];
         __syncwarp();
         const int col = n_blk * kNOut + c * 64 + (lane & 7) * 8;
         if (EPI == TILE_EPI_RESIDUAL) {
@@ -383,7 +475,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[ab]), 0u));
+        if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[ab]), lead));
         else mbar_arrive(&tmem_empty[ab]);
       }
     }
@@ -391,6 +483,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   // ------------------------------------------------------------------- teardown
   tc_fence_before_sync();
   __syncwarp();
+  pdl_wait();  // no thread leaves before the predecessor has finished
   if (PAIR) cluster_sync_all();
   else __syncthreads();
   if (warp == 1) {
@@ -401,7 +494,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
 }
 
 template <int BN, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTileThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 1)
 gemm_tile_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const TileArgs a,
                uint32_t* error_word) {
   gemm_tile_body<true, BN, EPI>(map_a, map_b, a, error_word);

@@ -7,6 +7,7 @@
 
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 namespace penny {
@@ -56,6 +57,36 @@ inline KernelSetup kernel_setup(const void* kernel, int smem_bytes, int threads_
   }
   done[{dev, kernel}] = ks;
   return ks;
+}
+
+// Clusters of `cluster` CTAs of this kernel that are resident at a time on the current device (asked once per
+// combination): clusters live inside a GPC, so larger ones leave SMs unused.  0 if the query fails.
+inline int max_clusters(const void* kernel, int cluster, int threads, size_t smem_bytes) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, size_t>, int> done;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(dev, kernel, cluster, smem_bytes);
+  auto it = done.find(key);
+  if (it != done.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(cluster * 128), 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  return done[key] = n;
 }
 
 }  // namespace penny

@@ -36,11 +36,12 @@ PENNY_STREAM_HD int stream_pairs(int units, int max_pairs) {
 }
 // Pairs per cluster.  With fewer tiles than pairs every tile is shared, and pairs of one cluster add their
 // parts through each other's shared memory instead of the workspace: the most (up to 4) that are resident
-// together with at least four K steps each.  1: the flat split (also for groups: tiles = 0).
-PENNY_STREAM_HD int stream_cluster(int tiles, int num_kb, int max_pairs) {
+// together (clusters[c]: how many clusters of c pairs the GPU holds) with at least four K steps each.
+// 1: the flat split.
+PENNY_STREAM_HD int stream_cluster(int tiles, int num_kb, const int* clusters) {
   int cl = 1;
   for (int c = 2; c <= 4; ++c)
-    if (tiles > 0 && tiles * c <= max_pairs && num_kb / c >= 4) cl = c;
+    if (tiles <= clusters[c] && num_kb / c >= 4) cl = c;
   return cl;
 }
 // units * pairs fits 32 bits (the launcher checks)
