@@ -7,7 +7,6 @@
 #include <torch/extension.h>
 
 #include "gemm_decode_sm100.h"
-#include "gemm_stream_sm100.h"
 #include "gemm_tile_sm100.h"
 #include "pdl.h"
 #include "gemm_sm100.h"
@@ -81,86 +80,10 @@ void bind_gemm(py::module_& m) {
     TORCH_CHECK(rc == cudaSuccess, "gemm_decode: ", cudaGetErrorString(rc));
   }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("silu_pairs") = false, py::arg("splits") = 0,
      py::arg("pdl") = true, py::arg("l2_budget") = -1, py::arg("smem_kb") = 0, py::arg("push") = py::none());
-  // Streamed GEMM for at most 256 rows of x per group (csrc/gemm_stream_sm100.cu).  epi: 0 plain, 1
-  // silu(gate) * up (up_offset: rows from a gate row to its up row, 64 or half of the weight rows), 2
-  // residual add + norm weight + sums of squares.  ranges: int32 row ranges of x (device), [groups, 2] or [groups + 1] borders;
-  // the weight is then [groups * rows, K] and max_rows bounds a group.  sumsq: the [parts, rows] fp32 sums
-  // of an earlier residual epilogue, whose 1 / rms multiplies this output.
-  m.def("gemm_stream", [](at::Tensor x, at::Tensor w, at::Tensor out, at::Tensor workspace, int64_t epi,
-                          int64_t up_offset, c10::optional<at::Tensor> ranges, int64_t max_rows,
-                          c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
-                          c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, bool pdl,
-                          int64_t smem_kb, int64_t cluster) {
-    auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
-    TORCH_CHECK(bf16(x) && bf16(w) && bf16(out) && x.dim() == 2 && w.dim() == 2 && out.dim() == 2,
-                "gemm_stream: 2-D bf16 CUDA tensors with contiguous rows");
-    penny::sm100::StreamGemm g = {};
-    g.x = x.data_ptr();
-    g.w = w.data_ptr();
-    g.out = out.data_ptr();
-    g.x_rows = (int)x.size(0);
-    g.K = (int)x.size(1);
-    g.groups = 0;
-    g.rows = g.x_rows;
-    g.w_rows = (int)w.size(0);
-    if (ranges.has_value()) {
-      // [groups, 2] starts and ends, or [groups + 1] borders
-      TORCH_CHECK(ranges->is_cuda() && ranges->scalar_type() == at::kInt && ranges->is_contiguous() &&
-                      (ranges->dim() == 1 || (ranges->dim() == 2 && ranges->size(1) == 2)),
-                  "gemm_stream: ranges must be [groups, 2] or [groups + 1] int32 CUDA");
-      g.groups = (int)(ranges->dim() == 1 ? ranges->size(0) - 1 : ranges->size(0));
-      g.range_stride = (int)ranges->dim();
-      TORCH_CHECK(g.groups > 0 && w.size(0) % g.groups == 0, "gemm_stream: the weight must be whole groups of rows");
-      g.ranges = ranges->data_ptr<int>();
-      g.rows = (int)max_rows;
-      g.w_rows = (int)(w.size(0) / g.groups);
-    }
-    TORCH_CHECK(g.rows >= 1 && g.rows <= penny::sm100::kStreamMaxRows, "gemm_stream: 1 <= rows <= 256 per group");
-    TORCH_CHECK(w.size(1) == g.K && out.size(0) == x.size(0) && out.size(1) == (epi == 1 ? g.w_rows / 2 : g.w_rows),
-                "gemm_stream: shape mismatch");
-    g.ldx = (int)x.stride(0);
-    g.ldw = (int)w.stride(0);
-    g.ldo = (int)out.stride(0);
-    g.epi = (int)epi;
-    g.up_offset = (int)up_offset;
-    g.eps = (float)eps;
-    if (sumsq.has_value()) {
-      TORCH_CHECK(sumsq->is_cuda() && sumsq->scalar_type() == at::kFloat && sumsq->is_contiguous() && sumsq->dim() == 2 &&
-                      sumsq->size(1) == g.rows, "gemm_stream: sumsq must be [parts, rows] fp32");
-      g.scale_sumsq = sumsq->data_ptr<float>();
-      g.scale_parts = (int)sumsq->size(0);
-      g.scale_width = g.K;
-    }
-    if (epi == 2) {
-      TORCH_CHECK(residual.has_value() && bf16(*residual) && residual->sizes() == out.sizes() &&
-                      residual->stride(0) == out.stride(0) && norm_w.has_value() == sumsq_out.has_value(),
-                  "gemm_stream: residual like out; norm_w and sumsq_out together");
-      g.residual = residual->data_ptr();
-      if (norm_w.has_value()) {
-        TORCH_CHECK(bf16(*norm_w) && norm_w->numel() == g.w_rows && sumsq_out->is_cuda() &&
-                        sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
-                        sumsq_out->numel() == (int64_t)(g.w_rows / 128) * g.rows,
-                    "gemm_stream: norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
-        g.norm_w = norm_w->data_ptr();
-        g.sumsq_out = sumsq_out->data_ptr<float>();
-      }
-    }
-    TORCH_CHECK(workspace.is_cuda() && workspace.is_contiguous(), "gemm_stream: CUDA workspace");
-    g.workspace = workspace.data_ptr();
-    g.workspace_bytes = workspace.nbytes();
-    g.pdl = pdl;
-    g.smem_kb = (int)smem_kb;
-    g.cluster = (int)cluster;
-    const at::cuda::OptionalCUDAGuard guard(x.device());
-    const cudaError_t rc =
-        penny::sm100::launch_gemm_stream(g, penny_gemm_error_word(), at::cuda::getCurrentCUDAStream().stream());
-    TORCH_CHECK(rc == cudaSuccess, "gemm_stream: ", cudaGetErrorString(rc));
-  }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("workspace"), py::arg("epi") = 0, py::arg("up_offset") = 64,
-     py::arg("ranges") = py::none(), py::arg("max_rows") = 0, py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5,
-     py::arg("residual") = py::none(), py::arg("norm_w") = py::none(), py::arg("sumsq_out") = py::none(),
-     py::arg("pdl") = true, py::arg("smem_kb") = 0, py::arg("cluster") = 0);
-  // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu): epi as gemm_stream, the gate rows of a
-  // weight before its up rows; ranges: as gemm_stream, of a and out; b [groups * rows, K].
+  // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
+  // rows before its up rows, out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
+  // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
+  // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
@@ -224,9 +147,6 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = true,
      py::arg("cluster") = 0);
-  m.def("gemm_stream_workspace_bytes", [](int64_t rows) {
-    return (int64_t)penny::sm100::stream_workspace_bytes((int)rows, penny::sm100::stream_max_pairs());
-  }, py::arg("rows"), "bytes of gemm_stream's workspace for up to `rows` rows per group; zero it once");
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K);
   });

@@ -15,7 +15,6 @@ template <bool PAIR, int BN, int EPI>
 cudaError_t launch_tile(const TileGemm& g, TileArgs a, int sms, uint32_t* error_word, cudaStream_t stream) {
   using Cfg = TileCfg<PAIR, BN>;
   constexpr bool kSilu = EPI == TILE_EPI_SILU;
-  constexpr int kPasses = (kSilu ? BN / 2 : BN) / 64;
   a.cl = 1;
   a.tiles_n = (a.n_out + (kSilu ? BN / 2 : BN) - 1) / (kSilu ? BN / 2 : BN);
   a.band = std::max(1, 2048 / Cfg::kRows);
@@ -33,23 +32,23 @@ cudaError_t launch_tile(const TileGemm& g, TileArgs a, int sms, uint32_t* error_
   // grouped: the tile count is only known on the device
   const long long tiles = (long long)((g.M + Cfg::kRows - 1) / Cfg::kRows) * a.tiles_n;
   const int slots = PAIR ? ks.pairs : sms;
-  if constexpr (PAIR) {
-    a.cl = std::min({std::max(1, g.cluster), kTileMaxCluster, kPasses / (EPI == TILE_EPI_RESIDUAL ? 2 : 1)});
-    if (a.cl > 1 && (g.groups > 0 || a.num_kb < a.cl)) return cudaErrorInvalidValue;
-  }
-  // (a cluster that splits its tiles works on one: its exchange areas are used once)
-  const int workers = a.cl > 1 ? (int)tiles : (g.groups > 0 ? slots : (int)std::min<long long>(slots, tiles));
+  a.cl = std::max(1, std::min({g.cluster, kTileMaxCluster, a.num_kb}));
+  // A cluster works on one tile, so with groups (whose tiles the device counts) no group may have two row tiles.
+  if (a.cl > 1 && g.groups > 0 && g.M > Cfg::kRows) return cudaErrorInvalidValue;
+  const int workers = a.cl > 1 ? (g.groups > 0 ? g.groups * a.tiles_n : (int)tiles) : (g.groups > 0 ? slots : (int)std::min<long long>(slots, tiles));
   if constexpr (PAIR)
     return launch_kernel_ex(gemm_tile_pair<BN, EPI>, dim3((unsigned)(2 * workers * a.cl)), dim3(kTileThreads),
                             Cfg::kSmemBytes, stream, g.pdl, 2 * a.cl, ma, mb, a, error_word);
   else
-    return launch_kernel_ex(gemm_tile_single<BN, EPI>, dim3((unsigned)workers), dim3(kTileThreads), Cfg::kSmemBytes,
-                            stream, g.pdl, 1, ma, mb, a, error_word);
+    return launch_kernel_ex(gemm_tile_single<BN, EPI>, dim3((unsigned)(workers * a.cl)), dim3(kTileThreads),
+                            Cfg::kSmemBytes, stream, g.pdl, a.cl, ma, mb, a, error_word);
 }
 
 // Tile and cluster by rounds times the time of a K step.  Steps measured on B200, one 4096-long K (us per
 // step, all operands through the 64 B / clk that an SM takes in): 128 x 128 0.32, 128 x 192 0.36, 128 x 256
-// 0.40, 256 x 256 on a pair 0.36; the exchange of a cluster's sums takes about as long as 11 steps.
+// 0.40, 256 x 256 on a pair 0.36.  The exchange of a cluster's sums takes about as long as 13 steps of single
+// CTAs (q / k / v of 128 tokens: 23.2 us whole, 17.5 in two; down 72.5 whole, 31.6 in four, 40.5 on pairs in
+// three) and 18 of a pair.
 void choose_tile(TileGemm& g, int sms, int pairs) {
   const long long m128 = (g.M + 127) / 128, m256 = (g.M + 255) / 256;
   const int num_kb = (g.K + kBlockK - 1) / kBlockK;
@@ -58,20 +57,26 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
     const double cost = (double)((tiles + slots - 1) / slots) * steps;
     if (g.block_n == 0 || cost < best) best = cost, g.block_n = block_n, g.cluster = cluster;
   };
-  auto clusters = [&](int c) {
-    return max_clusters(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>), 2 * c, kTileThreads,
-                        TileCfg<true, 256>::kSmemBytes);
+  auto clusters = [&](bool pair, int c) {
+    if (pair)
+      return max_clusters(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>), 2 * c, kTileThreads,
+                          TileCfg<true, 256>::kSmemBytes);
+    const void* fn = reinterpret_cast<const void*>(gemm_tile_single<128, TILE_EPI_PLAIN>);
+    if (kernel_setup(fn, TileCfg<false, 128>::kSmemBytes).rc != cudaSuccess) return 0;
+    return max_clusters(fn, c, kTileThreads, TileCfg<false, 128>::kSmemBytes);
   };
   auto cols = [&](int bn) { return (long long)((g.b_rows + bn - 1) / bn); };
   offer(128, 1, m128 * cols(128), sms, 0.32 * num_kb);
   if (g.epi == TILE_EPI_PLAIN) offer(192, 1, m128 * cols(192), sms, 0.36 * num_kb);
   offer(256, 1, m128 * cols(256), sms, 0.40 * num_kb);
+  for (int c = 2; c <= kTileMaxCluster && g.groups == 0; ++c)
+    if (m128 * cols(128) <= clusters(false, c) && num_kb >= 4 * c)
+      offer(128, c, m128 * cols(128), sms, 0.32 * ((num_kb + c - 1) / c + 13));
   if (pairs > 0 && pair_kernel_enabled()) {
     const long long tiles = m256 * cols(256);
     offer(512, 1, tiles, pairs, 0.36 * num_kb);
-    const int most = g.epi == TILE_EPI_PLAIN ? kTileMaxCluster : 2;
-    for (int c = 2; c <= most && g.groups == 0; ++c)
-      if (tiles <= clusters(c) && num_kb >= 4 * c) offer(512, c, tiles, pairs, 0.36 * ((num_kb + c - 1) / c + 11));
+    for (int c = 2; c <= kTileMaxCluster && g.groups == 0; ++c)
+      if (tiles <= clusters(true, c) && num_kb >= 4 * c) offer(512, c, tiles, pairs, 0.36 * ((num_kb + c - 1) / c + 18));
   }
 }
 

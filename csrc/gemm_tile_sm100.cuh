@@ -11,9 +11,9 @@
 //              epilogue of a tile runs under the next tile's MMAs
 //   warps 2-9  epilogue: TMEM -> registers (thread = row) -> swizzled staging rows ->
 //              128-byte row segments; two warps per lane quarter share the columns
-// Few tiles with a long K (o_proj and down of a few hundred tokens): the pairs of a
-// cluster split the K steps of a tile and exchange their fp32 sums through each
-// other's shared memory, every CTA finishing a part of the columns.
+// Few tiles with a long K (the linears of a few hundred tokens): the pairs or CTAs of
+// a cluster split the K steps of a tile and hand each other their fp32 sums through
+// shared memory, each finishing the rows of its share of the four TMEM quarters.
 // SILU: a b tile is BN / 2 gate rows and the BN / 2 up rows of the same features, so
 // both halves of a product are columns of one accumulator and only the activation
 // is written.  RESIDUAL: the output is added to the residual stream, which is kept
@@ -26,21 +26,20 @@
 #include "gemm_kernel_sm100.cuh"
 #include "gemm_tile_sm100.h"
 #include "pdl.h"
-#include "stream_gemm_plan.h"
 
 namespace penny {
 namespace sm100 {
 
 constexpr int kTileThreads = 320;
 constexpr int kTileMaxGroups = 256;
-constexpr int kTileMaxCluster = 4;  // pairs
+constexpr int kTileMaxCluster = 4;  // pairs or single CTAs: a TMEM quarter each
 
 struct TileArgs {
   __nv_bfloat16* out;
   int ldo, M, n_out;     // n_out: columns of out
   int num_kb, tiles_n, band;
   int groups, b_rows;
-  int cl;                // pairs per cluster; above 1 a cluster splits the K steps of every tile
+  int cl;                // pairs (or CTAs) per cluster; above 1 a cluster splits the K steps of its tile
   const int* ranges;
   int range_stride;
   const float* scale_sumsq;
@@ -80,6 +79,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   __shared__ uint64_t s_bars[2 * kStages + 4];
   __shared__ uint64_t s_peer_ready[kTileMaxCluster], s_recv;
   __shared__ short s_group[kTileMaxGroups];
+  __shared__ float s_half[2][kBlockM];  // RESIDUAL, 128 columns: sums of squares of the second 64
   __shared__ uint32_t s_tmem;
   __shared__ int s_active, s_tiles;
   __shared__ volatile int s_abort;
@@ -93,10 +93,11 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t crank = PAIR ? cluster_ctarank() : 0u, r = crank & 1u, lead = crank & ~1u;
-  const int cl = PAIR ? a.cl : 1, cs = (int)(crank >> 1);  // this pair's K range in a cluster that shares a tile
-  const int worker = PAIR ? ((int)blockIdx.x >> 1) / cl : (int)blockIdx.x;
-  const int workers = PAIR ? ((int)gridDim.x >> 1) / cl : (int)gridDim.x;
+  const uint32_t crank = cluster_ctarank(), r = PAIR ? crank & 1u : 0u, lead = PAIR ? crank & ~1u : crank;
+  const int cl = a.cl, cs = (int)(PAIR ? crank >> 1 : crank);  // K range in a cluster that shares a tile
+  const int worker = (PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x) / cl;
+  const int workers = (PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x) / cl;
+  auto cta_of = [&](int d) { return PAIR ? 2u * (uint32_t)d + r : (uint32_t)d; };  // same rows, K range d
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&full[i], 1);
@@ -142,16 +143,16 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   }
   tc_fence_before_sync();
   __syncwarp();
-  if (PAIR) cluster_sync_all();
+  if (PAIR || cl > 1) cluster_sync_all();
   else __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = s_tmem;
   const int num_tiles = s_tiles, active = s_active;
 
-  const int kb0 = stream_begin(a.num_kb, cl, PAIR ? cs : 0), kb1 = stream_begin(a.num_kb, cl, PAIR ? cs + 1 : 1);
+  const int kb0 = a.num_kb * cs / cl, kb1 = a.num_kb * (cs + 1) / cl;
   auto fail = [&](uint32_t code) {
     s_abort = 1;
-    for (uint32_t c = 0; PAIR && c < 2u * (uint32_t)cl; ++c)
+    for (uint32_t c = 0; c < (PAIR ? 2u : 1u) * (uint32_t)cl; ++c)
       if (c != crank) st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(&s_abort)), c), 1u);
     atomicCAS(error_word, 0u, code);
   };
@@ -293,14 +294,15 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     // ---------------------------------------------- epilogue (this CTA's 128 rows)
     const int q = warp & 3, h = (warp - 2) >> 2;  // TMEM lane quarter; which of the two warps of it
     unsigned char* stg = epi_stage + (warp - 2) * (32 * kStageRowBytes);
-    // 64-column passes of this warp (the residual's sums of squares want both passes of 128 columns).  In a
-    // cluster CTA cs finishes passes [cs * per, + per) of its rows.
+    // 64-column passes of this warp.  (RESIDUAL writes a sum of squares per 128 columns: both passes of them, or
+    // with 128 columns in all the two warps of a quarter add theirs.)
     constexpr int kPasses = kNOut / 64;
-    constexpr int kGrain = EPI == TILE_EPI_RESIDUAL ? 2 : 1;
-    const int per = (kPasses / kGrain + cl - 1) / cl * kGrain;
-    const int own0 = min(kPasses, cs * per), own1 = min(kPasses, own0 + per);
-    const int half = (((own1 - own0) / kGrain + 1) / 2) * kGrain;
-    const int c_begin = own0 + h * half, c_end = min(own1, c_begin + half);
+    constexpr bool kHalves = EPI == TILE_EPI_RESIDUAL && kPasses == 2;
+    constexpr int kGrain = EPI == TILE_EPI_RESIDUAL && !kHalves ? 2 : 1;
+    constexpr int kHalf = (kPasses / kGrain + 1) / 2 * kGrain;
+    const int c_begin = h * kHalf, c_end = min(kPasses, c_begin + kHalf);
+    // in a cluster the quarters [q0, q1) of the rows are finished here
+    const int q0 = (4 * cs + cl - 1) / cl, q1 = (4 * (cs + 1) + cl - 1) / cl, owner = q * cl / 4;
     TileCursor cur;
     start(cur);
     pdl_wait();
@@ -319,48 +321,61 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
         for (int p = 0; p < a.scale_parts; ++p) s += __ldcg(a.scale_sumsq + (size_t)p * a.M + rr);
         scale = rsqrtf(s * a.inv_width + a.eps);
       }
+      // RESIDUAL (the launcher wants whole, aligned rows of 64 columns here): the stream and the norm's weight
+      // travel while the product is finished, a pass ahead (behind it they were 3 us of the tail)
+      uint4 res[8], nw = make_uint4(0, 0, 0, 0);
+      auto load_residual = [&](int c) {
+        const int col = n_blk * kNOut + c * 64 + (lane & 7) * 8;
+        const __nv_bfloat16* rp = a.residual + (size_t)(row + (lane >> 3)) * a.ldo + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (row + i * 4 + (lane >> 3) < row_end && col < a.n_out) res[i] = *reinterpret_cast<const uint4*>(rp + (size_t)(i * 4) * a.ldo);
+        if (a.norm_w != nullptr && col < a.n_out) nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + col));
+      };
+      if (EPI == TILE_EPI_RESIDUAL && owner == cs && c_begin < c_end) load_residual(c_begin);
       bool ok = !s_abort && mbar_wait_abortable(&tmem_full[ab], ((uint32_t)it >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
       if (!__all_sync(0xffffffffu, ok)) break;
       tc_fence_after_sync();
       const uint32_t tacc = tmem_base + (uint32_t)(ab * BN) + ((uint32_t)(q * 32) << 16);
-      // Cluster: every CTA hands its peers (same rows, other K ranges) the columns they finish, as
-      // [peer][per passes][accumulator columns of a pass / 4][128 rows] float4 in the ring of a CTA that has
-      // said that its MMAs are complete (a cluster works on one tile).
-      constexpr int kAcc = kSilu ? 128 : 64;  // accumulator columns of a pass
-      float4* s_in = reinterpret_cast<float4*>(tiles) + q * 32 + lane;
-      if constexpr (PAIR) if (cl > 1) {
-        if (threadIdx.x == 64)
-          mbar_expect_tx(&s_recv, (uint32_t)((own1 - own0) * (cl - 1) * kAcc * kBlockM * 4));
-        if (warp == 2 && lane < cl && lane != cs)
-          mbar_arrive_cluster(map_to_cta(smem_u32(&s_peer_ready[cs]), 2u * (uint32_t)lane + r));
-        for (int d = 1; d < cl && ok; ++d) {
-          const int dst = (cs + d) % cl;  // everybody starts with another peer
-          ok = mbar_wait_cluster(&s_peer_ready[dst], 0u, abort_flag);
-          const uint32_t bar = map_to_cta(smem_u32(&s_recv), 2u * (uint32_t)dst + r);
-          const uint32_t remote = map_to_cta(smem_u32(s_in), 2u * (uint32_t)dst + r) +
-                                  (uint32_t)((cs - (cs > dst ? 1 : 0)) * per * kAcc * kBlockM * 4);
-          for (int c = dst * per; ok && c < min(kPasses, (dst + 1) * per); ++c)
+      // Cluster: a quarter's sums go to its owner, as [sender][accumulator column / 4][its rows] float4 in the
+      // ring of a CTA that has said that its MMAs are complete (a cluster works on one tile).
+      auto slot = [&](int from, int to, int rows, int q_first) {  // of this thread's row
+        return ((from - (from > to ? 1 : 0)) * (BN / 4)) * rows + (q - q_first) * 32 + lane;
+      };
+      const int own_rows = (q1 - q0) * 32;
+      const float4* s_in = reinterpret_cast<const float4*>(tiles);
+      if (cl > 1) {
+        if (threadIdx.x == 64) mbar_expect_tx(&s_recv, (uint32_t)(own_rows * BN * 4 * (cl - 1)));
+        if (warp == 2 && lane < cl && lane != cs) mbar_arrive_cluster(map_to_cta(smem_u32(&s_peer_ready[cs]), cta_of(lane)));
+        if (owner != cs) {
+          const int d0 = (4 * owner + cl - 1) / cl, rows = ((4 * (owner + 1) + cl - 1) / cl - d0) * 32;
+          ok = mbar_wait_cluster(&s_peer_ready[owner], 0u, abort_flag);
+          if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
+          if (!__all_sync(0xffffffffu, ok)) break;
+          const uint32_t bar = map_to_cta(smem_u32(&s_recv), cta_of(owner));
+          const uint32_t remote = map_to_cta(smem_u32(tiles), cta_of(owner)) + (uint32_t)slot(cs, owner, rows, d0) * 16;
 #pragma unroll 1
-            for (int k = h * (kAcc / 2); k < (h + 1) * (kAcc / 2); k += 32) {
-              uint32_t x[32];
-              tmem_ld_32x32(tacc + (k < 64 ? c * 64 + k : BN / 2 + c * 64 + k - 64), x);
-              tmem_ld_wait();
+          for (int k = h * (BN / 2); k < (h + 1) * (BN / 2); k += 32) {
+            uint32_t x[32];
+            tmem_ld_32x32(tacc + k, x);
+            tmem_ld_wait();
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                st_async_v4(remote + (uint32_t)((((c - dst * per) * kAcc + k) / 4 + j) * kBlockM * 16), bar, x[4 * j],
-                            x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
-            }
+            for (int j = 0; j < 8; ++j)
+              st_async_v4(remote + (uint32_t)((k / 4 + j) * rows * 16), bar, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+          }
+          break;
         }
-        if (own1 > own0) ok = ok && mbar_wait_cluster(&s_recv, 0u, abort_flag);
+        ok = mbar_wait_cluster(&s_recv, 0u, abort_flag);
         if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
         if (!__all_sync(0xffffffffu, ok)) break;
       }
       // 32 accumulator columns of pass c of the finished tile: k in [0, kAcc)
       auto load32 = [&](int c, int k, uint32_t (&x)[32]) {
-        tmem_ld_32x32(tacc + (k < 64 ? c * 64 + k : BN / 2 + c * 64 + k - 64), x);
+        const int col = k < 64 ? c * 64 + k : BN / 2 + c * 64 + k - 64;
+        tmem_ld_32x32(tacc + col, x);
         tmem_ld_wait();
-        if (!PAIR || cl == 1) return;
+        if (cl == 1) return;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = 0.f;
@@ -369,10 +384,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(x[j]);
           } else {
-            const float4* src = s_in + (((p - (p > cs ? 1 : 0)) * per + c - own0) * kAcc + k) / 4 * kBlockM;
+            const float4* src = s_in + slot(p, cs, own_rows, q0) + col / 4 * own_rows;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const float4 y = src[j * kBlockM];
+              const float4 y = src[j * own_rows];
               v[4 * j] += y.x;
               v[4 * j + 1] += y.y;
               v[4 * j + 2] += y.z;
@@ -418,15 +433,6 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
         __syncwarp();
         const int col = n_blk * kNOut + c * 64 + (lane & 7) * 8;
         if (EPI == TILE_EPI_RESIDUAL) {
-          // (the launcher wants whole, aligned rows of 64 columns here)
-          uint4 res[8];
-          const __nv_bfloat16* rp = a.residual + (size_t)(row + (lane >> 3)) * a.ldo + col;
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (row + i * 4 + (lane >> 3) < row_end && col < a.n_out)
-              res[i] = *reinterpret_cast<const uint4*>(rp + (size_t)(i * 4) * a.ldo);
-          uint4 nw = make_uint4(0, 0, 0, 0);
-          if (a.norm_w != nullptr && col < a.n_out) nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + col));
           const uint32_t ww[4] = {nw.x, nw.y, nw.z, nw.w};
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -448,6 +454,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
             *reinterpret_cast<uint4*>(a.residual + off) = make_uint4(zo[0], zo[1], zo[2], zo[3]);
             if (a.norm_w != nullptr) *reinterpret_cast<uint4*>(a.out + off) = make_uint4(wo[0], wo[1], wo[2], wo[3]);
           }
+          if (c + 1 < c_end) load_residual(c + 1);
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -457,8 +464,9 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           }
         }
         __syncwarp();
-        if (EPI == TILE_EPI_RESIDUAL && a.norm_w != nullptr && (c & 1)) {
+        if (EPI == TILE_EPI_RESIDUAL && a.norm_w != nullptr && (kHalves || (c & 1))) {
           // 128 columns done: sum over the eight lanes of a row
+          if (kHalves && h == 0) named_bar_sync(1 + q, 64);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             float s = ss[i];
@@ -466,10 +474,16 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
             s += __shfl_xor_sync(0xffffffffu, s, 2);
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             const int rr = row + i * 4 + (lane >> 3);
-            if ((lane & 7) == 0 && rr < row_end && col < a.n_out)
+            float* other = &s_half[it & 1][q * 32 + i * 4 + (lane >> 3)];
+            if (kHalves && h == 1) {
+              if ((lane & 7) == 0) *other = s;
+            } else if ((lane & 7) == 0 && rr < row_end && col < a.n_out) {
+              if (kHalves) s += *other;
               a.sumsq_out[(size_t)(n_blk * (BN / 128) + (c >> 1)) * a.M + rr] = s;
+            }
             ss[i] = 0.f;
           }
+          if (kHalves && h == 1) named_bar_sync(1 + q, 64);
         }
       }
       tc_fence_before_sync();
@@ -484,7 +498,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   tc_fence_before_sync();
   __syncwarp();
   pdl_wait();  // no thread leaves before the predecessor has finished
-  if (PAIR) cluster_sync_all();
+  if (PAIR || cl > 1) cluster_sync_all();
   else __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();

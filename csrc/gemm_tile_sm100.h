@@ -34,7 +34,8 @@ struct TileGemm {
   const void* norm_w;   // [b_rows]; null: only the residual add (out unused)
   float* sumsq_out;     // [b_rows / 128][M]
   int block_n;          // 0: choose; 128 / 192 / 256: single CTAs; 512: CTA pairs, 256 x 256
-  int cluster;          // CTA pairs that split the K steps of a tile (block_n 512, one round of tiles); 0, 1: none
+  int cluster;          // pairs (block_n 512) or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
+                        // groups only for M <= the tile's rows
   bool pdl;
 };
 

@@ -103,9 +103,6 @@ class LlamaSPPrefill:
         self.local = backend == "penny" and world == 1 and not self.cpu and (2 * self.F) % 128 == 0
         if self.local:
             self.sumsq = [torch.empty(n, tokens, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
-            self.workspace = None
-            if tokens <= 128:
-                self.workspace = torch.zeros(ops.gemm_stream_workspace_bytes(tokens), dtype=torch.uint8, device=self.dev)
         # kernels of this library per forward: per layer 2 norms, RoPE, silu*mul and (penny) 4 fused GEMMs
         self.kernels_per_forward = self.L * (4 + (4 if backend == "penny" else 0))
 
@@ -178,16 +175,9 @@ class LlamaSPPrefill:
 
     # ------------------------------------------------------------------ forward
     def _gemm(self, x, w, out, epi=0, sumsq=None, residual=None, norm_w=None, sumsq_out=None):
-        """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual).  Up to 128 tokens a narrow weight
-        is a stream that many CTA pairs share (streamed GEMM: o_proj 17 us against 22 us tiled, down 36 / 46 at
-        128 tokens); the wide gate/up weight has a tile for nearly every SM (63 us streamed, 45 tiled), and
-        above 128 tokens all of them are tiled."""
-        if self.workspace is not None and epi != 1:
-            ops.gemm_stream(x, w, out, self.workspace, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual,
-                            norm_w=norm_w, sumsq_out=sumsq_out)
-        else:
-            ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
-                          sumsq_out=sumsq_out)
+        """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual)."""
+        ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
+                      sumsq_out=sumsq_out)
 
     def _forward_local(self, x: torch.Tensor) -> torch.Tensor:
         """One rank.  h holds the residual stream times the next norm's weight, sumsq its sums of squares; the

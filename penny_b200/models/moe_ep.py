@@ -158,13 +158,6 @@ class MoeEPLayer:
                 w2[le] = torch.randn(cfg.hidden, cfg.ffn, device=dev, generator=g) * cfg.init_std
             self.w13.append(list(w13))
             self.w2.append(list(w2))
-        # Rows one expert can receive: a token picks it at most once.  Up to 256 the streamed GEMM reads every
-        # expert's weights once; more rows make the experts tensor-core work for the tiled one.
-        self.expert_rows = min(self.world * tokens, self.cap_rows)
-        self.workspace = None
-        if backend == "penny" and use_own_gemm and 0 < self.expert_rows <= 256:
-            self.workspace = torch.zeros(ops.gemm_stream_workspace_bytes(self.expert_rows), dtype=torch.uint8, device=dev)
-
     def _as_views(self, t) -> List[torch.Tensor]:
         return list(t) if isinstance(t, (list, tuple)) else [t]
 
@@ -195,15 +188,15 @@ class MoeEPLayer:
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
         w13, w2 = self._stack(self.w13[v]), self._stack(self.w2[v])
-        if self.workspace is not None:
-            ops.gemm_stream(rows, w13, act, self.workspace, 1, cfg.ffn, ranges, self.expert_rows)
-            ops.gemm_stream(act, w2, y, self.workspace, 0, 64, ranges, self.expert_rows)
-        else:
-            # 256-row tiles of CTA pairs, or 128-row ones where the average expert would leave half of those
-            # empty (the weights are read once per row tile either way)
-            block_n = 512 if self.world * self.tokens * cfg.topk > 160 * cfg.experts else 256
-            ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
-            ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n)
+        # 128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of
+        # CTA pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against
+        # 857, 2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678).  Up to four rows the down projection (16 tiles
+        # of K 14336 per expert) leaves more than half of the SMs idle: two CTAs share a tile's K steps (4 experts
+        # 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then).
+        pairs = self.world * self.tokens * cfg.topk
+        block_n = 512 if pairs > 640 * cfg.experts else 256
+        ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
+        ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=2 if rows.shape[0] <= 4 else 0)
         return y
 
     def _experts(self, v: int, rows: torch.Tensor, ranges):

@@ -36,7 +36,6 @@ CUDA_SOURCES = [
     "csrc/gemm_sm100.cu",
     "csrc/gemm_fused_sm100.cu",
     "csrc/gemm_decode_sm100.cu",
-    "csrc/gemm_stream_sm100.cu",
     "csrc/gemm_tile_sm100.cu",
     "csrc/moe_dispatch_combine.cu",
     "csrc/moe_routing.cu",

@@ -1,0 +1,114 @@
+"""The tiled GEMM with fused epilogues against fp32 PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(rows, N, K, scale=0.05):
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + N * 3 + K)
+    x = torch.randn(rows, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * scale).bfloat16()
+    return x, w
+
+
+def _close(out, want):
+    rel = ((out.float() - want).norm() / want.norm()).item()
+    assert rel < 4e-3, rel
+    torch.testing.assert_close(out.float(), want, atol=2e-2 * want.std().item(), rtol=1e-2)
+
+
+TILES = [128, 192, 256, 512, 0]
+
+
+@pytest.mark.parametrize("cluster", [0, 1, 2, 3, 4])  # pairs or CTAs that split a tile's K steps
+@pytest.mark.parametrize("block_n", TILES)
+@pytest.mark.parametrize("shape", [(1152, 768, 1024), (130, 200, 264), (2304, 1280, 512), (7, 64, 64), (256, 512, 8192)])
+def test_tile_plain(shape, block_n, cluster):
+    from penny_b200._ext import ops
+    M, N, K = shape
+    if cluster > K // 64:
+        pytest.skip("a cluster splits at least as many K steps")
+    a, b = _data(M, N, K)
+    for _ in range(2):
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.gemm_tile(a, b, out, block_n=block_n, cluster=cluster)
+        assert ops.gemm_error() == 0
+        _close(out, a.float() @ b.float().t())
+
+
+@pytest.mark.parametrize("block_n", [128, 256, 512])
+@pytest.mark.parametrize("shape", [(384, 704, 512), (129, 1792, 320)])
+def test_tile_silu_row_scale(shape, block_n):
+    from penny_b200._ext import ops
+    M, F, K = shape
+    a, b = _data(M, 2 * F, K, 0.02)
+    sumsq = torch.rand(5, M, device="cuda") * K / 5 + 1
+    y = (a.float() @ b.float().t()) * torch.rsqrt(sumsq.sum(0) / K + 1e-5)[:, None]
+    out = torch.full((M, F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.gemm_tile(a, b, out, 1, sumsq=sumsq, block_n=block_n, cluster=2)
+    assert ops.gemm_error() == 0
+    _close(out, torch.nn.functional.silu(y[:, :F]) * y[:, F:])
+
+
+@pytest.mark.parametrize("cluster", [2, 3, 4])
+@pytest.mark.parametrize("block_n", [128, 256, 512])
+@pytest.mark.parametrize("shape", [(384, 1024, 512), (1000, 384, 1088)])
+def test_tile_residual(shape, block_n, cluster):
+    from penny_b200._ext import ops
+    M, N, K = shape
+    a, b = _data(M, N, K)
+    res = torch.randn(M, N, device="cuda").bfloat16()
+    plain = res.clone()
+    nw = (1 + 0.1 * torch.randn(N, device="cuda")).bfloat16()
+    z = res.float() + a.float() @ b.float().t()
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ss = torch.full((N // 128, M), float("nan"), device="cuda")
+    ops.gemm_tile(a, b, out, 2, residual=res, norm_w=nw, sumsq_out=ss, block_n=block_n, cluster=cluster)
+    ops.gemm_tile(a, b, plain, 2, residual=plain, block_n=block_n)
+    assert ops.gemm_error() == 0
+    _close(res, z)
+    _close(out, z * nw.float())
+    _close(plain, z)
+    torch.testing.assert_close(ss, z.pow(2).view(M, N // 128, 128).sum(-1).t(), atol=1e-1, rtol=1e-2)
+
+
+@pytest.mark.parametrize("block_n", [128, 256, 512])
+@pytest.mark.parametrize("counts", [[300, 0, 1, 129, 0, 1024], [0, 0], [0, 256, 256], [3, 0, 1, 40]])
+@pytest.mark.parametrize("cluster", [0, 2])
+def test_tile_groups(counts, block_n, cluster):
+    from penny_b200._ext import ops
+    if cluster and sum(counts) > 100:
+        pytest.skip("clusters want one row tile per group")
+    F, K, E = 384, 320, len(counts)
+    ends = torch.tensor(counts).cumsum(0) + 3
+    ranges = torch.stack([ends - torch.tensor(counts), ends], 1).to(torch.int32)
+    rows = int(ends[-1]) + 5
+    x, w = _data(rows, E * 2 * F, K, 0.05)
+    out = torch.full((rows, F), -7.0, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_tile(x, w, out, 1, ranges=ranges.cuda(), block_n=block_n, cluster=cluster)
+    assert ops.gemm_error() == 0
+    want = torch.full((rows, F), -7.0, device="cuda")
+    for e in range(E):
+        s, t = ranges[e].tolist()
+        y = x[s:t].float() @ w[e * 2 * F:(e + 1) * 2 * F].float().t()
+        want[s:t] = torch.nn.functional.silu(y[:, :F]) * y[:, F:]
+    _close(out, want)
+
+
+@pytest.mark.parametrize("tokens", [128, 384])  # clusters that split K, and whole tiles
+def test_prefill_one_rank_matches_fp32(tokens):
+    from penny_b200.models.llama_sp import LlamaSPPrefill
+    from penny_b200.models.llama_tp import LlamaConfig
+    from penny_b200.parallel.comm import Communicator
+    cfg, layers = LlamaConfig.tiny(), 2
+    x = torch.randn(tokens, cfg.hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).bfloat16()
+    want = LlamaSPPrefill.reference_forward(cfg, x, layers, seed=1)
+    comm = Communicator.emulated(1, heap_bytes=64 << 20)
+    try:
+        m = LlamaSPPrefill(cfg, comm=comm, tokens=tokens, layers=layers, seed=1)
+        for _ in range(2):
+            got = m.forward(x).float()
+            assert ((got - want).norm() / want.norm()).item() < 1.5e-2
+    finally:
+        comm.close()
