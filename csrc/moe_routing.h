@@ -15,6 +15,9 @@ cudaError_t launch_moe_topk(const void* logits, int tokens, int experts, int top
 // expert_sorted[pairs], send_off[experts + 1] (exclusive prefix of counts), counts[experts].
 cudaError_t launch_moe_tables(const int* ids, int pairs, int experts, int* order, int* expert_sorted, int* send_off,
                               int* counts, cudaStream_t stream);
+// Both of the above.
+cudaError_t launch_moe_route_tables(const void* logits, int tokens, int experts, int topk, int* ids, float* gates,
+                                    int* order, int* expert_sorted, int* send_off, int* counts, cudaStream_t stream);
 // counts_all [world, experts] -> dst_base [world, experts] (row at the expert's owner where the rows of
 // (source rank, expert) start; rows ordered by local expert, then source rank), rows_per_rank [world],
 // expert_ranges [experts, 2] (start, end at the owner).

@@ -20,6 +20,7 @@ list).  The reference has no MoE path; its exchange is a pairwise swap
 """
 from __future__ import annotations
 
+import operator
 from dataclasses import dataclass
 from typing import List
 
@@ -144,7 +145,7 @@ class MoeEPLayer:
         # weights: router replicated; experts sharded
         self.ranks = list(range(self.world)) if comm.emulated else [comm.rank]
         g = torch.Generator(device=dev)
-        self.router, self.w13, self.w2 = [], [], []
+        self.router, self.w13, self.w2, self._whole = [], [], [], []
         for r in self.ranks:
             g.manual_seed(seed * 7919 + 1)
             self.router.append((torch.randn(cfg.experts, cfg.hidden, device=dev, generator=g) * cfg.init_std).to(dt))
@@ -158,6 +159,7 @@ class MoeEPLayer:
                 w2[le] = torch.randn(cfg.hidden, cfg.ffn, device=dev, generator=g) * cfg.init_std
             self.w13.append(list(w13))
             self.w2.append(list(w2))
+            self._whole.append([(list(self.w13[-1]), w13.view(-1, cfg.hidden)), (list(self.w2[-1]), w2.view(-1, cfg.ffn))])
     def _as_views(self, t) -> List[torch.Tensor]:
         return list(t) if isinstance(t, (list, tuple)) else [t]
 
@@ -171,15 +173,20 @@ class MoeEPLayer:
             torch.matmul(a, w.t(), out=out)
         return out
 
-    @staticmethod
-    def _stack(mats: List[torch.Tensor]) -> torch.Tensor:
-        """[experts * rows, K] over the experts' matrices: the tensor they are views of, or a copy when a
-        caller has put other tensors into the list."""
-        m = mats[0]
-        step = m.numel() * m.element_size()
-        if all(t.data_ptr() == m.data_ptr() + i * step and t.is_contiguous() for i, t in enumerate(mats)):
-            return m.as_strided((len(mats) * m.shape[0], m.shape[1]), (m.shape[1], 1))
-        return torch.cat(mats)
+    def _stacked(self, v: int) -> List[torch.Tensor]:
+        """Gate/up and down weights of this rank's experts as [experts * rows, K]: the tensors that the lists'
+        entries are views of, or a copy when a caller has put other tensors into a list."""
+        return [whole if all(map(operator.is_, mats, views)) else torch.cat(mats)
+                for mats, (views, whole) in zip((self.w13[v], self.w2[v]), self._whole[v])]
+
+    def _tiles(self, rows: int):
+        """Tile of the grouped GEMMs and cluster of the down projection for up to `rows` received rows.
+        128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of CTA
+        pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against 857,
+        2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678).  Up to four rows the down projection (16 tiles of
+        K 14336 per expert) leaves more than half of the SMs idle: two CTAs share a tile's K steps (4 experts
+        156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then)."""
+        return (512 if self.world * self.tokens * self.cfg.topk > 640 * self.cfg.experts else 256), (2 if rows <= 4 else 0)
 
     def _experts_grouped(self, v: int, rows: torch.Tensor, ranges: torch.Tensor):
         """SwiGLU FFN of this rank's local experts over its received rows in two launches; `ranges`
@@ -187,16 +194,10 @@ class MoeEPLayer:
         cfg = self.cfg
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
-        w13, w2 = self._stack(self.w13[v]), self._stack(self.w2[v])
-        # 128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of
-        # CTA pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against
-        # 857, 2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678).  Up to four rows the down projection (16 tiles
-        # of K 14336 per expert) leaves more than half of the SMs idle: two CTAs share a tile's K steps (4 experts
-        # 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then).
-        pairs = self.world * self.tokens * cfg.topk
-        block_n = 512 if pairs > 640 * cfg.experts else 256
+        w13, w2 = self._stacked(v)
+        block_n, down_cluster = self._tiles(rows.shape[0])
         ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
-        ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=2 if rows.shape[0] <= 4 else 0)
+        ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=down_cluster)
         return y
 
     def _experts(self, v: int, rows: torch.Tensor, ranges):
@@ -215,14 +216,20 @@ class MoeEPLayer:
         """x: [tokens, hidden] (a list with one tensor per virtual rank when emulated)."""
         cfg, comm = self.cfg, self.comm
         xs = self._as_views(x)
+        x0, pairs = xs[0], xs[0].shape[0] * cfg.topk
+        if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
+                and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
+                and cfg.topk <= 8 and cfg.experts <= 256):
+            w13, w2 = self._stacked(0)
+            out = ops.comm_moe_layer(comm._h, x0, self.router[0], w13, w2, self.dst_row_of_pair[0], self.recv[0],
+                                     self.meta[0], self.comb[0], cfg.topk, *self._tiles(pairs))
+            return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):
             i, g = route(torch.matmul(xv, self.router[v].t()), cfg.topk)
             ids.append(i)
             gates.append(g)
             tables.append(build_routing(i, cfg.experts))
-        if self.world == 1 and self.backend == "penny" and self.use_own_gemm and ids[0].numel() <= self.cap_rows:
-            return self._forward_one_rank(xs[0], ids[0], gates[0], tables[0])
         # every rank learns how many rows each rank sends to each expert
         if self.world > 1:
             for v in range(len(xs)):
@@ -256,19 +263,6 @@ class MoeEPLayer:
                              else rows_per_rank[self.ranks[0]], cfg.experts)
             return outs if comm.emulated else outs[0]
         return self._forward_nccl(xs[0], ids[0], gates[0], tables[0], counts_all, rows_per_rank, expert_ranges)
-
-    def _forward_one_rank(self, x, ids, gates, table):
-        """A world of one: the rows received are the pairs in sorted order, so their placement is the sender's
-        table, no capacity can be exceeded and nothing has to come back to the host between the kernels."""
-        cfg, comm = self.cfg, self.comm
-        order, expert_sorted, borders, _ = table
-        comm.moe_dispatch(x, order, expert_sorted, borders, borders[:cfg.experts], self.dst_row_of_pair[0],
-                          self.recv[0], self.meta[0], cfg.topk, cfg.experts)
-        y = self._experts_grouped(0, self.recv[0][:ids.numel()], borders)
-        out = torch.empty_like(x)
-        comm.moe_combine(y, out, ids.reshape(-1), gates.reshape(-1), self.meta[0], self.dst_row_of_pair[0], self.comb[0],
-                         0, cfg.experts)
-        return [out] if comm.emulated else out
 
     def _forward_nccl(self, x, ids, gates, table, counts_all, rows_per_rank, expert_ranges):
         """Baseline: the same layer with NCCL all_to_all_single for both exchanges."""
