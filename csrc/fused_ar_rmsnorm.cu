@@ -50,10 +50,10 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
   return t;
 }
 
-// z (fp32, K vectors per thread) -> residual_out / out for one row.
-template <typename T, int K>
-__device__ __forceinline__ void norm_and_store(float (&z)[K][16 / sizeof(T)], int nv, int HV,
-                                               const FusedNormArgs& a, size_t row, float* smem) {
+// z (fp32, K vectors per thread) -> residual_out / out for one row; weight(k, v): 16 bytes of the norm's weight.
+template <typename T, int K, class Weight>
+__device__ __forceinline__ void norm_and_store(float (&z)[K][16 / sizeof(T)], int nv, int HV, const FusedNormArgs& a,
+                                               size_t row, float* smem, Weight&& weight) {
   constexpr int E = 16 / sizeof(T);
   float ss = 0.f;
 #pragma unroll
@@ -67,14 +67,13 @@ __device__ __forceinline__ void norm_and_store(float (&z)[K][16 / sizeof(T)], in
   const float rstd = rsqrtf(ss / (float)a.hidden + a.eps);
   T* out = reinterpret_cast<T*>(a.out) + row * (size_t)a.hidden;
   T* rout = a.residual_out ? reinterpret_cast<T*>(a.residual_out) + row * (size_t)a.hidden : nullptr;
-  const T* w = reinterpret_cast<const T*>(a.weight);
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     if (k < nv) {
       const int v = threadIdx.x + k * blockDim.x;
       if (rout) st16(rout + (size_t)v * E, pack<T>(z[k]));
       float wv[E], o[E];
-      unpack_set<T>(ld16(w + (size_t)v * E), wv);
+      unpack_set<T>(weight(k, v), wv);
 #pragma unroll
       for (int i = 0; i < E; ++i) o[i] = z[k][i] * rstd * wv[i];
       st16(out + (size_t)v * E, pack<T>(o));
@@ -93,21 +92,30 @@ __global__ void __launch_bounds__(512) k_add_rmsnorm(const FusedNormArgs a) {
   pdl_launch_dependents();
   const int HV = a.hidden / E;
   pdl_wait();
+  // One row costs a few latencies and nothing else: all its loads leave together, the weight's too (loaded
+  // behind the block sum it was a third of the kernel's memory time).
   for (size_t row = blockIdx.x; row < (size_t)a.rows; row += gridDim.x) {
     float z[kMaxVecPerThread][E];
+    V16 x[kMaxVecPerThread], r[kMaxVecPerThread], w[kMaxVecPerThread];
     int nv = 0;
 #pragma unroll
     for (int k = 0; k < kMaxVecPerThread; ++k) {
       const int v = threadIdx.x + k * blockDim.x;
       if (v < HV) {
         nv = k + 1;
-        unpack_set<T>(ld16(reinterpret_cast<const T*>(a.in) + row * a.hidden + (size_t)v * E), z[k]);
-        if (a.residual)
-          unpack_add<T>(ld16(reinterpret_cast<const T*>(a.residual) + row * a.hidden + (size_t)v * E),
-                        z[k]);
+        x[k] = ld16(reinterpret_cast<const T*>(a.in) + row * a.hidden + (size_t)v * E);
+        if (a.residual) r[k] = ld16(reinterpret_cast<const T*>(a.residual) + row * a.hidden + (size_t)v * E);
+        w[k] = ld16(reinterpret_cast<const T*>(a.weight) + (size_t)v * E);
       }
     }
-    norm_and_store<T, kMaxVecPerThread>(z, nv, HV, a, row, smem);
+#pragma unroll
+    for (int k = 0; k < kMaxVecPerThread; ++k) {
+      if (k < nv) {
+        unpack_set<T>(x[k], z[k]);
+        if (a.residual) unpack_add<T>(r[k], z[k]);
+      }
+    }
+    norm_and_store<T, kMaxVecPerThread>(z, nv, HV, a, row, smem, [&](int k, int) { return w[k]; });
   }
 }
 
@@ -203,7 +211,9 @@ struct FusedOneShotNorm {
         // a timeout anywhere in the block abandons the row for the whole block
         if (__syncthreads_or(ok ? 0 : 1)) return;
       }
-      norm_and_store<T, kMaxVecPerThread>(z, nv, HV, a, row, smem);
+      norm_and_store<T, kMaxVecPerThread>(z, nv, HV, a, row, smem, [&](int, int v) {
+        return ld16(reinterpret_cast<const T*>(a.weight) + (size_t)v * E);
+      });
     }
   }
   static __device__ void run(const CommCtx& c, int rank, const FusedNormArgs& a, const Blk& b) {

@@ -493,11 +493,14 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
     a.push = *push;
   else
     a.push.world = 0;
-  // ring depth: what fits next to the receive area in ~106 KB (two kernels per SM); with a
-  // 128-wide batch tile one kernel per SM and as deep as the range needs
+  // ring depth: what fits next to the receive area in ~106 KB (two CTAs per SM, of this kernel or the next:
+  // one sets up and fills its ring while the other drains).  With a 128-wide batch tile and no more CTAs than
+  // SMs one per SM and as deep as the range needs.  A second round of CTAs wants the two as well (the step
+  // of 128 sequences, gate/up 62.8 us -> 45, the LM head at one sequence 176 -> 163, at 64 195 -> 181, at 128
+  // 232 -> 209).
   const int kb_per = (a.num_kb + splits - 1) / splits;
   // (measured, whole N = 1 decode step: 106 KB 6.08 ms, 75 KB 6.40, 56 KB 6.72, 150 KB 7.40)
-  const size_t budget = smem_kb > 0 ? (size_t)std::min(smem_kb, 226) << 10 : (BT <= 64 ? (size_t)106 << 10 : (size_t)200 << 10);
+  const size_t budget = smem_kb > 0 ? (size_t)std::min(smem_kb, 226) << 10 : (BT <= 64 || tiles * slabs * splits > sms ? (size_t)106 << 10 : (size_t)200 << 10);
   int stages = Cfg::min_stages();
   while (stages < kMaxStages && stages < kb_per && Cfg::smem_bytes(stages + 1, splits) <= budget) ++stages;
   a.stages = stages;

@@ -283,12 +283,12 @@ class LlamaTPDecoder:
             dist.all_reduce(part, group=self.pg)
             ops.add_rmsnorm(part, self.residual, weight, self.x, self.residual, self.cfg.eps)
 
-    def _linear(self, x, w, out, silu_pairs=False, smem_kb=0, push=None):
+    def _linear(self, x, w, out, silu_pairs=False, push=None):
         """out = x @ w^T on this library's decode GEMM: one launch (batches above 128 rows run as
         slabs of 128 rows inside it, 1024 rows per launch at most)."""
         B = x.shape[0]
         for r in range(0, B, 1024):
-            ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, smem_kb, push)
+            ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, 0, push)
 
     def _step_impl(self):
         cfg = self.cfg
@@ -317,8 +317,7 @@ class LlamaTPDecoder:
             nxt = self.layers[li + 1]["norm1"] if li + 1 < cfg.layers else self.final_norm
             self._reduce_norm(self.parts[1], nxt)
         if self.linears == "penny":
-            # nothing of the step needs to overlap with the LM head: give it the whole shared memory
-            self._linear(self.x, self.lm_head, self.logits, smem_kb=200)
+            self._linear(self.x, self.lm_head, self.logits)
         else:
             torch.matmul(self.x, self.lm_head.t(), out=self.logits)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
