@@ -110,7 +110,9 @@ void bind_decode(py::module_& m) {
   });
   m.def("argmax_workspace_bytes", [](int64_t rows) { return (int64_t)argmax_workspace_bytes((int)rows); });
   m.def("argmax_rows", [](at::Tensor logits, at::Tensor out_val, at::Tensor out_idx, int64_t index_base,
-                          c10::optional<at::Tensor> workspace, c10::optional<at::Tensor> pair) {
+                          c10::optional<at::Tensor> workspace, c10::optional<at::Tensor> pair,
+                          c10::optional<at::Tensor> next_tokens, c10::optional<at::Tensor> tokens,
+                          c10::optional<at::Tensor> positions) {
     need(bf16_cuda(logits) && logits.dim() == 2, "argmax_rows expects [rows, cols] bf16");
     const int64_t rows = logits.size(0);
     need(out_val.is_cuda() && out_val.scalar_type() == at::kFloat && out_val.numel() == rows, "out_val [rows] fp32");
@@ -128,12 +130,22 @@ void bind_decode(py::module_& m) {
            "pair [2 * rows] fp32");
       pp = pair->data_ptr<float>();
     }
+    GreedyStep step = {};
+    if (next_tokens.has_value()) {
+      need(tokens.has_value() && positions.has_value() && next_tokens->is_cuda() && tokens->is_cuda() && positions->is_cuda() &&
+               next_tokens->scalar_type() == at::kLong && tokens->scalar_type() == at::kLong &&
+               positions->scalar_type() == at::kInt && next_tokens->numel() == rows && tokens->numel() == rows &&
+               positions->numel() == rows && next_tokens->is_contiguous() && tokens->is_contiguous() && positions->is_contiguous(),
+           "next_tokens / tokens [rows] int64, positions [rows] int32, together");
+      step = {(long long*)next_tokens->data_ptr<int64_t>(), (long long*)tokens->data_ptr<int64_t>(), positions->data_ptr<int>()};
+    }
     const at::cuda::OptionalCUDAGuard guard(logits.device());
     ck(launch_argmax(logits.data_ptr(), (int)rows, (int)logits.size(1), out_val.data_ptr<float>(),
-                     (long long*)out_idx.data_ptr<int64_t>(), pp, (long long)index_base, ws, cur()),
+                     (long long*)out_idx.data_ptr<int64_t>(), pp, (long long)index_base, ws, step, cur()),
        "argmax_rows");
   }, py::arg("logits"), py::arg("out_val"), py::arg("out_idx"), py::arg("index_base"),
-     py::arg("workspace") = py::none(), py::arg("pair") = py::none());
+     py::arg("workspace") = py::none(), py::arg("pair") = py::none(), py::arg("next_tokens") = py::none(),
+     py::arg("tokens") = py::none(), py::arg("positions") = py::none());
   // Expert-parallel MoE routing on the device (csrc/moe_routing.cu)
   m.def("moe_route", [](at::Tensor logits, int64_t topk) {
     need(bf16_cuda(logits) && logits.dim() == 2, "moe_route expects [tokens, experts] bf16");

@@ -417,13 +417,15 @@ __device__ __forceinline__ void argmax_take(float v, int i, float& best, int& bi
 __global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* __restrict__ logits, int cols, int per,
                                                 float* __restrict__ out_val, long long* __restrict__ out_idx,
                                                 float* __restrict__ pair, long long index_base,
-                                                unsigned int* __restrict__ workspace) {
+                                                unsigned int* __restrict__ workspace, const GreedyStep step) {
   __shared__ float sval[8];
   __shared__ int sidx[8];
   __shared__ bool s_last;
   const int rows = (int)gridDim.y, chunks = (int)gridDim.x, r = (int)blockIdx.y, ch = (int)blockIdx.x;
   const __nv_bfloat16* row = logits + (size_t)r * cols;
   const int c0 = ch * per, c1 = min(cols, c0 + per);
+  pdl_launch_dependents();
+  pdl_wait();
   float best = -INFINITY;
   int bi = 0x7fffffff;
   if ((reinterpret_cast<uintptr_t>(row + c0) & 15u) == 0) {
@@ -493,6 +495,10 @@ __global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* __restrict_
     if (pair != nullptr) {
       pair[r] = best;
       pair[rows + r] = (float)(index_base + bi);  // vocabularies stay below 2^24: exact
+    }
+    if (step.next_tokens != nullptr) {
+      step.next_tokens[r] = step.tokens[r] = index_base + bi;
+      step.positions[r] += 1;
     }
   }
 }
@@ -604,7 +610,7 @@ size_t argmax_workspace_bytes(int rows) {
 }
 
 cudaError_t launch_argmax(const void* logits, int rows, int cols, float* out_val, long long* out_idx, float* pair,
-                          long long index_base, void* workspace, cudaStream_t stream) {
+                          long long index_base, void* workspace, const GreedyStep& step, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0 || rows > 65535) return cudaErrorInvalidValue;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -613,10 +619,9 @@ cudaError_t launch_argmax(const void* logits, int rows, int cols, float* out_val
   chunks = std::max(chunks, 1);
   int per = ((cols + chunks - 1) / chunks + 7) / 8 * 8;
   chunks = (cols + per - 1) / per;
-  k_argmax<<<dim3((unsigned)chunks, (unsigned)rows), 256, 0, stream>>>((const __nv_bfloat16*)logits, cols, per, out_val,
-                                                                     out_idx, pair, index_base,
-                                                                     (unsigned int*)workspace);
-  return cudaGetLastError();
+  return launch_kernel_ex(k_argmax, dim3((unsigned)chunks, (unsigned)rows), dim3(256), 0, stream, true, 1,
+                          (const __nv_bfloat16*)logits, cols, per, out_val, out_idx, pair, index_base,
+                          (unsigned int*)workspace, step);
 }
 
 cudaError_t launch_sample_finish(const float* pairs, int world, int B, long long* next_tokens, long long* tokens,

@@ -47,10 +47,15 @@ cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cud
 
 // logits: [rows, cols] bf16 -> per-row max value and index (+ index_base).  workspace: zeroed once,
 // argmax_workspace_bytes(rows) bytes (nullptr: one block per row); pair: optional [2 * rows] fp32
-// (values, then indices).
+// (values, then indices); step: where the winners are the next tokens of a greedy step (one rank, no
+// sample_finish launch behind it), the buffers that take them and the positions to advance.
+struct GreedyStep {
+  long long *next_tokens, *tokens;  // [rows]; next_tokens == nullptr: none of this
+  int* positions;
+};
 size_t argmax_workspace_bytes(int rows);
 cudaError_t launch_argmax(const void* logits, int rows, int cols, float* out_val, long long* out_idx, float* pair,
-                          long long index_base, void* workspace, cudaStream_t stream);
+                          long long index_base, void* workspace, const GreedyStep& step, cudaStream_t stream);
 // pairs: [world][2][B] fp32 (values, indices) -> next_tokens[B] = tokens[B] = index of the largest
 // value over the ranks; positions[B] += 1.
 cudaError_t launch_sample_finish(const float* pairs, int world, int B, long long* next_tokens, long long* tokens,

@@ -85,7 +85,8 @@ __device__ __forceinline__ void norm_and_store(float (&z)[K][16 / sizeof(T)], in
 // ---------------------------------------------------------------------------
 // communication-free: out = rmsnorm(in + residual)
 // ---------------------------------------------------------------------------
-template <typename T>
+// K: vectors per thread; one where the block covers the row (registers for four leave one block per SM).
+template <typename T, int K>
 __global__ void __launch_bounds__(512) k_add_rmsnorm(const FusedNormArgs a) {
   constexpr int E = 16 / sizeof(T);
   __shared__ float smem[32];
@@ -95,11 +96,11 @@ __global__ void __launch_bounds__(512) k_add_rmsnorm(const FusedNormArgs a) {
   // One row costs a few latencies and nothing else: all its loads leave together, the weight's too (loaded
   // behind the block sum it was a third of the kernel's memory time).
   for (size_t row = blockIdx.x; row < (size_t)a.rows; row += gridDim.x) {
-    float z[kMaxVecPerThread][E];
-    V16 x[kMaxVecPerThread], r[kMaxVecPerThread], w[kMaxVecPerThread];
+    float z[K][E];
+    V16 x[K], r[K], w[K];
     int nv = 0;
 #pragma unroll
-    for (int k = 0; k < kMaxVecPerThread; ++k) {
+    for (int k = 0; k < K; ++k) {
       const int v = threadIdx.x + k * blockDim.x;
       if (v < HV) {
         nv = k + 1;
@@ -109,13 +110,13 @@ __global__ void __launch_bounds__(512) k_add_rmsnorm(const FusedNormArgs a) {
       }
     }
 #pragma unroll
-    for (int k = 0; k < kMaxVecPerThread; ++k) {
+    for (int k = 0; k < K; ++k) {
       if (k < nv) {
         unpack_set<T>(x[k], z[k]);
         if (a.residual) unpack_add<T>(r[k], z[k]);
       }
     }
-    norm_and_store<T, kMaxVecPerThread>(z, nv, HV, a, row, smem, [&](int k, int) { return w[k]; });
+    norm_and_store<T, K>(z, nv, HV, a, row, smem, [&](int k, int) { return w[k]; });
   }
 }
 
@@ -508,7 +509,11 @@ cudaError_t launch_add_rmsnorm(int dtype, const FusedNormArgs& a, int blocks, in
                                cudaStream_t stream) {
   if (!shape_ok(dtype, a, threads)) return cudaErrorInvalidValue;
   cudaError_t rc = cudaErrorInvalidValue;
-  PENNY_DISPATCH_DTYPE(dtype, T, rc = launch_kernel_ex(k_add_rmsnorm<T>, dim3(blocks), dim3(threads), 0, stream, true, 1, a));
+  const bool one = (size_t)a.hidden * dtype_size(dtype) <= (size_t)threads * 16;
+  PENNY_DISPATCH_DTYPE(dtype, T, {
+    rc = one ? launch_kernel_ex(k_add_rmsnorm<T, 1>, dim3(blocks), dim3(threads), 0, stream, true, 1, a)
+             : launch_kernel_ex(k_add_rmsnorm<T, kMaxVecPerThread>, dim3(blocks), dim3(threads), 0, stream, true, 1, a);
+  });
   return rc;
 }
 
