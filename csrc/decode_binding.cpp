@@ -5,10 +5,13 @@
 #include <torch/extension.h>
 
 #include "decode_kernels.h"
+#include "gemm_tile_sm100.h"
 #include "moe_routing.h"
 
 namespace py = pybind11;
 using namespace penny;
+
+uint32_t* penny_gemm_error_word();  // gemm_binding.cpp
 
 namespace {
 cudaStream_t cur() { return at::cuda::getCurrentCUDAStream().stream(); }
@@ -182,6 +185,56 @@ void bind_decode(py::module_& m) {
        "moe_placement");
     return std::make_tuple(dst_base, rows, ranges);
   });
+  // A MoE layer of one rank: router, rows by expert, expert SwiGLU FFNs, gate-weighted sum.  Nothing comes
+  // back to the host, and it is one call: as Python calls the launches took 113 us of host time, of which a
+  // layer of a few tokens hid half.  w13 [experts * 2 ffn, hidden] (gate rows, then up rows),
+  // w2 [experts * hidden, ffn]; block_n and down_cluster as in gemm_tile.
+  m.def("moe_layer", [](at::Tensor x, at::Tensor router, at::Tensor w13, at::Tensor w2, int64_t topk, int64_t block_n,
+                        int64_t down_cluster) {
+    for (const at::Tensor* t : {&x, &router, &w13, &w2})
+      need(bf16_cuda(*t) && t->dim() == 2 && ((uintptr_t)t->data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 tensors");
+    const int T = (int)x.size(0), H = (int)x.size(1), E = (int)router.size(0), F = (int)w2.size(1), P = T * (int)topk;
+    need(router.size(1) == H && w13.size(0) == (int64_t)E * 2 * F && w13.size(1) == H && w2.size(0) == (int64_t)E * H && T > 0,
+         "moe_layer shapes");
+    const at::cuda::OptionalCUDAGuard guard(x.device());
+    const cudaStream_t stream = cur();
+    const at::Tensor logits = at::matmul(x, router.t());
+    // [ids | order | expert of sorted | row of pair | borders | counts], then the gates
+    const at::Tensor tables = at::empty({4 * (int64_t)P + 2 * E + 1}, x.options().dtype(at::kInt));
+    const at::Tensor gates = at::empty({P}, x.options().dtype(at::kFloat));
+    const at::Tensor rows = at::empty({P, H}, x.options()), act = at::empty({P, F}, x.options()), out = at::empty_like(x);
+    int* ids = tables.data_ptr<int>();
+    int *order = ids + P, *sorted = order + P, *row_of_pair = sorted + P, *borders = row_of_pair + P, *counts = borders + E + 1;
+    ck(launch_moe_route_tables(logits.data_ptr(), T, E, (int)topk, ids, gates.data_ptr<float>(), order, sorted, borders, counts,
+                               stream), "moe_layer: routing");
+    ck(launch_moe_gather(x.data_ptr(), order, P, (int)topk, H, rows.data_ptr(), row_of_pair, stream), "moe_layer: rows");
+    sm100::TileGemm g = {};
+    g.a = rows.data_ptr();
+    g.b = w13.data_ptr();
+    g.out = act.data_ptr();
+    g.M = P;
+    g.b_rows = 2 * F;
+    g.K = g.lda = g.ldb = H;
+    g.ldo = F;
+    g.epi = sm100::TILE_EPI_SILU;
+    g.groups = E;
+    g.ranges = borders;
+    g.range_stride = 1;
+    g.block_n = (int)block_n;
+    g.pdl = true;
+    ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "moe_layer: gate / up");
+    g.a = act.data_ptr();
+    g.b = w2.data_ptr();
+    g.out = rows.data_ptr();  // (their inputs are used up)
+    g.b_rows = H;
+    g.K = g.lda = g.ldb = F;
+    g.ldo = H;
+    g.epi = sm100::TILE_EPI_PLAIN;
+    g.cluster = (int)down_cluster;
+    ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "moe_layer: down");
+    ck(launch_moe_sum(rows.data_ptr(), row_of_pair, gates.data_ptr<float>(), T, (int)topk, H, out.data_ptr(), stream), "moe_layer: sum");
+    return out;
+  }, py::arg("x"), py::arg("router"), py::arg("w13"), py::arg("w2"), py::arg("topk"), py::arg("block_n"), py::arg("down_cluster"));
   m.def("sample_finish", [](at::Tensor pairs, int64_t world, at::Tensor next_tokens, at::Tensor tokens,
                             at::Tensor positions) {
     const int64_t B = next_tokens.numel();

@@ -11,6 +11,9 @@
 //                    lanes of its own warp that hold the same expert, from __match_any_sync), so the
 //                    order of equal keys is the original order.  Outputs: order[P] (pair index by
 //                    sorted position), expert_sorted[P], send_off[E + 1], counts[E].
+//   k_moe_gather,    one rank: the rows in sorted order, and the gate-weighted sum of the experts' outputs.
+//   k_moe_sum        The exchange kernels do the same with their call sequence and barriers around it
+//                    (7 us each for a few tokens, against 3 and a start under the predecessor).
 //   k_moe_placement  one block: from every rank's counts (counts_all[W][E]) the row where each
 //                    (source rank, expert) block starts at the expert's owner - rows ordered by
 //                    local expert, then by source rank - plus rows per rank and per-expert ranges.
@@ -22,6 +25,7 @@
 #include <stdint.h>
 
 #include "moe_routing.h"
+#include "pdl.h"
 
 namespace penny {
 namespace {
@@ -74,6 +78,8 @@ __global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat1
                                                               int* __restrict__ order, int* __restrict__ expert_sorted,
                                                               int* __restrict__ send_off, int* __restrict__ counts) {
   extern __shared__ int sm[];
+  pdl_launch_dependents();
+  pdl_wait();
   int* hist = sm;                       // [E] pairs per expert, then the running write position
   int* warp_cnt = sm + experts;         // [warps][E] of the current tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -128,6 +134,71 @@ __global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat1
   }
 }
 
+// One warp per 128 vectors (2 KB) of a row: a few tokens still fill the GPU, a lane has four loads in flight.
+constexpr int kRowVecs = 4 * 32;
+
+__global__ void __launch_bounds__(256) k_moe_gather(const uint4* __restrict__ x, const int* __restrict__ order, int pairs,
+                                                    int topk, int hv, uint4* __restrict__ rows, int* __restrict__ row_of_pair) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pieces = (hv + kRowVecs - 1) / kRowVecs, u = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  if (u >= pairs * pieces) return;
+  const int i = u / pieces, v0 = (u - i * pieces) * kRowVecs + lane, pair = order[i];
+  if (v0 == 0) row_of_pair[pair] = i;
+  const uint4* src = x + (size_t)(pair / topk) * hv;
+  uint4 r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (v0 + k * 32 < hv) r[k] = src[v0 + k * 32];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (v0 + k * 32 < hv) rows[(size_t)i * hv + v0 + k * 32] = r[k];
+}
+
+__global__ void __launch_bounds__(256) k_moe_sum(const uint4* __restrict__ y, const int* __restrict__ row_of_pair,
+                                                 const float* __restrict__ gates, int tokens, int topk, int hv,
+                                                 uint4* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pieces = (hv + kRowVecs - 1) / kRowVecs, u = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  if (u >= tokens * pieces) return;
+  const int t = u / pieces, v0 = (u - t * pieces) * kRowVecs + lane;
+  float acc[4][8];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[k][j] = 0.f;
+  for (int e = 0; e < topk; ++e) {
+    const uint4* src = y + (size_t)row_of_pair[t * topk + e] * hv;
+    const float g = gates[t * topk + e];
+    uint4 r[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (v0 + k * 32 < hv) r[k] = src[v0 + k * 32];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (v0 + k * 32 < hv) {
+        const uint32_t w[4] = {r[k].x, r[k].y, r[k].z, r[k].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[k][2 * j] += g * __uint_as_float(w[j] << 16);
+          acc[k][2 * j + 1] += g * __uint_as_float(w[j] & 0xffff0000u);
+        }
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (v0 + k * 32 < hv) {
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(acc[k][2 * j], acc[k][2 * j + 1]);
+        w[j] = *reinterpret_cast<const uint32_t*>(&b);
+      }
+      out[(size_t)t * hv + v0 + k * 32] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 __global__ void k_moe_placement(const int* __restrict__ counts_all, int world, int experts, int* __restrict__ dst_base,
                                 int* __restrict__ rows_per_rank, int* __restrict__ expert_ranges) {
   // one thread per destination rank: a few hundred additions at most
@@ -160,9 +231,8 @@ cudaError_t launch_moe_tables(const int* ids, int pairs, int experts, int* order
                               int* counts, cudaStream_t stream) {
   if (pairs <= 0 || experts <= 0 || experts > kMoeMaxExperts) return cudaErrorInvalidValue;
   const size_t smem = (size_t)(1 + kRouteWarps) * experts * sizeof(int);
-  k_moe_tables<<<1, kRouteThreads, smem, stream>>>(nullptr, 1, const_cast<int*>(ids), nullptr, pairs, experts, order,
-                                                   expert_sorted, send_off, counts);
-  return cudaGetLastError();
+  return launch_kernel_ex(k_moe_tables, dim3(1), dim3(kRouteThreads), smem, stream, true, 1, (const __nv_bfloat16*)nullptr, 1,
+                          const_cast<int*>(ids), (float*)nullptr, pairs, experts, order, expert_sorted, send_off, counts);
 }
 
 cudaError_t launch_moe_route_tables(const void* logits, int tokens, int experts, int topk, int* ids, float* gates,
@@ -174,9 +244,24 @@ cudaError_t launch_moe_route_tables(const void* logits, int tokens, int experts,
   }
   if (tokens <= 0 || experts <= 0 || topk <= 0 || topk > kMoeMaxTopk || topk > experts) return cudaErrorInvalidValue;
   const size_t smem = (size_t)(1 + kRouteWarps) * experts * sizeof(int);
-  k_moe_tables<<<1, kRouteThreads, smem, stream>>>((const __nv_bfloat16*)logits, topk, ids, gates, tokens * topk, experts,
-                                                   order, expert_sorted, send_off, counts);
-  return cudaGetLastError();
+  return launch_kernel_ex(k_moe_tables, dim3(1), dim3(kRouteThreads), smem, stream, true, 1, (const __nv_bfloat16*)logits, topk,
+                          ids, gates, tokens * topk, experts, order, expert_sorted, send_off, counts);
+}
+
+cudaError_t launch_moe_gather(const void* x, const int* order, int pairs, int topk, int hidden, void* rows, int* row_of_pair,
+                              cudaStream_t stream) {
+  if (pairs <= 0 || topk <= 0 || hidden <= 0 || hidden % 8 != 0) return cudaErrorInvalidValue;
+  const int hv = hidden / 8, pieces = (hv + kRowVecs - 1) / kRowVecs;
+  return launch_kernel_ex(k_moe_gather, dim3((unsigned)(((long long)pairs * pieces + 7) / 8)), dim3(256), 0, stream, true, 1,
+                          (const uint4*)x, order, pairs, topk, hv, (uint4*)rows, row_of_pair);
+}
+
+cudaError_t launch_moe_sum(const void* y, const int* row_of_pair, const float* gates, int tokens, int topk, int hidden, void* out,
+                           cudaStream_t stream) {
+  if (tokens <= 0 || topk <= 0 || hidden <= 0 || hidden % 8 != 0) return cudaErrorInvalidValue;
+  const int hv = hidden / 8, pieces = (hv + kRowVecs - 1) / kRowVecs;
+  return launch_kernel_ex(k_moe_sum, dim3((unsigned)(((long long)tokens * pieces + 7) / 8)), dim3(256), 0, stream, true, 1,
+                          (const uint4*)y, row_of_pair, gates, tokens, topk, hv, (uint4*)out);
 }
 
 cudaError_t launch_moe_placement(const int* counts_all, int world, int experts, int* dst_base, int* rows_per_rank,

@@ -18,6 +18,12 @@ cudaError_t launch_moe_tables(const int* ids, int pairs, int experts, int* order
 // Both of the above.
 cudaError_t launch_moe_route_tables(const void* logits, int tokens, int experts, int topk, int* ids, float* gates,
                                     int* order, int* expert_sorted, int* send_off, int* counts, cudaStream_t stream);
+// One rank, bf16 rows of a multiple of 8 elements, 16-byte aligned: rows[i] = x[order[i] / topk] and
+// row_of_pair[order[i]] = i; out[t] = sum over k of gates[t, k] * y[row_of_pair[t, k]].
+cudaError_t launch_moe_gather(const void* x, const int* order, int pairs, int topk, int hidden, void* rows, int* row_of_pair,
+                              cudaStream_t stream);
+cudaError_t launch_moe_sum(const void* y, const int* row_of_pair, const float* gates, int tokens, int topk, int hidden, void* out,
+                           cudaStream_t stream);
 // counts_all [world, experts] -> dst_base [world, experts] (row at the expert's owner where the rows of
 // (source rank, expert) start; rows ordered by local expert, then source rank), rows_per_rank [world],
 // expert_ranges [experts, 2] (start, end at the owner).

@@ -23,8 +23,6 @@
 #include <unordered_map>
 
 #include "comm.h"
-#include "gemm_tile_sm100.h"
-#include "moe_routing.h"
 #include "schedule.h"
 
 namespace py = pybind11;
@@ -498,95 +496,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     c->moe_combine(dtype_of(out[0]), a, t, current_stream());
   }, py::arg("comm"), py::arg("y"), py::arg("out"), py::arg("topk_ids"), py::arg("gates"), py::arg("meta"),
      py::arg("dst_row_of_pair"), py::arg("comb"), py::arg("recv_rows"), py::arg("experts"), py::arg("blocks") = 0);
-
-  // A MoE layer of a world of one: router, dispatch, expert SwiGLU FFNs, combine.  The rows received are the
-  // pairs in sorted order, so their placement is the sender's table, no capacity can be exceeded beyond the
-  // caller's check and nothing has to come back to the host.  One call: as Python calls the six launches took
-  // 113 us of host time, of which a layer of a few tokens hid half.
-  // w13 [experts * 2 ffn, hidden] (gate rows, then up rows), w2 [experts * hidden, ffn]; block_n and
-  // down_cluster as in gemm_tile.
-  m.def("comm_moe_layer", [](int64_t h, at::Tensor x, at::Tensor router, at::Tensor w13, at::Tensor w2,
-                             at::Tensor dst_row_of_pair, at::Tensor recv, at::Tensor meta, at::Tensor comb, int topk,
-                             int block_n, int down_cluster) {
-    Communicator* c = as_comm(h);
-    const int T = (int)x.size(0), H = (int)x.size(1), E = (int)router.size(0), F = (int)w2.size(1), P = T * topk;
-    for (const at::Tensor* t : {&x, &router, &w13, &w2, &recv, &comb}) {
-      check_dense(*t, "comm_moe_layer tensors");
-      TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->dim() == 2, "comm_moe_layer: 2-D bf16 tensors");
-    }
-    TORCH_CHECK(c->views() == 1 && c->world() == 1, "comm_moe_layer: a world of one");
-    TORCH_CHECK(router.size(1) == H && w13.size(0) == (int64_t)E * 2 * F && w13.size(1) == H && w2.size(0) == (int64_t)E * H &&
-                    recv.size(1) == H && recv.size(0) >= P && comb.size(0) >= P && comb.size(1) == H && T > 0,
-                "comm_moe_layer: shapes");
-    for (const at::Tensor* t : {&dst_row_of_pair, &meta})
-      TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kInt && t->is_contiguous() && t->numel() >= P,
-                  "comm_moe_layer: int32 CUDA tables");
-    const at::cuda::OptionalCUDAGuard guard(x.device());
-    const cudaStream_t stream = current_stream();
-    auto ck = [](cudaError_t rc, const char* what) { TORCH_CHECK(rc == cudaSuccess, "comm_moe_layer: ", what, ": ", cudaGetErrorString(rc)); };
-    const at::Tensor logits = at::matmul(x, router.t());
-    // [ids | order | expert of sorted | borders | counts], then the gates
-    const at::Tensor tables = at::empty({3 * (int64_t)P + 2 * E + 1}, x.options().dtype(at::kInt));
-    const at::Tensor gates = at::empty({P}, x.options().dtype(at::kFloat));
-    int* ids = tables.data_ptr<int>();
-    int *order = ids + P, *sorted = order + P, *borders = sorted + P, *counts = borders + E + 1;
-    ck(launch_moe_route_tables(logits.data_ptr(), T, E, topk, ids, gates.data_ptr<float>(), order, sorted, borders, counts, stream),
-       "routing");
-    MoeArgs a;
-    memset(&a, 0, sizeof(a));
-    a.x = x.data_ptr();
-    a.order = order;
-    a.expert_of_sorted = sorted;
-    a.send_off = borders;
-    a.dst_base = borders;
-    a.dst_row_of_pair = dst_row_of_pair.data_ptr<int>();
-    a.recv_off = c->heap_offset_of(recv.data_ptr(), 0);
-    a.meta_off = c->heap_offset_of(meta.data_ptr(), 0);
-    a.comb_off = c->heap_offset_of(comb.data_ptr(), 0);
-    TORCH_CHECK(a.recv_off != kNotInHeap && a.meta_off != kNotInHeap && a.comb_off != kNotInHeap,
-                "comm_moe_layer: recv, meta and comb must be symmetric heap tensors");
-    a.tokens = T;
-    a.topk = topk;
-    a.hidden = H;
-    a.experts = E;
-    a.cap_rows = (int)recv.size(0);
-    const Tuning t;
-    c->moe_dispatch(DT_BF16, &a, t, stream);
-    const at::Tensor act = at::empty({P, F}, x.options()), y = at::empty({P, H}, x.options()), out = at::empty_like(x);
-    sm100::TileGemm g = {};
-    g.a = recv.data_ptr();
-    g.b = w13.data_ptr();
-    g.out = act.data_ptr();
-    g.M = P;
-    g.b_rows = 2 * F;
-    g.K = g.lda = g.ldb = H;
-    g.ldo = F;
-    g.epi = sm100::TILE_EPI_SILU;
-    g.groups = E;
-    g.ranges = borders;
-    g.range_stride = 1;
-    g.block_n = block_n;
-    g.pdl = true;
-    ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "gate / up");
-    g.a = act.data_ptr();
-    g.b = w2.data_ptr();
-    g.out = y.data_ptr();
-    g.b_rows = H;
-    g.K = g.lda = g.ldb = F;
-    g.ldo = H;
-    g.epi = sm100::TILE_EPI_PLAIN;
-    g.cluster = down_cluster;
-    ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "down");
-    a.x = y.data_ptr();
-    a.out = out.data_ptr();
-    a.topk_ids = ids;
-    a.gates = gates.data_ptr<float>();
-    a.meta = meta.data_ptr<int>();
-    a.recv_rows = 0;
-    c->moe_combine(DT_BF16, &a, t, stream);
-    return out;
-  }, py::arg("comm"), py::arg("x"), py::arg("router"), py::arg("w13"), py::arg("w2"), py::arg("dst_row_of_pair"),
-     py::arg("recv"), py::arg("meta"), py::arg("comb"), py::arg("topk"), py::arg("block_n"), py::arg("down_cluster"));
 
   // out[M / world, N] = this rank's row shard of sum_r a_r[M, K_r] @ b_r[N, K_r]^T
   m.def("comm_gemm_rs", [](int64_t h, at::Tensor a, at::Tensor b, at::Tensor out) {

@@ -221,8 +221,7 @@ class MoeEPLayer:
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
                 and cfg.topk <= 8 and cfg.experts <= 256):
             w13, w2 = self._stacked(0)
-            out = ops.comm_moe_layer(comm._h, x0, self.router[0], w13, w2, self.dst_row_of_pair[0], self.recv[0],
-                                     self.meta[0], self.comb[0], cfg.topk, *self._tiles(pairs))
+            out = ops.moe_layer(x0, self.router[0], w13, w2, cfg.topk, *self._tiles(pairs))
             return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):
