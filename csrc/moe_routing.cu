@@ -139,7 +139,8 @@ constexpr int kRowVecs = 4 * 32;
 
 __global__ void __launch_bounds__(256) k_moe_gather(const uint4* __restrict__ x, const int* __restrict__ order, int pairs,
                                                     int topk, int hv, uint4* __restrict__ rows, int* __restrict__ row_of_pair) {
-  pdl_launch_dependents();
+  // (a GEMM that sets up early leaves registers for one block per SM: only where one is enough)
+  if (gridDim.x <= 148) pdl_launch_dependents();
   pdl_wait();
   const int pieces = (hv + kRowVecs - 1) / kRowVecs, u = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if (u >= pairs * pieces) return;
