@@ -13,20 +13,11 @@
 
 namespace py = pybind11;
 
-namespace {
-// One error word per device, zeroed at creation; a non-zero value means a
-// pipeline wait ran out inside a GEMM kernel.
-at::Tensor& error_word() {
-  static std::vector<at::Tensor> words(64);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!words[dev].defined())
-    words[dev] = torch::zeros({4}, torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, dev));
-  return words[dev];
+uint32_t* penny_gemm_error_word() {
+  uint32_t* word = penny::sm100::gemm_error_word();
+  TORCH_CHECK(word != nullptr, "gemm: no error word on this device");
+  return word;
 }
-}  // namespace
-
-uint32_t* penny_gemm_error_word() { return reinterpret_cast<uint32_t*>(error_word().data_ptr<int>()); }
 
 void bind_gemm(py::module_& m) {
   // out[M, N] = a[M, K] @ b[N, K]^T (the nn.Linear convention: b is the weight)
@@ -166,9 +157,19 @@ void bind_gemm(py::module_& m) {
         "1 / 0: split (or not) the ragged last wave of the CTA-pair GEMM along K; -1: PENNY_GEMM_SPLIT_TAIL decides");
   // Synchronises; returns and clears the error code of the GEMM kernels (0 = fine).
   m.def("gemm_error", []() {
-    at::Tensor& w = error_word();
-    int v = w[0].item<int>();
-    if (v != 0) w.zero_();
+    uint32_t* word = penny_gemm_error_word();
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    int v = 0;
+    cudaError_t rc = cudaMemcpyAsync(&v, word, sizeof(v), cudaMemcpyDeviceToHost, stream);
+    if (rc == cudaSuccess) rc = cudaStreamSynchronize(stream);
+    if (rc == cudaSuccess && v != 0) rc = cudaMemsetAsync(word, 0, sizeof(v), stream);
+    TORCH_CHECK(rc == cudaSuccess, "gemm_error: ", cudaGetErrorString(rc));
     return v;
+  });
+  // The word itself as an int32 tensor [1] of the current device, to be looked at without a synchronisation.
+  m.def("gemm_error_word", []() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return at::from_blob(penny_gemm_error_word(), {1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev));
   });
 }

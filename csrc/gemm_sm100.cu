@@ -42,6 +42,25 @@ namespace penny {
 namespace sm100 {
 
 namespace {
+__device__ uint32_t g_gemm_error;
+}  // namespace
+
+uint32_t* gemm_error_word() {
+  static std::atomic<void*> address[64];  // (fixed once the library is loaded on a device)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  void* p = address[dev].load();
+  if (p == nullptr) {
+    if (cudaGetSymbolAddress(&p, g_gemm_error) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    address[dev].store(p);
+  }
+  return reinterpret_cast<uint32_t*>(p);
+}
+
+namespace {
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,

@@ -22,6 +22,11 @@ cudaError_t launch_gemm_bf16(const void* a, const void* b, void* c, int M, int N
                              int ldb, int ldc, int block_n, uint32_t* error_word,
                              cudaStream_t stream);
 
+// The error word of the current device (nullptr if the query fails): zero from the start, part of the library's
+// own device image.  (Allocated and zeroed on first use, it would live in the graph of a process whose first
+// GEMM is captured, and every replay would zero it before anyone reads it.)
+uint32_t* gemm_error_word();
+
 // False when PENNY_GEMM_PAIR=0 forces the single-CTA kernels everywhere.
 bool pair_kernel_enabled();
 // Whether the ragged last wave of the pair kernel is split along K over the idle

@@ -319,11 +319,13 @@ class LlamaTPDecoder:
         if self.linears == "penny":
             self._linear(self.x, self.lm_head, self.logits)
         else:
-            # (256 rows: 217 us on this library's tiles, 264-323 on the library's; level at 192.  The warm-up
-            # steps stay with the library throughout: they are there for its handle and workspace.)
-            if self.B > 192 and self.V >= 1 << 16 and not warm_up:
+            # (256 rows: 201 us on this library's tiles, 264 on the library's; level at 192.  A warm-up step runs
+            # both, so that neither's first launch is a captured one; the library's logits come last, and what
+            # the warm-up leaves behind the current positions is the same with either head.)
+            own_head = self.B > 192 and self.V >= 1 << 16
+            if own_head:
                 ops.gemm_tile(self.x, self.lm_head, self.logits)
-            else:
+            if warm_up or not own_head:
                 torch.matmul(self.x, self.lm_head.t(), out=self.logits)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
         # in fp32), gathered over the ranks; one kernel then picks the best rank per sequence, feeds the

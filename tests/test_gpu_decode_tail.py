@@ -1,5 +1,8 @@
 """The end of a greedy decode step on one GPU: LM head of a large batch, arg-max that hands the tokens on."""
 import dataclasses
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -37,3 +40,23 @@ def test_lm_head_of_a_large_batch(batch):
     err = (m.logits.float() - want).abs().max().item()
     assert err < 0.05 * want.std().item() + 0.02, err
     assert torch.equal(m.positions, positions + 1) and torch.equal(m.next_tokens, m.tokens)
+
+
+def test_gemm_error_outlives_a_captured_first_gemm():
+    """The first GEMM of a process is a captured one: its error word is zero before any replay, and a replay
+    leaves an error that is already there to be read."""
+    code = """if True:
+        import dataclasses, torch
+        from penny_b200._ext import ops
+        from penny_b200.models.llama_tp import LlamaConfig, LlamaTPDecoder
+        cfg = dataclasses.replace(LlamaConfig.tiny(), vocab=1 << 16)
+        m = LlamaTPDecoder(cfg, world=1, max_batch=200, max_len=40)
+        m.fill_synthetic_kv(20)
+        m.capture()
+        assert ops.gemm_error() == 0
+        ops.gemm_error_word().fill_(7)
+        m.step_device()
+        assert ops.gemm_error() == 7 and ops.gemm_error() == 0
+    """
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], cwd=root, check=True, timeout=300)
