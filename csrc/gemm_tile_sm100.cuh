@@ -303,6 +303,12 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     const int c_begin = h * kHalf, c_end = min(kPasses, c_begin + kHalf);
     // in a cluster the quarters [q0, q1) of the rows are finished here
     const int q0 = (4 * cs + cl - 1) / cl, q1 = (4 * (cs + 1) + cl - 1) / cl, owner = q * cl / 4;
+    // The two warps of a quarter that meet at a barrier below leave this loop together: a bounded wait that ran
+    // out in one of them, or an abort that only one has seen, ends it for both.
+    auto agree = [&](bool ok) {
+      ok = __all_sync(0xffffffffu, ok);
+      return kHalves ? named_bar_all(1 + q, 64, ok) : ok;
+    };
     TileCursor cur;
     start(cur);
     pdl_wait();
@@ -335,7 +341,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       if (EPI == TILE_EPI_RESIDUAL && owner == cs && c_begin < c_end) load_residual(c_begin);
       bool ok = !s_abort && mbar_wait_abortable(&tmem_full[ab], ((uint32_t)it >> 1) & 1u, abort_flag);
       if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!agree(ok)) break;
       tc_fence_after_sync();
       const uint32_t tacc = tmem_base + (uint32_t)(ab * BN) + ((uint32_t)(q * 32) << 16);
       // Cluster: a quarter's sums go to its owner, as [sender][accumulator column / 4][its rows] float4 in the
@@ -352,7 +358,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           const int d0 = (4 * owner + cl - 1) / cl, rows = ((4 * (owner + 1) + cl - 1) / cl - d0) * 32;
           ok = mbar_wait_cluster(&s_peer_ready[owner], 0u, abort_flag);
           if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
-          if (!__all_sync(0xffffffffu, ok)) break;
+          if (!__all_sync(0xffffffffu, ok)) break;  // (this branch leaves the loop before the barrier anyway)
           const uint32_t bar = map_to_cta(smem_u32(&s_recv), cta_of(owner));
           const uint32_t remote = map_to_cta(smem_u32(tiles), cta_of(owner)) + (uint32_t)slot(cs, owner, rows, d0) * 16;
 #pragma unroll 1
@@ -368,7 +374,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
         }
         ok = mbar_wait_cluster(&s_recv, 0u, abort_flag);
         if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        if (!agree(ok)) break;
       }
       // 32 accumulator columns of pass c of the finished tile: k in [0, kAcc)
       auto load32 = [&](int c, int k, uint32_t (&x)[32]) {
