@@ -185,6 +185,19 @@ void bind_decode(py::module_& m) {
        "moe_placement");
     return std::make_tuple(dst_base, rows, ranges);
   });
+  // Matrices of one shape that lie back to back in one storage, as one matrix of all their rows; None if they
+  // don't.  Looked at on every call: entries of a caller's list may be other tensors by now, or the same ones
+  // over other memory (tensor.data = ...).
+  m.def("stacked_rows", [](const std::vector<at::Tensor>& mats) -> c10::optional<at::Tensor> {
+    if (mats.empty() || !bf16_cuda(mats[0]) || mats[0].dim() != 2 || ((uintptr_t)mats[0].data_ptr() & 15) != 0) return c10::nullopt;
+    const at::Tensor& t0 = mats[0];
+    for (size_t i = 1; i < mats.size(); ++i)
+      if (!bf16_cuda(mats[i]) || mats[i].sizes() != t0.sizes() ||
+          mats[i].storage().unsafeGetStorageImpl() != t0.storage().unsafeGetStorageImpl() ||
+          mats[i].storage_offset() != t0.storage_offset() + (int64_t)i * t0.numel())
+        return c10::nullopt;
+    return t0.detach().as_strided({(int64_t)mats.size() * t0.size(0), t0.size(1)}, {t0.size(1), 1});
+  });
   // A MoE layer of one rank: router, rows by expert, expert SwiGLU FFNs, gate-weighted sum.  Nothing comes
   // back to the host, and it is one call: as Python calls the launches took 113 us of host time, of which a
   // layer of a few tokens hid half.  w13 [experts * 2 ffn, hidden] (gate rows, then up rows),

@@ -20,7 +20,6 @@ list).  The reference has no MoE path; its exchange is a pairwise swap
 """
 from __future__ import annotations
 
-import operator
 from dataclasses import dataclass
 from typing import List
 
@@ -145,12 +144,13 @@ class MoeEPLayer:
         # weights: router replicated; experts sharded
         self.ranks = list(range(self.world)) if comm.emulated else [comm.rank]
         g = torch.Generator(device=dev)
-        self.router, self.w13, self.w2, self._whole = [], [], [], []
+        self.router, self.w13, self.w2 = [], [], []
         for r in self.ranks:
             g.manual_seed(seed * 7919 + 1)
             self.router.append((torch.randn(cfg.experts, cfg.hidden, device=dev, generator=g) * cfg.init_std).to(dt))
             # one tensor per kind and rank, the experts' matrices are views of it: the grouped GEMMs address
-            # all of them through one descriptor
+            # all of them through one descriptor.  (Weights copied into the views keep that; a list whose entries
+            # are replaced by other tensors is taken one expert after another.)
             w13 = torch.empty(self.epr, 2 * cfg.ffn, cfg.hidden, dtype=dt, device=dev)
             w2 = torch.empty(self.epr, cfg.hidden, cfg.ffn, dtype=dt, device=dev)
             for le in range(self.epr):
@@ -159,7 +159,7 @@ class MoeEPLayer:
                 w2[le] = torch.randn(cfg.hidden, cfg.ffn, device=dev, generator=g) * cfg.init_std
             self.w13.append(list(w13))
             self.w2.append(list(w2))
-            self._whole.append([(list(self.w13[-1]), w13.view(-1, cfg.hidden)), (list(self.w2[-1]), w2.view(-1, cfg.ffn))])
+
     def _as_views(self, t) -> List[torch.Tensor]:
         return list(t) if isinstance(t, (list, tuple)) else [t]
 
@@ -173,11 +173,11 @@ class MoeEPLayer:
             torch.matmul(a, w.t(), out=out)
         return out
 
-    def _stacked(self, v: int) -> List[torch.Tensor]:
-        """Gate/up and down weights of this rank's experts as [experts * rows, K]: the tensors that the lists'
-        entries are views of, or a copy when a caller has put other tensors into a list."""
-        return [whole if all(map(operator.is_, mats, views)) else torch.cat(mats)
-                for mats, (views, whole) in zip((self.w13[v], self.w2[v]), self._whole[v])]
+    def _stacked(self, v: int):
+        """Gate/up and down weights of this rank's experts as [experts * rows, K], or None where an entry of the
+        lists does not lie behind the one before it (any more)."""
+        w13, w2 = ops.stacked_rows(self.w13[v][:self.epr]), ops.stacked_rows(self.w2[v][:self.epr])
+        return None if w13 is None or w2 is None else (w13, w2)
 
     def _tiles(self, rows: int):
         """Tile of the grouped GEMMs and cluster of the down projection for up to `rows` received rows.
@@ -188,13 +188,12 @@ class MoeEPLayer:
         156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then)."""
         return (512 if self.world * self.tokens * self.cfg.topk > 640 * self.cfg.experts else 256), (2 if rows <= 4 else 0)
 
-    def _experts_grouped(self, v: int, rows: torch.Tensor, ranges: torch.Tensor):
-        """SwiGLU FFN of this rank's local experts over its received rows in two launches; `ranges`
+    def _experts_grouped(self, w13: torch.Tensor, w2: torch.Tensor, rows: torch.Tensor, ranges: torch.Tensor):
+        """SwiGLU FFN of this rank's local experts (stacked) over its received rows in two launches; `ranges`
         [local experts, 2] stays on the device."""
         cfg = self.cfg
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
-        w13, w2 = self._stacked(v)
         block_n, down_cluster = self._tiles(rows.shape[0])
         ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
         ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=down_cluster)
@@ -219,9 +218,8 @@ class MoeEPLayer:
         x0, pairs = xs[0], xs[0].shape[0] * cfg.topk
         if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
-                and cfg.topk <= 8 and cfg.experts <= 256):
-            w13, w2 = self._stacked(0)
-            out = ops.moe_layer(x0, self.router[0], w13, w2, cfg.topk, *self._tiles(pairs))
+                and cfg.topk <= 8 and cfg.experts <= 256 and (stacked := self._stacked(0)) is not None):
+            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *self._tiles(pairs))
             return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):
@@ -251,8 +249,9 @@ class MoeEPLayer:
             ys = []
             for v, r in enumerate(self.ranks):
                 rows = self.recv[v][:rows_per_rank[r]]
-                if self.use_own_gemm and rows.shape[0] > 0:
-                    ys.append(self._experts_grouped(v, rows, ranges_dev[r * self.epr:(r + 1) * self.epr]))
+                stacked = self._stacked(v) if self.use_own_gemm and rows.shape[0] > 0 else None
+                if stacked is not None:
+                    ys.append(self._experts_grouped(*stacked, rows, ranges_dev[r * self.epr:(r + 1) * self.epr]))
                 else:
                     ys.append(self._experts(v, rows, expert_ranges[r]))
             outs = [torch.empty_like(xv) for xv in xs]

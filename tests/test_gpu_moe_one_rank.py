@@ -27,3 +27,49 @@ def test_one_rank(tokens, topk):
             torch.testing.assert_close(got.float(), want, atol=3e-3, rtol=3e-2)
     finally:
         comm.close()
+
+
+def _layer(cfg, tokens, world=1, **kw):
+    from penny_b200.models.moe_ep import MoeEPLayer
+    from penny_b200.parallel.comm import Communicator
+    comm = Communicator.emulated(world, heap_bytes=256 << 20, timeout_ms=3000)
+    return comm, MoeEPLayer(cfg, comm, tokens=tokens, **kw)
+
+
+def _check(layer, xs):
+    w13, w2 = sum(layer.w13, []), sum(layer.w2, [])
+    for got, want in zip(layer.forward(xs), layer.reference(xs, w13, w2, layer.router[0])):
+        torch.testing.assert_close(got.float(), want, atol=3e-3, rtol=3e-2)
+
+
+@pytest.mark.parametrize("world", [1, 2])
+def test_weights_are_those_of_the_lists(world):
+    """Entries replaced, given other memory, swapped or written to after construction: every forward uses what the
+    lists hold then, without a copy of the experts, and what they no longer hold is freed."""
+    from penny_b200.models.moe_ep import MoeConfig
+    cfg = MoeConfig(hidden=512, ffn=1024, experts=8, topk=2)
+    comm, layer = _layer(cfg, 64, world, cap_factor=float(world))
+    try:
+        xs = [torch.randn(64, cfg.hidden, device="cuda").bfloat16() for _ in range(world)]
+        fresh = lambda t: torch.randn_like(t) * 0.02  # noqa: E731
+        _check(layer, xs)
+        layer.w13[0][1].copy_(fresh(layer.w13[0][1]))
+        _check(layer, xs)
+        layer.w13[0][2].data = fresh(layer.w13[0][2])
+        _check(layer, xs)
+        layer.w2[-1][0], layer.w2[-1][1] = layer.w2[-1][1], layer.w2[-1][0]
+        _check(layer, xs)
+        both = sum(t.numel() for t in sum(layer.w13 + layer.w2, [])) * 2
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        layer.forward(xs)
+        assert torch.cuda.max_memory_allocated() - before < both // 4
+        for lists in (layer.w13, layer.w2):
+            for mats in lists:
+                mats[:] = [fresh(t) for t in mats]
+        del mats, lists
+        assert torch.cuda.memory_allocated() < before + both // 4  # (the tensors that the lists held are gone)
+        _check(layer, xs)
+    finally:
+        comm.close()
