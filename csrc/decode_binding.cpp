@@ -201,17 +201,19 @@ void bind_decode(py::module_& m) {
   // A MoE layer of one rank: router, rows by expert, expert SwiGLU FFNs, gate-weighted sum.  Nothing comes
   // back to the host, and it is one call: as Python calls the launches took 113 us of host time, of which a
   // layer of a few tokens hid half.  w13 [experts * 2 ffn, hidden] (gate rows, then up rows),
-  // w2 [experts * hidden, ffn]; block_n and down_cluster as in gemm_tile.
+  // w2 [experts * hidden, ffn]; block_n and down_cluster as in gemm_tile.  The router meets the library's GEMM only
+  // and may have any strides.
   m.def("moe_layer", [](at::Tensor x, at::Tensor router, at::Tensor w13, at::Tensor w2, int64_t topk, int64_t block_n,
                         int64_t down_cluster) {
-    for (const at::Tensor* t : {&x, &router, &w13, &w2})
+    for (const at::Tensor* t : {&x, &w13, &w2})
       need(bf16_cuda(*t) && t->dim() == 2 && ((uintptr_t)t->data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 tensors");
+    need(router.is_cuda() && router.scalar_type() == at::kBFloat16 && router.dim() == 2, "moe_layer: 2-D bf16 router");
     const int T = (int)x.size(0), H = (int)x.size(1), E = (int)router.size(0), F = (int)w2.size(1), P = T * (int)topk;
     need(router.size(1) == H && w13.size(0) == (int64_t)E * 2 * F && w13.size(1) == H && w2.size(0) == (int64_t)E * H && T > 0,
          "moe_layer shapes");
     const at::cuda::OptionalCUDAGuard guard(x.device());
     const cudaStream_t stream = cur();
-    const at::Tensor logits = at::matmul(x, router.t());
+    const at::Tensor logits = at::matmul(x, router.t()).contiguous();
     // [ids | order | expert of sorted | row of pair | borders | counts], then the gates
     const at::Tensor tables = at::empty({4 * (int64_t)P + 2 * E + 1}, x.options().dtype(at::kInt));
     const at::Tensor gates = at::empty({P}, x.options().dtype(at::kFloat));

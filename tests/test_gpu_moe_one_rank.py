@@ -73,3 +73,17 @@ def test_weights_are_those_of_the_lists(world):
         _check(layer, xs)
     finally:
         comm.close()
+
+
+def test_router_of_any_strides():
+    from penny_b200.models.moe_ep import MoeConfig
+    comm, layer = _layer(MoeConfig(hidden=256, ffn=640), 40)
+    try:
+        x = torch.randn(40, 256, device="cuda").bfloat16()
+        wide = torch.zeros(8, 257, device="cuda", dtype=torch.bfloat16)
+        wide[:, 1:] = layer.router[0]
+        for router in (layer.router[0].t().contiguous().t(), wide[:, 1:]):  # column-major; padded and unaligned
+            layer.router[0] = router
+            _check(layer, [x])
+    finally:
+        comm.close()
