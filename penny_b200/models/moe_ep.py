@@ -212,9 +212,12 @@ class MoeEPLayer:
         return y
 
     def forward(self, x):
-        """x: [tokens, hidden] (a list with one tensor per virtual rank when emulated)."""
+        """x: [tokens, hidden], tokens at most those the layer was built for (a list with one tensor per virtual rank
+        when emulated)."""
         cfg, comm = self.cfg, self.comm
         xs = self._as_views(x)
+        if max(xv.shape[0] for xv in xs) > self.tokens:  # the exchange's buffers and tables are that long
+            raise RuntimeError(f"MoE layer built for {self.tokens} tokens, called with {max(xv.shape[0] for xv in xs)}")
         x0, pairs = xs[0], xs[0].shape[0] * cfg.topk
         if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0

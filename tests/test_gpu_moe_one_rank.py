@@ -87,3 +87,16 @@ def test_router_of_any_strides():
             _check(layer, [x])
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("world", [1, 2])
+def test_more_tokens_than_built_for_are_refused(world):
+    from penny_b200.models.moe_ep import MoeConfig
+    comm, layer = _layer(MoeConfig(hidden=256, ffn=640), 40, world, cap_factor=float(world))
+    try:
+        xs = [torch.randn(41 if v == 0 else 40, 256, device="cuda").bfloat16() for v in range(world)]
+        with pytest.raises(RuntimeError, match="built for 40 tokens"):
+            layer.forward(xs)
+        _check(layer, [x[:40] for x in xs])
+    finally:
+        comm.close()
