@@ -252,7 +252,8 @@ class MoeEPLayer:
             ys = []
             for v, r in enumerate(self.ranks):
                 rows = self.recv[v][:rows_per_rank[r]]
-                stacked = self._stacked(v) if self.use_own_gemm and rows.shape[0] > 0 else None
+                # (one grouped launch holds up to 256 groups)
+                stacked = self._stacked(v) if self.use_own_gemm and rows.shape[0] > 0 and self.epr <= 256 else None
                 if stacked is not None:
                     ys.append(self._experts_grouped(*stacked, rows, ranges_dev[r * self.epr:(r + 1) * self.epr]))
                 else:

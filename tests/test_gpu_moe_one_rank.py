@@ -100,3 +100,13 @@ def test_more_tokens_than_built_for_are_refused(world):
         _check(layer, [x[:40] for x in xs])
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("experts", [256, 264])  # the most groups of a launch, and more
+def test_many_experts(experts):
+    from penny_b200.models.moe_ep import MoeConfig
+    comm, layer = _layer(MoeConfig(hidden=256, ffn=256, experts=experts), 200)
+    try:
+        _check(layer, [torch.randn(200, 256, device="cuda").bfloat16()])
+    finally:
+        comm.close()
