@@ -119,6 +119,17 @@ def placement(counts_all: torch.Tensor, world: int):
     return dst_base, rows_per_rank, expert_ranges
 
 
+def expert_tiles(rows: int, experts: int):
+    """Tile of the grouped GEMMs and cluster of the down projection for `rows` rows on a rank's `experts` experts.
+    128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of CTA
+    pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against 857,
+    2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678; at 5 to 500 tokens pairs cost 70 to 90 us of 334 to 510).
+    Up to four rows the down projection (16 tiles of K 14336 per expert) leaves more than half of the SMs idle:
+    two CTAs share a tile's K steps (4 experts 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles
+    then)."""
+    return (512 if rows > 640 * experts else 256), (2 if rows <= 4 else 0)
+
+
 class MoeEPLayer:
     def __init__(self, cfg: MoeConfig, comm, tokens: int, cap_factor: float = 2.0, backend: str = "penny",
                  seed: int = 0, use_own_gemm: bool = True):
@@ -179,22 +190,13 @@ class MoeEPLayer:
         w13, w2 = ops.stacked_rows(self.w13[v][:self.epr]), ops.stacked_rows(self.w2[v][:self.epr])
         return None if w13 is None or w2 is None else (w13, w2)
 
-    def _tiles(self, rows: int):
-        """Tile of the grouped GEMMs and cluster of the down projection for up to `rows` received rows.
-        128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of CTA
-        pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against 857,
-        2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678).  Up to four rows the down projection (16 tiles of
-        K 14336 per expert) leaves more than half of the SMs idle: two CTAs share a tile's K steps (4 experts
-        156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then)."""
-        return (512 if self.world * self.tokens * self.cfg.topk > 640 * self.cfg.experts else 256), (2 if rows <= 4 else 0)
-
     def _experts_grouped(self, w13: torch.Tensor, w2: torch.Tensor, rows: torch.Tensor, ranges: torch.Tensor):
         """SwiGLU FFN of this rank's local experts (stacked) over its received rows in two launches; `ranges`
         [local experts, 2] stays on the device."""
         cfg = self.cfg
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
-        block_n, down_cluster = self._tiles(rows.shape[0])
+        block_n, down_cluster = expert_tiles(rows.shape[0], self.epr)
         ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
         ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=down_cluster)
         return y
@@ -222,7 +224,7 @@ class MoeEPLayer:
         if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
                 and cfg.topk <= 8 and cfg.experts <= 256 and (stacked := self._stacked(0)) is not None):
-            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *self._tiles(pairs))
+            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *expert_tiles(pairs, self.epr))
             return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):

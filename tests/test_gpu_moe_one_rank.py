@@ -110,3 +110,23 @@ def test_many_experts(experts):
         _check(layer, [torch.randn(200, 256, device="cuda").bfloat16()])
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("world", [1, 2])
+def test_fewer_tokens_than_built_for(world, monkeypatch):
+    """A call's tiles follow its own rows: a layer built for a prefill batch decodes on the tiles of a small one."""
+    from penny_b200.models import moe_ep
+    cfg = moe_ep.MoeConfig(hidden=256, ffn=640)
+    comm, layer = _layer(cfg, 3000, world, cap_factor=float(world))
+    asked, rule = [], moe_ep.expert_tiles
+    monkeypatch.setattr(moe_ep, "expert_tiles", lambda rows, *a: asked.append((rows, rule(rows, *a)[0])) or rule(rows, *a))
+    try:
+        for tokens in (3000, 5, 700, 1):
+            asked.clear()
+            _check(layer, [torch.randn(tokens, cfg.hidden, device="cuda").bfloat16() for _ in range(world)])
+            comm.check()
+            assert sum(r for r, _ in asked) == world * tokens * cfg.topk
+            assert all(t == (512 if r > 640 * layer.epr else 256) for r, t in asked)
+            assert tokens == 3000 or {t for _, t in asked} == {256}
+    finally:
+        comm.close()
