@@ -119,15 +119,20 @@ def placement(counts_all: torch.Tensor, world: int):
     return dst_base, rows_per_rank, expert_ranges
 
 
-def expert_tiles(rows: int, experts: int):
+def expert_tiles(rows: int, experts: int, hidden: int, ffn: int, sms: int):
     """Tile of the grouped GEMMs and cluster of the down projection for `rows` rows on a rank's `experts` experts.
+
     128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of CTA
     pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against 857,
     2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678; at 5 to 500 tokens pairs cost 70 to 90 us of 334 to 510).
-    Up to four rows the down projection (16 tiles of K 14336 per expert) leaves more than half of the SMs idle:
-    two CTAs share a tile's K steps (4 experts 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles
-    then)."""
-    return (512 if rows > 640 * experts else 256), (2 if rows <= 4 else 0)
+
+    Where at most half of the SMs have a tile of the down projection, two CTAs share a tile's K steps (hidden 4096, ffn
+    14336, down alone: 4 experts 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then; whole layer
+    of 4 experts and 100 rows 292 -> 275).  Handing the sums over costs about 13 of the steps of 64 that half of K
+    must save (whole layer, 2 tokens, ffn 1024 / 1664 / 2048 / 4096: 68.3 / 76.0 / 79.3 / 120.1 us without, 69.4 /
+    75.8 / 77.7 / 108.4 with), and a cluster works on one row tile."""
+    shared = rows <= 128 and 2 * min(rows, experts) * -(-hidden // 256) <= sms and ffn > 2 * 13 * 64
+    return (512 if rows > 640 * experts else 256), (2 if shared else 0)
 
 
 class MoeEPLayer:
@@ -142,6 +147,7 @@ class MoeEPLayer:
         self.use_own_gemm = use_own_gemm
         dev = torch.device("cuda", torch.cuda.current_device())
         self.dev = dev
+        self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
         pairs = tokens * cfg.topk
         self.cap_rows = int(cap_factor * pairs) // 8 * 8
         dt = torch.bfloat16
@@ -196,7 +202,7 @@ class MoeEPLayer:
         cfg = self.cfg
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
-        block_n, down_cluster = expert_tiles(rows.shape[0], self.epr)
+        block_n, down_cluster = expert_tiles(rows.shape[0], self.epr, cfg.hidden, cfg.ffn, self.sms)
         ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
         ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=down_cluster)
         return y
@@ -224,7 +230,7 @@ class MoeEPLayer:
         if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
                 and cfg.topk <= 8 and cfg.experts <= 256 and (stacked := self._stacked(0)) is not None):
-            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *expert_tiles(pairs, self.epr))
+            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms))
             return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):

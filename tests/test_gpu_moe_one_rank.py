@@ -130,3 +130,17 @@ def test_fewer_tokens_than_built_for(world, monkeypatch):
             assert tokens == 3000 or {t for _, t in asked} == {256}
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("experts,tokens", [(8, 2), (8, 3), (4, 2), (4, 64), (4, 65), (2, 33)])
+def test_down_projection_in_clusters(experts, tokens):
+    """Around the borders of the rule for two CTAs per tile of the down projection (long K)."""
+    from penny_b200.models.moe_ep import MoeConfig, expert_tiles
+    cfg = MoeConfig(hidden=512, ffn=2048, experts=experts)
+    comm, layer = _layer(cfg, tokens)
+    try:
+        assert expert_tiles(2 * tokens, experts, 512, 2048, layer.sms)[1] == (0 if tokens == 65 else 2)
+        _check(layer, [torch.randn(tokens, cfg.hidden, device="cuda").bfloat16()])
+        assert comm.gemm_error() == 0
+    finally:
+        comm.close()
