@@ -74,7 +74,9 @@ void bind_gemm(py::module_& m) {
   // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
   // rows before its up rows, out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
   // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
-  // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).
+  // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).  pdl: may start,
+  // and without ranges load b, while the kernel before it on the stream still runs, so that kernel must not write
+  // b (a weight); everything else is waited for.
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
@@ -136,7 +138,7 @@ void bind_gemm(py::module_& m) {
     TORCH_CHECK(rc == cudaSuccess, "gemm_tile: ", cudaGetErrorString(rc));
   }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epi") = 0, py::arg("ranges") = py::none(),
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
-     py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = true,
+     py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
      py::arg("cluster") = 0);
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K);

@@ -36,7 +36,8 @@ struct TileGemm {
   int block_n;          // 0: choose; 128 / 192 / 256: single CTAs; 512: CTA pairs, 256 x 256
   int cluster;          // pairs (block_n 512) or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
                         // groups only for M <= the tile's rows
-  bool pdl;
+  bool pdl;             // may start, and without groups load b, while the kernel before it on the stream still runs:
+                        // that kernel must not write b
 };
 
 cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream);

@@ -177,7 +177,7 @@ class LlamaSPPrefill:
     def _gemm(self, x, w, out, epi=0, sumsq=None, residual=None, norm_w=None, sumsq_out=None):
         """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual)."""
         ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
-                      sumsq_out=sumsq_out)
+                      sumsq_out=sumsq_out, pdl=True)
 
     def _forward_local(self, x: torch.Tensor) -> torch.Tensor:
         """One rank.  h holds the residual stream times the next norm's weight, sumsq its sums of squares; the

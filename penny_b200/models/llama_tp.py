@@ -324,7 +324,7 @@ class LlamaTPDecoder:
             # the warm-up leaves behind the current positions is the same with either head.)
             own_head = self.B > 192 and self.V >= 1 << 16
             if own_head:
-                ops.gemm_tile(self.x, self.lm_head, self.logits)
+                ops.gemm_tile(self.x, self.lm_head, self.logits, pdl=self.pdl)
             if warm_up or not own_head:
                 torch.matmul(self.x, self.lm_head.t(), out=self.logits)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact

@@ -203,8 +203,8 @@ class MoeEPLayer:
         act = torch.empty(rows.shape[0], cfg.ffn, dtype=rows.dtype, device=rows.device)
         y = torch.empty_like(rows)
         block_n, down_cluster = expert_tiles(rows.shape[0], self.epr, cfg.hidden, cfg.ffn, self.sms)
-        ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n)
-        ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, cluster=down_cluster)
+        ops.gemm_tile(rows, w13, act, 1, ranges, block_n=block_n, pdl=True)
+        ops.gemm_tile(act, w2, y, 0, ranges, block_n=block_n, pdl=True, cluster=down_cluster)
         return y
 
     def _experts(self, v: int, rows: torch.Tensor, ranges):

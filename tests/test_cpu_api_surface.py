@@ -214,3 +214,10 @@ def test_attention_split_rule_reproduces_the_measured_choices():
         for kv in (16, 2048, 32768):
             s = f(items, kv)
             assert 1 <= s <= 16
+
+
+def test_gemm_tile_waits_for_both_operands_by_default():
+    """Loading b early is for weights: a caller has to say so (gemm_tile(..., pdl=True))."""
+    import torch  # noqa: F401  (the extension links against its libraries)
+    import penny_cpp
+    assert "pdl: bool = False" in penny_cpp.gemm_tile.__doc__

@@ -112,3 +112,20 @@ def test_prefill_one_rank_matches_fp32(tokens):
             assert ((got - want).norm() / want.norm()).item() < 1.5e-2
     finally:
         comm.close()
+
+
+def test_b_written_by_the_kernel_before():
+    """Unless told otherwise the GEMM waits for what wrote either operand, also a kernel that releases it early."""
+    from penny_b200._ext import ops
+    N, K = 2048, 4096
+    a = torch.randn(128, K, device="cuda").bfloat16()
+    ones = torch.ones(K, device="cuda", dtype=torch.bfloat16)
+    b, h, ss = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16), torch.empty(N, K, device="cuda").bfloat16(), \
+        torch.empty(N, device="cuda")
+    out = torch.empty(128, N, device="cuda", dtype=torch.bfloat16)
+    for i in range(8):
+        src = (torch.randn(N, K, device="cuda") * 0.05).bfloat16()
+        torch.cuda.synchronize()
+        ops.norm_prep(src, None, ones, b, h, ss)  # b = src
+        ops.gemm_tile(a, b, out)
+        _close(out, a.float() @ src.float().t())
