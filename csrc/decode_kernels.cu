@@ -555,7 +555,9 @@ cudaError_t launch_norm_prep(const void* src, const long long* index, const void
                              float* sumsq, int rows, int H, cudaStream_t stream) {
   if (rows < 1 || H < 8 || H % 8 != 0) return cudaErrorInvalidValue;
   const int threads = std::min(512, (H / 8 + 31) / 32 * 32);
-  return launch_kernel_ex(k_norm_prep, dim3((unsigned)rows), dim3((unsigned)threads), 0, stream, true, 1,
+  // The one launch of the stack that starts when everything before it has completed: the linear behind it loads
+  // weights before its own wait, and a weight may have been written by the kernel before the stack.
+  return launch_kernel_ex(k_norm_prep, dim3((unsigned)rows), dim3((unsigned)threads), 0, stream, false, 1,
                           (const __nv_bfloat16*)src, index, (const __nv_bfloat16*)norm_w, (__nv_bfloat16*)residual,
                           (__nv_bfloat16*)out, sumsq, H);
 }

@@ -129,3 +129,27 @@ def test_b_written_by_the_kernel_before():
         ops.norm_prep(src, None, ones, b, h, ss)  # b = src
         ops.gemm_tile(a, b, out)
         _close(out, a.float() @ src.float().t())
+
+
+@pytest.mark.parametrize("tokens", [128, 512])
+def test_prefill_after_a_weight_update(tokens):
+    """A forward right behind the kernels that rewrite its weights, on one stream, uses the new ones."""
+    from penny_b200.models.llama_sp import LlamaSPPrefill
+    from penny_b200.models.llama_tp import LlamaConfig
+    from penny_b200.parallel.comm import Communicator
+    cfg = LlamaConfig.tiny()
+    x = torch.randn(tokens, cfg.hidden, device="cuda").bfloat16()
+    comm = Communicator.emulated(1, heap_bytes=64 << 20)
+    try:
+        new = LlamaSPPrefill(cfg, comm=comm, tokens=tokens, layers=1, seed=2)
+        m = LlamaSPPrefill(cfg, comm=comm, tokens=tokens, layers=1, seed=1)
+        want = new.forward(x)
+        stale = torch.zeros_like(m.layers[0]["wqkv"])
+        for _ in range(20):
+            m.layers[0]["wqkv"].copy_(stale)
+            torch.cuda.synchronize()
+            for k in ("norm1", "norm2", "wo", "wgu", "wd", "wqkv"):  # the first linear's weight last
+                m.layers[0][k].copy_(new.layers[0][k])
+            assert torch.equal(m.forward(x), want)
+    finally:
+        comm.close()
