@@ -123,11 +123,19 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     else tmem_alloc(&s_tmem, Cfg::kTmemCols);
   }
   if (a.groups > 0) pdl_wait();  // the row ranges come from the kernel before this one
+  // Only rows that a and out have: a range that leaves them would be stored past out, and in a cluster bring a
+  // second tile that nobody waits for.
+  auto group_rows = [&](int g, int& r0, int& r1) {
+    r0 = min(max(a.ranges[a.range_stride * g], 0), a.M);
+    r1 = min(max(a.ranges[a.range_stride * g + 1], r0), a.M);
+  };
   if (a.groups > 0 && warp == 0) {
     int n = 0, tot = 0;
     for (int g0 = 0; g0 < a.groups; g0 += 32) {
       const int g = g0 + lane;
-      const int rows = g < a.groups ? max(0, a.ranges[a.range_stride * g + 1] - a.ranges[a.range_stride * g]) : 0;
+      int r0 = 0, r1 = 0;
+      if (g < a.groups) group_rows(g, r0, r1);
+      const int rows = r1 - r0;
       const unsigned m = __ballot_sync(0xffffffffu, rows > 0);
       if (rows > 0) s_group[n + __popc(m & ((1u << lane) - 1u))] = (short)g;
       n += __popc(m);
@@ -158,8 +166,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
   };
   auto open_group = [&](TileCursor& c) {
     if (a.groups > 0) {
-      c.rows0 = a.ranges[a.range_stride * s_group[c.g]];
-      c.rows1 = a.ranges[a.range_stride * s_group[c.g] + 1];
+      group_rows(s_group[c.g], c.rows0, c.rows1);
     } else {
       c.rows0 = 0;
       c.rows1 = a.M;

@@ -21,7 +21,7 @@ struct TileGemm {
   int lda, ldb, ldo;
   int epi;
   // groups > 0: rows ranges[s g] .. ranges[s g + 1] of a and out (device memory, s = range_stride) meet b rows
-  // g * b_rows ..
+  // g * b_rows ..  (what lies outside [0, M) is left out)
   int groups;
   const int* ranges;
   int range_stride;  // 2: (start, end) pairs; 1: group g ends where g + 1 starts

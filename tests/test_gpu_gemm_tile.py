@@ -153,3 +153,21 @@ def test_prefill_after_a_weight_update(tokens):
             assert torch.equal(m.forward(x), want)
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("cluster", [0, 2])
+def test_tile_groups_outside_the_rows(cluster):
+    """Ranges that leave the rows of a are cut to them: nothing is read or written outside."""
+    from penny_b200._ext import ops
+    K, N, M = 320, 256, 100
+    ranges = torch.tensor([[-40, 10], [10, 10], [10, 30], [60, 30], [90, 400], [120, 500]], dtype=torch.int32)
+    x, w = _data(M, 6 * N, K)
+    whole = torch.full((M + 400, N), -7.0, device="cuda", dtype=torch.bfloat16)
+    out = whole[200:200 + M]
+    ops.gemm_tile(x, w, out, 0, ranges=ranges.cuda(), block_n=256, cluster=cluster)
+    assert ops.gemm_error() == 0
+    want = torch.full((M, N), -7.0, device="cuda")
+    for g, (s, t) in enumerate([(0, 10), (10, 10), (10, 30), (0, 0), (90, M), (0, 0)]):
+        want[s:t] = x[s:t].float() @ w[g * N:(g + 1) * N].float().t()
+    _close(out, want)
+    assert (whole[:200] == -7).all() and (whole[200 + M:] == -7).all()
