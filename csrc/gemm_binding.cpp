@@ -121,10 +121,10 @@ void bind_gemm(py::module_& m) {
                   "gemm_tile: residual like out; norm_w and sumsq_out together");
       g.residual = residual->data_ptr();
       if (norm_w.has_value()) {
-        TORCH_CHECK(bf16(*norm_w) && norm_w->numel() == g.b_rows && sumsq_out->is_cuda() &&
+        TORCH_CHECK(bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == g.b_rows && sumsq_out->is_cuda() &&
                         sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
                         sumsq_out->numel() == (int64_t)(g.b_rows / 128) * g.M,
-                    "gemm_tile: norm_w [rows of b], sumsq_out [rows of b / 128, rows]");
+                    "gemm_tile: contiguous norm_w [rows of b], sumsq_out [rows of b / 128, rows]");
         g.norm_w = norm_w->data_ptr();
         g.sumsq_out = sumsq_out->data_ptr<float>();
       }

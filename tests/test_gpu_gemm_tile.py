@@ -171,3 +171,14 @@ def test_tile_groups_outside_the_rows(cluster):
         want[s:t] = x[s:t].float() @ w[g * N:(g + 1) * N].float().t()
     _close(out, want)
     assert (whole[:200] == -7).all() and (whole[200 + M:] == -7).all()
+
+
+def test_tile_norm_weight_must_be_contiguous():
+    from penny_b200._ext import ops
+    a, b = _data(128, 256, 64)
+    res, out, ss = torch.zeros(128, 256, device="cuda").bfloat16(), torch.zeros(128, 256, device="cuda").bfloat16(), \
+        torch.zeros(2, 128, device="cuda")
+    row = torch.ones(1, 128, device="cuda").bfloat16()
+    for nw in (row.expand(2, 128), torch.ones(2, 192, device="cuda").bfloat16()[:, :128]):  # 256 elements, but not in a row
+        with pytest.raises(RuntimeError, match="contiguous norm_w"):
+            ops.gemm_tile(a, b, out, 2, residual=res, norm_w=nw, sumsq_out=ss)
