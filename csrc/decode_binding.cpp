@@ -22,6 +22,18 @@ void ck(cudaError_t rc, const char* what) {
 bool bf16_cuda(const at::Tensor& t) {
   return t.is_cuda() && t.is_contiguous() && t.scalar_type() == at::kBFloat16;
 }
+// Matrices of one shape that lie back to back in one storage.  Looked at on every call: entries of a caller's list
+// may be other tensors by now, or the same ones over other memory (tensor.data = ...).
+bool stacked(const std::vector<at::Tensor>& mats) {
+  if (mats.empty() || !bf16_cuda(mats[0]) || mats[0].dim() != 2 || ((uintptr_t)mats[0].data_ptr() & 15) != 0) return false;
+  const at::Tensor& t0 = mats[0];
+  for (size_t i = 1; i < mats.size(); ++i)
+    if (!bf16_cuda(mats[i]) || mats[i].sizes() != t0.sizes() ||
+        mats[i].storage().unsafeGetStorageImpl() != t0.storage().unsafeGetStorageImpl() ||
+        mats[i].storage_offset() != t0.storage_offset() + (int64_t)i * t0.numel())
+      return false;
+  return true;
+}
 }  // namespace
 
 void bind_decode(py::module_& m) {
@@ -185,32 +197,25 @@ void bind_decode(py::module_& m) {
        "moe_placement");
     return std::make_tuple(dst_base, rows, ranges);
   });
-  // Matrices of one shape that lie back to back in one storage, as one matrix of all their rows; None if they
-  // don't.  Looked at on every call: entries of a caller's list may be other tensors by now, or the same ones
-  // over other memory (tensor.data = ...).
+  // stacked() as one matrix of all rows, or None.
   m.def("stacked_rows", [](const std::vector<at::Tensor>& mats) -> c10::optional<at::Tensor> {
-    if (mats.empty() || !bf16_cuda(mats[0]) || mats[0].dim() != 2 || ((uintptr_t)mats[0].data_ptr() & 15) != 0) return c10::nullopt;
-    const at::Tensor& t0 = mats[0];
-    for (size_t i = 1; i < mats.size(); ++i)
-      if (!bf16_cuda(mats[i]) || mats[i].sizes() != t0.sizes() ||
-          mats[i].storage().unsafeGetStorageImpl() != t0.storage().unsafeGetStorageImpl() ||
-          mats[i].storage_offset() != t0.storage_offset() + (int64_t)i * t0.numel())
-        return c10::nullopt;
-    return t0.detach().as_strided({(int64_t)mats.size() * t0.size(0), t0.size(1)}, {t0.size(1), 1});
+    if (!stacked(mats)) return c10::nullopt;
+    const int64_t K = mats[0].size(1);
+    return mats[0].detach().as_strided({(int64_t)mats.size() * mats[0].size(0), K}, {K, 1});
   });
   // A MoE layer of one rank: router, rows by expert, expert SwiGLU FFNs, gate-weighted sum.  Nothing comes
   // back to the host, and it is one call: as Python calls the launches took 113 us of host time, of which a
-  // layer of a few tokens hid half.  w13 [experts * 2 ffn, hidden] (gate rows, then up rows),
-  // w2 [experts * hidden, ffn]; block_n and down_cluster as in gemm_tile.  The router meets the library's GEMM only
-  // and may have any strides.
-  m.def("moe_layer", [](at::Tensor x, at::Tensor router, at::Tensor w13, at::Tensor w2, int64_t topk, int64_t block_n,
-                        int64_t down_cluster) {
-    for (const at::Tensor* t : {&x, &w13, &w2})
-      need(bf16_cuda(*t) && t->dim() == 2 && ((uintptr_t)t->data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 tensors");
+  // layer of a few tokens hid half.  w13: per expert [2 ffn, hidden] (gate rows, then up rows), w2: [hidden, ffn], each
+  // list one stack, else None is returned and nothing runs; block_n and down_cluster as in gemm_tile.  The router meets
+  // the library's GEMM only and may have any strides.
+  m.def("moe_layer", [](at::Tensor x, at::Tensor router, const std::vector<at::Tensor>& w13, const std::vector<at::Tensor>& w2,
+                        int64_t topk, int64_t block_n, int64_t down_cluster) -> c10::optional<at::Tensor> {
+    if (!stacked(w13) || !stacked(w2)) return c10::nullopt;
+    need(bf16_cuda(x) && x.dim() == 2 && ((uintptr_t)x.data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 x");
     need(router.is_cuda() && router.scalar_type() == at::kBFloat16 && router.dim() == 2, "moe_layer: 2-D bf16 router");
-    const int T = (int)x.size(0), H = (int)x.size(1), E = (int)router.size(0), F = (int)w2.size(1), P = T * (int)topk;
-    need(router.size(1) == H && w13.size(0) == (int64_t)E * 2 * F && w13.size(1) == H && w2.size(0) == (int64_t)E * H && T > 0,
-         "moe_layer shapes");
+    const int T = (int)x.size(0), H = (int)x.size(1), E = (int)router.size(0), F = (int)w2[0].size(1), P = T * (int)topk;
+    need(router.size(1) == H && (int)w13.size() == E && (int)w2.size() == E && w13[0].size(0) == 2 * (int64_t)F &&
+             w13[0].size(1) == H && w2[0].size(0) == H && T > 0, "moe_layer shapes");
     const at::cuda::OptionalCUDAGuard guard(x.device());
     const cudaStream_t stream = cur();
     const at::Tensor logits = at::matmul(x, router.t()).contiguous();
@@ -225,7 +230,7 @@ void bind_decode(py::module_& m) {
     ck(launch_moe_gather(x.data_ptr(), order, P, (int)topk, H, rows.data_ptr(), row_of_pair, stream), "moe_layer: rows");
     sm100::TileGemm g = {};
     g.a = rows.data_ptr();
-    g.b = w13.data_ptr();
+    g.b = w13[0].data_ptr();
     g.out = act.data_ptr();
     g.M = P;
     g.b_rows = 2 * F;
@@ -239,7 +244,7 @@ void bind_decode(py::module_& m) {
     g.pdl = true;
     ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "moe_layer: gate / up");
     g.a = act.data_ptr();
-    g.b = w2.data_ptr();
+    g.b = w2[0].data_ptr();
     g.out = rows.data_ptr();  // (their inputs are used up)
     g.b_rows = H;
     g.K = g.lda = g.ldb = F;

@@ -224,14 +224,17 @@ class MoeEPLayer:
         when emulated)."""
         cfg, comm = self.cfg, self.comm
         xs = self._as_views(x)
-        if max(xv.shape[0] for xv in xs) > self.tokens:  # the exchange's buffers and tables are that long
-            raise RuntimeError(f"MoE layer built for {self.tokens} tokens, called with {max(xv.shape[0] for xv in xs)}")
+        for xv in xs:
+            if xv.shape[0] > self.tokens:  # the exchange's buffers and tables are that long
+                raise RuntimeError(f"MoE layer built for {self.tokens} tokens, called with {xv.shape[0]}")
         x0, pairs = xs[0], xs[0].shape[0] * cfg.topk
         if (self.world == 1 and self.backend == "penny" and self.use_own_gemm and 0 < pairs <= self.cap_rows
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
-                and cfg.topk <= 8 and cfg.experts <= 256 and (stacked := self._stacked(0)) is not None):
-            out = ops.moe_layer(x0, self.router[0], *stacked, cfg.topk, *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms))
-            return [out] if comm.emulated else out
+                and cfg.topk <= 8 and cfg.experts <= 256):
+            out = ops.moe_layer(x0, self.router[0], self.w13[0][:self.epr], self.w2[0][:self.epr], cfg.topk,
+                                *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms))
+            if out is not None:
+                return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
         for v, xv in enumerate(xs):
             i, g = route(torch.matmul(xv, self.router[v].t()), cfg.topk)
