@@ -103,8 +103,9 @@ class LlamaSPPrefill:
         self.local = backend == "penny" and world == 1 and not self.cpu and (2 * self.F) % 128 == 0
         if self.local:
             self.sumsq = [torch.empty(n, tokens, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
-        # kernels of this library per forward: per layer 2 norms, RoPE, silu*mul and (penny) 4 fused GEMMs
-        self.kernels_per_forward = self.L * (4 + (4 if backend == "penny" else 0))
+        # kernels of this library per forward: per layer 2 norms, RoPE, silu*mul and (penny) 4 fused GEMMs; on one
+        # rank RoPE and 4 GEMMs with the rest in their epilogues, behind one norm
+        self.kernels_per_forward = 1 + 5 * self.L if self.local else self.L * (4 + (4 if backend == "penny" else 0))
 
     # ------------------------------------------------------------------ linears
     def _col(self, h_shard: torch.Tensor, w: torch.Tensor, out: torch.Tensor):

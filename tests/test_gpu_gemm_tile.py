@@ -182,3 +182,33 @@ def test_tile_norm_weight_must_be_contiguous():
     for nw in (row.expand(2, 128), torch.ones(2, 192, device="cuda").bfloat16()[:, :128]):  # 256 elements, but not in a row
         with pytest.raises(RuntimeError, match="contiguous norm_w"):
             ops.gemm_tile(a, b, out, 2, residual=res, norm_w=nw, sumsq_out=ss)
+
+
+@pytest.mark.parametrize("backend,local", [("penny", True), ("penny", False), ("nccl", False)])
+def test_kernels_per_forward(backend, local, monkeypatch):
+    from penny_b200.models import llama_sp
+    from penny_b200.models.llama_tp import LlamaConfig
+    from penny_b200.parallel.comm import Communicator
+    cfg, calls = LlamaConfig.tiny(), []
+
+    class Counted:
+        def __init__(self, inner):
+            self.inner = inner
+
+        def __getattr__(self, name):
+            f = getattr(self.inner, name)
+            return (lambda *a, **k: calls.append(name) or f(*a, **k)) if callable(f) else f
+    comm = Communicator.emulated(1, heap_bytes=64 << 20)
+    try:
+        m = llama_sp.LlamaSPPrefill(cfg, comm=comm, tokens=128, layers=3, backend=backend)
+        assert m.local == (backend == "penny")
+        if m.local and not local:  # the fused GEMM + collective kernels, as several ranks run them
+            x = torch.empty(128 * cfg.hidden + 1, device="cuda", dtype=torch.bfloat16)[1:].view(128, cfg.hidden).normal_()
+        else:
+            x = torch.randn(128, cfg.hidden, device="cuda").bfloat16()
+        monkeypatch.setattr(llama_sp, "ops", Counted(llama_sp.ops))
+        m.comm = Counted(comm)
+        m.forward(x)
+        assert len(calls) == (m.kernels_per_forward if m.local == local else 3 * 8), calls
+    finally:
+        comm.close()
