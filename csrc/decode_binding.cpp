@@ -56,21 +56,17 @@ void bind_decode(py::module_& m) {
     ck(launch_rope_rows(qkv.data_ptr(), (int)qkv.size(0), (int)Hq, (int)Hkv, (int)D, (int)pos0, (float)theta, cur()),
        "rope_rows");
   });
-  m.def("norm_prep", [](at::Tensor src, c10::optional<at::Tensor> index, at::Tensor norm_w, at::Tensor residual,
-                        at::Tensor out, at::Tensor sumsq) {
-    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2 && residual.dim() == 2,
+  m.def("norm_prep", [](at::Tensor src, at::Tensor norm_w, at::Tensor residual, at::Tensor out, at::Tensor sumsq) {
+    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2,
          "norm_prep expects contiguous bf16 CUDA tensors");
-    const int64_t rows = residual.size(0), H = src.size(1);
-    need(residual.size(1) == H && out.sizes() == residual.sizes() && norm_w.numel() == H && sumsq.is_cuda() &&
+    const int64_t rows = src.size(0), H = src.size(1);
+    need(residual.sizes() == src.sizes() && out.sizes() == src.sizes() && norm_w.numel() == H && sumsq.is_cuda() &&
              sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous() && sumsq.numel() == rows, "norm_prep shapes");
-    need(index.has_value() ? index->is_cuda() && index->scalar_type() == at::kLong && index->is_contiguous() &&
-                                 index->numel() == rows : src.size(0) == rows, "norm_prep: one source row per output row");
     for (const at::Tensor* t : {&src, &norm_w, &residual, &out})
       need(((uintptr_t)t->data_ptr() & 15) == 0, "norm_prep: 16-byte aligned tensors");
     const at::cuda::OptionalCUDAGuard guard(src.device());
-    ck(launch_norm_prep(src.data_ptr(), index.has_value() ? (const long long*)index->data_ptr<int64_t>() : nullptr,
-                        norm_w.data_ptr(), residual.data_ptr(), out.data_ptr(), sumsq.data_ptr<float>(), (int)rows, (int)H,
-                        cur()),
+    ck(launch_norm_prep(src.data_ptr(), norm_w.data_ptr(), residual.data_ptr(), out.data_ptr(), sumsq.data_ptr<float>(),
+                        (int)rows, (int)H, cur()),
        "norm_prep");
   });
   m.def("decode_attn_workspace_bytes", [](int64_t B, int64_t Hq, int64_t splits) {

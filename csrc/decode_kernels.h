@@ -16,11 +16,11 @@ cudaError_t launch_rope_append(void* qkv, void* kcache, void* vcache, const int*
 cudaError_t launch_rope_rows(void* qkv, int T, int Hq, int Hkv, int D, int pos0, float theta,
                              cudaStream_t stream);
 
-// residual[r] = src[index ? index[r] : r], out[r] = residual[r] * norm_w, sumsq[r] = sum residual[r]^2: what the
+// residual[r] = src[r], out[r] = residual[r] * norm_w, sumsq[r] = sum residual[r]^2: what the
 // first linear of a stack with norms in the GEMM epilogues starts from.  Rows of H bf16, H % 8 == 0, all
 // pointers 16-byte aligned.
-cudaError_t launch_norm_prep(const void* src, const long long* index, const void* norm_w, void* residual, void* out,
-                             float* sumsq, int rows, int H, cudaStream_t stream);
+cudaError_t launch_norm_prep(const void* src, const void* norm_w, void* residual, void* out, float* sumsq, int rows, int H,
+                             cudaStream_t stream);
 
 // Scratch the split-KV attention needs: per (row, head, split) an unnormalised
 // fp32 output row plus (max, sum).

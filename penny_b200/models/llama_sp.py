@@ -184,7 +184,7 @@ class LlamaSPPrefill:
         """One rank.  h holds the residual stream times the next norm's weight, sumsq its sums of squares; the
         linear that reads h scales its output rows by 1 / rms, so a norm costs no pass of its own."""
         res, h, ss = torch.empty_like(x), self.h, self.sumsq[0]
-        ops.norm_prep(x, None, self.layers[0]["norm1"], res, h, ss)
+        ops.norm_prep(x, self.layers[0]["norm1"], res, h, ss)
         for li, l in enumerate(self.layers):
             self._gemm(h, l["wqkv"], self.qkv, sumsq=ss)
             attn = self._attention()

@@ -126,7 +126,7 @@ def test_b_written_by_the_kernel_before():
     for i in range(8):
         src = (torch.randn(N, K, device="cuda") * 0.05).bfloat16()
         torch.cuda.synchronize()
-        ops.norm_prep(src, None, ones, b, h, ss)  # b = src
+        ops.norm_prep(src, ones, b, h, ss)  # b = src
         ops.gemm_tile(a, b, out)
         _close(out, a.float() @ src.float().t())
 
