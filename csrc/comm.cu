@@ -630,7 +630,13 @@ LaunchCfg Communicator::moe_cfg(const Tuning& t, cudaStream_t stream) const {
   cfg.emu_world = emu_ && world_ > 1 ? world_ : 0;
   cfg.pdl = world_ == 1;
   // every block polls blocks * world flags of its peers; a world of one has none and takes what the GPU holds
-  const int cap = world_ == 1 ? 3 * 148 : (emu_ ? std::max(1, 128 / world_) : 64);
+  int cap = emu_ ? std::max(1, 128 / world_) : 64;
+  if (world_ == 1) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cap = std::min(kMaxBlocks, std::max(1, 3 * sms));
+  }
   cfg.blocks = std::min(cap, t.blocks > 0 ? t.blocks : cap);
   return cfg;
 }

@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat1
 constexpr int kRowVecs = 4 * 32;
 
 __global__ void __launch_bounds__(256) k_moe_gather(const uint4* __restrict__ x, const int* __restrict__ order, int pairs,
-                                                    int topk, int hv, uint4* __restrict__ rows, int* __restrict__ row_of_pair) {
-  // (a GEMM that sets up early leaves registers for one block per SM: only where one is enough)
-  if (gridDim.x <= 148) pdl_launch_dependents();
+                                                    int topk, int hv, uint4* __restrict__ rows, int* __restrict__ row_of_pair,
+                                                    bool early) {
+  if (early) pdl_launch_dependents();
   pdl_wait();
   const int pieces = (hv + kRowVecs - 1) / kRowVecs, u = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if (u >= pairs * pieces) return;
@@ -253,8 +253,13 @@ cudaError_t launch_moe_gather(const void* x, const int* order, int pairs, int to
                               cudaStream_t stream) {
   if (pairs <= 0 || topk <= 0 || hidden <= 0 || hidden % 8 != 0) return cudaErrorInvalidValue;
   const int hv = hidden / 8, pieces = (hv + kRowVecs - 1) / kRowVecs;
-  return launch_kernel_ex(k_moe_gather, dim3((unsigned)(((long long)pairs * pieces + 7) / 8)), dim3(256), 0, stream, true, 1,
-                          (const uint4*)x, order, pairs, topk, hv, (uint4*)rows, row_of_pair);
+  const long long blocks = ((long long)pairs * pieces + 7) / 8;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // A GEMM that sets up early leaves registers for one block per SM, so it is released early only where one is enough.
+  return launch_kernel_ex(k_moe_gather, dim3((unsigned)blocks), dim3(256), 0, stream, true, 1, (const uint4*)x, order, pairs,
+                          topk, hv, (uint4*)rows, row_of_pair, blocks <= sms);
 }
 
 cudaError_t launch_moe_sum(const void* y, const int* row_of_pair, const float* gates, int tokens, int topk, int hidden, void* out,
