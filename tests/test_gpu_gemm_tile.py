@@ -96,7 +96,7 @@ def test_tile_groups(counts, block_n, cluster):
     _close(out, want)
 
 
-@pytest.mark.parametrize("tokens", [128, 384])  # clusters that split K, and whole tiles
+@pytest.mark.parametrize("tokens", [128, 384])  # one row tile, and several
 def test_prefill_one_rank_matches_fp32(tokens):
     from penny_b200.models.llama_sp import LlamaSPPrefill
     from penny_b200.models.llama_tp import LlamaConfig
@@ -212,3 +212,59 @@ def test_kernels_per_forward(backend, local, monkeypatch):
         assert len(calls) == (m.kernels_per_forward if m.local == local else 3 * 8), calls
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("block_n", [128, 256, 512, 0])
+def test_tile_residual_over_several_rounds(block_n):
+    """More than two tiles for every CTA or pair, ragged rows: accumulators, sums of squares and the residual that is
+    loaded ahead are used again and again, with the norm and without."""
+    from penny_b200._ext import ops
+    M, N, K = 4200, 2560, 256
+    a, b = _data(M, N, K)
+    res = torch.randn(M, N, device="cuda").bfloat16()
+    plain = res.clone()
+    nw = (1 + 0.1 * torch.randn(N, device="cuda")).bfloat16()
+    z = res.float() + a.float() @ b.float().t()
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ss = torch.full((N // 128, M), float("nan"), device="cuda")
+    ops.gemm_tile(a, b, out, 2, residual=res, norm_w=nw, sumsq_out=ss, block_n=block_n)
+    ops.gemm_tile(a, b, plain, 2, residual=plain, block_n=block_n)
+    assert ops.gemm_error() == 0
+    _close(res, z)
+    _close(out, z * nw.float())
+    _close(plain, z)
+    # the sums are over the product rounded to bf16 plus the residual: 2 * 2^-9 of each of 128 squares at most
+    torch.testing.assert_close(ss, z.pow(2).view(M, N // 128, 128).sum(-1).t(), atol=0, rtol=2 ** -8)
+
+
+def _prefill(cfg, tokens, layers, local, limit):
+    from penny_b200.models.llama_sp import LlamaSPPrefill
+    from penny_b200.parallel.comm import Communicator
+    x = torch.randn(tokens, cfg.hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).bfloat16()
+    want = LlamaSPPrefill.reference_forward(cfg, x, layers, seed=1)
+    comm = Communicator.emulated(1, heap_bytes=256 << 20, timeout_ms=2000)
+    try:
+        m = LlamaSPPrefill(cfg, comm=comm, tokens=tokens, layers=layers, seed=1)
+        assert m.local
+        m.local = local
+        for _ in range(2):
+            got = m.forward(x).float()
+            comm.check()
+            assert comm.gemm_error() == 0
+            assert ((got - want).norm() / want.norm()).item() < limit
+    finally:
+        comm.close()
+
+
+@pytest.mark.parametrize("tokens", [128, 384, 2432])
+def test_prefill_one_rank_long_k(tokens):
+    """K of 2048 and 4096: at 128 and 384 tokens clusters split it (more than the 26 steps of 64 from which that
+    pays); 2432 tokens are several rounds of tiles per SM in gate/up."""
+    from penny_b200.models.llama_tp import LlamaConfig
+    _prefill(LlamaConfig(hidden=2048, layers=2, heads=16, kv_heads=4, head_dim=128, ffn=4096, vocab=2048), tokens, 2, True, 1.5e-2)
+
+
+def test_prefill_fused_kernels_on_one_rank():
+    """The GEMM + collective kernels that several ranks run (heap slots, flags, gathered-buffer TMA), on one."""
+    from penny_b200.models.llama_tp import LlamaConfig
+    _prefill(LlamaConfig.tiny(), 512, 2, False, 3e-2)

@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# clusters for a handful of rows; routing in one block (up to 1024 tokens) or two launches; pair tiles
+# routing in one block (up to 1024 tokens) or two launches; pair tiles
 @pytest.mark.parametrize("tokens", [4, 5, 1024, 1032, 2700])
 @pytest.mark.parametrize("topk", [1, 2])
 def test_one_rank(tokens, topk):
