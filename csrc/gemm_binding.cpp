@@ -157,6 +157,8 @@ void bind_gemm(py::module_& m) {
   m.def("pdl_enabled", []() { return penny::pdl_enabled(); });
   m.def("gemm_set_split_tail", [](int64_t on) { penny::sm100::set_split_tail((int)on); }, py::arg("on"),
         "1 / 0: split (or not) the ragged last wave of the CTA-pair GEMM along K; -1: PENNY_GEMM_SPLIT_TAIL decides");
+  m.def("gemm_pair_enabled", []() { return penny::sm100::pair_kernel_enabled(); },
+        "False when PENNY_GEMM_PAIR=0 keeps the GEMMs on single-CTA tiles");
   // Synchronises; returns and clears the error code of the GEMM kernels (0 = fine).
   m.def("gemm_error", []() {
     uint32_t* word = penny_gemm_error_word();

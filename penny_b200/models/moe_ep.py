@@ -125,6 +125,7 @@ def expert_tiles(rows: int, experts: int, hidden: int, ffn: int, sms: int):
     128-row tiles of single CTAs, 256 columns wide: most experts' rows fill one or two.  256-row tiles of CTA
     pairs once the average expert fills three (8 experts, gate/up + down: 1000 tokens 804 us against 857,
     2000 tokens 1278 / 1379, 3000 tokens 1723 / 1678; at 5 to 500 tokens pairs cost 70 to 90 us of 334 to 510).
+    PENNY_GEMM_PAIR=0 leaves them out.
 
     Where at most half of the SMs have a tile of the down projection, two CTAs share a tile's K steps (hidden 4096, ffn
     14336, down alone: 4 experts 156 us -> 97; with 6 of them 125 -> 146, there are enough tiles then; whole layer
@@ -132,7 +133,7 @@ def expert_tiles(rows: int, experts: int, hidden: int, ffn: int, sms: int):
     must save (whole layer, 2 tokens, ffn 1024 / 1664 / 2048 / 4096: 68.3 / 76.0 / 79.3 / 120.1 us without, 69.4 /
     75.8 / 77.7 / 108.4 with), and a cluster works on one row tile."""
     shared = rows <= 128 and 2 * min(rows, experts) * -(-hidden // 256) <= sms and ffn > 2 * 13 * 64
-    return (512 if rows > 640 * experts else 256), (2 if shared else 0)
+    return (512 if rows > 640 * experts and ops.gemm_pair_enabled() else 256), (2 if shared else 0)
 
 
 class MoeEPLayer:

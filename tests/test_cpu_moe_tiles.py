@@ -1,4 +1,8 @@
 """Tiles of the MoE layer's grouped GEMMs: the rule against the sizes it was measured at."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 from penny_b200.models.moe_ep import expert_tiles
@@ -12,3 +16,9 @@ from penny_b200.models.moe_ep import expert_tiles
 ])
 def test_expert_tiles(rows, experts, hidden, ffn, want):
     assert expert_tiles(rows, experts, hidden, ffn, 148) == want
+
+
+def test_no_pairs_where_they_are_switched_off():
+    code = "from penny_b200.models.moe_ep import expert_tiles; assert expert_tiles(9000, 8, 4096, 14336, 148) == (256, 0)"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, PENNY_GEMM_PAIR="0"), check=True, timeout=300)
