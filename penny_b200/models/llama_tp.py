@@ -83,10 +83,18 @@ class LlamaTPDecoder:
         if linears == "auto":
             # measured (one layer's four linears replayed from a graph, batch 256): this library's decode
             # GEMM is a weight-streaming kernel with a 128-row batch tile, 56.9 vs 34.3 us at TP 8 and 231 vs
-            # 119 us at TP 1 against the library GEMM once the problem is compute-bound; up to 128 rows it
-            # is level (95 vs 92 us at TP 1, batch 64) and lets the epilogues fuse
+            # 119 us at TP 1 against the library GEMM once the problem is compute-bound (the tiled GEMM was
+            # measured there on the LM head only, see own_head); up to 128 rows it is level (95 vs 92 us
+            # at TP 1, batch 64) and lets the epilogues fuse
             linears = "penny" if max_batch <= 128 else "cublas"
         self.linears, self.pdl = linears, pdl
+        # LM head beside the library's linears: on this library's tiles while one row tile of a CTA pair holds the batch.
+        # Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 / 217 / 222 us against the library's
+        # 224 / 293 / 238 / 328; vocabularies of 65536 to 151936 and hidden 2048 to 8192: 0.95 to 1.5 times as fast,
+        # 1.2 on average.  Level at 192.  A second row tile that is partly filled costs a whole one: 257 / 384 / 512
+        # / 1024 rows 359 / 374 / 524 / 858 against 263 / 307 / 499 / 836.  Smaller vocabulary shards (32000: 0.84 to
+        # 1.2 times as fast, by hidden and rows) stay with the library.
+        self.own_head = linears == "cublas" and 192 < max_batch <= 256 and cfg.vocab // world >= 1 << 16
         if world > 1 and backend != "nccl":
             assert comm is not None, "a Communicator is required for the penny backends"
         self.cfg, self.comm, self.rank, self.world = cfg, comm, rank, world
@@ -166,7 +174,7 @@ class LlamaTPDecoder:
         if backend == "penny_unfused" and world > 1:
             norms += 2 * cfg.layers  # separate all-reduce kernels
         # + arg-max (+ the all-gather of the ranks' candidates and the choice among them) + LM head
-        own_head = chunks if self.linears == "penny" else int(B > 192 and self.V >= 1 << 16)
+        own_head = chunks if self.linears == "penny" else int(self.own_head)
         self.kernels_per_step = cfg.layers * per_layer + norms + 1 + (2 if world > 1 else 0) + own_head
 
     # ------------------------------------------------------------------ weights
@@ -319,13 +327,11 @@ class LlamaTPDecoder:
         if self.linears == "penny":
             self._linear(self.x, self.lm_head, self.logits)
         else:
-            # (256 rows: 201 us on this library's tiles, 264 on the library's; level at 192.  A warm-up step runs
-            # both, so that neither's first launch is a captured one; the library's logits come last, and what
-            # the warm-up leaves behind the current positions is the same with either head.)
-            own_head = self.B > 192 and self.V >= 1 << 16
-            if own_head:
+            # (a warm-up step runs both heads, so that neither's first launch is a captured one; the library's logits
+            # come last, and what the warm-up leaves behind the current positions is the same with either)
+            if self.own_head:
                 ops.gemm_tile(self.x, self.lm_head, self.logits, pdl=self.pdl)
-            if warm_up or not own_head:
+            if warm_up or not self.own_head:
                 torch.matmul(self.x, self.lm_head.t(), out=self.logits)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
         # in fp32), gathered over the ranks; one kernel then picks the best rank per sequence, feeds the

@@ -60,3 +60,24 @@ def test_gemm_error_outlives_a_captured_first_gemm():
     """
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", code], cwd=root, check=True, timeout=300)
+
+
+@pytest.mark.parametrize("batch,own", [(192, 0), (193, 1), (256, 1), (257, 0), (512, 0)])
+def test_which_head_and_how_many_kernels(batch, own, monkeypatch):
+    from penny_b200.models import llama_tp
+    cfg = dataclasses.replace(llama_tp.LlamaConfig.tiny(), vocab=1 << 16)
+    m = llama_tp.LlamaTPDecoder(cfg, world=1, max_batch=batch, max_len=24, use_graph=False, full_init=True)
+    m.fill_synthetic_kv(8)
+    tokens, positions = m.tokens.clone(), m.positions.clone()
+    calls, inner = [], llama_tp.ops
+
+    class Counted:
+        def __getattr__(self, name):
+            return lambda *a, **k: calls.append(name) or getattr(inner, name)(*a, **k)
+    monkeypatch.setattr(llama_tp, "ops", Counted())
+    m.step_device()
+    monkeypatch.undo()
+    assert calls.count("gemm_tile") == own and len(calls) == m.kernels_per_step
+    want = m.reference_logits(tokens, positions, m.kcache, m.vcache)
+    err = (m.logits.float() - want).abs().max().item()
+    assert err < 0.05 * want.std().item() + 0.02, err
