@@ -31,8 +31,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 // First 1024-byte boundary at or after `p` (the 128-byte swizzle's period).  An offset and not a rounded
 // pointer: rounding goes through an integer, after which the compiler no longer knows that the result
-// is shared memory and every access to it becomes a generic one (the sum of a cluster's parts in the
-// streamed GEMM's epilogue took 3.5 us that way and 0.7 us with shared loads).
+// is shared memory and every access to it becomes a generic one (summing a cluster's parts in an epilogue
+// took 3.5 us that way and 0.7 us with shared loads).
 __device__ __forceinline__ unsigned char* align_tiles(unsigned char* p) {
   return p + ((1024u - (smem_u32(p) & 1023u)) & 1023u);
 }
