@@ -56,19 +56,25 @@ void bind_decode(py::module_& m) {
     ck(launch_rope_rows(qkv.data_ptr(), (int)qkv.size(0), (int)Hq, (int)Hkv, (int)D, (int)pos0, (float)theta, cur()),
        "rope_rows");
   });
-  m.def("norm_prep", [](at::Tensor src, at::Tensor norm_w, at::Tensor residual, at::Tensor out, at::Tensor sumsq) {
-    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2,
+  // ids [rows] int64: the rows of src (an embedding table) that become the stream
+  m.def("norm_prep", [](at::Tensor src, at::Tensor norm_w, at::Tensor residual, at::Tensor out, at::Tensor sumsq,
+                        c10::optional<at::Tensor> ids) {
+    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2 && residual.dim() == 2,
          "norm_prep expects contiguous bf16 CUDA tensors");
-    const int64_t rows = src.size(0), H = src.size(1);
-    need(residual.sizes() == src.sizes() && out.sizes() == src.sizes() && norm_w.numel() == H && sumsq.is_cuda() &&
-             sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous() && sumsq.numel() == rows, "norm_prep shapes");
+    const int64_t rows = ids.has_value() ? ids->numel() : src.size(0), H = src.size(1);
+    if (ids.has_value())
+      need(ids->is_cuda() && ids->scalar_type() == at::kLong && ids->is_contiguous(), "norm_prep: ids must be int64 CUDA");
+    need(residual.size(0) == rows && residual.size(1) == H && out.sizes() == residual.sizes() && norm_w.numel() == H &&
+             sumsq.is_cuda() && sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous() && sumsq.numel() == rows,
+         "norm_prep shapes");
     for (const at::Tensor* t : {&src, &norm_w, &residual, &out})
       need(((uintptr_t)t->data_ptr() & 15) == 0, "norm_prep: 16-byte aligned tensors");
     const at::cuda::OptionalCUDAGuard guard(src.device());
-    ck(launch_norm_prep(src.data_ptr(), norm_w.data_ptr(), residual.data_ptr(), out.data_ptr(), sumsq.data_ptr<float>(),
-                        (int)rows, (int)H, cur()),
+    ck(launch_norm_prep(src.data_ptr(), ids.has_value() ? (const long long*)ids->data_ptr<int64_t>() : nullptr, src.size(0),
+                        norm_w.data_ptr(), residual.data_ptr(), out.data_ptr(), sumsq.data_ptr<float>(), (int)rows, (int)H,
+                        cur()),
        "norm_prep");
-  });
+  }, py::arg("src"), py::arg("norm_w"), py::arg("residual"), py::arg("out"), py::arg("sumsq"), py::arg("ids") = py::none());
   m.def("decode_attn_workspace_bytes", [](int64_t B, int64_t Hq, int64_t splits) {
     return (int64_t)decode_attn_workspace_bytes((int)B, (int)Hq, (int)splits);
   });

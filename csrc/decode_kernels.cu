@@ -15,6 +15,9 @@
 
 #include "decode_attn_common.cuh"
 #include "decode_kernels.h"
+
+#undef NDEBUG  // an embedding row that does not exist stops the kernel in every build
+#include <cassert>
 #include "pdl.h"
 
 #include <stdio.h>
@@ -126,8 +129,10 @@ __global__ void __launch_bounds__(320) k_rope_rows_vec(__nv_bfloat16* __restrict
 
 // Start of a stack whose norms ride in the GEMM epilogues: row r of src becomes residual row r, its product with
 // the first norm's weight the first linear's input, and its sum of squares what that linear scales its rows by.
-// One block per row.
-__global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restrict__ src,
+// One block per row.  ids: row r is row ids[r] of src (a token's embedding; an id that src does not have stops the
+// kernel, as in torch.index_select).
+__global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restrict__ src, const long long* __restrict__ ids,
+                                                   long long src_rows,
                                                    const __nv_bfloat16* __restrict__ norm_w,
                                                    __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out,
                                                    float* __restrict__ sumsq, int H) {
@@ -135,7 +140,9 @@ __global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restri
   pdl_launch_dependents();
   pdl_wait();
   const size_t r = blockIdx.x;
-  const uint4* in = reinterpret_cast<const uint4*>(src + r * H);
+  const long long from = ids != nullptr ? ids[r] : (long long)r;
+  assert(from >= 0 && from < src_rows);
+  const uint4* in = reinterpret_cast<const uint4*>(src + (size_t)from * H);
   const uint4* w = reinterpret_cast<const uint4*>(norm_w);
   float ss = 0.f;
   for (int v = threadIdx.x; v < H / 8; v += blockDim.x) {
@@ -551,14 +558,14 @@ cudaError_t launch_rope_rows(void* qkv, int T, int Hq, int Hkv, int D, int pos0,
   return cudaGetLastError();
 }
 
-cudaError_t launch_norm_prep(const void* src, const void* norm_w, void* residual, void* out, float* sumsq, int rows, int H,
-                             cudaStream_t stream) {
+cudaError_t launch_norm_prep(const void* src, const long long* ids, long long src_rows, const void* norm_w, void* residual,
+                             void* out, float* sumsq, int rows, int H, cudaStream_t stream) {
   if (rows < 1 || H < 8 || H % 8 != 0) return cudaErrorInvalidValue;
   const int threads = std::min(512, (H / 8 + 31) / 32 * 32);
   // The one launch of the stack that starts when everything before it has completed: the linear behind it loads
   // weights before its own wait, and a weight may have been written by the kernel before the stack.
   return launch_kernel_ex(k_norm_prep, dim3((unsigned)rows), dim3((unsigned)threads), 0, stream, false, 1,
-                          (const __nv_bfloat16*)src, (const __nv_bfloat16*)norm_w, (__nv_bfloat16*)residual,
+                          (const __nv_bfloat16*)src, ids, src_rows, (const __nv_bfloat16*)norm_w, (__nv_bfloat16*)residual,
                           (__nv_bfloat16*)out, sumsq, H);
 }
 

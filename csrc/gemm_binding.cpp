@@ -39,9 +39,11 @@ void bind_gemm(py::module_& m) {
   // range); the K ranges of a tile are reduced inside a thread-block cluster through distributed shared
   // memory.  pdl: may start (and load w) while the previous kernel on the stream still runs, so w must not
   // be written by that kernel.  silu_pairs: w's rows are blocks of 64 gate + 64 up rows and out is
-  // [B, N / 2] = silu(gate) * up.
+  // [B, N / 2] = silu(gate) * up.  sumsq, residual, norm_w, sumsq_out: as in gemm_tile below.
   m.def("gemm_decode", [](at::Tensor x, at::Tensor w, at::Tensor out, bool silu_pairs, int64_t splits, bool pdl,
-                          int64_t l2_budget, int64_t smem_kb, c10::optional<at::Tensor> push) {
+                          int64_t l2_budget, int64_t smem_kb, c10::optional<at::Tensor> push,
+                          c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
+                          c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out) {
     TORCH_CHECK(x.is_cuda() && w.is_cuda() && out.is_cuda(), "gemm_decode: CUDA tensors");
     TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
                     out.scalar_type() == at::kBFloat16, "gemm_decode: bf16 only");
@@ -63,14 +65,37 @@ void bind_gemm(py::module_& m) {
       memcpy(&pd, push->data_ptr(), sizeof(pd));
       pp = &pd;
     }
+    penny::sm100::DecodeFold fold = {};
+    fold.eps = (float)eps;
+    if (sumsq.has_value()) {
+      TORCH_CHECK(sumsq->is_cuda() && sumsq->scalar_type() == at::kFloat && sumsq->is_contiguous() && sumsq->dim() == 2 &&
+                      sumsq->size(1) == B, "gemm_decode: sumsq must be [parts, rows] fp32");
+      fold.scale_sumsq = sumsq->data_ptr<float>();
+      fold.scale_parts = (int)sumsq->size(0);
+    }
+    int epi = silu_pairs ? penny::sm100::DECODE_EPI_SILU_PAIRS : penny::sm100::DECODE_EPI_PLAIN;
+    if (residual.has_value()) {
+      auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
+      TORCH_CHECK(!silu_pairs && bf16(*residual) && residual->sizes() == out.sizes() && residual->stride(0) == out.stride(0) &&
+                      norm_w.has_value() && bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == N &&
+                      sumsq_out.has_value() && sumsq_out->is_cuda() && sumsq_out->scalar_type() == at::kFloat &&
+                      sumsq_out->is_contiguous() && N % 128 == 0 && sumsq_out->numel() == N / 128 * B,
+                  "gemm_decode: residual like out, contiguous norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
+      epi = penny::sm100::DECODE_EPI_RESIDUAL;
+      fold.residual = residual->data_ptr();
+      fold.norm_w = norm_w->data_ptr();
+      fold.sumsq_out = sumsq_out->data_ptr<float>();
+    }
     cudaError_t rc = penny::sm100::launch_gemm_decode(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), (int)B, (int)N, (int)K, (int)x.stride(0), (int)w.stride(0),
-        (int)out.stride(0), silu_pairs ? 1 : 0, (int)splits, pdl, (long long)l2_budget, (int)smem_kb, pp,
+        (int)out.stride(0), epi, (int)splits, pdl, (long long)l2_budget, (int)smem_kb, pp, &fold,
         penny_gemm_error_word(),
         at::cuda::getCurrentCUDAStream().stream());
     TORCH_CHECK(rc == cudaSuccess, "gemm_decode: ", cudaGetErrorString(rc));
   }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("silu_pairs") = false, py::arg("splits") = 0,
-     py::arg("pdl") = true, py::arg("l2_budget") = -1, py::arg("smem_kb") = 0, py::arg("push") = py::none());
+     py::arg("pdl") = true, py::arg("l2_budget") = -1, py::arg("smem_kb") = 0, py::arg("push") = py::none(),
+     py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
+     py::arg("sumsq_out") = py::none());
   // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
   // rows before its up rows, out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
   // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq

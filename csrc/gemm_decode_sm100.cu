@@ -12,8 +12,8 @@
 //   * One CTA per (W tile, K range).  The K ranges of a tile belong to the CTAs
 //     of one thread-block cluster (1-8 CTAs), which add their fp32 partials
 //     through distributed shared memory: every CTA owns a slice of the batch
-//     columns, receives that slice from its peers (st.shared::cluster + one
-//     mbarrier arrival per peer), adds in rank order and stores bf16.  No global
+//     columns, receives that slice from its peers (st.async, the bytes counted
+//     on its mbarrier), adds in rank order and stores bf16.  No global
 //     workspace, no atomics, no second pass, deterministic.  The cluster size is
 //     chosen per shape from a small time model (decode_gemm_plan.h).
 //   * Programmatic dependent launch: the kernel may start while its predecessor
@@ -25,7 +25,7 @@
 //   * 3-4 stage TMA ring of 24 KB (B <= 64), at most ~106 KB of shared memory, so
 //     two of these kernels (or one and the decode attention) are resident per SM:
 //     that is what lets the next kernel's prologue overlap this one.
-//   * warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: epilogue.  Every wait
+//   * warp 0: TMA producer, warp 1: MMA issuer, warps 2-9: epilogue.  Every wait
 //     is bounded; TMEM is always freed.
 //
 // Epilogues: plain store, or silu(gate) * up for a gate/up weight whose rows are
@@ -72,7 +72,8 @@ namespace sm100 {
 
 namespace {
 
-constexpr int kDecThreads = 192;
+constexpr int kDecEpiThreads = 256;  // eight epilogue warps
+constexpr int kDecThreads = 64 + kDecEpiThreads;
 constexpr int kMaxStages = 8;
 
 // Diagnostics: with PENNY_DEC_STAMPS=1 the first 512 CTAs of a launch record
@@ -94,6 +95,12 @@ struct DecodeArgs {
   int epi;          // DECODE_EPI_*
   int slabs;        // batch slabs of BT rows (1 unless B > 128)
   DecodePush push;  // world == 0: plain store
+  const float* scale_sumsq;
+  int scale_parts;
+  float inv_width, eps;
+  __nv_bfloat16* residual;
+  const __nv_bfloat16* norm_w;
+  float* sumsq_out;
 };
 
 template <int BT>
@@ -102,20 +109,16 @@ struct DecodeCfg {
   static constexpr int kXBytes = BT * kBlockK * 2;
   static constexpr int kStageBytes = kWBytes + kXBytes;
   static constexpr int kTmemCols = BT < 32 ? 32 : BT;
+  static constexpr int kBarBytes = 256;
   // the peers' partials of this CTA's column slice: [splits - 1][slice][128 rows] fp32
   __host__ __device__ static size_t recv_floats(int splits) { return decode_recv_floats(BT, splits); }
   // The ring doubles as the [BT][128] fp32 staging area of the epilogue, so it is never smaller than that.
   __host__ __device__ static int min_stages() { return (BT * kBlockM * 4 + kStageBytes - 1) / kStageBytes; }
   static size_t smem_bytes(int stages, int splits) {
-    return (size_t)stages * kStageBytes + recv_floats(splits) * 4 + 1024 /*alignment*/ + 256 /*barriers*/;
+    return (size_t)stages * kStageBytes + recv_floats(splits) * 4 + 1024 /*alignment*/ + kBarBytes + BT * 4 /*s_scale*/;
   }
 };
 
-__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, const float4& v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z),
-               "f"(v.w)
-               : "memory");
-}
 // One [128 x 64] box of W into L2 only (no shared memory, no barrier).
 __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
@@ -135,9 +138,10 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   uint64_t* full = bars;
   uint64_t* empty = bars + kMaxStages;
   uint64_t* tmem_full = bars + 2 * kMaxStages;
-  uint64_t* recv_bar = bars + 2 * kMaxStages + 1;  // [4]: one per epilogue warp (row quarter)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 5);
+  uint64_t* recv_bar = bars + 2 * kMaxStages + 1;  // the peers' partials of my columns, counted in bytes
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  float* s_scale = reinterpret_cast<float*>(bars + Cfg::kBarBytes / 8);  // [BT] 1 / rms of this CTA's columns
 
   pdl_launch_dependents();
   const int cta_lin = (int)(blockIdx.y * gridDim.x + blockIdx.x);
@@ -154,7 +158,10 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int row0 = ((int)blockIdx.y % a.slabs) * BT;
   const int kb0 = decode_kb_begin(a.num_kb, S, (int)crank), kb1 = decode_kb_begin(a.num_kb, S, (int)crank + 1);
   const int nkb = kb1 - kb0;
-  const int sl = decode_slice(BT, S);
+  // the batch rows of this slab are dealt out over the cluster: columns [lo, hi) are finished here
+  const int nB = min(BT, a.B - row0);
+  const int sl = decode_slice(nB, S);
+  const int lo = (int)crank * sl, hi = min(nB, lo + sl);
   // Tiles walk their K range from different starting points (and wrap around), so that at any
   // moment the CTAs of a wave read different column ranges of W rather than the same few
   // hundred bytes of every row.
@@ -172,9 +179,10 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       mbar_init(&empty[i], 1);
     }
     mbar_init(tmem_full, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&recv_bar[i], S > 1 ? (uint32_t)(S - 1) : 1u);
+    mbar_init(recv_bar, 1);
     *s_abort = 0;
     mbar_fence_init();
+    if (S > 1 && lo < hi) mbar_expect_tx(recv_bar, (uint32_t)((S - 1) * (hi - lo) * kBlockM * 4));
     // The first ring-full of W tiles is requested before anything else happens in
     // the CTA (TMEM allocation, the block and cluster barriers): its HBM latency
     // runs under the rest of the prologue.  W never depends on the predecessor.
@@ -273,75 +281,92 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // ------------------------------------------------------------------ epilogue
     // Everything after the TMEM read works on shared memory with run-time loops:
     // the code stays small (an unrolled per-column epilogue costs more in
-    // instruction-cache misses than the whole GEMM takes).  Each warp owns a
-    // quarter of the tile's rows from TMEM to the final store, so the four warps
-    // never wait for one another (except for the gate/up pairing).
-    const int q = warp & 3;         // TMEM lane quarter of this warp
+    // instruction-cache misses than the whole GEMM takes).  What is left is a chain of
+    // latencies, so eight warps share it, two per TMEM lane quarter.
+    const int q = warp & 3, h = (warp - 2) >> 2;
     const int row = q * 32 + lane;  // weight row inside the tile = output column
-    const bool silu = a.epi == DECODE_EPI_SILU_PAIRS;
+    const int tid = (int)threadIdx.x - 64;
+    const bool silu = a.epi == DECODE_EPI_SILU_PAIRS, resid = a.epi == DECODE_EPI_RESIDUAL;
+    pdl_wait();  // this thread's stores (and the loads below) come after everything the predecessor did
+    if (a.scale_sumsq != nullptr && lo < hi) {
+      // 1 / rms of my columns, under the product: several threads per column where there are few
+      const int n = hi - lo;
+      int tpc = 32;
+      while (n * tpc > kDecEpiThreads) tpc >>= 1;
+      const int c = tid / tpc;
+      float s = 0.f;
+      if (c < n) {
+        const float* p = a.scale_sumsq + row0 + lo + c;
+#pragma unroll 8
+        for (int i = tid % tpc; i < a.scale_parts; i += tpc) s += __ldcg(p + (size_t)i * a.B);
+      }
+      for (int o = tpc >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (c < n && tid % tpc == 0) s_scale[c] = rsqrtf(s * a.inv_width + a.eps);
+    }
+    // A work item is 8 consecutive rows (output columns) of one batch column; a thread's items are of one row group.
+    const int groups = silu ? 8 : 16;
+    const int g = tid % groups, n0 = tile * (silu ? kBlockM / 2 : kBlockM) + g * 8;
+    // RESIDUAL: the stream's rows travel an item ahead, the first ones and the norm's weight under the product
+    uint4 r_next = make_uint4(0, 0, 0, 0), nw = r_next;
+    auto load_residual = [&](int j) {
+      if (j < hi) r_next = *reinterpret_cast<const uint4*>(a.residual + (size_t)(row0 + j) * a.ldo + n0);
+    };
+    if (resid) {
+      nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + n0));
+      load_residual(lo + tid / groups);
+    }
     bool ok = mbar_wait_abortable(tmem_full, 0u, s_abort);
     if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
     ok = __all_sync(0xffffffffu, ok);
-    if (q == 0 && lane == 0) stamp(5);  // accumulator complete
+    if (tid == 0) stamp(5);  // accumulator complete
     tc_fence_after_sync();
-    pdl_wait();  // this thread's stores come after everything the predecessor did
     // accumulator -> shared memory, column-major [BT columns][128 rows] fp32, in the
     // pipeline stages (every MMA that read them has completed)
     float* s_acc = reinterpret_cast<float*>(tiles);
+    const float4* s_acc4 = reinterpret_cast<const float4*>(s_acc);
+    const int c_begin = h * (BT / 2), c_end = min(nB, c_begin + BT / 2);
     if (ok) {
       const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BT / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tacc + c * 32, r);
+      for (int c = c_begin; c < c_end; c += 16) {
+        uint32_t r[16];
+        tmem_ld_32x16(tacc + c, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) s_acc[(c * 32 + j) * kBlockM + row] = __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) s_acc[(c + j) * kBlockM + row] = __uint_as_float(r[j]);
       }
     }
     __syncwarp();
-    const float4* s_acc4 = reinterpret_cast<const float4*>(s_acc);
     if (S > 1) {
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // the peers' barriers exist
       if (ok) {
-        // ---- hand every other CTA the rows of this warp of its column slice: a store
-        // instruction covers 4 columns x 128 bytes; then one release-arrive per peer ----
-        const uint32_t recv_local = smem_u32(s_recv);
-        const int rv = q * 8 + (lane & 7), cl = lane >> 3;  // float4 of my quarter, column within a group of 4
-        for (int d = 0; d < S; ++d) {
+        // ---- hand every other CTA the columns of its slice that this warp has: a store instruction
+        // covers 4 columns x 128 bytes and counts its bytes on the owner's barrier, so nothing waits
+        // for the stores (an arrival behind them was 1.5-2 us of a split GEMM's 3 us exchange) ----
+        const uint32_t recv_local = smem_u32(s_recv), bar_local = smem_u32(recv_bar);
+        const int rv = q * 8 + (lane & 7);  // float4 of my quarter
+        const uint32_t per = (65536u + (uint32_t)sl - 1u) / (uint32_t)sl;
+        for (int c = c_begin + (lane >> 3); c < c_end; c += 4) {
+          const int d = (int)(((uint32_t)c * per) >> 16);  // owner: c / sl
           if (d == (int)crank) continue;
-          const int lo = d * sl, hi = min(BT, lo + sl);
-          const uint32_t remote =
-              map_to_cta(recv_local, (uint32_t)d) + (uint32_t)(decode_recv_slot((int)crank, d) * sl * kBlockM * 4);
-          for (int c = lo + cl; c < hi; c += 4)
-            st_cluster_v4(remote + (uint32_t)(((c - lo) * (kBlockM / 4) + rv) * 16), s_acc4[c * (kBlockM / 4) + rv]);
-        }
-        __syncwarp();
-        if (lane == 0) {
-          for (int d = 0; d < S; ++d)
-            if (d != (int)crank) mbar_arrive_cluster(map_to_cta(smem_u32(&recv_bar[q]), (uint32_t)d));
+          const float4 v = s_acc4[c * (kBlockM / 4) + rv];
+          st_async_v4(map_to_cta(recv_local, (uint32_t)d) +
+                          (uint32_t)(((decode_recv_slot((int)crank, d) * sl + c - d * sl) * (kBlockM / 4) + rv) * 16),
+                      map_to_cta(bar_local, (uint32_t)d), __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z),
+                      __float_as_uint(v.w));
         }
       }
     }
-    if (silu) named_bar_sync(1, 128);  // gate rows meet the up rows another warp staged
-    if (ok && S > 1) {
-      // my rows of the peers' partials (gate/up pairing: every quarter)
-      for (int w = 0; w < 4; ++w) {
-        if (!silu && w != q) continue;
-        if (!mbar_wait_cluster(&recv_bar[w], 0u, s_abort)) ok = false;
-      }
+    named_bar_sync(1, kDecEpiThreads);  // all rows and columns staged, s_scale written
+    if (ok && S > 1 && lo < hi) {
+      ok = mbar_wait_cluster(recv_bar, 0u, s_abort);
       if (!ok && lane == 0) fail(GEMM_ERR_EPILOGUE_WAIT);
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (q == 0 && lane == 0) stamp(6);  // peers' partials received
+    if (tid == 0) stamp(6);  // peers' partials received
     if (ok) {
-      // ---- my slice: add the peers' partials in rank order, apply the epilogue, store.
-      // A work item is 8 consecutive rows (output columns) of one batch column; a warp takes the
-      // items of its own row quarter (gate/up: gate rows 16 q .. 16 q + 15 and their up rows).
-      const int lo = (int)crank * sl, hi = min(min(BT, lo + sl), a.B - row0);
-      const int groups = silu ? 2 : 4;  // row groups of 8 per column in this warp's share
+      // ---- my slice: add the peers' partials in rank order, apply the epilogue, store ----
       const int n_out = silu ? a.N / 2 : a.N;
-      const int n_tile0 = tile * (silu ? kBlockM / 2 : kBlockM);
       const bool vec_ok = (a.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.out) & 15u) == 0);
       // push mode: the call number of the all-reduce that follows (final: the predecessor has
       // finished) selects the scratch half and stamps the lines
@@ -351,8 +376,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         push_seq = *reinterpret_cast<const volatile unsigned long long*>(a.push.call_seq);
         push_base = scratch_half(a.push.scratch_off, a.push.scratch_bytes, push_seq);
       }
-      for (int idx = lane; idx < (hi - lo) * groups; idx += 32) {
-        const int j = lo + idx / groups, g = q * groups + idx % groups;
+      for (int j = lo + tid / groups; j < hi; j += kDecEpiThreads / groups) {
         // sum over the cluster of rows r0 .. r0 + 7 of column j
         auto sum8 = [&](int r0, float (&acc)[8]) {
 #pragma unroll
@@ -369,14 +393,42 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         };
         float v[8];
         sum8(g * 8, v);
+        const float sc = a.scale_sumsq != nullptr ? s_scale[j - lo] : 1.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] *= sc;
+        if (resid) {
+          const uint32_t rw[4] = {r_next.x, r_next.y, r_next.z, r_next.w}, ww[4] = {nw.x, nw.y, nw.z, nw.w};
+          load_residual(j + kDecEpiThreads / groups);
+          uint32_t zo[4], ho[4];
+          float ss = 0.f;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float z0 = v[2 * k] + __uint_as_float(rw[k] << 16);
+            const float z1 = v[2 * k + 1] + __uint_as_float(rw[k] & 0xffff0000u);
+            ss += z0 * z0 + z1 * z1;
+            zo[k] = pack_bf16x2(__float_as_uint(z0), __float_as_uint(z1));
+            ho[k] = pack_bf16x2(__float_as_uint(z0 * __uint_as_float(ww[k] << 16)),
+                                __float_as_uint(z1 * __uint_as_float(ww[k] & 0xffff0000u)));
+          }
+          const size_t off = (size_t)(row0 + j) * a.ldo + n0;
+          *reinterpret_cast<uint4*>(a.residual + off) = make_uint4(zo[0], zo[1], zo[2], zo[3]);
+          *reinterpret_cast<uint4*>(a.out + off) = make_uint4(ho[0], ho[1], ho[2], ho[3]);
+          const unsigned half = 0xffffu << (lane & 16);  // the sixteen row groups of this column
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(half, ss, o);
+          if (g == 0) a.sumsq_out[(size_t)tile * a.B + row0 + j] = ss;
+          continue;
+        }
         if (silu) {
           // rows 0-63 of the tile are gate, rows 64-127 the matching up rows
           float u[8];
           sum8(64 + g * 8, u);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = v[k] / (1.f + __expf(-v[k])) * u[k];
+          for (int k = 0; k < 8; ++k) {
+            const float e = 1.f + __expf(-v[k]);
+            v[k] = (a.scale_sumsq != nullptr ? __fdividef(v[k], e) : v[k] / e) * (u[k] * sc);
+          }
         }
-        const int n0 = n_tile0 + g * 8;
         __nv_bfloat16* dst = a.out + (size_t)(row0 + j) * a.ldo + n0;
         if (vec_ok && n0 + 8 <= n_out) {
           uint4 o;
@@ -465,9 +517,8 @@ const int* decode_capacity(int sms) {
 
 template <int BT>
 cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int N, int K, int ldx, int ldw, int ldo,
-                             int epi, int splits, bool pdl, long long l2_budget, int smem_kb, const DecodePush* push, int sms,
-                             uint32_t* error_word,
-                             cudaStream_t stream) {
+                             int epi, int splits, bool pdl, long long l2_budget, int smem_kb, const DecodePush* push,
+                             const DecodeFold* fold, int sms, uint32_t* error_word, cudaStream_t stream) {
   using Cfg = DecodeCfg<BT>;
   CUtensorMap mw, mx;
   cudaError_t rc = make_tile_map(&mw, w, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, kBlockM);
@@ -493,6 +544,14 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
     a.push = *push;
   else
     a.push.world = 0;
+  const DecodeFold f = fold != nullptr ? *fold : DecodeFold{};
+  a.scale_sumsq = f.scale_sumsq;
+  a.scale_parts = f.scale_parts;
+  a.inv_width = 1.f / (float)K;
+  a.eps = f.eps;
+  a.residual = reinterpret_cast<__nv_bfloat16*>(f.residual);
+  a.norm_w = reinterpret_cast<const __nv_bfloat16*>(f.norm_w);
+  a.sumsq_out = f.sumsq_out;
   // ring depth: what fits next to the receive area in ~106 KB (two CTAs per SM, of this kernel or the next:
   // one sets up and fills its ring while the other drains).  With a 128-wide batch tile and no more CTAs than
   // SMs one per SM and as deep as the range needs.  A second round of CTAs wants the two as well (the step
@@ -527,11 +586,18 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
 
 cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, int N, int K, int ldx, int ldw,
                                int ldo, int epi, int splits, bool pdl, long long l2_budget_bytes,
-                               int smem_kb, const DecodePush* push, uint32_t* error_word, cudaStream_t stream) {
+                               int smem_kb, const DecodePush* push, const DecodeFold* fold, uint32_t* error_word,
+                               cudaStream_t stream) {
   if (B <= 0 || B > kDecodeMaxBatch || N <= 0 || K <= 0 || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0)
     return cudaErrorInvalidValue;
   if (push != nullptr && B > 128) return cudaErrorInvalidValue;  // the owners' receive lines cover one slab
-  if (epi != DECODE_EPI_PLAIN && epi != DECODE_EPI_SILU_PAIRS) return cudaErrorInvalidValue;
+  if (epi != DECODE_EPI_PLAIN && epi != DECODE_EPI_SILU_PAIRS && epi != DECODE_EPI_RESIDUAL) return cudaErrorInvalidValue;
+  if (epi == DECODE_EPI_RESIDUAL &&
+      (N % kBlockM != 0 || ldo % 8 != 0 || push != nullptr || fold == nullptr || fold->residual == nullptr ||
+       fold->norm_w == nullptr || fold->sumsq_out == nullptr ||
+       ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(fold->residual) |
+         reinterpret_cast<uintptr_t>(fold->norm_w)) & 15u) != 0))
+    return cudaErrorInvalidValue;
   if (epi == DECODE_EPI_SILU_PAIRS && N % kBlockM != 0) return cudaErrorInvalidValue;
   if ((N + kBlockM - 1) / kBlockM > 65535) return cudaErrorInvalidValue;
   if (push != nullptr && (push->world < 2 || push->world > 8 || epi != DECODE_EPI_PLAIN || N % 8 != 0 || ldo % 8 != 0 ||
@@ -542,10 +608,10 @@ cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, i
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (l2_budget_bytes < 0) l2_budget_bytes = (long long)32 << 20;
   if (B <= 32)
-    return launch_decode_bt<32>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, sms, error_word, stream);
+    return launch_decode_bt<32>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
   if (B <= 64)
-    return launch_decode_bt<64>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, sms, error_word, stream);
-  return launch_decode_bt<128>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, sms, error_word, stream);
+    return launch_decode_bt<64>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
+  return launch_decode_bt<128>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
 }
 
 int gemm_decode_stamps(unsigned long long* out, int max_ctas) {

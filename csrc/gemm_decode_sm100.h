@@ -14,6 +14,20 @@ enum DecodeEpilogue : int {
   // the same features (N a multiple of 128); out is [B, N / 2] with
   // out[b][blk * 64 + i] = silu(gate) * up.
   DECODE_EPI_SILU_PAIRS = 1,
+  // z = acc + residual; residual = z; out = z * norm_w; sumsq_out = sum of z^2 per 128 columns (N a multiple of 128)
+  DECODE_EPI_RESIDUAL = 2,
+};
+
+// What rides in the epilogue of a linear that stands next to a norm.
+struct DecodeFold {
+  // null, or [scale_parts][B] sums of squares of the rows of x before their norm weight: every output is
+  // multiplied by rsqrt(sum / K + eps)
+  const float* scale_sumsq;
+  int scale_parts;
+  float eps;
+  void* residual;      // DECODE_EPI_RESIDUAL: [B, N], ldo
+  const void* norm_w;  // [N]
+  float* sumsq_out;    // [N / 128][B]
 };
 
 // Epilogue target of a row-parallel linear whose output goes into an all-reduce + RMSNorm of the
@@ -38,13 +52,15 @@ struct DecodePush {
 //   l2_budget_bytes a whole W no larger than this is prefetched into L2 before the
 //                   dependency wait (-1 = default, 0 = only a rolling window)
 //   push            null, or where rows owned by other ranks go (see DecodePush); plain epilogue only
+//   fold            null, or the row scale and the residual add of the norms around the linear (see DecodeFold)
 //   smem_kb         shared memory the TMA ring may grow to (0 = default: ~106 KB, so
 //                   that the next kernel of the step fits on the SM beside this one;
 //                   up to 226 for a kernel nothing needs to overlap with)
 // Allocates nothing; no workspace; safe to capture.  error_word as in launch_gemm_bf16.
 cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, int N, int K, int ldx, int ldw,
                                int ldo, int epi, int splits, bool pdl, long long l2_budget_bytes,
-                               int smem_kb, const DecodePush* push, uint32_t* error_word, cudaStream_t stream);
+                               int smem_kb, const DecodePush* push, const DecodeFold* fold, uint32_t* error_word,
+                               cudaStream_t stream);
 
 // Diagnostics (PENNY_DEC_STAMPS=1): copies the %globaltimer stamps of the last launch's first CTAs to
 // `out` ([ctas][8] nanoseconds: CTA start, prologue done, predecessor complete, last load issued, last

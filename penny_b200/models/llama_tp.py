@@ -9,7 +9,8 @@ One decode step for a batch of sequences on `world` GPUs:
                one kernel)--> ] x layers
           -> lm_head shard GEMM -> arg-max (local, then across ranks)
 
-Seven launches per layer, all of them this library's kernels: the linears are
+Seven launches per layer (on one rank five: the residual adds and norms ride in
+the GEMM epilogues), all of them this library's kernels: the linears are
 the tcgen05 decode GEMM (`ops.gemm_decode`; `linears="cublas"` swaps in
 torch.matmul for comparison), and every kernel is launched with programmatic
 stream serialization, so inside the captured CUDA graph a kernel's prologue and
@@ -129,6 +130,9 @@ class LlamaTPDecoder:
         if (comm is not None and world > 1 and backend == "penny" and proto == "ll_twoshot" and linears == "penny"
                 and max_batch <= 128 and hasattr(comm, "fused_norm_push_target")):
             self._push = comm.fused_norm_push_target(max_batch, H)
+        # One rank on this library's linears: the residual add and the norms ride in the GEMM epilogues (two launches
+        # of 2 us each less per layer).
+        self.fold = world == 1 and linears == "penny" and max_batch <= 1024 and cfg.hidden % 128 == 0
         self._init_weights(seed, full_init)
 
         def buf(*shape, dtype=dt, heap=False):
@@ -147,6 +151,8 @@ class LlamaTPDecoder:
         # buffers, so consecutive all-reduces never read the same one
         self.parts = [buf(B, H, heap=True), buf(B, H, heap=True)]
         self.part = self.parts[0]
+        if self.fold:
+            self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
         self.gu = buf(B, 2 * self.F) if linears == "cublas" else None
         self.act = buf(B, self.F)
         self.logits = buf(B, self.V)
@@ -176,6 +182,8 @@ class LlamaTPDecoder:
         # + arg-max (+ the all-gather of the ranks' candidates and the choice among them) + LM head
         own_head = chunks if self.linears == "penny" else int(self.own_head)
         self.kernels_per_step = cfg.layers * per_layer + norms + 1 + (2 if world > 1 else 0) + own_head
+        if self.fold:
+            self.kernels_per_step = 5 * cfg.layers + 3
 
     # ------------------------------------------------------------------ weights
     def _init_weights(self, seed: int, full_init: bool):
@@ -298,7 +306,23 @@ class LlamaTPDecoder:
         for r in range(0, B, 1024):
             ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, 0, push)
 
-    def _step_impl(self, warm_up: bool = False):
+    def _layers_folded(self):
+        """One rank: five launches per layer.  x holds the residual stream times the next norm's weight, sumsq its
+        sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
+        x, ss, eps, pdl = self.x, self.sumsq[0], self.cfg.eps, self.pdl
+        ops.norm_prep(self.embed, self.layers[0]["norm1"], self.residual, x, ss, ids=self.tokens)
+        for li, L in enumerate(self.layers):
+            ops.gemm_decode(x, L["wqkv"], self.qkv, pdl=pdl, sumsq=ss, eps=eps)
+            ops.decode_attention_fused(self.qkv, self.kcache[li], self.vcache[li], self.positions, self.attn,
+                                       self.workspace, self.Hq, self.Hkv, self.splits, self.scale, self.cfg.rope_theta, pdl)
+            ss = self.sumsq[1]
+            ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=self.residual, norm_w=L["norm2"], sumsq_out=ss)
+            ops.gemm_decode(x, L["wgu"], self.act, True, pdl=pdl, sumsq=ss, eps=eps)
+            nxt = self.layers[li + 1]["norm1"] if li + 1 < self.cfg.layers else self.final_norm
+            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=self.residual, norm_w=nxt, sumsq_out=ss)
+        ops.gemm_decode(x, self.lm_head, self.logits, pdl=pdl, sumsq=ss, eps=eps)
+
+    def _layers(self, warm_up: bool):
         cfg = self.cfg
         torch.index_select(self.embed, 0, self.tokens, out=self.residual)
         ops.add_rmsnorm(self.residual, None, self.layers[0]["norm1"], self.x, None, cfg.eps)
@@ -333,6 +357,12 @@ class LlamaTPDecoder:
                 ops.gemm_tile(self.x, self.lm_head, self.logits, pdl=self.pdl)
             if warm_up or not self.own_head:
                 torch.matmul(self.x, self.lm_head.t(), out=self.logits)
+
+    def _step_impl(self, warm_up: bool = False, separate: bool = False):
+        if self.fold and not separate:
+            self._layers_folded()
+        else:
+            self._layers(warm_up)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
         # in fp32), gathered over the ranks; one kernel then picks the best rank per sequence, feeds the
         # token back (step() overwrites self.tokens with the caller's tokens) and advances the positions
@@ -355,8 +385,10 @@ class LlamaTPDecoder:
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
-            for _ in range(2):
-                self._step_impl(warm_up=True)
+            # (the first warm-up step on separate norms, whichever route the step takes: the second one's tokens, and
+            # with them the rows that it leaves behind the current positions, do not depend on the route)
+            for i in range(2):
+                self._step_impl(warm_up=True, separate=i == 0)
         torch.cuda.current_stream().wait_stream(s)
         torch.cuda.synchronize()
         if self.use_graph:

@@ -1,0 +1,64 @@
+"""The decode GEMM's row scale and residual epilogue (the norms on either side of a linear)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (rows, columns, K): one row, an odd number with a ragged last slice, whole and just exceeded batch tiles, two slabs;
+# K of one step, of a partial last step, and more K steps than the ring is deep
+SHAPES = [(1, 128, 64), (5, 256, 520), (33, 512, 1024), (64, 384, 4096), (128, 256, 2048), (129, 256, 1032)]
+
+
+def _inputs(B, N, K, parts):
+    g = torch.Generator(device="cuda").manual_seed(B * 7 + N + K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    return r(B, K).bfloat16(), (r(N, K) * K ** -0.5).bfloat16(), r(parts, B).square() * K / parts
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("splits", [0, 1, 3, 8])
+def test_residual_epilogue(shape, splits):
+    from penny_b200._ext import ops
+    B, N, K = shape
+    x, w, _ = _inputs(B, N, K, 1)
+    res, norm_w = torch.randn(B, N, device="cuda").bfloat16(), torch.rand(N, device="cuda").bfloat16()
+    z = res.double() + x.double() @ w.double().t()
+    out, ss = torch.empty_like(res), torch.full((N // 128, B), float("nan"), device="cuda")
+    ops.gemm_decode(x, w, out, False, splits, residual=res, norm_w=norm_w, sumsq_out=ss)
+    assert ops.gemm_error() == 0
+    # fp32 sums of up to 4096 products of size K ** -0.5: 1e-5 at most; then one bf16 rounding (2 ** -9)
+    tol = z.abs() * 2.0 ** -8 + 1e-4
+    assert ((res.double() - z).abs() <= tol).all()
+    assert ((out.double() - z * norm_w.double()).abs() <= tol * norm_w.double() + 1e-6).all()
+    want = z.square().view(B, N // 128, 128).sum(-1).t()
+    torch.testing.assert_close(ss.double(), want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("silu,parts,splits", [(False, 1, 0), (False, 32, 2), (True, 3, 0), (True, 32, 4)])
+def test_row_scale(shape, silu, parts, splits):
+    from penny_b200._ext import ops
+    B, N, K = shape
+    x, w, ss = _inputs(B, N, K, parts)
+    scale = torch.rsqrt(ss.double().sum(0) / K + 1e-5)
+    want = (x.double() @ w.double().t()) * scale[:, None]
+    if silu:
+        v = want.view(B, N // 128, 2, 64)
+        want = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(B, N // 2)
+    out = torch.empty(B, N // 2 if silu else N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_decode(x, w, out, silu, splits, sumsq=ss, eps=1e-5)
+    assert ops.gemm_error() == 0
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4 * scale.max()).all()
+
+
+def test_embedding_rows_start_the_stream():
+    from penny_b200._ext import ops
+    table = torch.randn(50, 512, device="cuda").bfloat16()
+    ids = torch.tensor([49, 0, 7, 7, 31], device="cuda")
+    w = torch.rand(512, device="cuda").bfloat16()
+    res, out = (torch.empty(5, 512, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ss = torch.empty(1, 5, device="cuda")
+    ops.norm_prep(table, w, res, out, ss, ids=ids)
+    want = table[ids]
+    assert torch.equal(res, want) and torch.equal(out, (want.float() * w.float()).bfloat16())
+    torch.testing.assert_close(ss[0], want.float().square().sum(-1), rtol=1e-5, atol=0)
