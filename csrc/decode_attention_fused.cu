@@ -12,12 +12,21 @@
 //     softmax from shared memory.  q is rotated in registers by every CTA.
 //   * The last CTA of a (row, KV head) to finish merges the split partials: a
 //     self-resetting arrival counter per (row, KV head), no second launch.
+//   * The pieces of a row: `splits` equal ones (grid z), or with balance as many as its length
+//     asks for.  What bounds the kernel is the cache's stream while about 150 CTAs are at work,
+//     and otherwise one CTA's: a position per 10 ns.  Rows of one length stay whole once they
+//     fill half of the GPU (37 rows of 4096: 92 us whole, 98 in two or three pieces), a few
+//     long ones are cut to fill it, and of rows of mixed lengths the long ones, which would
+//     run on alone (64 rows of 1 to 2048: 50.8 -> 47.4 us of 41.7 for the bytes).  Every CTA reads
+//     all positions under the dependency wait and finds its own piece.
 //   * Programmatic dependent launch: the kernel may start while the QKV GEMM is
 //     still running.  Its first K / V tiles - written by earlier decode steps,
 //     never by the kernels just before it - are requested BEFORE the dependency
 //     wait; q, k, v of the new token are read after it.
 //
 // The reference has no attention (it is used inside vLLM / SGLang, README.md:20-33).
+#include <algorithm>
+
 #include "decode_attn_common.cuh"
 #include "decode_kernels.h"
 #include "kernel_setup.h"
@@ -28,24 +37,104 @@ namespace penny {
 namespace {
 using namespace attn;
 
+// Shortest piece and most pieces of a row: a merge is 2 us.  One row of 2048 positions in 1 / 4 / 8 / 16 pieces: 17.3 /
+// 8.0 / 6.9 / 7.7 us, of 16000 in 8 / 16 / 37: 23.6 / 17.7 / 19.5, of 100 in 1 / 8 / 16: 2.7 / 5.1 / 6.5.
+constexpr int kMinPiece = 256, kMaxPieces = 16;
+
+// Piece `idx` of a batch whose rows are cut by length: row, KV head, piece and pieces of that row.  A piece is the
+// batch's positions over `slots` (the CTAs that the GPU holds at a time), over twice as many where the rows are of mixed
+// lengths and alone fill half of them, and a row has as many as fit it whole.  At most 2 slots more than (row, KV head)
+// pairs; idx past the last one: row -1.  Called by every thread of the block.
+struct Piece {
+  int b, kh, sp, n;
+};
+__device__ __forceinline__ Piece find_piece(const int* __restrict__ positions, int B, int Hkv, int slots, int idx) {
+  __shared__ int s_part[2][kAttnWarps];
+  __shared__ Piece s_piece;
+  const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int per = (B + kAttnWarps * 32 - 1) / (kAttnWarps * 32), r0 = min(B, tid * per), r1 = min(B, r0 + per);
+  int sum = 0, top = 0;
+  for (int r = r0; r < r1; ++r) {
+    sum += positions[r];
+    top = max(top, positions[r]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+  }
+  if (lane == 0) {
+    s_part[0][warp] = sum;
+    s_part[1][warp] = top;
+  }
+  if (tid == 0) s_piece.b = -1;
+  __syncthreads();
+  long long total = 0;
+#pragma unroll
+  for (int w = 0; w < kAttnWarps; ++w) {
+    total += s_part[0][w];
+    top = max(top, s_part[1][w]);
+  }
+  const bool mixed = (long long)top * B * 4 > total * 5 && B * Hkv * 2 > slots;
+  const int target = mixed ? 2 * slots : slots;
+  const int len = max(kMinPiece, (int)((total * Hkv + target - 1) / target));
+  auto pieces_of = [&](int r) { return min(kMaxPieces, max(1, positions[r] / len)); };
+  __syncthreads();
+  int mine = 0;
+  for (int r = r0; r < r1; ++r) mine += pieces_of(r);
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) s_part[0][warp] = incl;
+  __syncthreads();
+  int first = incl - mine;
+  for (int w = 0; w < warp; ++w) first += s_part[0][w];
+  int at = idx - first * Hkv;
+  if (at >= 0 && at < mine * Hkv) {
+    for (int r = r0; r < r1; ++r) {
+      const int n = pieces_of(r);
+      if (at < n * Hkv) {
+        s_piece = {r, at % Hkv, at / Hkv, n};
+        break;
+      }
+      at -= n * Hkv;
+    }
+  }
+  __syncthreads();
+  return s_piece;
+}
+
 template <int G>
 __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
-    const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache,
+    const __nv_bfloat16* qkv /* written by the predecessor: a restrict pointer's loads may move above the wait */,
+    __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache,
     const int* __restrict__ positions, __nv_bfloat16* __restrict__ out, float* __restrict__ part_o,
-    float* __restrict__ part_ml, unsigned* __restrict__ counters, int Hq, int Hkv, int max_len, int splits,
-    float scale, float theta) {
+    float* __restrict__ part_ml, unsigned* __restrict__ counters, int B, int Hq, int Hkv, int max_len, int splits,
+    int slots, float scale, float theta) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ float s_new[2 * kD];  // rotated k (as stored: bf16-rounded) and v of the new token
   __shared__ int s_last;
   pdl_launch_dependents();
-  const int b = blockIdx.x, kh = blockIdx.y, sp = blockIdx.z;
+  Piece pc{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, splits};
+  if (slots > 0) pc = find_piece(positions, B, Hkv, slots, (int)blockIdx.x);
+  if (pc.b < 0) {
+    pdl_wait();
+    return;
+  }
+  const int b = pc.b, kh = pc.kh, sp = pc.sp, pieces = pc.n;
+  // partial rows: head hh of piece p of this (row, KV head) is row slot0 + p * slot_p + hh * slot_h
+  const size_t slot0 = slots > 0 ? (size_t)(blockIdx.x - sp * Hkv) * G : ((size_t)b * Hq + kh * G) * pieces;
+  const int slot_p = slots > 0 ? Hkv * G : 1, slot_h = slots > 0 ? 1 : pieces;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   // positions[] was advanced at the end of the previous step, long before any kernel
   // that may still be running when this one starts
   const int pos = positions[b];
   const int len = pos;  // old rows; the new token is handled separately
-  const int per = ((len + splits - 1) / splits + kTile - 1) / kTile * kTile;
+  const int per = ((len + pieces - 1) / pieces + kTile - 1) / kTile * kTile;
   const int t0 = sp * per;
   const int t1 = min(len, t0 + per);
   const int ntiles = t1 > t0 ? (t1 - t0 + kTile - 1) / kTile : 0;
@@ -74,6 +163,15 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
   };
   issue(0);
   issue(1);
+  // the rotation needs the position alone: its powers, sines and cosines under the dependency wait
+  float rot_c[16], rot_s[16], k_c = 0.f, k_s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int d = (i >> 2) * 16 + ((i >> 1) & 1) * 8 + 2 * t + (i & 1);
+    __sincosf((float)pos * __powf(theta, -2.0f * (float)d / (float)kD), &rot_s[i], &rot_c[i]);
+  }
+  if (sp == 0 && threadIdx.x < kD / 2)
+    __sincosf((float)pos * __powf(theta, -2.0f * (float)threadIdx.x / (float)kD), &k_s, &k_c);
   pdl_wait();
 
   const size_t qkv_row = (size_t)b * (Hq + 2 * Hkv) * kD;
@@ -94,9 +192,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
         const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(qp + d + kD / 2);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const float inv_freq = __powf(theta, -2.0f * (float)(d + e) / (float)kD);
-          float sn, cs;
-          __sincosf((float)pos * inv_freq, &sn, &cs);
+          const float sn = rot_s[kc * 4 + h * 2 + e], cs = rot_c[kc * 4 + h * 2 + e];
           const float a = bf2f(e ? lo.y : lo.x), bb = bf2f(e ? hi.y : hi.x);
           ra[h * 2 + e] = (a * cs - bb * sn) * qs;
           rb[h * 2 + e] = (bb * cs + a * sn) * qs;
@@ -114,9 +210,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
     const int tid = (int)threadIdx.x;
     if (tid < kD / 2) {
       const __nv_bfloat16* kp = qkv + qkv_row + (size_t)(Hq + kh) * kD;
-      const float inv_freq = __powf(theta, -2.0f * (float)tid / (float)kD);
-      float sn, cs;
-      __sincosf((float)pos * inv_freq, &sn, &cs);
+      const float sn = k_s, cs = k_c;
       const float a = bf2f(kp[tid]), bb = bf2f(kp[tid + kD / 2]);
       const __nv_bfloat16 ka = __float2bfloat16_rn(a * cs - bb * sn), kb = __float2bfloat16_rn(bb * cs + a * sn);
       kcache[coff + tid] = ka;
@@ -259,14 +353,14 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
       acc[0] += wgt * ov.x; acc[1] += wgt * ov.y; acc[2] += wgt * ov.z; acc[3] += wgt * ov.w;
     }
     const int hq = kh * G + hh;
-    if (splits == 1) {
+    if (pieces == 1) {
       const float inv = L > 0.f ? 1.f / L : 0.f;
       uint2 raw;
       raw.x = pack2(acc[0] * inv, acc[1] * inv);
       raw.y = pack2(acc[2] * inv, acc[3] * inv);
       *reinterpret_cast<uint2*>(out + ((size_t)b * Hq + hq) * kD + d4) = raw;
     } else {
-      const size_t slot = ((size_t)b * Hq + hq) * splits + sp;
+      const size_t slot = slot0 + (size_t)sp * slot_p + (size_t)hh * slot_h;
       *reinterpret_cast<float4*>(part_o + slot * kD + d4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
       if (d4 == 0) {
         part_ml[slot * 2] = M;
@@ -274,32 +368,52 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
       }
     }
   }
-  if (splits == 1) return;
-  // ---- the last split of this (row, KV head) to get here merges them all ----
+  if (pieces == 1) return;
+  // ---- the last piece of this (row, KV head) to get here merges them all ----
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned* cnt = counters + (size_t)b * Hkv + kh;
     const unsigned old = atomicAdd(cnt, 1u);
-    const int last = old == (unsigned)(splits - 1);
-    if (last) *cnt = 0u;  // every split has arrived: ready for the next launch
+    const int last = old == (unsigned)(pieces - 1);
+    if (last) *cnt = 0u;  // every piece has arrived: ready for the next launch
     s_last = last;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // (eight pieces' loads at a time: one after another they were 3 us of a step of one short sequence)
   for (int item = threadIdx.x; item < G * 32; item += kAttnWarps * 32) {
     const int hq = kh * G + (item >> 5), d4 = (item & 31) * 4;
-    const size_t base = ((size_t)b * Hq + hq) * splits;
+    const size_t base = slot0 + (size_t)(item >> 5) * slot_h;
+    auto ml_of = [&](int s) {
+      return s < pieces ? __ldcg(reinterpret_cast<const float2*>(part_ml + (base + (size_t)s * slot_p) * 2))
+                        : make_float2(-INFINITY, 0.f);
+    };
     float M = -INFINITY;
-    for (int s = 0; s < splits; ++s) M = fmaxf(M, __ldcg(part_ml + (base + s) * 2));
+    for (int s0 = 0; s0 < pieces; s0 += 8) {
+      float ms[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ms[i] = ml_of(s0 + i).x;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) M = fmaxf(M, ms[i]);
+    }
     float L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < splits; ++s) {
-      const float ms = __ldcg(part_ml + (base + s) * 2);
-      const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - M);
-      L += w * __ldcg(part_ml + (base + s) * 2 + 1);
-      const float4 ov = __ldcg(reinterpret_cast<const float4*>(part_o + (base + s) * kD + d4));
-      acc[0] += w * ov.x; acc[1] += w * ov.y; acc[2] += w * ov.z; acc[3] += w * ov.w;
+    for (int s0 = 0; s0 < pieces; s0 += 8) {
+      float2 ml[8];
+      float4 ov[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        ml[i] = ml_of(s0 + i);
+        ov[i] = s0 + i < pieces ? __ldcg(reinterpret_cast<const float4*>(part_o + (base + (size_t)(s0 + i) * slot_p) * kD + d4))
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float w = (ml[i].x == -INFINITY) ? 0.f : exp2f(ml[i].x - M);
+        L += w * ml[i].y;
+        acc[0] += w * ov[i].x; acc[1] += w * ov[i].y; acc[2] += w * ov[i].z; acc[3] += w * ov[i].w;
+      }
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
     uint2 raw;
@@ -311,20 +425,49 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
 
 }  // namespace
 
+namespace {
+size_t counter_bytes(int B, int Hkv) { return ((size_t)B * Hkv * sizeof(unsigned) + 15) / 16 * 16; }
+
+// CTAs that a balanced launch counts on; 0, no pieces, where there are four rounds of (row, KV head) pairs anyhow, which
+// the GPU deals out as they end.
+int balance_slots(int items, int sms) { return items > 8 * sms ? 0 : 2 * sms; }
+int balance_extra(int items, int slots) { return items * 2 > slots ? 2 * slots : slots; }  // pieces beyond one per pair
+int device_sms() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+  return sms;
+}
+}  // namespace
+
 size_t decode_attn_fused_workspace_bytes(int B, int Hq, int Hkv, int splits) {
-  // partial rows + (max, sum) per (row, head, split), then one arrival counter per (row, KV head)
-  return decode_attn_workspace_bytes(B, Hq, splits) + (size_t)B * Hkv * sizeof(unsigned);
+  // one arrival counter per (row, KV head), then partial rows + (max, sum) per (row, head, split)
+  return counter_bytes(B, Hkv) + decode_attn_workspace_bytes(B, Hq, splits);
+}
+
+int decode_attn_balanced_splits(int B, int Hkv) {
+  const int items = B * Hkv;
+  const int slots = balance_slots(items, device_sms());
+  return slots == 0 ? 1 : 1 + (balance_extra(items, slots) + items - 1) / items;
 }
 
 cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* vcache, const int* positions,
                                           void* out, void* workspace, int B, int Hq, int Hkv, int D, int max_len,
-                                          int splits, float scale, float theta, bool pdl, cudaStream_t stream) {
+                                          int splits, float scale, float theta, bool pdl, bool balance,
+                                          cudaStream_t stream) {
   if (D != kD || Hkv < 1 || Hq % Hkv != 0 || splits < 1 || B < 1) return cudaErrorInvalidValue;
-  const int G = Hq / Hkv;
-  float* part_o = reinterpret_cast<float*>(workspace);
+  const int G = Hq / Hkv, items = B * Hkv;
+  unsigned* counters = reinterpret_cast<unsigned*>(workspace);
+  float* part_o = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + counter_bytes(B, Hkv));
   float* part_ml = part_o + (size_t)B * Hq * splits * kD;
-  unsigned* counters = reinterpret_cast<unsigned*>(part_ml + (size_t)B * Hq * splits * 2);
-  dim3 grid(B, Hkv, splits);
+  int slots = 0, extra = 0;
+  if (balance) {
+    slots = balance_slots(items, device_sms());
+    extra = balance_extra(items, slots);
+    // (a workspace for fewer pieces than the cut may take: whole rows)
+    if (slots == 0 || (long long)items * (splits - 1) < extra) slots = 0, splits = 1;
+  }
+  const dim3 grid = slots > 0 ? dim3((unsigned)(items + extra)) : dim3(B, Hkv, splits);
   cudaError_t rc = cudaSuccess;
 #define PENNY_ATTN_FUSED(GG)                                                                                  \
   do {                                                                                                        \
@@ -332,8 +475,8 @@ cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* v
     if (rc != cudaSuccess) return rc;                                                                         \
     rc = launch_kernel_ex(k_decode_attn_fused<GG>, grid, dim3(kAttnWarps * 32), (size_t)kAttnSmem, stream,    \
                           pdl, 1, (const __nv_bfloat16*)qkv, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache,  \
-                          positions, (__nv_bfloat16*)out, part_o, part_ml, counters, Hq, Hkv, max_len, splits, \
-                          scale, theta);                                                                      \
+                          positions, (__nv_bfloat16*)out, part_o, part_ml, counters, B, Hq, Hkv, max_len,     \
+                          splits, slots, scale, theta);                                                                      \
   } while (0)
   switch (G) {
     case 1: PENNY_ATTN_FUSED(1); break;

@@ -100,7 +100,7 @@ void bind_decode(py::module_& m) {
   // rope + KV append + split-KV attention + merge in one launch; qkv is the raw projection of the new token
   m.def("decode_attention_fused", [](at::Tensor qkv, at::Tensor kcache, at::Tensor vcache, at::Tensor positions,
                                      at::Tensor out, at::Tensor workspace, int64_t Hq, int64_t Hkv, int64_t splits,
-                                     double scale, double theta, bool pdl) {
+                                     double scale, double theta, bool pdl, bool balance) {
     need(bf16_cuda(qkv) && bf16_cuda(kcache) && bf16_cuda(vcache) && bf16_cuda(out), "decode_attention_fused expects contiguous bf16 CUDA tensors");
     need(positions.is_cuda() && positions.scalar_type() == at::kInt && positions.is_contiguous(), "positions must be int32 CUDA");
     need(kcache.dim() == 4 && vcache.sizes() == kcache.sizes(), "caches must be [B, Hkv, max_len, D]");
@@ -114,10 +114,15 @@ void bind_decode(py::module_& m) {
     const at::cuda::OptionalCUDAGuard guard(qkv.device());
     ck(launch_decode_attention_fused(qkv.data_ptr(), kcache.data_ptr(), vcache.data_ptr(), positions.data_ptr<int>(),
                                      out.data_ptr(), workspace.data_ptr(), (int)B, (int)Hq, (int)Hkv, (int)D,
-                                     (int)kcache.size(2), (int)splits, (float)scale, (float)theta, pdl, cur()),
+                                     (int)kcache.size(2), (int)splits, (float)scale, (float)theta, pdl, balance, cur()),
        "decode_attention_fused");
   }, py::arg("qkv"), py::arg("kcache"), py::arg("vcache"), py::arg("positions"), py::arg("out"), py::arg("workspace"),
-     py::arg("Hq"), py::arg("Hkv"), py::arg("splits"), py::arg("scale"), py::arg("theta"), py::arg("pdl") = true);
+     py::arg("Hq"), py::arg("Hkv"), py::arg("splits"), py::arg("scale"), py::arg("theta"), py::arg("pdl") = true,
+     py::arg("balance") = false);
+  m.def("decode_attn_balanced_splits", [](int64_t B, int64_t Hkv) {
+    need(B >= 1 && Hkv >= 1, "decode_attn_balanced_splits: rows and KV heads");
+    return (int64_t)decode_attn_balanced_splits((int)B, (int)Hkv);
+  });
   m.def("silu_mul", [](at::Tensor gate_up, at::Tensor out) {
     need(bf16_cuda(gate_up) && bf16_cuda(out) && gate_up.dim() == 2, "silu_mul expects [rows, 2F] bf16");
     const int64_t rows = gate_up.size(0), F = gate_up.size(1) / 2;

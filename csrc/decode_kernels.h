@@ -35,12 +35,16 @@ cudaError_t launch_decode_attention(const void* qkv, const void* kcache, const v
 // One launch for rope + KV append + split-KV attention + merge (csrc/decode_attention_fused.cu).
 // qkv holds the UNROTATED projections of the new token; rows [0, positions[b]) of the caches are
 // attended to together with the new token, whose rotated k and v are stored at row positions[b].
-// workspace: decode_attn_fused_workspace_bytes, zeroed once before the first call (its tail holds
-// self-resetting arrival counters).  pdl: launch with programmatic stream serialization.
+// workspace: decode_attn_fused_workspace_bytes, zeroed once before the first call (it begins with
+// self-resetting arrival counters).  pdl: launch with programmatic stream serialization.  balance: the
+// rows are cut by their lengths instead of into `splits` equal parts each; splits is then what the workspace
+// was sized for (decode_attn_balanced_splits gives what the best cut needs).
 size_t decode_attn_fused_workspace_bytes(int B, int Hq, int Hkv, int splits);
 cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* vcache, const int* positions,
                                           void* out, void* workspace, int B, int Hq, int Hkv, int D, int max_len,
-                                          int splits, float scale, float theta, bool pdl, cudaStream_t stream);
+                                          int splits, float scale, float theta, bool pdl, bool balance,
+                                          cudaStream_t stream);
+int decode_attn_balanced_splits(int B, int Hkv);
 
 // gate_up: [rows, 2F] (gate | up) -> out [rows, F] = silu(gate) * up
 cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cudaStream_t stream);

@@ -165,8 +165,10 @@ class LlamaTPDecoder:
         self.kcache = [torch.zeros(B, self.Hkv, max_len, D, dtype=dt, device=self.dev) for _ in range(cfg.layers)]
         self.vcache = [torch.zeros(B, self.Hkv, max_len, D, dtype=dt, device=self.dev) for _ in range(cfg.layers)]
         self.splits = self.attention_splits(B * self.Hkv, max_len)
+        # (the folded step has the rows cut by their lengths: how many partial rows that takes at most)
+        self.pieces = ops.decode_attn_balanced_splits(B, self.Hkv) if self.fold else 1
         # split partials + self-resetting arrival counters (zero before the first use)
-        self.workspace = torch.zeros(ops.decode_attn_fused_workspace_bytes(B, self.Hq, self.Hkv, self.splits),
+        self.workspace = torch.zeros(ops.decode_attn_fused_workspace_bytes(B, self.Hq, self.Hkv, max(self.splits, self.pieces)),
                                      dtype=torch.uint8, device=self.dev)
         self.scale = 1.0 / math.sqrt(D)
         self._graph = None
@@ -309,17 +311,18 @@ class LlamaTPDecoder:
     def _layers_folded(self):
         """One rank: five launches per layer.  x holds the residual stream times the next norm's weight, sumsq its
         sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
-        x, ss, eps, pdl = self.x, self.sumsq[0], self.cfg.eps, self.pdl
-        ops.norm_prep(self.embed, self.layers[0]["norm1"], self.residual, x, ss, ids=self.tokens)
+        x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.residual, self.pdl
+        ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=self.tokens)
         for li, L in enumerate(self.layers):
             ops.gemm_decode(x, L["wqkv"], self.qkv, pdl=pdl, sumsq=ss, eps=eps)
             ops.decode_attention_fused(self.qkv, self.kcache[li], self.vcache[li], self.positions, self.attn,
-                                       self.workspace, self.Hq, self.Hkv, self.splits, self.scale, self.cfg.rope_theta, pdl)
+                                       self.workspace, self.Hq, self.Hkv, self.pieces, self.scale, self.cfg.rope_theta,
+                                       pdl, balance=True)
             ss = self.sumsq[1]
-            ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=self.residual, norm_w=L["norm2"], sumsq_out=ss)
+            ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=res, norm_w=L["norm2"], sumsq_out=ss)
             ops.gemm_decode(x, L["wgu"], self.act, True, pdl=pdl, sumsq=ss, eps=eps)
             nxt = self.layers[li + 1]["norm1"] if li + 1 < self.cfg.layers else self.final_norm
-            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=self.residual, norm_w=nxt, sumsq_out=ss)
+            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=res, norm_w=nxt, sumsq_out=ss)
         ops.gemm_decode(x, self.lm_head, self.logits, pdl=pdl, sumsq=ss, eps=eps)
 
     def _layers(self, warm_up: bool):
