@@ -421,7 +421,7 @@ __device__ __forceinline__ void argmax_take(float v, int i, float& best, int& bi
   }
 }
 
-__global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* __restrict__ logits, int cols, int per,
+__global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* logits /* not restrict */, int cols, int per,
                                                 float* __restrict__ out_val, long long* __restrict__ out_idx,
                                                 float* __restrict__ pair, long long index_base,
                                                 unsigned int* __restrict__ workspace, const GreedyStep step) {

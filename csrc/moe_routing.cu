@@ -30,10 +30,12 @@
 namespace penny {
 namespace {
 
+// (What a predecessor writes is read through plain pointers: the compiler takes a const restrict pointer's loads for
+// constant and may move them above the dependency wait.)
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteWarps = kRouteThreads / 32;
 
-__device__ __forceinline__ void topk_of_token(const __nv_bfloat16* __restrict__ logits, int t, int experts, int topk, int* ids,
+__device__ __forceinline__ void topk_of_token(const __nv_bfloat16* logits, int t, int experts, int topk, int* ids,
                                               float* gates) {
   const __nv_bfloat16* row = logits + (size_t)t * experts;
   float best[kMoeMaxTopk];
@@ -73,7 +75,7 @@ __global__ void k_moe_topk(const __nv_bfloat16* __restrict__ logits, int tokens,
 }
 
 // logits != nullptr: ids and gates are made here first, topk of each token.
-__global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat16* __restrict__ logits, int topk, int* ids,
+__global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat16* logits, int topk, int* ids,
                                                               float* gates, int pairs, int experts,
                                                               int* __restrict__ order, int* __restrict__ expert_sorted,
                                                               int* __restrict__ send_off, int* __restrict__ counts) {
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(kRouteThreads) k_moe_tables(const __nv_bfloat1
 // One warp per 128 vectors (2 KB) of a row: a few tokens still fill the GPU, a lane has four loads in flight.
 constexpr int kRowVecs = 4 * 32;
 
-__global__ void __launch_bounds__(256) k_moe_gather(const uint4* __restrict__ x, const int* __restrict__ order, int pairs,
+__global__ void __launch_bounds__(256) k_moe_gather(const uint4* x, const int* order, int pairs,
                                                     int topk, int hv, uint4* __restrict__ rows, int* __restrict__ row_of_pair,
                                                     bool early) {
   if (early) pdl_launch_dependents();
@@ -156,8 +158,8 @@ __global__ void __launch_bounds__(256) k_moe_gather(const uint4* __restrict__ x,
     if (v0 + k * 32 < hv) rows[(size_t)i * hv + v0 + k * 32] = r[k];
 }
 
-__global__ void __launch_bounds__(256) k_moe_sum(const uint4* __restrict__ y, const int* __restrict__ row_of_pair,
-                                                 const float* __restrict__ gates, int tokens, int topk, int hv,
+__global__ void __launch_bounds__(256) k_moe_sum(const uint4* y, const int* row_of_pair,
+                                                 const float* gates, int tokens, int topk, int hv,
                                                  uint4* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
