@@ -62,6 +62,20 @@ PENNY_PLAN_HD int decode_choose_splits(int tiles, int num_kb, const int* capacit
   return best;
 }
 
+// The same for a linear between the folded norms of one rank's step, whose clusters were timed in its chain of launches:
+// up to five CTAs on three SMs.  The stream runs at 32 GB/s per CTA, so a sixth and a seventh range pay (down of 8 rows
+// 21.9 us in six, 20.7 in seven, 20.8 in eight; o 9.0 / 8.6 / 8.8) where the occupancy query, which wants whole
+// clusters per GPC, stops at six; 288 CTAs no longer run side by side (q / k / v 11.0 us in five, 16.1 in six).
+// Batch tiles of 128 rows hold one CTA per SM and keep to the rule above.
+PENNY_PLAN_HD int decode_choose_splits_chain(int tiles, int num_kb, int sms) {
+  int best = 1;
+  for (int s = 2; s <= kDecodeMaxSplits; ++s) {
+    if (num_kb / s < 6) break;
+    if ((long long)tiles * s * 3 <= (long long)sms * 5) best = s;
+  }
+  return best;
+}
+
 // capacity[] stand-in for a GPU of `sms` SMs in GPCs of `gpc_sms`, two CTAs per SM,
 // whole clusters per GPC (used by the CPU tests; the launcher uses the real figure).
 PENNY_PLAN_HD void decode_model_capacity(int sms, int gpc_sms, int* capacity) {

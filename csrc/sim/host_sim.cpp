@@ -343,6 +343,9 @@ int penny_decode_choose_splits(int tiles, int num_kb, int sms, int gpc_sms) {
   penny::sm100::decode_model_capacity(sms, gpc_sms, cap);
   return penny::sm100::decode_choose_splits(tiles, num_kb, cap);
 }
+int penny_decode_choose_splits_chain(int tiles, int num_kb, int sms) {
+  return penny::sm100::decode_choose_splits_chain(tiles, num_kb, sms);
+}
 // Tile -> (row block, column block) of the persistent GEMM kernels; pair_rank < 0
 // selects the single-CTA kernel, 0 / 1 the CTA of a pair.  Returns the number of
 // tiles (pair tiles) of the grid.

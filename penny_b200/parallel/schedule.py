@@ -131,3 +131,8 @@ def decode_choose_splits(tiles: int, num_kb: int, sms: int = 148, gpc_sms: int =
     """Cluster size the decode GEMM picks for `tiles` weight tiles of 128 rows and `num_kb` K steps of
     64 on a GPU of `sms` SMs in GPCs of `gpc_sms` (the launcher uses the occupancy API's figure)."""
     return sim_lib().penny_decode_choose_splits(tiles, num_kb, sms, gpc_sms)
+
+
+def decode_choose_splits_chain(tiles: int, num_kb: int, sms: int = 148) -> int:
+    """The same for the linears of one rank's step, between folded norms."""
+    return sim_lib().penny_decode_choose_splits_chain(tiles, num_kb, sms)
