@@ -76,15 +76,19 @@ void bind_gemm(py::module_& m) {
     int epi = silu_pairs ? penny::sm100::DECODE_EPI_SILU_PAIRS : penny::sm100::DECODE_EPI_PLAIN;
     if (residual.has_value()) {
       auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
-      TORCH_CHECK(!silu_pairs && bf16(*residual) && residual->sizes() == out.sizes() && residual->stride(0) == out.stride(0) &&
-                      norm_w.has_value() && bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == N &&
-                      sumsq_out.has_value() && sumsq_out->is_cuda() && sumsq_out->scalar_type() == at::kFloat &&
-                      sumsq_out->is_contiguous() && N % 128 == 0 && sumsq_out->numel() == N / 128 * B,
-                  "gemm_decode: residual like out, contiguous norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
+      TORCH_CHECK(epi == penny::sm100::DECODE_EPI_PLAIN && N % 128 == 0 && bf16(*residual) && residual->sizes() == out.sizes() &&
+                      residual->stride(0) == out.stride(0) && norm_w.has_value() == sumsq_out.has_value(),
+                  "gemm_decode: residual like out, rows of w a multiple of 128; norm_w and sumsq_out together");
       epi = penny::sm100::DECODE_EPI_RESIDUAL;
       fold.residual = residual->data_ptr();
-      fold.norm_w = norm_w->data_ptr();
-      fold.sumsq_out = sumsq_out->data_ptr<float>();
+      if (norm_w.has_value()) {
+        TORCH_CHECK(bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == N && sumsq_out->is_cuda() &&
+                        sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
+                        sumsq_out->numel() == N / 128 * B,
+                    "gemm_decode: contiguous norm_w [rows of w], sumsq_out [rows of w / 128, rows]");
+        fold.norm_w = norm_w->data_ptr();
+        fold.sumsq_out = sumsq_out->data_ptr<float>();
+      }
     }
     cudaError_t rc = penny::sm100::launch_gemm_decode(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), (int)B, (int)N, (int)K, (int)x.stride(0), (int)w.stride(0),

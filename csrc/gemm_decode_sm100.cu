@@ -28,9 +28,10 @@
 //   * warp 0: TMA producer, warp 1: MMA issuer, warps 2-9: epilogue.  Every wait
 //     is bounded; TMEM is always freed.
 //
-// Epilogues: plain store, or silu(gate) * up for a gate/up weight whose rows are
+// Epilogues: plain store; silu(gate) * up for a gate/up weight whose rows are
 // interleaved in blocks of 64 (tile = 64 gate rows + the 64 up rows of the same
-// features; out is [B, N / 2]).
+// features; out is [B, N / 2]); residual add with what the next norm needs
+// (DecodeFold).
 //
 // The reference has no GEMM of any kind (it is a collectives library used
 // inside vLLM / SGLang, README.md:20-33); this kernel is what lets the TP-decode
@@ -312,7 +313,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (j < hi) r_next = *reinterpret_cast<const uint4*>(a.residual + (size_t)(row0 + j) * a.ldo + n0);
     };
     if (resid) {
-      nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + n0));
+      if (a.norm_w != nullptr) nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + n0));
       load_residual(lo + tid / groups);
     }
     bool ok = mbar_wait_abortable(tmem_full, 0u, s_abort);
@@ -412,6 +413,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           }
           const size_t off = (size_t)(row0 + j) * a.ldo + n0;
           *reinterpret_cast<uint4*>(a.residual + off) = make_uint4(zo[0], zo[1], zo[2], zo[3]);
+          if (a.norm_w == nullptr) continue;
           *reinterpret_cast<uint4*>(a.out + off) = make_uint4(ho[0], ho[1], ho[2], ho[3]);
           const unsigned half = 0xffffu << (lane & 16);  // the sixteen row groups of this column
 #pragma unroll
@@ -593,10 +595,10 @@ cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, i
   if (B <= 0 || B > kDecodeMaxBatch || N <= 0 || K <= 0 || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0)
     return cudaErrorInvalidValue;
   if (push != nullptr && B > 128) return cudaErrorInvalidValue;  // the owners' receive lines cover one slab
-  if (epi != DECODE_EPI_PLAIN && epi != DECODE_EPI_SILU_PAIRS && epi != DECODE_EPI_RESIDUAL) return cudaErrorInvalidValue;
+  if (epi < DECODE_EPI_PLAIN || epi > DECODE_EPI_RESIDUAL) return cudaErrorInvalidValue;
   if (epi == DECODE_EPI_RESIDUAL &&
       (N % kBlockM != 0 || ldo % 8 != 0 || push != nullptr || fold == nullptr || fold->residual == nullptr ||
-       fold->norm_w == nullptr || fold->sumsq_out == nullptr ||
+       (fold->norm_w != nullptr && (out == nullptr || fold->sumsq_out == nullptr)) ||
        ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(fold->residual) |
          reinterpret_cast<uintptr_t>(fold->norm_w)) & 15u) != 0))
     return cudaErrorInvalidValue;

@@ -26,7 +26,7 @@ struct DecodeFold {
   int scale_parts;
   float eps;
   void* residual;      // DECODE_EPI_RESIDUAL: [B, N], ldo
-  const void* norm_w;  // [N]
+  const void* norm_w;  // [N]; null: only the residual add (out and sumsq_out unused)
   float* sumsq_out;    // [N / 128][B]
 };
 

@@ -22,12 +22,16 @@ def test_residual_epilogue(shape, splits):
     B, N, K = shape
     x, w, _ = _inputs(B, N, K, 1)
     res, norm_w = torch.randn(B, N, device="cuda").bfloat16(), torch.rand(N, device="cuda").bfloat16()
+    res0 = res.clone()
     z = res.double() + x.double() @ w.double().t()
     out, ss = torch.empty_like(res), torch.full((N // 128, B), float("nan"), device="cuda")
     ops.gemm_decode(x, w, out, False, splits, residual=res, norm_w=norm_w, sumsq_out=ss)
     assert ops.gemm_error() == 0
     # fp32 sums of up to 4096 products of size K ** -0.5: 1e-5 at most; then one bf16 rounding (2 ** -9)
     tol = z.abs() * 2.0 ** -8 + 1e-4
+    alone = res0.clone()
+    ops.gemm_decode(x, w, torch.empty_like(res), False, splits, residual=alone)  # without a norm behind it
+    assert torch.equal(alone, res)
     assert ((res.double() - z).abs() <= tol).all()
     assert ((out.double() - z * norm_w.double()).abs() <= tol * norm_w.double() + 1e-6).all()
     want = z.square().view(B, N // 128, 128).sum(-1).t()
