@@ -438,11 +438,37 @@ __global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* logits /* n
   if ((reinterpret_cast<uintptr_t>(row + c0) & 15u) == 0) {
     const int nvec = (c1 - c0) / 8;
     const uint4* vp = reinterpret_cast<const uint4*>(row + c0);
-    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-      const uint4 q = vp[i];
-      const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
+    // Four vectors at a time, their largest value by packed maxima (which, like the comparisons, pass over NaN); only one
+    // that beats the best is looked for.  A comparison and a choice of index per element were 0.9 us per vector and
+    // thread: 34 us for 256 rows of 128256 logits, 11 for 64.
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += 4 * blockDim.x) {
+      uint4 q[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) argmax_take(bf2f(e[k]), c0 + i * 8 + k, best, bi);
+      for (int u = 0; u < 4; ++u) q[u] = vp[min(i0 + u * (int)blockDim.x, nvec - 1)];  // (past the end: the last one again)
+      __nv_bfloat162 top = *reinterpret_cast<const __nv_bfloat162*>(&q[0].x);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) top = __hmax2(top, e[k]);
+      }
+      const float m = bf2f(__hmax(top.x, top.y));
+      if (m > best || (m == best && bi == 0x7fffffff)) {
+        bool found = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q[u]);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float v = bf2f(e[k]);
+            if (!found && v == m) {
+              found = true;
+              best = v;
+              bi = c0 + min(i0 + u * (int)blockDim.x, nvec - 1) * 8 + k;
+            }
+          }
+        }
+      }
     }
     for (int i = c0 + nvec * 8 + threadIdx.x; i < c1; i += blockDim.x) argmax_take(bf2f(row[i]), i, best, bi);
   } else {
