@@ -56,14 +56,16 @@ void bind_decode(py::module_& m) {
     ck(launch_rope_rows(qkv.data_ptr(), (int)qkv.size(0), (int)Hq, (int)Hkv, (int)D, (int)pos0, (float)theta, cur()),
        "rope_rows");
   });
-  // ids [rows] int64: the rows of src (an embedding table) that become the stream
+  // ids [rows] int64: the rows of src (an embedding table) that become the stream; in pinned host memory they are read
+  // from there when the kernel runs
   m.def("norm_prep", [](at::Tensor src, at::Tensor norm_w, at::Tensor residual, at::Tensor out, at::Tensor sumsq,
                         c10::optional<at::Tensor> ids) {
     need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2 && residual.dim() == 2,
          "norm_prep expects contiguous bf16 CUDA tensors");
     const int64_t rows = ids.has_value() ? ids->numel() : src.size(0), H = src.size(1);
     if (ids.has_value())
-      need(ids->is_cuda() && ids->scalar_type() == at::kLong && ids->is_contiguous(), "norm_prep: ids must be int64 CUDA");
+      need((ids->is_cuda() || ids->is_pinned()) && ids->scalar_type() == at::kLong && ids->is_contiguous(),
+           "norm_prep: ids must be int64, CUDA or pinned");
     need(residual.size(0) == rows && residual.size(1) == H && out.sizes() == residual.sizes() && norm_w.numel() == H &&
              sumsq.is_cuda() && sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous() && sumsq.numel() == rows,
          "norm_prep shapes");
@@ -134,7 +136,7 @@ void bind_decode(py::module_& m) {
   m.def("argmax_rows", [](at::Tensor logits, at::Tensor out_val, at::Tensor out_idx, int64_t index_base,
                           c10::optional<at::Tensor> workspace, c10::optional<at::Tensor> pair,
                           c10::optional<at::Tensor> next_tokens, c10::optional<at::Tensor> tokens,
-                          c10::optional<at::Tensor> positions) {
+                          c10::optional<at::Tensor> positions, c10::optional<at::Tensor> host_tokens) {
     need(bf16_cuda(logits) && logits.dim() == 2, "argmax_rows expects [rows, cols] bf16");
     const int64_t rows = logits.size(0);
     need(out_val.is_cuda() && out_val.scalar_type() == at::kFloat && out_val.numel() == rows, "out_val [rows] fp32");
@@ -159,7 +161,12 @@ void bind_decode(py::module_& m) {
                positions->scalar_type() == at::kInt && next_tokens->numel() == rows && tokens->numel() == rows &&
                positions->numel() == rows && next_tokens->is_contiguous() && tokens->is_contiguous() && positions->is_contiguous(),
            "next_tokens / tokens [rows] int64, positions [rows] int32, together");
-      step = {(long long*)next_tokens->data_ptr<int64_t>(), (long long*)tokens->data_ptr<int64_t>(), positions->data_ptr<int>()};
+      step = {(long long*)next_tokens->data_ptr<int64_t>(), (long long*)tokens->data_ptr<int64_t>(), positions->data_ptr<int>(), nullptr};
+      if (host_tokens.has_value()) {
+        need(host_tokens->is_pinned() && host_tokens->scalar_type() == at::kLong && host_tokens->is_contiguous() &&
+                 host_tokens->numel() == rows, "host_tokens: pinned [rows] int64");
+        step.host_tokens = (long long*)host_tokens->data_ptr<int64_t>();
+      }
     }
     const at::cuda::OptionalCUDAGuard guard(logits.device());
     ck(launch_argmax(logits.data_ptr(), (int)rows, (int)logits.size(1), out_val.data_ptr<float>(),
@@ -167,7 +174,7 @@ void bind_decode(py::module_& m) {
        "argmax_rows");
   }, py::arg("logits"), py::arg("out_val"), py::arg("out_idx"), py::arg("index_base"),
      py::arg("workspace") = py::none(), py::arg("pair") = py::none(), py::arg("next_tokens") = py::none(),
-     py::arg("tokens") = py::none(), py::arg("positions") = py::none());
+     py::arg("tokens") = py::none(), py::arg("positions") = py::none(), py::arg("host_tokens") = py::none());
   // Expert-parallel MoE routing on the device (csrc/moe_routing.cu)
   m.def("moe_route", [](at::Tensor logits, int64_t topk) {
     need(bf16_cuda(logits) && logits.dim() == 2, "moe_route expects [tokens, experts] bf16");

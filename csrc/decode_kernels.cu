@@ -531,6 +531,7 @@ __global__ void __launch_bounds__(256) k_argmax(const __nv_bfloat16* logits /* n
     }
     if (step.next_tokens != nullptr) {
       step.next_tokens[r] = step.tokens[r] = index_base + bi;
+      if (step.host_tokens != nullptr) step.host_tokens[r] = index_base + bi;
       step.positions[r] += 1;
     }
   }

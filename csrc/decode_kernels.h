@@ -56,6 +56,7 @@ cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cud
 struct GreedyStep {
   long long *next_tokens, *tokens;  // [rows]; next_tokens == nullptr: none of this
   int* positions;
+  long long* host_tokens;  // null, or pinned host memory that takes the winners too
 };
 size_t argmax_workspace_bytes(int rows);
 cudaError_t launch_argmax(const void* logits, int rows, int cols, float* out_val, long long* out_idx, float* pair,

@@ -171,7 +171,7 @@ class LlamaTPDecoder:
         self.workspace = torch.zeros(ops.decode_attn_fused_workspace_bytes(B, self.Hq, self.Hkv, max(self.splits, self.pieces)),
                                      dtype=torch.uint8, device=self.dev)
         self.scale = 1.0 / math.sqrt(D)
-        self._graph = None
+        self._graph = self._host_graph = None
         self._host_in = torch.zeros(B, dtype=torch.int64).pin_memory()
         self._host_out = torch.zeros(B, dtype=torch.int64).pin_memory()
         # kernels of this library launched per step (the few torch glue ops excluded)
@@ -308,11 +308,11 @@ class LlamaTPDecoder:
         for r in range(0, B, 1024):
             ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, 0, push)
 
-    def _layers_folded(self):
+    def _layers_folded(self, tokens):
         """One rank: five launches per layer.  x holds the residual stream times the next norm's weight, sumsq its
         sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
         x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.residual, self.pdl
-        ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=self.tokens)
+        ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
         for li, L in enumerate(self.layers):
             ops.gemm_decode(x, L["wqkv"], self.qkv, pdl=pdl, sumsq=ss, eps=eps)
             ops.decode_attention_fused(self.qkv, self.kcache[li], self.vcache[li], self.positions, self.attn,
@@ -361,9 +361,9 @@ class LlamaTPDecoder:
             if warm_up or not self.own_head:
                 torch.matmul(self.x, self.lm_head.t(), out=self.logits)
 
-    def _step_impl(self, warm_up: bool = False, separate: bool = False):
+    def _step_impl(self, warm_up: bool = False, separate: bool = False, host: bool = False):
         if self.fold and not separate:
-            self._layers_folded()
+            self._layers_folded(self._host_in if host else self.tokens)
         else:
             self._layers(warm_up)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
@@ -372,7 +372,7 @@ class LlamaTPDecoder:
         # (one rank: the winners are the tokens, the same kernel hands them on)
         if self.world == 1:
             ops.argmax_rows(self.logits, self.max_val, self.max_idx, 0, self.argmax_ws, None, self.next_tokens, self.tokens,
-                            self.positions)
+                            self.positions, self._host_out if host else None)
         else:
             ops.argmax_rows(self.logits, self.max_val, self.max_idx, self.rank * self.V, self.argmax_ws, self.pair)
             if self.backend == "nccl":
@@ -398,6 +398,12 @@ class LlamaTPDecoder:
             self._graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self._graph):
                 self._step_impl()
+            if self.fold:
+                # step()'s own graph: the first kernel reads the caller's tokens from pinned memory, the last one leaves
+                # the next ones there.  Two copies around the graph were 10 us of a step's 20 outside its layers.
+                self._host_graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(self._host_graph):
+                    self._step_impl(host=True)
             torch.cuda.synchronize()
         self.positions.copy_(saved[0])
         self.tokens.copy_(saved[1])
@@ -414,9 +420,12 @@ class LlamaTPDecoder:
         next token of every sequence as a CPU tensor.  Host -> device copy of the
         inputs from pinned memory, the step, device -> host read of the result."""
         self._host_in.copy_(tokens)
-        self.tokens.copy_(self._host_in, non_blocking=True)
-        self.step_device()
-        self._host_out.copy_(self.next_tokens, non_blocking=True)
+        if self._host_graph is not None:
+            self._host_graph.replay()
+        else:
+            self.tokens.copy_(self._host_in, non_blocking=True)
+            self.step_device()
+            self._host_out.copy_(self.next_tokens, non_blocking=True)
         torch.cuda.current_stream().synchronize()
         return self._host_out
 
