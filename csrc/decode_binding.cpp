@@ -56,11 +56,12 @@ void bind_decode(py::module_& m) {
     ck(launch_rope_rows(qkv.data_ptr(), (int)qkv.size(0), (int)Hq, (int)Hkv, (int)D, (int)pos0, (float)theta, cur()),
        "rope_rows");
   });
-  // ids [rows] int64: the rows of src (an embedding table) that become the stream; in pinned host memory they are read
+  // residual: bf16 or fp32.  ids [rows] int64: the rows of src (an embedding table) that become the stream; in pinned host memory they are read
   // from there when the kernel runs
   m.def("norm_prep", [](at::Tensor src, at::Tensor norm_w, at::Tensor residual, at::Tensor out, at::Tensor sumsq,
                         c10::optional<at::Tensor> ids) {
-    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(residual) && bf16_cuda(out) && src.dim() == 2 && residual.dim() == 2,
+    need(bf16_cuda(src) && bf16_cuda(norm_w) && bf16_cuda(out) &&
+             (bf16_cuda(residual) || (residual.is_cuda() && residual.scalar_type() == at::kFloat && residual.is_contiguous())) && src.dim() == 2 && residual.dim() == 2,
          "norm_prep expects contiguous bf16 CUDA tensors");
     const int64_t rows = ids.has_value() ? ids->numel() : src.size(0), H = src.size(1);
     if (ids.has_value())
@@ -73,7 +74,7 @@ void bind_decode(py::module_& m) {
       need(((uintptr_t)t->data_ptr() & 15) == 0, "norm_prep: 16-byte aligned tensors");
     const at::cuda::OptionalCUDAGuard guard(src.device());
     ck(launch_norm_prep(src.data_ptr(), ids.has_value() ? (const long long*)ids->data_ptr<int64_t>() : nullptr, src.size(0),
-                        norm_w.data_ptr(), residual.data_ptr(), out.data_ptr(), sumsq.data_ptr<float>(), (int)rows, (int)H,
+                        norm_w.data_ptr(), residual.data_ptr(), residual.scalar_type() == at::kFloat, out.data_ptr(), sumsq.data_ptr<float>(), (int)rows, (int)H,
                         cur()),
        "norm_prep");
   }, py::arg("src"), py::arg("norm_w"), py::arg("residual"), py::arg("out"), py::arg("sumsq"), py::arg("ids") = py::none());

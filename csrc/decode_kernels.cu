@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(320) k_rope_rows_vec(__nv_bfloat16* __restrict
 // kernel, as in torch.index_select).
 __global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restrict__ src, const long long* __restrict__ ids,
                                                    long long src_rows,
-                                                   const __nv_bfloat16* __restrict__ norm_w,
-                                                   __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out,
+                                                   const __nv_bfloat16* __restrict__ norm_w, void* __restrict__ residual,
+                                                   bool residual_fp32, __nv_bfloat16* __restrict__ out,
                                                    float* __restrict__ sumsq, int H) {
   __shared__ float s_part[16];
   pdl_launch_dependents();
@@ -157,7 +157,13 @@ __global__ void __launch_bounds__(512) k_norm_prep(const __nv_bfloat16* __restri
       ss += a * a + b * b;
       oe[k] = pack2(a * bf2f(ne[k].x), b * bf2f(ne[k].y));
     }
-    reinterpret_cast<uint4*>(residual + r * H)[v] = x;
+    if (residual_fp32) {
+      float4* rp = reinterpret_cast<float4*>(residual) + (r * H / 8 + v) * 2;
+      rp[0] = make_float4(bf2f(xe[0].x), bf2f(xe[0].y), bf2f(xe[1].x), bf2f(xe[1].y));
+      rp[1] = make_float4(bf2f(xe[2].x), bf2f(xe[2].y), bf2f(xe[3].x), bf2f(xe[3].y));
+    } else {
+      (reinterpret_cast<uint4*>(residual) + r * H / 8)[v] = x;
+    }
     reinterpret_cast<uint4*>(out + r * H)[v] = o;
   }
 #pragma unroll
@@ -586,13 +592,13 @@ cudaError_t launch_rope_rows(void* qkv, int T, int Hq, int Hkv, int D, int pos0,
 }
 
 cudaError_t launch_norm_prep(const void* src, const long long* ids, long long src_rows, const void* norm_w, void* residual,
-                             void* out, float* sumsq, int rows, int H, cudaStream_t stream) {
+                             bool residual_fp32, void* out, float* sumsq, int rows, int H, cudaStream_t stream) {
   if (rows < 1 || H < 8 || H % 8 != 0) return cudaErrorInvalidValue;
   const int threads = std::min(512, (H / 8 + 31) / 32 * 32);
   // The one launch of the stack that starts when everything before it has completed: the linear behind it loads
   // weights before its own wait, and a weight may have been written by the kernel before the stack.
   return launch_kernel_ex(k_norm_prep, dim3((unsigned)rows), dim3((unsigned)threads), 0, stream, false, 1,
-                          (const __nv_bfloat16*)src, ids, src_rows, (const __nv_bfloat16*)norm_w, (__nv_bfloat16*)residual,
+                          (const __nv_bfloat16*)src, ids, src_rows, (const __nv_bfloat16*)norm_w, residual, residual_fp32,
                           (__nv_bfloat16*)out, sumsq, H);
 }
 

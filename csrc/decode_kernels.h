@@ -20,7 +20,7 @@ cudaError_t launch_rope_rows(void* qkv, int T, int Hq, int Hkv, int D, int pos0,
 // first linear of a stack with norms in the GEMM epilogues starts from.  Rows of H bf16, H % 8 == 0, all
 // pointers 16-byte aligned.
 cudaError_t launch_norm_prep(const void* src, const long long* ids, long long src_rows, const void* norm_w, void* residual,
-                             void* out, float* sumsq, int rows, int H, cudaStream_t stream);
+                             bool residual_fp32, void* out, float* sumsq, int rows, int H, cudaStream_t stream);
 
 // Scratch the split-KV attention needs: per (row, head, split) an unnormalised
 // fp32 output row plus (max, sum).

@@ -39,11 +39,13 @@ void bind_gemm(py::module_& m) {
   // range); the K ranges of a tile are reduced inside a thread-block cluster through distributed shared
   // memory.  pdl: may start (and load w) while the previous kernel on the stream still runs, so w must not
   // be written by that kernel.  silu_pairs: w's rows are blocks of 64 gate + 64 up rows and out is
-  // [B, N / 2] = silu(gate) * up.  sumsq, residual, norm_w, sumsq_out: as in gemm_tile below.
+  // [B, N / 2] = silu(gate) * up.  sumsq, residual, norm_w, sumsq_out: as in gemm_tile below;
+  // the residual may be fp32, stream_out then takes the sum in bf16 as well.
   m.def("gemm_decode", [](at::Tensor x, at::Tensor w, at::Tensor out, bool silu_pairs, int64_t splits, bool pdl,
                           int64_t l2_budget, int64_t smem_kb, c10::optional<at::Tensor> push,
                           c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
-                          c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out) {
+                          c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out,
+                          c10::optional<at::Tensor> stream_out) {
     TORCH_CHECK(x.is_cuda() && w.is_cuda() && out.is_cuda(), "gemm_decode: CUDA tensors");
     TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
                     out.scalar_type() == at::kBFloat16, "gemm_decode: bf16 only");
@@ -76,11 +78,18 @@ void bind_gemm(py::module_& m) {
     int epi = silu_pairs ? penny::sm100::DECODE_EPI_SILU_PAIRS : penny::sm100::DECODE_EPI_PLAIN;
     if (residual.has_value()) {
       auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
-      TORCH_CHECK(epi == penny::sm100::DECODE_EPI_PLAIN && N % 128 == 0 && bf16(*residual) && residual->sizes() == out.sizes() &&
+      fold.residual_fp32 = residual->scalar_type() == at::kFloat;
+      TORCH_CHECK(epi == penny::sm100::DECODE_EPI_PLAIN && N % 128 == 0 && residual->is_cuda() && residual->stride(-1) == 1 &&
+                      (fold.residual_fp32 || bf16(*residual)) && residual->sizes() == out.sizes() &&
                       residual->stride(0) == out.stride(0) && norm_w.has_value() == sumsq_out.has_value(),
                   "gemm_decode: residual like out, rows of w a multiple of 128; norm_w and sumsq_out together");
       epi = penny::sm100::DECODE_EPI_RESIDUAL;
       fold.residual = residual->data_ptr();
+      if (stream_out.has_value()) {
+        TORCH_CHECK(fold.residual_fp32 && bf16(*stream_out) && stream_out->sizes() == out.sizes() &&
+                        stream_out->stride(0) == out.stride(0), "gemm_decode: stream_out like out, beside an fp32 residual");
+        fold.stream_out = stream_out->data_ptr();
+      }
       if (norm_w.has_value()) {
         TORCH_CHECK(bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == N && sumsq_out->is_cuda() &&
                         sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
@@ -99,7 +108,7 @@ void bind_gemm(py::module_& m) {
   }, py::arg("x"), py::arg("w"), py::arg("out"), py::arg("silu_pairs") = false, py::arg("splits") = 0,
      py::arg("pdl") = true, py::arg("l2_budget") = -1, py::arg("smem_kb") = 0, py::arg("push") = py::none(),
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
-     py::arg("sumsq_out") = py::none());
+     py::arg("sumsq_out") = py::none(), py::arg("stream_out") = py::none());
   // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
   // rows before its up rows, out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
   // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq

@@ -99,7 +99,9 @@ struct DecodeArgs {
   const float* scale_sumsq;
   int scale_parts;
   float inv_width, eps;
-  __nv_bfloat16* residual;
+  char* residual;
+  int res_bytes;  // of an element of the residual: 2 (bf16) or 4 (fp32)
+  __nv_bfloat16* stream_out;
   const __nv_bfloat16* norm_w;
   float* sumsq_out;
 };
@@ -308,9 +310,13 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int groups = silu ? 8 : 16;
     const int g = tid % groups, n0 = tile * (silu ? kBlockM / 2 : kBlockM) + g * 8;
     // RESIDUAL: the stream's rows travel an item ahead, the first ones and the norm's weight under the product
-    uint4 r_next = make_uint4(0, 0, 0, 0), nw = r_next;
+    uint4 r_next[2], nw = make_uint4(0, 0, 0, 0);
+    r_next[0] = r_next[1] = nw;
     auto load_residual = [&](int j) {
-      if (j < hi) r_next = *reinterpret_cast<const uint4*>(a.residual + (size_t)(row0 + j) * a.ldo + n0);
+      if (j >= hi) return;
+      const uint4* p = reinterpret_cast<const uint4*>(a.residual + ((size_t)(row0 + j) * a.ldo + n0) * a.res_bytes);
+      r_next[0] = p[0];
+      if (a.res_bytes == 4) r_next[1] = p[1];
     };
     if (resid) {
       if (a.norm_w != nullptr) nw = __ldg(reinterpret_cast<const uint4*>(a.norm_w + n0));
@@ -398,21 +404,33 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] *= sc;
         if (resid) {
-          const uint32_t rw[4] = {r_next.x, r_next.y, r_next.z, r_next.w}, ww[4] = {nw.x, nw.y, nw.z, nw.w};
+          const uint32_t rw[8] = {r_next[0].x, r_next[0].y, r_next[0].z, r_next[0].w, r_next[1].x, r_next[1].y, r_next[1].z, r_next[1].w};
+          const uint32_t ww[4] = {nw.x, nw.y, nw.z, nw.w};
+          const bool wide = a.res_bytes == 4;
           load_residual(j + kDecEpiThreads / groups);
           uint32_t zo[4], ho[4];
           float ss = 0.f;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const float z0 = v[2 * k] + __uint_as_float(rw[k] << 16);
-            const float z1 = v[2 * k + 1] + __uint_as_float(rw[k] & 0xffff0000u);
+            const float z0 = v[2 * k] + __uint_as_float(wide ? rw[2 * k] : rw[k] << 16);
+            const float z1 = v[2 * k + 1] + __uint_as_float(wide ? rw[2 * k + 1] : rw[k] & 0xffff0000u);
+            v[2 * k] = z0;
+            v[2 * k + 1] = z1;
             ss += z0 * z0 + z1 * z1;
             zo[k] = pack_bf16x2(__float_as_uint(z0), __float_as_uint(z1));
             ho[k] = pack_bf16x2(__float_as_uint(z0 * __uint_as_float(ww[k] << 16)),
                                 __float_as_uint(z1 * __uint_as_float(ww[k] & 0xffff0000u)));
           }
           const size_t off = (size_t)(row0 + j) * a.ldo + n0;
-          *reinterpret_cast<uint4*>(a.residual + off) = make_uint4(zo[0], zo[1], zo[2], zo[3]);
+          uint4* rp = reinterpret_cast<uint4*>(a.residual + off * a.res_bytes);
+          const uint4 zb = make_uint4(zo[0], zo[1], zo[2], zo[3]);
+          if (wide) {
+            rp[0] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+            rp[1] = make_uint4(__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7]));
+            if (a.stream_out != nullptr) *reinterpret_cast<uint4*>(a.stream_out + off) = zb;
+          } else {
+            rp[0] = zb;
+          }
           if (a.norm_w == nullptr) continue;
           *reinterpret_cast<uint4*>(a.out + off) = make_uint4(ho[0], ho[1], ho[2], ho[3]);
           const unsigned half = 0xffffu << (lane & 16);  // the sixteen row groups of this column
@@ -553,7 +571,9 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
   a.scale_parts = f.scale_parts;
   a.inv_width = 1.f / (float)K;
   a.eps = f.eps;
-  a.residual = reinterpret_cast<__nv_bfloat16*>(f.residual);
+  a.residual = reinterpret_cast<char*>(f.residual);
+  a.res_bytes = f.residual_fp32 ? 4 : 2;
+  a.stream_out = reinterpret_cast<__nv_bfloat16*>(f.stream_out);
   a.norm_w = reinterpret_cast<const __nv_bfloat16*>(f.norm_w);
   a.sumsq_out = f.sumsq_out;
   // ring depth: what fits next to the receive area in ~106 KB (two CTAs per SM, of this kernel or the next:
@@ -600,7 +620,7 @@ cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, i
       (N % kBlockM != 0 || ldo % 8 != 0 || push != nullptr || fold == nullptr || fold->residual == nullptr ||
        (fold->norm_w != nullptr && (out == nullptr || fold->sumsq_out == nullptr)) ||
        ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(fold->residual) |
-         reinterpret_cast<uintptr_t>(fold->norm_w)) & 15u) != 0))
+         reinterpret_cast<uintptr_t>(fold->stream_out) | reinterpret_cast<uintptr_t>(fold->norm_w)) & 15u) != 0))
     return cudaErrorInvalidValue;
   if (epi == DECODE_EPI_SILU_PAIRS && N % kBlockM != 0) return cudaErrorInvalidValue;
   if ((N + kBlockM - 1) / kBlockM > 65535) return cudaErrorInvalidValue;

@@ -25,7 +25,9 @@ struct DecodeFold {
   const float* scale_sumsq;
   int scale_parts;
   float eps;
-  void* residual;      // DECODE_EPI_RESIDUAL: [B, N], ldo
+  void* residual;      // DECODE_EPI_RESIDUAL: [B, N], ldo; bf16, or with residual_fp32 fp32
+  bool residual_fp32;
+  void* stream_out;    // residual_fp32: null, or [B, N], ldo: the sum once more in bf16
   const void* norm_w;  // [N]; null: only the residual add (out and sumsq_out unused)
   float* sumsq_out;    // [N / 128][B]
 };

@@ -153,6 +153,10 @@ class LlamaTPDecoder:
         self.part = self.parts[0]
         if self.fold:
             self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
+            # The folded step's stream stays fp32 from layer to layer (the residual buffer takes it in bf16 at the end): 16
+            # roundings fewer.  Distance of 8 random layers from 64 bits: 0.018 with norms of their own, 0.0145 folded,
+            # 0.012 with this, for 0.3 us a layer.
+            self.stream = torch.empty(B, H, dtype=torch.float32, device=self.dev)
         self.gu = buf(B, 2 * self.F) if linears == "cublas" else None
         self.act = buf(B, self.F)
         self.logits = buf(B, self.V)
@@ -311,7 +315,7 @@ class LlamaTPDecoder:
     def _layers_folded(self, tokens):
         """One rank: five launches per layer.  x holds the residual stream times the next norm's weight, sumsq its
         sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
-        x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.residual, self.pdl
+        x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.stream, self.pdl
         ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
         for li, L in enumerate(self.layers):
             ops.gemm_decode(x, L["wqkv"], self.qkv, pdl=pdl, sumsq=ss, eps=eps)
@@ -321,8 +325,10 @@ class LlamaTPDecoder:
             ss = self.sumsq[1]
             ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=res, norm_w=L["norm2"], sumsq_out=ss)
             ops.gemm_decode(x, L["wgu"], self.act, True, pdl=pdl, sumsq=ss, eps=eps)
-            nxt = self.layers[li + 1]["norm1"] if li + 1 < self.cfg.layers else self.final_norm
-            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=res, norm_w=nxt, sumsq_out=ss)
+            last = li + 1 == self.cfg.layers
+            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=res, sumsq_out=ss,
+                            norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
+                            stream_out=self.residual if last else None)
         ops.gemm_decode(x, self.lm_head, self.logits, pdl=pdl, sumsq=ss, eps=eps)
 
     def _layers(self, warm_up: bool):

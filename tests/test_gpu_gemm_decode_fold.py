@@ -36,6 +36,11 @@ def test_residual_epilogue(shape, splits):
     assert ((out.double() - z * norm_w.double()).abs() <= tol * norm_w.double() + 1e-6).all()
     want = z.square().view(B, N // 128, 128).sum(-1).t()
     torch.testing.assert_close(ss.double(), want, rtol=1e-4, atol=1e-4)
+    # the stream in fp32, with a copy in bf16
+    wide, copy, out2, ss2 = res0.float(), torch.empty_like(res), torch.empty_like(out), torch.empty_like(ss)
+    ops.gemm_decode(x, w, out2, False, splits, residual=wide, norm_w=norm_w, sumsq_out=ss2, stream_out=copy)
+    assert bool(((wide.double() - z).abs() <= 1e-4).all()) and torch.equal(copy, wide.bfloat16())
+    assert torch.equal(copy, res) and torch.equal(out2, out) and torch.equal(ss2, ss)
 
 
 @pytest.mark.parametrize("shape", SHAPES)
@@ -64,5 +69,8 @@ def test_embedding_rows_start_the_stream():
     ss = torch.empty(1, 5, device="cuda")
     ops.norm_prep(table, w, res, out, ss, ids=ids)
     want = table[ids]
+    wide = torch.empty(5, 512, device="cuda")
+    ops.norm_prep(table, w, wide, out, ss, ids=ids)
+    assert torch.equal(wide, want.float())
     assert torch.equal(res, want) and torch.equal(out, (want.float() * w.float()).bfloat16())
     torch.testing.assert_close(ss[0], want.float().square().sum(-1), rtol=1e-5, atol=0)
