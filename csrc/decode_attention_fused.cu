@@ -463,7 +463,11 @@ cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* v
   int slots = 0, extra = 0;
   if (balance) {
     slots = balance_slots(items, device_sms());
-    extra = balance_extra(items, slots);
+    // (no more than the cache's length allows: the launch behind this one begins when every CTA of this one has begun, so
+    // CTAs without a piece keep its weights waiting)
+    extra = (int)std::min<long long>(balance_extra(items, slots),
+                                     (long long)items * (std::min(kMaxPieces, std::max(1, (max_len - 1) / kMinPiece)) - 1));
+    if (extra == 0) slots = 0;
     // (a workspace for fewer pieces than the cut may take: whole rows)
     if (slots == 0 || (long long)items * (splits - 1) < extra) slots = 0, splits = 1;
   }
