@@ -113,12 +113,12 @@ struct DecodeCfg {
   static constexpr int kStageBytes = kWBytes + kXBytes;
   static constexpr int kTmemCols = BT < 32 ? 32 : BT;
   static constexpr int kBarBytes = 256;
-  // the peers' partials of this CTA's column slice: [splits - 1][slice][128 rows] fp32
-  __host__ __device__ static size_t recv_floats(int splits) { return decode_recv_floats(BT, splits); }
+  // the peers' partials of this CTA's column slice: [splits - 1][slice][128 rows] fp32, for the rows that a slab has
+  __host__ __device__ static size_t recv_floats(int splits, int B) { return decode_recv_floats(B < BT ? B : BT, splits); }
   // The ring doubles as the [BT][128] fp32 staging area of the epilogue, so it is never smaller than that.
   __host__ __device__ static int min_stages() { return (BT * kBlockM * 4 + kStageBytes - 1) / kStageBytes; }
-  static size_t smem_bytes(int stages, int splits) {
-    return (size_t)stages * kStageBytes + recv_floats(splits) * 4 + 1024 /*alignment*/ + kBarBytes + BT * 4 /*s_scale*/;
+  static size_t smem_bytes(int stages, int splits, int B = BT) {
+    return (size_t)stages * kStageBytes + recv_floats(splits, B) * 4 + 1024 /*alignment*/ + kBarBytes + BT * 4 /*s_scale*/;
   }
 };
 
@@ -137,7 +137,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int S = a.splits, stages = a.stages;
   float* aux = reinterpret_cast<float*>(tiles + (size_t)stages * Cfg::kStageBytes);
   float* s_recv = aux;  // [S - 1][slice][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(aux + Cfg::recv_floats(S));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(aux + Cfg::recv_floats(S, a.B));
   uint64_t* full = bars;
   uint64_t* empty = bars + kMaxStages;
   uint64_t* tmem_full = bars + 2 * kMaxStages;
@@ -576,18 +576,19 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
   a.stream_out = reinterpret_cast<__nv_bfloat16*>(f.stream_out);
   a.norm_w = reinterpret_cast<const __nv_bfloat16*>(f.norm_w);
   a.sumsq_out = f.sumsq_out;
-  // ring depth: what fits next to the receive area in ~106 KB (two CTAs per SM, of this kernel or the next:
+  // ring depth: what fits next to the receive area in 106 to 112 KB (two CTAs per SM, of this kernel or the next:
   // one sets up and fills its ring while the other drains).  With a 128-wide batch tile and no more CTAs than
   // SMs one per SM and as deep as the range needs.  A second round of CTAs wants the two as well (the step
   // of 128 sequences, gate/up 62.8 us -> 45, the LM head at one sequence 176 -> 163, at 64 195 -> 181, at 128
   // 232 -> 209).
   const int kb_per = (a.num_kb + splits - 1) / splits;
-  // (measured, whole N = 1 decode step: 106 KB 6.08 ms, 75 KB 6.40, 56 KB 6.72, 150 KB 7.40)
-  const size_t budget = smem_kb > 0 ? (size_t)std::min(smem_kb, 226) << 10 : (BT <= 64 || tiles * slabs * splits > sms ? (size_t)106 << 10 : (size_t)200 << 10);
+  // (measured, whole N = 1 decode step: 106 KB 6.08 ms, 75 KB 6.40, 56 KB 6.72, 150 KB 7.40.  112 KB is the most that two CTAs
+  // leave room for: with the receive area as large as the batch asks for, a fifth stage for up to 8 rows, 0.5 % of a step)
+  const size_t budget = smem_kb > 0 ? (size_t)std::min(smem_kb, 226) << 10 : (BT <= 64 || tiles * slabs * splits > sms ? (size_t)(BT <= 64 ? 112 : 106) << 10 : (size_t)200 << 10);
   int stages = Cfg::min_stages();
-  while (stages < kMaxStages && stages < kb_per && Cfg::smem_bytes(stages + 1, splits) <= budget) ++stages;
+  while (stages < kMaxStages && stages < kb_per && Cfg::smem_bytes(stages + 1, splits, B) <= budget) ++stages;
   a.stages = stages;
-  const size_t smem = Cfg::smem_bytes(stages, splits);
+  const size_t smem = Cfg::smem_bytes(stages, splits, B);
   if (smem > ((size_t)227 << 10)) return cudaErrorInvalidValue;
   // L2 prefetch of the rest of the weight range while the predecessor runs: only when
   // the whole matrix fits the budget (a shard of a tensor-parallel layer does; the

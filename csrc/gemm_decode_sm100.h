@@ -55,7 +55,7 @@ struct DecodePush {
 //                   dependency wait (-1 = default, 0 = only a rolling window)
 //   push            null, or where rows owned by other ranks go (see DecodePush); plain epilogue only
 //   fold            null, or the row scale and the residual add of the norms around the linear (see DecodeFold)
-//   smem_kb         shared memory the TMA ring may grow to (0 = default: ~106 KB, so
+//   smem_kb         shared memory the TMA ring may grow to (0 = default: ~110 KB, so
 //                   that the next kernel of the step fits on the SM beside this one;
 //                   up to 226 for a kernel nothing needs to overlap with)
 // Allocates nothing; no workspace; safe to capture.  error_word as in launch_gemm_bf16.
