@@ -45,6 +45,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "all_reduce_oneshot.cuh"
 #include "decode_gemm_plan.h"
@@ -111,7 +112,8 @@ struct DecodeCfg {
   static constexpr int kWBytes = kBlockM * kBlockK * 2;  // 16 KB of weights per stage
   static constexpr int kXBytes = BT * kBlockK * 2;
   static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kTmemCols = BT < 32 ? 32 : BT;
+  static constexpr int kTmemCols = BT <= 32 ? 32 : (BT <= 64 ? 64 : 128);
+  static constexpr int kHalf = (BT / 2 + 15) / 16 * 16;  // columns of the first of a quarter's two epilogue warps
   static constexpr int kBarBytes = 256;
   // the peers' partials of this CTA's column slice: [splits - 1][slice][128 rows] fp32, for the rows that a slab has
   __host__ __device__ static size_t recv_floats(int splits, int B) { return decode_recv_floats(B < BT ? B : BT, splits); }
@@ -331,7 +333,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // pipeline stages (every MMA that read them has completed)
     float* s_acc = reinterpret_cast<float*>(tiles);
     const float4* s_acc4 = reinterpret_cast<const float4*>(s_acc);
-    const int c_begin = h * (BT / 2), c_end = min(nB, c_begin + BT / 2);
+    const int c_begin = h * Cfg::kHalf, c_end = h == 0 ? min(nB, Cfg::kHalf) : nB;
     if (ok) {
       const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
@@ -632,11 +634,19 @@ cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, i
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (l2_budget_bytes < 0) l2_budget_bytes = (long long)32 << 20;
-  if (B <= 32)
-    return launch_decode_bt<32>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
-  if (B <= 64)
-    return launch_decode_bt<64>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
-  return launch_decode_bt<128>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push, fold, sms, error_word, stream);
+  // Batch tiles in steps of 16 rows where the launch is one of a chain of folded linears: fewer rows of x per K step and a
+  // smaller exchange leave a stage more for the weights (a step of 1 / 8 / 37 rows, the latter on 16 and 48 instead of 32 and
+  // 64: 792 -> 783, 913 -> 909, 1358 -> 1333 us).
+  const bool chain = fold != nullptr && (fold->scale_sumsq != nullptr || fold->residual != nullptr);
+  auto go = [&](auto bt) {
+    return launch_decode_bt<decltype(bt)::value>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push,
+                                                 fold, sms, error_word, stream);
+  };
+  if (chain && B <= 16) return go(std::integral_constant<int, 16>());
+  if (B <= 32) return go(std::integral_constant<int, 32>());
+  if (chain && B <= 48) return go(std::integral_constant<int, 48>());
+  if (B <= 64) return go(std::integral_constant<int, 64>());
+  return go(std::integral_constant<int, 128>());
 }
 
 int gemm_decode_stamps(unsigned long long* out, int max_ctas) {

@@ -4,9 +4,11 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# (rows, columns, K): one row, an odd number with a ragged last slice, whole and just exceeded batch tiles, two slabs;
+# (rows, columns, K): one row, an odd number with a ragged last slice, whole and just exceeded batch tiles (16, 32, 48, 64,
+# 128 rows), two slabs;
 # K of one step, of a partial last step, and more K steps than the ring is deep
-SHAPES = [(1, 128, 64), (5, 256, 520), (33, 512, 1024), (64, 384, 4096), (128, 256, 2048), (129, 256, 1032)]
+SHAPES = [(1, 128, 64), (5, 256, 520), (16, 256, 1024), (17, 128, 2048), (33, 512, 1024), (48, 256, 4096), (49, 128, 1024),
+          (64, 384, 4096), (128, 256, 2048), (129, 256, 1032)]
 
 
 def _inputs(B, N, K, parts):
