@@ -7,7 +7,7 @@
 //
 //   * Operands are swapped with respect to a large GEMM: the 128 rows of a W tile
 //     are the M side of tcgen05.mma (K-major as stored), the batch rows of x are
-//     the N side (32, 64 or 128 wide).  TMEM lane = output column n, TMEM column =
+//     the N side (16, 32, 48, 64 or 128 wide).  TMEM lane = output column n, TMEM column =
 //     batch row.
 //   * One CTA per (W tile, K range).  The K ranges of a tile belong to the CTAs
 //     of one thread-block cluster (1-8 CTAs), which add their fp32 partials
@@ -22,7 +22,7 @@
 //     CTA's W range (bounded by a byte budget) all happen BEFORE the dependency
 //     wait; only the x tiles wait for the predecessor.  W must therefore not be
 //     written by the kernel launched just before (weights never are).
-//   * 3-4 stage TMA ring of 24 KB (B <= 64), at most ~106 KB of shared memory, so
+//   * 3-5 stage TMA ring of 18-24 KB (B <= 64), at most 112 KB of shared memory, so
 //     two of these kernels (or one and the decode attention) are resident per SM:
 //     that is what lets the next kernel's prologue overlap this one.
 //   * warp 0: TMA producer, warp 1: MMA issuer, warps 2-9: epilogue.  Every wait
