@@ -25,9 +25,8 @@
 //     wait; q, k, v of the new token are read after it.
 //
 // The reference has no attention (it is used inside vLLM / SGLang, README.md:20-33).
-#include <algorithm>
-
 #include "decode_attn_common.cuh"
+#include "decode_attn_plan.h"
 #include "decode_kernels.h"
 #include "kernel_setup.h"
 #include "pdl.h"
@@ -37,26 +36,21 @@ namespace penny {
 namespace {
 using namespace attn;
 
-// Shortest piece and most pieces of a row: a merge is 2 us.  One row of 2048 positions in 1 / 4 / 8 / 16 pieces: 17.3 /
-// 8.0 / 6.9 / 7.7 us, of 16000 in 8 / 16 / 37: 23.6 / 17.7 / 19.5, of 100 in 1 / 8 / 16: 2.7 / 5.1 / 6.5.
-constexpr int kMinPiece = 256, kMaxPieces = 16;
-
-// Piece `idx` of a batch whose rows are cut by length: row, KV head, piece and pieces of that row.  A piece is the
-// batch's positions over `slots` (the CTAs that the GPU holds at a time), over twice as many where the rows are of mixed
-// lengths and alone fill half of them, and a row has as many as fit it whole.  At most 2 slots more than (row, KV head)
-// pairs; idx past the last one: row -1.  Called by every thread of the block.
+// Piece `idx` of a batch whose rows are cut by length (decode_attn_plan.h): row, KV head, piece and pieces of that row.  At
+// most balance_extra more than (row, KV head) pairs; idx past the last one: row -1.  Called by every thread of the block.
 struct Piece {
   int b, kh, sp, n;
 };
-__device__ __forceinline__ Piece find_piece(const int* __restrict__ positions, int B, int Hkv, int slots, int idx) {
+__device__ __forceinline__ Piece find_piece(const int* __restrict__ positions, int max_len, int B, int Hkv, int slots, int idx) {
   __shared__ int s_part[2][kAttnWarps];
   __shared__ Piece s_piece;
   const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per = (B + kAttnWarps * 32 - 1) / (kAttnWarps * 32), r0 = min(B, tid * per), r1 = min(B, r0 + per);
   int sum = 0, top = 0;
   for (int r = r0; r < r1; ++r) {
-    sum += positions[r];
-    top = max(top, positions[r]);
+    const int rows = cut_rows(positions[r], max_len);
+    sum += rows;
+    top = max(top, rows);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -75,13 +69,11 @@ __device__ __forceinline__ Piece find_piece(const int* __restrict__ positions, i
     total += s_part[0][w];
     top = max(top, s_part[1][w]);
   }
-  const bool mixed = (long long)top * B * 4 > total * 5 && B * Hkv * 2 > slots;
-  const int target = mixed ? 2 * slots : slots;
-  const int len = max(kMinPiece, (int)((total * Hkv + target - 1) / target));
-  auto pieces_of = [&](int r) { return min(kMaxPieces, max(1, positions[r] / len)); };
+  const int len = piece_len(total, top, B, Hkv, slots);
+  auto pieces_at = [&](int r) { return pieces_of(cut_rows(positions[r], max_len), len); };
   __syncthreads();
   int mine = 0;
-  for (int r = r0; r < r1; ++r) mine += pieces_of(r);
+  for (int r = r0; r < r1; ++r) mine += pieces_at(r);
   int incl = mine;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -95,7 +87,7 @@ __device__ __forceinline__ Piece find_piece(const int* __restrict__ positions, i
   int at = idx - first * Hkv;
   if (at >= 0 && at < mine * Hkv) {
     for (int r = r0; r < r1; ++r) {
-      const int n = pieces_of(r);
+      const int n = pieces_at(r);
       if (at < n * Hkv) {
         s_piece = {r, at % Hkv, at / Hkv, n};
         break;
@@ -119,7 +111,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
   __shared__ int s_last;
   pdl_launch_dependents();
   Piece pc{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, splits};
-  if (slots > 0) pc = find_piece(positions, B, Hkv, slots, (int)blockIdx.x);
+  if (slots > 0) pc = find_piece(positions, max_len, B, Hkv, slots, (int)blockIdx.x);
   if (pc.b < 0) {
     pdl_wait();
     return;
@@ -133,7 +125,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
   // positions[] was advanced at the end of the previous step, long before any kernel
   // that may still be running when this one starts
   const int pos = positions[b];
-  const int len = pos;  // old rows; the new token is handled separately
+  const int len = cached_rows(pos, max_len);  // old rows; the new token is handled separately
   const int per = ((len + pieces - 1) / pieces + kTile - 1) / kTile * kTile;
   const int t0 = sp * per;
   const int t1 = min(len, t0 + per);
@@ -204,8 +196,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
       qa[kc + 4][1] = (g < G) ? pack2(rb[2], rb[3]) : 0u;
     }
   }
-  // ---- the new token: split 0 appends it to the cache and keeps it in shared memory ----
+  // ---- the new token: split 0 appends it to the cache and keeps it in shared memory.  A position past the cache's
+  // end has no row there: the token attends to all cached rows and itself, and is not kept. ----
   if (sp == 0) {
+    const bool keep = pos >= 0 && pos < max_len;
     const size_t coff = (cache_row0 + (size_t)pos) * kD;
     const int tid = (int)threadIdx.x;
     if (tid < kD / 2) {
@@ -213,15 +207,17 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
       const float sn = k_s, cs = k_c;
       const float a = bf2f(kp[tid]), bb = bf2f(kp[tid + kD / 2]);
       const __nv_bfloat16 ka = __float2bfloat16_rn(a * cs - bb * sn), kb = __float2bfloat16_rn(bb * cs + a * sn);
-      kcache[coff + tid] = ka;
-      kcache[coff + tid + kD / 2] = kb;
+      if (keep) {
+        kcache[coff + tid] = ka;
+        kcache[coff + tid + kD / 2] = kb;
+      }
       s_new[tid] = bf2f(ka);
       s_new[tid + kD / 2] = bf2f(kb);
     } else {
       const __nv_bfloat16* vp = qkv + qkv_row + (size_t)(Hq + Hkv + kh) * kD;
       const int j = (tid - kD / 2) * 2;
       const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(vp + j);
-      *reinterpret_cast<__nv_bfloat162*>(vcache + coff + j) = v2;
+      if (keep) *reinterpret_cast<__nv_bfloat162*>(vcache + coff + j) = v2;
       s_new[kD + j] = bf2f(v2.x);
       s_new[kD + j + 1] = bf2f(v2.y);
     }
@@ -428,10 +424,6 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn_fused(
 namespace {
 size_t counter_bytes(int B, int Hkv) { return ((size_t)B * Hkv * sizeof(unsigned) + 15) / 16 * 16; }
 
-// CTAs that a balanced launch counts on; 0, no pieces, where there are four rounds of (row, KV head) pairs anyhow, which
-// the GPU deals out as they end.
-int balance_slots(int items, int sms) { return items > 8 * sms ? 0 : 2 * sms; }
-int balance_extra(int items, int slots) { return items * 2 > slots ? 2 * slots : slots; }  // pieces beyond one per pair
 int device_sms() {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -463,10 +455,7 @@ cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* v
   int slots = 0, extra = 0;
   if (balance) {
     slots = balance_slots(items, device_sms());
-    // (no more than the cache's length allows: the launch behind this one begins when every CTA of this one has begun, so
-    // CTAs without a piece keep its weights waiting)
-    extra = (int)std::min<long long>(balance_extra(items, slots),
-                                     (long long)items * (std::min(kMaxPieces, std::max(1, (max_len - 1) / kMinPiece)) - 1));
+    extra = grid_extra(items, slots, max_len);
     if (extra == 0) slots = 0;
     // (a workspace for fewer pieces than the cut may take: whole rows)
     if (slots == 0 || (long long)items * (splits - 1) < extra) slots = 0, splits = 1;

@@ -24,6 +24,7 @@
 
 #include "../algos.h"
 #include "../gemm_tile_order.h"
+#include "../decode_attn_plan.h"
 #include "../decode_gemm_plan.h"
 #include "../all_reduce_oneshot.cuh"
 #include "../all_reduce_ring.cuh"
@@ -345,6 +346,23 @@ int penny_decode_choose_splits(int tiles, int num_kb, int sms, int gpc_sms) {
 }
 int penny_decode_choose_splits_chain(int tiles, int num_kb, int sms) {
   return penny::sm100::decode_choose_splits_chain(tiles, num_kb, sms);
+}
+// The decode attention's cut by lengths (decode_attn_plan.h): pieces of every row, as the kernel counts them; returns the
+// pieces beyond one per (row, KV head) that the launcher's grid has room for, -1 where rows stay whole.
+int penny_decode_attn_cut(const int* positions, int B, int Hkv, int max_len, int sms, int* pieces) {
+  using namespace penny::attn;
+  const int slots = balance_slots(B * Hkv, sms);
+  if (slots == 0) return -1;
+  long long total = 0;
+  int top = 0;
+  for (int r = 0; r < B; ++r) {
+    const int rows = cut_rows(positions[r], max_len);
+    total += rows;
+    top = at_least(top, rows);
+  }
+  const int len = piece_len(total, top, B, Hkv, slots);
+  for (int r = 0; r < B; ++r) pieces[r] = pieces_of(cut_rows(positions[r], max_len), len);
+  return grid_extra(B * Hkv, slots, max_len);
 }
 // Tile -> (row block, column block) of the persistent GEMM kernels; pair_rank < 0
 // selects the single-CTA kernel, 0 / 1 the CTA of a pair.  Returns the number of

@@ -136,3 +136,12 @@ def decode_choose_splits(tiles: int, num_kb: int, sms: int = 148, gpc_sms: int =
 def decode_choose_splits_chain(tiles: int, num_kb: int, sms: int = 148) -> int:
     """The same for the linears of one rank's step, between folded norms."""
     return sim_lib().penny_decode_choose_splits_chain(tiles, num_kb, sms)
+
+
+def decode_attn_cut(positions, kv_heads: int, max_len: int, sms: int = 148):
+    """The decode attention's cut of a batch's rows by their lengths (csrc/decode_attn_plan.h): (pieces of every row,
+    pieces beyond one per (row, KV head) that the grid has room for), or None where all rows stay whole."""
+    n = len(positions)
+    pos, pieces = (ctypes.c_int * n)(*positions), (ctypes.c_int * n)()
+    extra = sim_lib().penny_decode_attn_cut(pos, n, kv_heads, max_len, sms, pieces)
+    return None if extra < 0 else (list(pieces), extra)

@@ -54,3 +54,55 @@ def test_pieces_by_length(B, Hq, Hkv, L, kind):
     want = torch.einsum("hgt,htd->hgd", s.softmax(-1), v2[b, :, :p + 1].double()).reshape(Hq * D)
     # (as above, and q rounded to bf16 before the scores, angles of up to 5000 rad in fp32)
     torch.testing.assert_close(out[b].double(), want, atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("balance", [True, False])
+def test_position_past_the_cache(balance):
+    """A row that the cache cannot hold attends to all cached rows and itself and is stored nowhere, and the rows' arrival
+    counters serve the next launch."""
+    from penny_b200._ext import ops
+    B, Hq, Hkv, L = 2, 8, 8, 768
+    g = torch.Generator(device="cuda").manual_seed(9)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    kf, vf = r(B + 1, Hkv, L, D), r(B + 1, Hkv, L, D)  # (a row of slack behind the caches)
+    kc, vc, splits = kf[:B], vf[:B], ops.decode_attn_balanced_splits(B, Hkv)
+    ws = torch.zeros(ops.decode_attn_fused_workspace_bytes(B, Hq, Hkv, splits), dtype=torch.uint8, device="cuda")
+    for last in (L, L + 300, L - 1):
+        pos = torch.tensor([40, last], dtype=torch.int32, device="cuda")
+        qkv, k0, v0 = r(B, (Hq + 2 * Hkv) * D), kf.clone(), vf.clone()
+        out = torch.full((B, Hq * D), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.decode_attention_fused(qkv, kc, vc, pos, out, ws, Hq, Hkv, splits, D ** -0.5, 1e4, balance=balance)
+        for b, p in enumerate(pos.tolist()):
+            ang = p * 1e4 ** (-torch.arange(64, device="cuda", dtype=torch.float64) / 64)
+            rot = lambda t: torch.cat([t[:, :64] * ang.cos() - t[:, 64:] * ang.sin(), t[:, 64:] * ang.cos() + t[:, :64] * ang.sin()], -1)  # noqa: E731
+            q, k, v = (t.view(Hkv, D) for t in qkv[b].double().split(Hkv * D))
+            q, k = rot(q), rot(k)
+            rows = min(p, L)
+            keys = torch.cat([k0[b, :, :rows].double(), k.bfloat16().double()[:, None]], 1)
+            vals = torch.cat([v0[b, :, :rows].double(), v[:, None]], 1)
+            s = torch.einsum("hd,htd->ht", q, keys) / math.sqrt(D)
+            want = torch.einsum("ht,htd->hd", s.softmax(-1), vals).reshape(Hq * D)
+            # (tolerance as in test_pieces_by_length)
+            torch.testing.assert_close(out[b].double(), want, atol=2e-2, rtol=2e-2)
+            if p < L:
+                torch.testing.assert_close(kf[b, :, p].double(), k, atol=3e-2, rtol=2e-2)
+                assert torch.equal(vf[b, :, p].double(), v)
+                k0[b, :, p], v0[b, :, p] = kf[b, :, p], vf[b, :, p]
+        assert torch.equal(kf, k0) and torch.equal(vf, v0)  # nothing else was written
+
+
+def test_decoder_up_to_the_caches_last_row():
+    """A cache filled up to its last row: the warm-up's second step has no row left, and none of it shows later."""
+    from penny_b200.models.llama_tp import LlamaConfig, LlamaTPDecoder
+    for L in (768, 300):
+        m = LlamaTPDecoder(LlamaConfig.tiny(), world=1, max_batch=3, max_len=L, full_init=True)
+        m.fill_synthetic_kv(L - 1)
+        before = [c.clone() for c in m.kcache + m.vcache]
+        m.capture()
+        for c, old in zip(m.kcache + m.vcache, before):
+            assert torch.equal(c[:, :, :L - 1], old[:, :, :L - 1])
+        tokens, positions = m.tokens.clone(), m.positions.clone()
+        m.step_device()
+        want = m.reference_logits(tokens, positions, m.kcache, m.vcache)
+        assert (m.logits.float() - want).abs().max().item() < 0.05 * want.std().item() + 0.02
+        assert torch.equal(m.positions, positions + 1)
