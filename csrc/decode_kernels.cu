@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "decode_attn_common.cuh"
+#include "decode_attn_plan.h"
 #include "decode_kernels.h"
 
 #undef NDEBUG  // an embedding row that does not exist stops the kernel in every build
@@ -57,6 +58,7 @@ __global__ void k_rope_append(__nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __
     x[i] = __float2bfloat16_rn(ra);
     x[i + half] = __float2bfloat16_rn(rb);
   } else {
+    if (pos < 0 || pos >= max_len) return;  // the cache has no such row
     const int kh = h - Hq;
     const size_t coff = (((size_t)b * Hkv + kh) * max_len + pos) * D;
     kcache[coff + i] = __float2bfloat16_rn(ra);
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) k_decode_attn(
   const int b = blockIdx.x, kh = blockIdx.y, sp = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int len = positions[b] + 1;  // the new token was appended at positions[b]
+  const int len = cached_rows(positions[b] + 1, max_len);  // the new token was appended at positions[b]
   const int per = ((len + splits - 1) / splits + kTile - 1) / kTile * kTile;
   const int t0 = sp * per;
   const int t1 = min(len, t0 + per);

@@ -106,3 +106,26 @@ def test_decoder_up_to_the_caches_last_row():
         want = m.reference_logits(tokens, positions, m.kcache, m.vcache)
         assert (m.logits.float() - want).abs().max().item() < 0.05 * want.std().item() + 0.02
         assert torch.equal(m.positions, positions + 1)
+
+
+def test_separate_kernels_past_the_cache():
+    """rope_append stores no row that the cache does not have; the attention reads the rows that there are."""
+    from penny_b200._ext import ops
+    B, Hq, Hkv, L = 3, 8, 2, 100
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    kf, vf, qkv = r(B + 1, Hkv, L, D), r(B + 1, Hkv, L, D), r(B, (Hq + 2 * Hkv) * D)
+    pos = torch.tensor([L - 1, L, L + 500], dtype=torch.int32, device="cuda")
+    k0, v0 = kf.clone(), vf.clone()
+    ops.rope_append(qkv, kf[:B], vf[:B], pos, Hq, Hkv, D, 1e4)
+    assert not torch.equal(kf[0, :, L - 1], k0[0, :, L - 1])
+    k0[0, :, L - 1], v0[0, :, L - 1] = kf[0, :, L - 1], vf[0, :, L - 1]
+    assert torch.equal(kf, k0) and torch.equal(vf, v0)
+    for splits in (1, 3):
+        out = torch.empty(B, Hq * D, device="cuda", dtype=torch.bfloat16)
+        ws = torch.empty(ops.decode_attn_workspace_bytes(B, Hq, splits), dtype=torch.uint8, device="cuda")
+        ops.decode_attention(qkv, kf[:B], vf[:B], pos, out, ws, Hq, Hkv, splits, D ** -0.5)
+        q = qkv[:, :Hq * D].view(B, Hkv, Hq // Hkv, D).double()
+        s = torch.einsum("bhgd,bhtd->bhgt", q, kf[:B].double()) / math.sqrt(D)
+        want = torch.einsum("bhgt,bhtd->bhgd", s.softmax(-1), vf[:B].double()).reshape(B, Hq * D)
+        torch.testing.assert_close(out.double(), want, atol=2e-2, rtol=2e-2)  # (as above)
