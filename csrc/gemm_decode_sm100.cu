@@ -446,10 +446,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           float u[8];
           sum8(64 + g * 8, u);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float e = 1.f + __expf(-v[k]);
-            v[k] = (a.scale_sumsq != nullptr ? __fdividef(v[k], e) : v[k] / e) * (u[k] * sc);
-          }
+          for (int k = 0; k < 8; ++k) v[k] = v[k] / (1.f + __expf(-v[k])) * (u[k] * sc);
         }
         __nv_bfloat16* dst = a.out + (size_t)(row0 + j) * a.ldo + n0;
         if (vec_ok && n0 + 8 <= n_out) {

@@ -62,6 +62,21 @@ def test_row_scale(shape, silu, parts, splits):
     assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4 * scale.max()).all()
 
 
+@pytest.mark.parametrize("B", [1, 40, 130])
+def test_silu_of_large_negative_gates(B):
+    """silu(g) * up far out on the negative side, where exp(-g) is near the largest fp32: small, not zero."""
+    from penny_b200._ext import ops
+    K, gates = 64, torch.arange(64, device="cuda") * 0.5 - 88.5
+    x, w = torch.zeros(B, K, device="cuda"), torch.zeros(128, K, device="cuda")
+    x[:, 0], w[:64, 0], w[64:, 0] = 1.0, gates, 1.0
+    ss, out = torch.full((1, B), float(K), device="cuda"), torch.empty(B, 64, device="cuda", dtype=torch.bfloat16)
+    for sumsq, scale in ((None, 1.0), (ss, (1.0 + 1e-5) ** -0.5)):
+        ops.gemm_decode(x.bfloat16(), w.bfloat16(), out, True, sumsq=sumsq, eps=1e-5)
+        want = torch.nn.functional.silu(gates.double() * scale) * scale
+        # one bf16 rounding; the fast exponential is off by 2 + 1.173 * 88.5 ulp (2 ** -16) at most, CUDA's bound for it
+        torch.testing.assert_close(out.double(), want.expand(B, 64), rtol=2.0 ** -8 + 2.0 ** -15, atol=0)
+
+
 def test_embedding_rows_start_the_stream():
     from penny_b200._ext import ops
     table = torch.randn(50, 512, device="cuda").bfloat16()
