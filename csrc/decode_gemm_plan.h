@@ -63,15 +63,22 @@ PENNY_PLAN_HD int decode_choose_splits(int tiles, int num_kb, const int* capacit
 }
 
 // The same for a linear between the folded norms of one rank's step, whose clusters were timed in its chain of launches:
-// up to five CTAs on three SMs.  The stream runs at 32 GB/s per CTA, so a sixth and a seventh range pay (down of 8 rows
-// 21.9 us in six, 20.7 in seven, 20.8 in eight; o 9.0 / 8.6 / 8.8) where the occupancy query, which wants whole
-// clusters per GPC, stops at six; 288 CTAs no longer run side by side (q / k / v 11.0 us in five, 16.1 in six).
+// either rule is enough, the device's answer or up to five CTAs on three SMs.
+//   * The stream runs at 32 GB/s per CTA, so at 31 to 35 tiles a seventh range pays although the occupancy query, which
+//     wants whole clusters per GPC, has room for 210 CTAs in sevens (a layer's linears at hidden 4096, o and down of 32
+//     tiles in six / seven, 1 row: 78.8 / 77.9 us, 40 rows 87.0 / 85.7; 34 tiles level); 288 CTAs no longer run side by
+//     side (q / k / v 11.0 us in five, 16.1 in six).
+//   * Five on three alone keeps clusters small that the device has room for: 64 tiles, K 4096, gate/up and down in three /
+//     four 25.0 / 23.7 us, 128 tiles in one / two 39.8 / 38.7, a layer of hidden 5376 123.3 / 121.4.
+//   * Its room filled to the last cluster is too much for a chain, where CTAs of the launch before are still at work (44
+//     tiles in six, 264 of 264 CTAs: 153.3 us a layer, in five 150.6; 90 in three, 270 of 270: 31.4, in two 30.3).
 // Batch tiles of 128 rows hold one CTA per SM and keep to the rule above.
-PENNY_PLAN_HD int decode_choose_splits_chain(int tiles, int num_kb, int sms) {
+PENNY_PLAN_HD int decode_choose_splits_chain(int tiles, int num_kb, int sms, const int* capacity) {
   int best = 1;
   for (int s = 2; s <= kDecodeMaxSplits; ++s) {
     if (num_kb / s < 6) break;
-    if ((long long)tiles * s * 3 <= (long long)sms * 5) best = s;
+    const long long ctas = (long long)tiles * s;
+    if (ctas < (long long)capacity[s] || ctas * 3 <= (long long)sms * 5) best = s;
   }
   return best;
 }

@@ -556,7 +556,7 @@ cudaError_t launch_decode_bt(const void* x, const void* w, void* out, int B, int
   if ((long long)tiles * slabs > 65535) return cudaErrorInvalidValue;
   a.slabs = slabs;
   if (splits <= 0 && BT <= 64 && fold != nullptr && (fold->scale_sumsq != nullptr || fold->residual != nullptr))
-    splits = decode_choose_splits_chain(tiles * slabs, a.num_kb, sms);
+    splits = decode_choose_splits_chain(tiles * slabs, a.num_kb, sms, decode_capacity<BT>(sms));
   if (splits <= 0) splits = decode_choose_splits(tiles * slabs, a.num_kb, decode_capacity<BT>(sms));
   splits = std::max(1, std::min(splits, std::min(kDecodeMaxSplits, a.num_kb)));
   a.splits = splits;

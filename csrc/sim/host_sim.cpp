@@ -344,8 +344,9 @@ int penny_decode_choose_splits(int tiles, int num_kb, int sms, int gpc_sms) {
   penny::sm100::decode_model_capacity(sms, gpc_sms, cap);
   return penny::sm100::decode_choose_splits(tiles, num_kb, cap);
 }
-int penny_decode_choose_splits_chain(int tiles, int num_kb, int sms) {
-  return penny::sm100::decode_choose_splits_chain(tiles, num_kb, sms);
+// capacity: [kDecodeMaxSplits + 1], CTAs that the device holds in clusters of s
+int penny_decode_choose_splits_chain(int tiles, int num_kb, int sms, const int* capacity) {
+  return penny::sm100::decode_choose_splits_chain(tiles, num_kb, sms, capacity);
 }
 // The decode attention's cut by lengths (decode_attn_plan.h): pieces of every row, as the kernel counts them; returns the
 // pieces beyond one per (row, KV head) that the launcher's grid has room for, -1 where rows stay whole.

@@ -133,9 +133,13 @@ def decode_choose_splits(tiles: int, num_kb: int, sms: int = 148, gpc_sms: int =
     return sim_lib().penny_decode_choose_splits(tiles, num_kb, sms, gpc_sms)
 
 
-def decode_choose_splits_chain(tiles: int, num_kb: int, sms: int = 148) -> int:
-    """The same for the linears of one rank's step, between folded norms."""
-    return sim_lib().penny_decode_choose_splits_chain(tiles, num_kb, sms)
+B200_CLUSTER_CTAS = (0, 296, 296, 270, 264, 260, 264, 210, 240)  # ops.gemm_decode_capacity up to 64 rows, by cluster size
+
+
+def decode_choose_splits_chain(tiles: int, num_kb: int, sms: int = 148, capacity=B200_CLUSTER_CTAS) -> int:
+    """The same for the linears of one rank's step, between folded norms; `capacity`: CTAs that the device holds in
+    clusters of 0 to 8."""
+    return sim_lib().penny_decode_choose_splits_chain(tiles, num_kb, sms, (ctypes.c_int * 9)(*capacity))
 
 
 def decode_attn_cut(positions, kv_heads: int, max_len: int, sms: int = 148):
