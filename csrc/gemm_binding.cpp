@@ -178,9 +178,10 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
      py::arg("cluster") = 0);
-  m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K) {
-    return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K);
-  });
+  m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K, bool folded) {
+    return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K, folded);
+  }, py::arg("B"), py::arg("N"), py::arg("K"), py::arg("folded") = false,
+     "cluster size of gemm_decode(splits=0); folded: with sumsq or residual");
   m.def("gemm_decode_capacity", [](int64_t B, int64_t splits) {
     return penny::sm100::gemm_decode_capacity((int)B, (int)splits);
   });

@@ -655,23 +655,31 @@ int gemm_decode_stamps(unsigned long long* out, int max_ctas) {
   return n;
 }
 
-int gemm_decode_capacity(int B, int splits) {
+namespace {
+const int* capacity_of(int B, bool folded, int sms) {
+  if (folded && B <= 16) return decode_capacity<16>(sms);
+  if (B <= 32) return decode_capacity<32>(sms);
+  if (folded && B <= 48) return decode_capacity<48>(sms);
+  return B <= 64 ? decode_capacity<64>(sms) : decode_capacity<128>(sms);
+}
+int current_sms() {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   (void)cudaGetLastError();
+  return sms > 0 ? sms : 148;
+}
+}  // namespace
+
+int gemm_decode_capacity(int B, int splits) {
   if (splits < 1 || splits > kDecodeMaxSplits) return 0;
-  const int* cap = B <= 32 ? decode_capacity<32>(sms) : (B <= 64 ? decode_capacity<64>(sms) : decode_capacity<128>(sms));
-  return cap[splits];
+  return capacity_of(B, false, current_sms())[splits];
 }
 
-int gemm_decode_splits(int B, int N, int K) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  (void)cudaGetLastError();
-  if (sms <= 0) sms = 148;
+int gemm_decode_splits(int B, int N, int K, bool folded) {
+  const int sms = current_sms();
   const int num_kb = (K + kBlockK - 1) / kBlockK, tiles = (N + kBlockM - 1) / kBlockM * ((std::max(B, 1) + 127) / 128);
-  const int* cap = B <= 32 ? decode_capacity<32>(sms) : (B <= 64 ? decode_capacity<64>(sms) : decode_capacity<128>(sms));
-  return decode_choose_splits(tiles, num_kb, cap);
+  const int* cap = capacity_of(B, folded, sms);
+  return folded && B <= 64 ? decode_choose_splits_chain(tiles, num_kb, sms, cap) : decode_choose_splits(tiles, num_kb, cap);
 }
 
 }  // namespace sm100

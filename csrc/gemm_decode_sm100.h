@@ -71,8 +71,9 @@ int gemm_decode_stamps(unsigned long long* out, int max_ctas);
 
 // CTAs of the decode GEMM the current device holds at once when they come in clusters of `splits`.
 int gemm_decode_capacity(int B, int splits);
-// The cluster size launch_gemm_decode(splits = 0) uses for this shape on the current device.
-int gemm_decode_splits(int B, int N, int K);
+// The cluster size launch_gemm_decode(splits = 0) uses for this shape on the current device; folded: with a row scale or a
+// residual.
+int gemm_decode_splits(int B, int N, int K, bool folded = false);
 
 }  // namespace sm100
 }  // namespace penny

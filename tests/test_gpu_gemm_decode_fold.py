@@ -77,6 +77,26 @@ def test_silu_of_large_negative_gates(B):
         torch.testing.assert_close(out.double(), want.expand(B, 64), rtol=2.0 ** -8 + 2.0 ** -15, atol=0)
 
 
+@pytest.mark.parametrize("B,N,K", [(1, 4096, 4096), (16, 1024, 2048), (40, 4096, 4096), (64, 8192, 4096), (65, 4096, 4096)])
+def test_splits_query_is_what_a_launch_takes(B, N, K):
+    """Sums of a launch with splits=0 have the bits of the cluster size that the query names, with and without a fold."""
+    from penny_b200._ext import ops
+    x, w, ss = _inputs(B, N, K, 1)
+    for folded in (False, True):
+        def run(splits):
+            out = torch.empty(B, N, device="cuda", dtype=torch.bfloat16)
+            wide = torch.zeros(B, N, device="cuda")  # (fp32 sums, where another order of adding shows)
+            if folded:
+                ops.gemm_decode(x, w, out, False, splits, residual=wide)
+            else:
+                ops.gemm_decode(x, w, out, False, splits)
+            return wide if folded else out
+        took, named = run(0), ops.gemm_decode_splits(B, N, K, folded)
+        assert torch.equal(took, run(named))
+        if folded:
+            assert [s for s in range(1, 9) if torch.equal(took, run(s))] == [named]
+
+
 def test_embedding_rows_start_the_stream():
     from penny_b200._ext import ops
     table = torch.randn(50, 512, device="cuda").bfloat16()
