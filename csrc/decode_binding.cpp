@@ -156,6 +156,7 @@ void bind_decode(py::module_& m) {
       pp = pair->data_ptr<float>();
     }
     GreedyStep step = {};
+    need(next_tokens.has_value() || !host_tokens.has_value(), "host_tokens: beside next_tokens");
     if (next_tokens.has_value()) {
       need(tokens.has_value() && positions.has_value() && next_tokens->is_cuda() && tokens->is_cuda() && positions->is_cuda() &&
                next_tokens->scalar_type() == at::kLong && tokens->scalar_type() == at::kLong &&

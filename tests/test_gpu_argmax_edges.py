@@ -29,3 +29,24 @@ def test_argmax_edges(cols, chunked):
     best = torch.where(v.isnan(), torch.full_like(v, float("-inf")), v).max(-1).values
     first = (v == best[:, None]).int().argmax(-1)  # (an all-NaN row: 0)
     assert torch.equal(val, best) and torch.equal(idx, first)
+
+
+def test_host_tokens_take_the_winners():
+    """Pinned host memory gets the ids that next_tokens gets, and is refused where there are none to get."""
+    from penny_b200._ext import ops
+    rows, cols = 5, 3001
+    logits = torch.randn(rows, cols, device="cuda").bfloat16()
+    val, idx = torch.empty(rows, device="cuda"), torch.empty(rows, dtype=torch.int64, device="cuda")
+    ws = torch.zeros(ops.argmax_workspace_bytes(rows), dtype=torch.uint8, device="cuda")
+    nxt, tok = (torch.full((rows,), -1, dtype=torch.int64, device="cuda") for _ in range(2))
+    pos, host = torch.arange(rows, dtype=torch.int32, device="cuda"), torch.full((rows,), -1, dtype=torch.int64).pin_memory()
+    with pytest.raises(RuntimeError, match="host_tokens"):
+        ops.argmax_rows(logits, val, idx, 0, ws, host_tokens=host)
+    ops.argmax_rows(logits, val, idx, 7, ws, None, nxt, tok, pos, host)
+    torch.cuda.synchronize()
+    assert torch.equal(idx, 7 + logits.float().argmax(-1)) or torch.equal(logits.gather(1, (idx - 7)[:, None])[:, 0].float(), val)
+    assert torch.equal(host, idx.cpu()) and torch.equal(nxt, idx) and torch.equal(tok, idx)
+    assert pos.tolist() == [r + 1 for r in range(rows)]
+    for bad in (host.clone(), host.to(torch.int32).pin_memory(), torch.zeros(rows + 1, dtype=torch.int64).pin_memory()):
+        with pytest.raises(RuntimeError, match="host_tokens"):
+            ops.argmax_rows(logits, val, idx, 7, ws, None, nxt, tok, pos, bad)
