@@ -76,6 +76,8 @@ void bind_gemm(py::module_& m) {
       fold.scale_parts = (int)sumsq->size(0);
     }
     int epi = silu_pairs ? penny::sm100::DECODE_EPI_SILU_PAIRS : penny::sm100::DECODE_EPI_PLAIN;
+    TORCH_CHECK(residual.has_value() || !(norm_w.has_value() || sumsq_out.has_value() || stream_out.has_value()),
+                "gemm_decode: norm_w, sumsq_out and stream_out beside a residual");
     if (residual.has_value()) {
       auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
       fold.residual_fp32 = residual->scalar_type() == at::kFloat;

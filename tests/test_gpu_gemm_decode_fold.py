@@ -97,6 +97,21 @@ def test_splits_query_is_what_a_launch_takes(B, N, K):
             assert [s for s in range(1, 9) if torch.equal(took, run(s))] == [named]
 
 
+def test_outputs_that_nothing_writes_are_refused():
+    from penny_b200._ext import ops
+    x, w, _ = _inputs(3, 128, 64, 1)
+    out, ss = torch.empty(3, 128, device="cuda", dtype=torch.bfloat16), torch.empty(1, 3, device="cuda")
+    norm_w = torch.ones(128, device="cuda", dtype=torch.bfloat16)
+    for kw in ({"norm_w": norm_w, "sumsq_out": ss}, {"sumsq_out": ss}, {"stream_out": torch.empty_like(out)}):
+        with pytest.raises(RuntimeError, match="beside a residual"):
+            ops.gemm_decode(x, w, out, **kw)
+    wide = torch.zeros(3, 128, device="cuda")
+    with pytest.raises(RuntimeError, match="together"):
+        ops.gemm_decode(x, w, out, residual=wide, norm_w=norm_w)
+    with pytest.raises(RuntimeError, match="stream_out"):
+        ops.gemm_decode(x, w, out, residual=torch.zeros_like(out), stream_out=torch.empty_like(out))
+
+
 def test_embedding_rows_start_the_stream():
     from penny_b200._ext import ops
     table = torch.randn(50, 512, device="cuda").bfloat16()
