@@ -1,0 +1,38 @@
+"""The public decode call: host tokens in, host tokens out, step after step."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _decoder(use_graph, linears, batch=5, max_len=1500):
+    from penny_b200.models.llama_tp import LlamaConfig, LlamaTPDecoder
+    m = LlamaTPDecoder(LlamaConfig.tiny(), world=1, max_batch=batch, max_len=max_len, use_graph=use_graph, full_init=True,
+                       linears=linears)
+    m.fill_synthetic_kv(max_len - 10)
+    # (mixed lengths: whole rows and rows of several pieces)
+    m.positions.copy_(torch.tensor([1400, 3, 600, 1, 900][:batch], dtype=torch.int32))
+    m.capture()
+    return m
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_ids_without_an_embedding_row_are_refused(use_graph):
+    """Before anything is launched: the state is what it was, and the next step runs."""
+    m = _decoder(use_graph, "auto")
+    good = torch.arange(m.B)
+    positions = m.positions.clone()
+    first = m.step(good).clone()
+    m.positions.copy_(positions)
+    for bad_id in (m.cfg.vocab, -1, 2 ** 62, -(2 ** 63)):
+        bad = good.clone()
+        bad[m.B - 1] = bad_id
+        with pytest.raises(IndexError):
+            m.step(bad)
+        torch.cuda.synchronize()
+        assert torch.equal(m.positions, positions)
+    edge = good.clone()
+    edge[0] = m.cfg.vocab - 1
+    m.step(edge)
+    m.positions.copy_(positions)
+    assert torch.equal(m.step(good), first)
