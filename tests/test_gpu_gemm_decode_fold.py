@@ -126,3 +126,12 @@ def test_embedding_rows_start_the_stream():
     assert torch.equal(wide, want.float())
     assert torch.equal(res, want) and torch.equal(out, (want.float() * w.float()).bfloat16())
     torch.testing.assert_close(ss[0], want.float().square().sum(-1), rtol=1e-5, atol=0)
+    # ids in pinned host memory are read when the kernel runs
+    host, again = ids.cpu().pin_memory(), torch.empty_like(wide)
+    for _ in range(2):
+        ops.norm_prep(table, w, again, out, ss, ids=host)
+        torch.cuda.synchronize()
+        assert torch.equal(again, table[host.cuda()].float())
+        host.copy_(torch.tensor([0, 1, 49, 30, 2]))
+    with pytest.raises(RuntimeError, match="ids"):
+        ops.norm_prep(table, w, again, out, ss, ids=host.clone())  # pageable
