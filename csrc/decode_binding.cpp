@@ -133,6 +133,16 @@ void bind_decode(py::module_& m) {
     const at::cuda::OptionalCUDAGuard guard(gate_up.device());
     ck(launch_silu_mul(gate_up.data_ptr(), out.data_ptr(), (int)rows, (int)F, cur()), "silu_mul");
   });
+  // dst (int64 in host memory) = src; returns whether every id lies in [0, rows).  One call from Python for both: a look at
+  // the ids by numpy beside the copy was 1.3 us of a step, more on a cold first one.
+  m.def("take_ids", [](at::Tensor src, at::Tensor dst, int64_t rows) {
+    need(dst.device().is_cpu() && dst.scalar_type() == at::kLong && dst.is_contiguous(), "take_ids: dst int64 on the host");
+    dst.copy_(src);
+    const int64_t *id = dst.data_ptr<int64_t>(), *end = id + dst.numel();
+    bool ok = true;
+    for (; id < end; ++id) ok &= *id >= 0 && *id < rows;
+    return ok;
+  });
   m.def("argmax_workspace_bytes", [](int64_t rows) { return (int64_t)argmax_workspace_bytes((int)rows); });
   m.def("argmax_rows", [](at::Tensor logits, at::Tensor out_val, at::Tensor out_idx, int64_t index_base,
                           c10::optional<at::Tensor> workspace, c10::optional<at::Tensor> pair,

@@ -178,7 +178,6 @@ class LlamaTPDecoder:
         self._graph = self._host_graph = None
         self._host_in = torch.zeros(B, dtype=torch.int64).pin_memory()
         self._host_out = torch.zeros(B, dtype=torch.int64).pin_memory()
-        self._host_ids = self._host_in.numpy().view("uint64")
         # kernels of this library launched per step (the few torch glue ops excluded)
         chunks = -(-B // 1024)  # the decode GEMM takes up to 1024 rows per launch
         gemms = 4 * chunks if self.linears == "penny" else 0
@@ -427,9 +426,8 @@ class LlamaTPDecoder:
         next token of every sequence as a CPU tensor.  The captured step of one rank
         reads the tokens from pinned memory and leaves the next ones there; the other
         forms copy them to the device and back around the step."""
-        self._host_in.copy_(tokens)
-        # (negative ids are the largest unsigned ones; on the device an id without an embedding row stops the context)
-        if self._host_ids.max() >= self.cfg.vocab:
+        # (on the device an id without an embedding row stops the context)
+        if not ops.take_ids(tokens, self._host_in, self.cfg.vocab):
             raise IndexError(f"token ids must lie in [0, {self.cfg.vocab})")
         if self._host_graph is not None:
             self._host_graph.replay()
