@@ -3,7 +3,7 @@
 // tests.
 //
 //   out[B, N] = x[B, K] W[N, K]^T for a decode batch (one slab of B <= 128 rows; larger batches run
-//   their slabs as grid z of the same launch, so the slabs of a weight tile read it from L2 together).
+//   their slabs side by side in the same launch, so the slabs of a weight tile read it from L2 together).
 //   * one CTA per (weight tile of 128 rows, K range); the `splits` CTAs of a tile
 //     form one thread-block cluster and reduce their fp32 partials through
 //     distributed shared memory: no global workspace, no counters, no fix-up pass;
@@ -11,7 +11,8 @@
 //     whose sizes differ by at most one;
 //   * after its MMAs a CTA keeps the accumulator columns (= batch rows) of its
 //     own slice and sends every other slice to the CTA that owns it: CTA r owns
-//     columns [r * slice, min(bt, (r + 1) * slice)) of the bt-wide batch tile.
+//     columns [r * slice, min(rows, (r + 1) * slice)) of the rows that the slab has
+//     (the last slab of a larger batch may have fewer than its tile is wide).
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -31,7 +32,7 @@ constexpr int kDecodeMaxBatch = 1024;  // rows of x per launch
 PENNY_PLAN_HD int decode_kb_begin(int num_kb, int splits, int r) {
   return (int)((long long)num_kb * r / splits);
 }
-// columns of the batch tile owned by one CTA of the cluster
+// columns owned by one CTA of the cluster, of `bt` that there are
 PENNY_PLAN_HD int decode_slice(int bt, int splits) { return (bt + splits - 1) / splits; }
 // slot of source CTA `src` in the receive area of CTA `dst` (src != dst): sources in rank order, dst left out
 PENNY_PLAN_HD int decode_recv_slot(int src, int dst) { return src - (src > dst ? 1 : 0); }

@@ -22,9 +22,9 @@
 //     CTA's W range (bounded by a byte budget) all happen BEFORE the dependency
 //     wait; only the x tiles wait for the predecessor.  W must therefore not be
 //     written by the kernel launched just before (weights never are).
-//   * 3-5 stage TMA ring of 18-24 KB (B <= 64), at most 112 KB of shared memory, so
-//     two of these kernels (or one and the decode attention) are resident per SM:
-//     that is what lets the next kernel's prologue overlap this one.
+//   * TMA ring of 18-24 KB stages (B <= 64): three or four at 64 rows, five or six up to 16, in at most
+//     112 KB of shared memory, so two of these kernels (or one and the decode attention) are resident per
+//     SM: that is what lets the next kernel's prologue overlap this one.
 //   * warp 0: TMA producer, warp 1: MMA issuer, warps 2-9: epilogue.  Every wait
 //     is bounded; TMEM is always freed.
 //
@@ -633,7 +633,7 @@ cudaError_t launch_gemm_decode(const void* x, const void* w, void* out, int B, i
   if (l2_budget_bytes < 0) l2_budget_bytes = (long long)32 << 20;
   // Batch tiles in steps of 16 rows where the launch is one of a chain of folded linears: fewer rows of x per K step and a
   // smaller exchange leave a stage more for the weights (a step of 1 / 8 / 37 rows, the latter on 16 and 48 instead of 32 and
-  // 64: 792 -> 783, 913 -> 909, 1358 -> 1333 us).
+  // 64: 792 -> 783, 913 -> 909, 1358 -> 1333 us).  Launches without a fold (several ranks) were not timed on them.
   const bool chain = fold != nullptr && (fold->scale_sumsq != nullptr || fold->residual != nullptr);
   auto go = [&](auto bt) {
     return launch_decode_bt<decltype(bt)::value>(x, w, out, B, N, K, ldx, ldw, ldo, epi, splits, pdl, l2_budget_bytes, smem_kb, push,

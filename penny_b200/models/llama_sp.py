@@ -179,7 +179,9 @@ class LlamaSPPrefill:
         """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual)."""
         # One row block: the narrow linears are a weight stream like a decode step's, and the decode GEMM's smaller CTAs
         # begin theirs under the launch before (128 tokens, a layer's q/k/v, o and down 19.6 + 19.3 + 37 us in the
-        # forward -> 18 + 12.3 + 28.6).  Gate/up has tiles for every SM and stays (45.4 there, 43.8 here).
+        # forward -> 16 + 17 + 27, 568 -> 498 us for four layers).  Gate/up has tiles for every SM and stays (45.4 there,
+        # 43.8 here).  Two row blocks are two slabs of the decode GEMM's grid: 256 tokens 666-711 us there, 700-771 here,
+        # 384 tokens 967-1004 there, 902-906 here; the line could lie at 256.
         if self.T <= 128 and epi != 1:
             ops.gemm_decode(x, w, out, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w, sumsq_out=sumsq_out)
             return

@@ -82,11 +82,12 @@ class LlamaTPDecoder:
         assert cfg.vocab % world == 0 and cfg.head_dim == 128 and (cfg.ffn // world) % 64 == 0
         assert backend in ("penny", "penny_unfused", "nccl") and linears in ("auto", "penny", "cublas")
         if linears == "auto":
-            # measured (one layer's four linears replayed from a graph, batch 256): this library's decode
-            # GEMM is a weight-streaming kernel with a 128-row batch tile, 56.9 vs 34.3 us at TP 8 and 231 vs
-            # 119 us at TP 1 against the library GEMM once the problem is compute-bound (the tiled GEMM was
-            # measured there on the LM head only, see own_head); up to 128 rows it is level (95 vs 92 us
-            # at TP 1, batch 64) and lets the epilogues fuse
+            # This library's decode GEMM is a weight-streaming kernel with a 128-row batch tile: above 128 rows a step of
+            # 8 Llama-3-8B-shaped layers, norms folded, takes 1651 / 1690 / 1834 / 1958 us at 129 / 160 / 192 / 256 rows
+            # (kv 100) against 1255 / 1295 / 1454 / 1498 with the library's linears (one layer's linears at TP 8 and 256
+            # rows, timed before the folds: 56.9 against 34.3).  The tiled GEMM with its epilogues is level there, 137
+            # against 132 us a layer at 256 rows.  Up to 128 rows the decode GEMM is level by itself (91.9 against 93.7 us
+            # a layer at 64 rows, with silu * up) and lets the norms ride in its epilogues.
             linears = "penny" if max_batch <= 128 else "cublas"
         self.linears, self.pdl = linears, pdl
         # LM head beside the library's linears: on this library's tiles while one row tile of a CTA pair holds the batch.
@@ -153,9 +154,9 @@ class LlamaTPDecoder:
         self.part = self.parts[0]
         if self.fold:
             self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
-            # The folded step's stream stays fp32 from layer to layer (the residual buffer takes it in bf16 at the end): 16
-            # roundings fewer.  Distance of 8 random layers from 64 bits: 0.018 with norms of their own, 0.0145 folded,
-            # 0.012 with this, for 0.3 us a layer.
+            # The folded step's stream stays fp32 from layer to layer (the residual buffer takes it in bf16 at the end), for
+            # 0.3 us a layer.  Logits of 8 / 32 random Llama-3-8B-shaped layers, distance from 64 bits (2-norm): 0.0142 /
+            # 0.0293, with norms of their own and a bf16 stream 0.0189 / 0.0417.
             self.stream = torch.empty(B, H, dtype=torch.float32, device=self.dev)
         self.gu = buf(B, 2 * self.F) if linears == "cublas" else None
         self.act = buf(B, self.F)
@@ -395,7 +396,8 @@ class LlamaTPDecoder:
         s.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(s):
             # (the first warm-up step on separate norms, whichever route the step takes: the second one's tokens, and
-            # with them the rows that it leaves behind the current positions, do not depend on the route)
+            # with them the rows that it leaves behind the current positions, do not depend on the route.  A cache that
+            # is full after the first step keeps none of the second's.)
             for i in range(2):
                 self._step_impl(warm_up=True, separate=i == 0)
         torch.cuda.current_stream().wait_stream(s)
