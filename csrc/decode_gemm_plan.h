@@ -29,9 +29,8 @@ namespace sm100 {
 constexpr int kDecodeMaxSplits = 8;  // portable cluster size
 constexpr int kDecodeMaxBatch = 1024;  // rows of x per launch
 
-PENNY_PLAN_HD int decode_kb_begin(int num_kb, int splits, int r) {
-  return (int)((long long)num_kb * r / splits);
-}
+// (num_kb < 2^25 and r <= 8: no 64-bit division in the kernel's prologue)
+PENNY_PLAN_HD int decode_kb_begin(int num_kb, int splits, int r) { return num_kb * r / splits; }
 // columns owned by one CTA of the cluster, of `bt` that there are
 PENNY_PLAN_HD int decode_slice(int bt, int splits) { return (bt + splits - 1) / splits; }
 // slot of source CTA `src` in the receive area of CTA `dst` (src != dst): sources in rank order, dst left out

@@ -142,6 +142,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
 __device__ __forceinline__ uint64_t advance_desc_k(uint64_t desc, int k) {
   return desc + (uint64_t)(k * (kUmmaK * 2 / 16));
 }
+// A descriptor from its two halves: the upper one is the same for every tile, the lower one is the address in 16-byte
+// units under the constants of make_smem_desc (an address step that stays inside shared memory carries into none of them).
+__device__ __forceinline__ uint64_t make_desc(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
 // kind::f16, A = B = bf16 (format 1), D = fp32 (format 1), both K-major.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -185,6 +188,13 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
 // before the other CTA's accesses.
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The rendezvous after barrier set-up: fence.mbarrier_init has already made the initialised barriers visible to the
+// cluster, so the arrival needs no release (a release held every warp of a prologue for about a microsecond).
+// Not for teardown, where remote arrivals and stores still have to be ordered.
+__device__ __forceinline__ void cluster_sync_after_init() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
