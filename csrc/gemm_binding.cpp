@@ -116,11 +116,14 @@ void bind_gemm(py::module_& m) {
   // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
   // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).  pdl: may start,
   // and without ranges load b, while the kernel before it on the stream still runs, so that kernel must not write
-  // b (a weight); everything else is waited for.
+  // b (a weight); everything else is waited for.  The residual may be fp32, stream_out then takes the sum in bf16 as
+  // well.  sumsq_out [rows of b / 128, M]: a sum for every 128 columns; [rows of b / 16, M]: as many rows as the call returns
+  // hold sums of some columns each, which leaves the width of the tiles free.  block_n, cluster: tile columns and CTAs (or
+  // pairs) that share a tile's K, 0: choose; pair 1 / -1: CTA pairs or single CTAs (0: pairs of 256 x 256 for block_n 512).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
-                        int64_t cluster) {
+                        int64_t cluster, c10::optional<at::Tensor> stream_out, int64_t pair) {
     auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
     TORCH_CHECK(bf16(a) && bf16(b) && bf16(out) && a.dim() == 2 && b.dim() == 2 && out.dim() == 2,
                 "gemm_tile: 2-D bf16 CUDA tensors with contiguous rows");
@@ -156,15 +159,24 @@ void bind_gemm(py::module_& m) {
       g.scale_parts = (int)sumsq->size(0);
     }
     if (epi == 2) {
-      TORCH_CHECK(residual.has_value() && bf16(*residual) && residual->sizes() == out.sizes() &&
+      g.residual_fp32 = residual.has_value() && residual->scalar_type() == at::kFloat;
+      TORCH_CHECK(residual.has_value() && residual->is_cuda() && residual->stride(-1) == 1 &&
+                      (g.residual_fp32 || bf16(*residual)) && residual->sizes() == out.sizes() &&
                       residual->stride(0) == out.stride(0) && norm_w.has_value() == sumsq_out.has_value(),
                   "gemm_tile: residual like out; norm_w and sumsq_out together");
       g.residual = residual->data_ptr();
+      if (stream_out.has_value()) {
+        TORCH_CHECK(g.residual_fp32 && bf16(*stream_out) && stream_out->sizes() == out.sizes() &&
+                        stream_out->stride(0) == out.stride(0), "gemm_tile: stream_out like out, beside an fp32 residual");
+        g.stream_out = stream_out->data_ptr();
+      }
       if (norm_w.has_value()) {
         TORCH_CHECK(bf16(*norm_w) && norm_w->is_contiguous() && norm_w->numel() == g.b_rows && sumsq_out->is_cuda() &&
                         sumsq_out->scalar_type() == at::kFloat && sumsq_out->is_contiguous() &&
-                        sumsq_out->numel() == (int64_t)(g.b_rows / 128) * g.M,
-                    "gemm_tile: contiguous norm_w [rows of b], sumsq_out [rows of b / 128, rows]");
+                        (sumsq_out->numel() == (int64_t)(g.b_rows / 128) * g.M ||
+                         sumsq_out->numel() == (int64_t)(g.b_rows / 16) * g.M),
+                    "gemm_tile: contiguous norm_w [rows of b], sumsq_out [rows of b / 128 or / 16, rows]");
+        g.sumsq_cap = sumsq_out->numel() == (int64_t)(g.b_rows / 128) * g.M ? 0 : g.b_rows / 16;
         g.norm_w = norm_w->data_ptr();
         g.sumsq_out = sumsq_out->data_ptr<float>();
       }
@@ -172,14 +184,18 @@ void bind_gemm(py::module_& m) {
     g.block_n = (int)block_n;
     g.pdl = pdl;
     g.cluster = (int)cluster;
+    g.pair = (int)pair;
+    TORCH_CHECK(epi == 2 || !stream_out.has_value(), "gemm_tile: stream_out beside a residual");
     const at::cuda::OptionalCUDAGuard guard(a.device());
-    const cudaError_t rc =
-        penny::sm100::launch_gemm_tile(g, penny_gemm_error_word(), at::cuda::getCurrentCUDAStream().stream());
+    int sumsq_rows = 0;
+    const cudaError_t rc = penny::sm100::launch_gemm_tile(g, penny_gemm_error_word(),
+                                                          at::cuda::getCurrentCUDAStream().stream(), &sumsq_rows);
     TORCH_CHECK(rc == cudaSuccess, "gemm_tile: ", cudaGetErrorString(rc));
+    return sumsq_rows;
   }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epi") = 0, py::arg("ranges") = py::none(),
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
-     py::arg("cluster") = 0);
+     py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0);
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K, bool folded) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K, folded);
   }, py::arg("B"), py::arg("N"), py::arg("K"), py::arg("folded") = false,

@@ -2,6 +2,9 @@
 #include "gemm_tile_sm100.cuh"
 
 #include <algorithm>
+#include <array>
+#include <map>
+#include <mutex>
 
 #include "gemm_sm100.h"
 #include "kernel_setup.h"
@@ -11,92 +14,151 @@ namespace sm100 {
 
 namespace {
 
-template <bool PAIR, int BN, int EPI>
-cudaError_t launch_tile(const TileGemm& g, TileArgs a, int sms, uint32_t* error_word, cudaStream_t stream) {
-  using Cfg = TileCfg<PAIR, BN>;
+constexpr int kTileSmem = 224 << 10;  // ring and staging of the one CTA of an SM
+
+template <bool PAIR, int EPI, bool SPLIT, int NSUB>
+cudaError_t launch_tile(const TileGemm& g, TileArgs a, TileShape t, int sms, uint32_t* error_word, cudaStream_t stream) {
   constexpr bool kSilu = EPI == TILE_EPI_SILU;
-  a.cl = 1;
-  a.tiles_n = (a.n_out + (kSilu ? BN / 2 : BN) - 1) / (kSilu ? BN / 2 : BN);
-  a.band = std::max(1, 2048 / Cfg::kRows);
+  const int sub_out = kSilu ? t.sub / 2 : t.sub;
+  a.sub = t.sub;
+  a.tiles_n = (a.n_out + t.nsub * sub_out - 1) / (t.nsub * sub_out);
+  a.band = std::max(1, 2048 / t.rows());
   CUtensorMap ma, mb;
   cudaError_t rc = make_tile_map(&ma, g.a, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda, kBlockM);
   if (rc != cudaSuccess) return rc;
   rc = make_tile_map(&mb, g.b, (uint64_t)std::max(1, g.groups) * g.b_rows, (uint64_t)g.K, (uint64_t)g.ldb,
-                     (uint32_t)(PAIR || kSilu ? BN / 2 : BN));
+                     (uint32_t)(PAIR || kSilu ? t.sub / 2 : t.sub));
   if (rc != cudaSuccess) return rc;
-  const void* fn = nullptr;
-  if constexpr (PAIR) fn = reinterpret_cast<const void*>(gemm_tile_pair<BN, EPI>);
-  else fn = reinterpret_cast<const void*>(gemm_tile_single<BN, EPI>);
-  const KernelSetup ks = kernel_setup(fn, Cfg::kSmemBytes, PAIR ? kTileThreads : 0);
+  const auto kernel = gemm_tile_kernel<PAIR, EPI, SPLIT, NSUB>;
+  const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(kernel), kTileSmem, PAIR ? kTileThreads : 0);
   if (ks.rc != cudaSuccess) return ks.rc;
   // grouped: the tile count is only known on the device
-  const long long tiles = (long long)((g.M + Cfg::kRows - 1) / Cfg::kRows) * a.tiles_n;
+  const long long tiles = (long long)((g.M + t.rows() - 1) / t.rows()) * a.tiles_n;
   const int slots = PAIR ? ks.pairs : sms;
-  a.cl = std::max(1, std::min({g.cluster, kTileMaxCluster, a.num_kb}));
   // A cluster works on one tile, so with groups (whose tiles the device counts) no group may have two row tiles.
-  if (a.cl > 1 && g.groups > 0 && g.M > Cfg::kRows) return cudaErrorInvalidValue;
-  const int workers = a.cl > 1 ? (g.groups > 0 ? g.groups * a.tiles_n : (int)tiles) : (g.groups > 0 ? slots : (int)std::min<long long>(slots, tiles));
-  if constexpr (PAIR)
-    return launch_kernel_ex(gemm_tile_pair<BN, EPI>, dim3((unsigned)(2 * workers * a.cl)), dim3(kTileThreads),
-                            Cfg::kSmemBytes, stream, g.pdl, 2 * a.cl, ma, mb, a, error_word);
-  else
-    return launch_kernel_ex(gemm_tile_single<BN, EPI>, dim3((unsigned)(workers * a.cl)), dim3(kTileThreads),
-                            Cfg::kSmemBytes, stream, g.pdl, a.cl, ma, mb, a, error_word);
+  if (SPLIT && g.groups > 0 && g.M > t.rows()) return cudaErrorInvalidValue;
+  long long workers = SPLIT ? (g.groups > 0 ? (long long)g.groups * a.tiles_n : tiles) : (g.groups > 0 ? slots : std::min<long long>(slots, tiles));
+  const int epi_bytes = TileEpi<EPI, SPLIT>::kBytes;
+  const int kb_per = (a.num_kb + a.cl - 1) / a.cl;
+  a.stages = std::min({kTileMaxStages, kb_per, (kTileSmem - epi_bytes - 1024) / t.stage_bytes()});
+  if (SPLIT) {  // the ring takes the peers' sums
+    const int own = (sub_out / 16 + a.cl - 1) / a.cl * 16;
+    const int recv = (a.cl - 1) * std::max(own, a.ss_cols) * (kSilu ? 2 : 1) * kBlockM * 4;
+    a.stages = std::max(a.stages, (recv + t.stage_bytes() - 1) / t.stage_bytes());
+  }
+  a.stages = std::max(a.stages, 2);
+  const int smem = a.stages * t.stage_bytes() + epi_bytes + 1024;
+  if (smem > kTileSmem) return cudaErrorInvalidValue;
+  const int cols = t.nsub * t.sub;
+  a.accs = 2 * cols <= 512 && (g.groups > 0 ? !SPLIT : tiles > workers) ? 2 : 1;
+  a.tmem_cols = 32;
+  while (a.tmem_cols < a.accs * cols) a.tmem_cols *= 2;
+  return launch_kernel_ex(kernel, dim3((unsigned)((PAIR ? 2 : 1) * workers * a.cl)), dim3(kTileThreads), (size_t)smem, stream, g.pdl,
+                          (PAIR ? 2 : 1) * a.cl, ma, mb, a, error_word);
 }
 
-// Tile and cluster by rounds times the time of a K step.  Steps measured on B200, one 4096-long K (us per
-// step, all operands through the 64 B / clk that an SM takes in): 128 x 128 0.32, 128 x 192 0.36, 128 x 256
-// 0.40, 256 x 256 on a pair 0.36.  The exchange of a cluster's sums takes about as long as 13 steps of single
-// CTAs (q / k / v of 128 tokens: 23.2 us whole, 17.5 in two; down 72.5 whole, 31.6 in four, 40.5 on pairs in
-// three) and 18 of a pair.
+// Width of the tiles, CTAs or pairs, and cluster, by a time model that was fitted to 3000 launches on B200 (M 128 to
+// 4096, eight weights of a layer, the three epilogues, chains of launches with weights from HBM).  Its choice took 1.4 %
+// longer than the best of the candidates on average; the figures below are the fit's, in cycles at 1.8 GHz and us:
+//   * a K step takes the MMAs' time (2 cycles a column) or that of filling its stage: 71 bytes a cycle and 64 cycles on
+//     pairs, 83 and 19 on single CTAs;
+//   * a round that is partly empty costs three quarters of a whole one (the rest comes back as clock or as memory
+//     bandwidth for the others);
+//   * the last epilogue, and each one where a single set of accumulators has to be drained first (above 256 columns), 0.6 us
+//     and 0.04 a column; handing the sums of a cluster over 3.2 and 0.03 a column of the share that is sent.
 void choose_tile(TileGemm& g, int sms, int pairs) {
-  const long long m128 = (g.M + 127) / 128, m256 = (g.M + 255) / 256;
   const int num_kb = (g.K + kBlockK - 1) / kBlockK;
-  double best = 0;
-  auto offer = [&](int block_n, int cluster, long long tiles, int slots, double steps) {
-    const double cost = (double)((tiles + slots - 1) / slots) * steps;
-    if (g.block_n == 0 || cost < best) best = cost, g.block_n = block_n, g.cluster = cluster;
-  };
+  const bool silu = g.epi == TILE_EPI_SILU, blocks = g.epi == TILE_EPI_RESIDUAL && g.norm_w != nullptr && g.sumsq_cap <= 0;
   auto clusters = [&](bool pair, int c) {
-    if (pair)
-      return max_clusters(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>), 2 * c, kTileThreads,
-                          TileCfg<true, 256>::kSmemBytes);
-    const void* fn = reinterpret_cast<const void*>(gemm_tile_single<128, TILE_EPI_PLAIN>);
-    if (kernel_setup(fn, TileCfg<false, 128>::kSmemBytes).rc != cudaSuccess) return 0;
-    return max_clusters(fn, c, kTileThreads, TileCfg<false, 128>::kSmemBytes);
+    const void* fn = pair ? reinterpret_cast<const void*>(gemm_tile_kernel<true, TILE_EPI_PLAIN, true, 1>)
+                          : reinterpret_cast<const void*>(gemm_tile_kernel<false, TILE_EPI_PLAIN, true, 1>);
+    if (kernel_setup(fn, kTileSmem).rc != cudaSuccess) return 0;
+    return max_clusters(fn, (pair ? 2 : 1) * c, kTileThreads, kTileSmem);
   };
-  auto cols = [&](int bn) { return (long long)((g.b_rows + bn - 1) / bn); };
-  offer(128, 1, m128 * cols(128), sms, 0.32 * num_kb);
-  if (g.epi == TILE_EPI_PLAIN) offer(192, 1, m128 * cols(192), sms, 0.36 * num_kb);
-  offer(256, 1, m128 * cols(256), sms, 0.40 * num_kb);
-  for (int c = 2; c <= kTileMaxCluster && g.groups == 0; ++c)
-    if (m128 * cols(128) <= clusters(false, c) && num_kb >= 4 * c)
-      offer(128, c, m128 * cols(128), sms, 0.32 * ((num_kb + c - 1) / c + 13));
-  if (pairs > 0 && pair_kernel_enabled()) {
-    const long long tiles = m256 * cols(256);
-    offer(512, 1, tiles, pairs, 0.36 * num_kb);
-    for (int c = 2; c <= kTileMaxCluster && g.groups == 0; ++c)
-      if (tiles <= clusters(true, c) && num_kb >= 4 * c) offer(512, c, tiles, pairs, 0.36 * ((num_kb + c - 1) / c + 18));
+  double best = 0;
+  g.block_n = 0;
+  for (int pair = 0; pair <= (pairs > 0 && pair_kernel_enabled() ? 1 : 0); ++pair) {
+    const int slots = pair ? pairs : sms, rows = pair ? 2 * kBlockM : kBlockM;
+    const double fill = pair ? 71. : 83., step0 = pair ? 64. : 19.;
+    for (int c = 1; c <= (g.groups == 0 ? kTileMaxCluster : 1); ++c) {
+      if (c > 1 && num_kb < 4 * c) break;
+      const int room = c > 1 ? clusters(pair != 0, c) : 0;
+      for (int bn = blocks ? 128 : 64; bn <= (c > 1 ? 256 : 512); bn += blocks ? 128 : (bn < 256 ? 16 : 32)) {
+        const TileShape t{pair != 0, bn > 256 ? bn / 2 : bn, bn > 256 ? 2 : 1};
+        if (blocks && t.sub % 128 != 0) continue;
+        const int sub_out = silu ? t.sub / 2 : t.sub, out = t.nsub * sub_out;
+        if (c > 1 && (sub_out % 16 != 0 || sub_out < 16 * c)) continue;
+        const int n_out = silu ? g.b_rows / 2 : g.b_rows;
+        const int tiles_n = (n_out + out - 1) / out;
+        if (g.sumsq_cap > 0 && tiles_n * c > g.sumsq_cap) continue;
+        const long long tiles = (long long)((g.M + rows - 1) / rows) * tiles_n;
+        if (c > 1 && tiles > room) continue;
+        const double share = (double)tiles * c / slots;
+        const double rounds = 0.75 * (double)((tiles * c + slots - 1) / slots) + 0.25 * std::max(1., share);
+        const double step = std::max(2.1 * bn, t.stage_bytes() / fill + step0) / 1800.;
+        const double drain = 0.6 + 0.04 * (silu ? 0.7 * bn : bn);
+        double cost = rounds * ((num_kb + c - 1) / c) * step + (pair ? 0.6 : 0.);
+        if (c > 1) cost += 3.2 + 0.03 * bn * (c - 1) / c + 0.04 * bn / c;
+        else cost += drain * (2 * bn > 512 ? (double)((tiles + slots - 1) / slots) : 1.);
+        if (g.block_n == 0 || cost < best) best = cost, g.block_n = bn, g.pair = pair ? 1 : -1, g.cluster = c;
+      }
+    }
   }
+}
+
+// The choice depends on the shape and the device alone and takes some 10 us: kept per shape, up to a bound.
+void choose_tile_once(TileGemm& g, int dev, int sms, int pairs) {
+  struct Choice {
+    int block_n, pair, cluster;
+  };
+  static std::mutex mu;
+  static std::map<std::array<int, 9>, Choice> kept;
+  const std::array<int, 9> key = {dev, g.M, g.b_rows, g.K, g.epi, g.groups > 0, g.norm_w != nullptr, g.sumsq_cap, pair_kernel_enabled()};
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = kept.find(key);
+    if (it != kept.end()) {
+      g.block_n = it->second.block_n;
+      g.pair = it->second.pair;
+      g.cluster = it->second.cluster;
+      return;
+    }
+  }
+  choose_tile(g, sms, pairs);
+  std::lock_guard<std::mutex> lock(mu);
+  if (kept.size() >= 4096) kept.clear();
+  kept[key] = Choice{g.block_n, g.pair, g.cluster};
 }
 
 template <int EPI>
-cudaError_t launch_tile_n(const TileGemm& g, const TileArgs& a, int block_n, int sms, uint32_t* error_word,
-                          cudaStream_t stream) {
-  switch (block_n) {
-    case 128: return launch_tile<false, 128, EPI>(g, a, sms, error_word, stream);
-    case 192:
-      if constexpr (EPI == TILE_EPI_PLAIN) return launch_tile<false, 192, EPI>(g, a, sms, error_word, stream);
-      return cudaErrorInvalidValue;
-    case 256: return launch_tile<false, 256, EPI>(g, a, sms, error_word, stream);
-    case 512: return launch_tile<true, 256, EPI>(g, a, sms, error_word, stream);
-    default: return cudaErrorInvalidValue;
-  }
+cudaError_t launch_tile_epi(const TileGemm& g, TileArgs a, int sms, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows) {
+  TileShape t;
+  t.pair = g.pair > 0 || (g.pair == 0 && g.block_n == 512);
+  const int block_n = g.pair == 0 && g.block_n == 512 ? 256 : g.block_n;
+  t.nsub = block_n > 256 ? 2 : 1;
+  t.sub = block_n / t.nsub;
+  if (block_n < 32 || block_n > 512 || block_n % (16 * t.nsub) != 0) return cudaErrorInvalidValue;
+  const int sub_out = EPI == TILE_EPI_SILU ? t.sub / 2 : t.sub;
+  a.cl = std::max(1, std::min({g.cluster, kTileMaxCluster, a.num_kb}));
+  a.ss_cols = EPI == TILE_EPI_RESIDUAL && g.norm_w != nullptr && g.sumsq_cap <= 0 ? 128 : 0;
+  if (a.ss_cols > 0 && t.sub % a.ss_cols != 0) return cudaErrorInvalidValue;
+  if (a.cl > 1 && (t.nsub > 1 || sub_out % 16 != 0 || sub_out < 16 * a.cl)) return cudaErrorInvalidValue;
+  const int ss_rows = a.ss_cols > 0 ? g.b_rows / a.ss_cols : (g.b_rows + t.nsub * t.sub - 1) / (t.nsub * t.sub) * a.cl;
+  if (EPI == TILE_EPI_RESIDUAL && g.norm_w != nullptr && a.ss_cols == 0 && ss_rows > g.sumsq_cap) return cudaErrorInvalidValue;
+  if (sumsq_rows != nullptr) *sumsq_rows = EPI == TILE_EPI_RESIDUAL && g.norm_w != nullptr ? ss_rows : 0;
+  if (a.cl > 1)
+    return t.pair ? launch_tile<true, EPI, true, 1>(g, a, t, sms, error_word, stream)
+                  : launch_tile<false, EPI, true, 1>(g, a, t, sms, error_word, stream);
+  if (t.nsub > 1)
+    return t.pair ? launch_tile<true, EPI, false, 2>(g, a, t, sms, error_word, stream)
+                  : launch_tile<false, EPI, false, 2>(g, a, t, sms, error_word, stream);
+  return t.pair ? launch_tile<true, EPI, false, 1>(g, a, t, sms, error_word, stream)
+                : launch_tile<false, EPI, false, 1>(g, a, t, sms, error_word, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream) {
+cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows) {
   if (g.M <= 0 || g.b_rows <= 0 || g.K <= 0 || g.K % 8 != 0 || g.lda % 8 != 0 || g.ldb % 8 != 0 || g.groups < 0 ||
       g.groups > kTileMaxGroups || (g.groups > 0 && (g.ranges == nullptr || g.scale_sumsq != nullptr)))
     return cudaErrorInvalidValue;
@@ -104,7 +166,8 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   if (g.epi == TILE_EPI_RESIDUAL &&
       (g.groups > 0 || g.b_rows % 128 != 0 || g.ldo % 8 != 0 || g.residual == nullptr ||
        (g.norm_w != nullptr && (g.out == nullptr || g.sumsq_out == nullptr)) ||
-       ((reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.residual) | reinterpret_cast<uintptr_t>(g.norm_w)) & 15u) != 0))
+       ((reinterpret_cast<uintptr_t>(g.out) | reinterpret_cast<uintptr_t>(g.residual) | reinterpret_cast<uintptr_t>(g.stream_out) |
+         reinterpret_cast<uintptr_t>(g.norm_w)) & 15u) != 0))
     return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -123,19 +186,22 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   a.scale_parts = g.scale_parts;
   a.inv_width = 1.f / (float)g.K;
   a.eps = g.eps;
-  a.residual = reinterpret_cast<__nv_bfloat16*>(g.residual);
+  a.residual = reinterpret_cast<char*>(g.residual);
+  a.res_bytes = g.residual_fp32 ? 4 : 2;
+  a.stream_out = reinterpret_cast<__nv_bfloat16*>(g.stream_out);
   a.norm_w = reinterpret_cast<const __nv_bfloat16*>(g.norm_w);
   a.sumsq_out = g.sumsq_out;
   TileGemm c = g;
   if (g.block_n == 0) {
-    const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_pair<256, TILE_EPI_PLAIN>),
-                                        TileCfg<true, 256>::kSmemBytes, kTileThreads);
-    choose_tile(c, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
+    const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_kernel<true, TILE_EPI_PLAIN, false, 1>), kTileSmem,
+                                        kTileThreads);
+    choose_tile_once(c, dev, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
+    if (c.block_n == 0) return cudaErrorInvalidValue;
   }
   switch (g.epi) {
-    case TILE_EPI_PLAIN: return launch_tile_n<TILE_EPI_PLAIN>(c, a, c.block_n, sms, error_word, stream);
-    case TILE_EPI_SILU: return launch_tile_n<TILE_EPI_SILU>(c, a, c.block_n, sms, error_word, stream);
-    case TILE_EPI_RESIDUAL: return launch_tile_n<TILE_EPI_RESIDUAL>(c, a, c.block_n, sms, error_word, stream);
+    case TILE_EPI_PLAIN: return launch_tile_epi<TILE_EPI_PLAIN>(c, a, sms, error_word, stream, sumsq_rows);
+    case TILE_EPI_SILU: return launch_tile_epi<TILE_EPI_SILU>(c, a, sms, error_word, stream, sumsq_rows);
+    case TILE_EPI_RESIDUAL: return launch_tile_epi<TILE_EPI_RESIDUAL>(c, a, sms, error_word, stream, sumsq_rows);
     default: return cudaErrorInvalidValue;
   }
 }

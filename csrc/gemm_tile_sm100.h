@@ -30,17 +30,25 @@ struct TileGemm {
   const float* scale_sumsq;
   int scale_parts;
   float eps;
-  void* residual;       // [M, b_rows], ldo
+  void* residual;       // [M, b_rows], ldo; bf16, or with residual_fp32 fp32
+  bool residual_fp32;
+  void* stream_out;     // residual_fp32: null, or [M, b_rows], ldo: the sum once more in bf16
   const void* norm_w;   // [b_rows]; null: only the residual add (out unused)
-  float* sumsq_out;     // [b_rows / 128][M]
-  int block_n;          // 0: choose; 128 / 192 / 256: single CTAs; 512: CTA pairs, 256 x 256
-  int cluster;          // pairs (block_n 512) or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
+  float* sumsq_out;     // [b_rows / 128][M], or with sumsq_cap > 0 [sumsq_cap][M]
+  int sumsq_cap;        // above 0: the first rows of sumsq_out take one sum per tile, or CTA of a cluster, of its columns
+                        // (launch_gemm_tile says how many rows): any width of tile will do, and a cluster shares out a
+                        // tile's columns evenly
+  int block_n;          // 0: choose; else the columns of a tile: a multiple of 16 up to 256, or of 32 up to 512 (two
+                        // accumulators).  pair = 0: 512 stands for CTA pairs, 256 x 256
+  int pair;             // 0: by block_n; 1: CTA pairs, tiles of 256 rows; -1: single CTAs
+  int cluster;          // pairs or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
                         // groups only for M <= the tile's rows
   bool pdl;             // may start, and without groups load b, while the kernel before it on the stream still runs:
                         // that kernel must not write b
 };
 
-cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream);
+// sumsq_rows: null, or the rows of sumsq_out that the launch writes.
+cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows = nullptr);
 
 }  // namespace sm100
 }  // namespace penny

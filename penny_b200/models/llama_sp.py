@@ -102,7 +102,8 @@ class LlamaSPPrefill:
         # residual add, silu * mul and the norms (see _forward_local)
         self.local = backend == "penny" and world == 1 and not self.cpu and (2 * self.F) % 128 == 0
         if self.local:
-            self.sumsq = [torch.empty(n, tokens, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
+            # (the linears say how many rows of the second one their tiles filled)
+            self.sumsq = [torch.empty(n, tokens, dtype=torch.float32, device=self.dev) for n in (1, H // 16)]
         # kernels of this library per forward: per layer 2 norms, RoPE, silu*mul and (penny) 4 fused GEMMs; on one
         # rank RoPE and 4 GEMMs with the rest in their epilogues, behind one norm
         self.kernels_per_forward = 1 + 5 * self.L if self.local else self.L * (4 + (4 if backend == "penny" else 0))
@@ -176,17 +177,10 @@ class LlamaSPPrefill:
 
     # ------------------------------------------------------------------ forward
     def _gemm(self, x, w, out, epi=0, sumsq=None, residual=None, norm_w=None, sumsq_out=None):
-        """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual)."""
-        # One row block: the narrow linears are a weight stream like a decode step's, and the decode GEMM's smaller CTAs
-        # begin theirs under the launch before (128 tokens, a layer's q/k/v, o and down 19.6 + 19.3 + 37 us in the
-        # forward -> 16 + 17 + 27, 568 -> 498 us for four layers).  Gate/up has tiles for every SM and stays (45.4 there,
-        # 43.8 here).  Two row blocks are two slabs of the decode GEMM's grid: 256 tokens 666-711 us there, 700-771 here,
-        # 384 tokens 967-1004 there, 902-906 here; the line could lie at 256.
-        if self.T <= 128 and epi != 1:
-            ops.gemm_decode(x, w, out, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w, sumsq_out=sumsq_out)
-            return
-        ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
-                      sumsq_out=sumsq_out, pdl=True)
+        """One linear with its epilogue (0 plain, 1 silu * mul, 2 residual); the part of sumsq_out that it wrote."""
+        rows = ops.gemm_tile(x, w, out, epi, sumsq=sumsq, eps=self.cfg.eps, residual=residual, norm_w=norm_w,
+                             sumsq_out=sumsq_out, pdl=True)
+        return sumsq_out[:rows] if sumsq_out is not None else None
 
     def _forward_local(self, x: torch.Tensor) -> torch.Tensor:
         """One rank.  h holds the residual stream times the next norm's weight, sumsq its sums of squares; the
@@ -196,11 +190,11 @@ class LlamaSPPrefill:
         for li, l in enumerate(self.layers):
             self._gemm(h, l["wqkv"], self.qkv, sumsq=ss)
             attn = self._attention()
-            ss = self.sumsq[1]
-            self._gemm(attn, l["wo"], h, 2, residual=res, norm_w=l["norm2"], sumsq_out=ss)
+            ss = self._gemm(attn, l["wo"], h, 2, residual=res, norm_w=l["norm2"], sumsq_out=self.sumsq[1])
             self._gemm(h, l["wgu"], self.act, 1, sumsq=ss)
             if li + 1 < len(self.layers):
-                self._gemm(self.act, l["wd"], h, 2, residual=res, norm_w=self.layers[li + 1]["norm1"], sumsq_out=ss)
+                ss = self._gemm(self.act, l["wd"], h, 2, residual=res, norm_w=self.layers[li + 1]["norm1"],
+                                sumsq_out=self.sumsq[1])
             else:
                 self._gemm(self.act, l["wd"], h, 2, residual=res)
         return res
