@@ -81,17 +81,19 @@ class LlamaTPDecoder:
         assert cfg.heads % world == 0 and cfg.kv_heads % world == 0 and cfg.ffn % world == 0
         assert cfg.vocab % world == 0 and cfg.head_dim == 128 and (cfg.ffn // world) % 64 == 0
         assert backend in ("penny", "penny_unfused", "nccl") and linears in ("auto", "penny", "cublas")
+        # One rank: the linears of the folded step that the tiled GEMM takes (see _layers_folded).
+        self.tiled = self.tiled_linears(cfg, max_batch) if linears == "auto" and world == 1 else frozenset()
         if linears == "auto":
-            # This library's decode GEMM is a weight-streaming kernel with a 128-row batch tile: above 128 rows a step of
-            # 8 Llama-3-8B-shaped layers, norms folded, takes 1651 / 1690 / 1834 / 1958 us at 129 / 160 / 192 / 256 rows
-            # (kv 100) against 1255 / 1295 / 1454 / 1498 with the library's linears (one layer's linears at TP 8 and 256
-            # rows, timed before the folds: 56.9 against 34.3).  The tiled GEMM with its epilogues is level there, 137
-            # against 132 us a layer at 256 rows.  Up to 128 rows the decode GEMM is level by itself (91.9 against 93.7 us
-            # a layer at 64 rows, with silu * up) and lets the norms ride in its epilogues.
+            # Several ranks, and what one rank's step does not have on the tiled GEMM: this library's decode GEMM is a
+            # weight-streaming kernel with a 128-row batch tile, above 128 rows a step of 8 Llama-3-8B-shaped layers, norms
+            # folded, takes 1651 / 1690 / 1834 / 1958 us at 129 / 160 / 192 / 256 rows (kv 100) against 1255 / 1295 / 1454 /
+            # 1498 with the library's linears (one layer's linears at TP 8 and 256 rows, timed before the folds: 56.9
+            # against 34.3).  Up to 128 rows it is level by itself (91.9 against 93.7 us a layer at 64 rows, with silu * up)
+            # and lets the norms ride in its epilogues.
             linears = "penny" if max_batch <= 128 else "cublas"
         self.linears, self.pdl = linears, pdl
-        # LM head beside the library's linears: on this library's tiles while one row tile of a CTA pair holds the batch.
-        # Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 / 217 / 222 us against the library's
+        # LM head beside the library's linears (layers under hidden 2048, several ranks): on this library's tiles while one
+        # row tile of a CTA pair holds the batch.  Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 / 217 / 222 us against the library's
         # 224 / 293 / 238 / 328; vocabularies of 65536 to 151936 and hidden 2048 to 8192: 0.95 to 1.5 times as fast,
         # 1.2 on average.  Level at 192.  A second row tile that is partly filled costs a whole one: 257 / 384 / 512
         # / 1024 rows 359 / 374 / 524 / 858 against 263 / 307 / 499 / 836.  Smaller vocabulary shards (32000: 0.84 to
@@ -133,7 +135,7 @@ class LlamaTPDecoder:
             self._push = comm.fused_norm_push_target(max_batch, H)
         # One rank on this library's linears: the residual add and the norms ride in the GEMM epilogues (two launches
         # of 2 us each less per layer).
-        self.fold = world == 1 and linears == "penny" and max_batch <= 1024 and cfg.hidden % 128 == 0
+        self.fold = bool(self.tiled) or (world == 1 and linears == "penny" and max_batch <= 1024 and cfg.hidden % 128 == 0)
         self._init_weights(seed, full_init)
 
         def buf(*shape, dtype=dt, heap=False):
@@ -153,7 +155,8 @@ class LlamaTPDecoder:
         self.parts = [buf(B, H, heap=True), buf(B, H, heap=True)]
         self.part = self.parts[0]
         if self.fold:
-            self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
+            # (the tiled GEMM says how many rows of the second one its tiles filled)
+            self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // (16 if self.tiled else 128))]
             # The folded step's stream stays fp32 from layer to layer (the residual buffer takes it in bf16 at the end), for
             # 0.3 us a layer.  Logits of 8 / 32 random Llama-3-8B-shaped layers, distance from 64 bits (2-norm): 0.0142 /
             # 0.0293, with norms of their own and a bf16 stream 0.0189 / 0.0417.
@@ -191,6 +194,26 @@ class LlamaTPDecoder:
         self.kernels_per_step = cfg.layers * per_layer + norms + 1 + (2 if world > 1 else 0) + own_head
         if self.fold:
             self.kernels_per_step = 5 * cfg.layers + 3
+
+    @staticmethod
+    def tiled_linears(cfg: LlamaConfig, batch: int) -> frozenset:
+        """The linears of one rank's folded step that run on the tiled GEMM, the others on the decode GEMM.
+
+        8 Llama-3-8B-shaped layers and the head, kv 100, us.  Up to 64 rows none (64: 948, with q/k/v, gate/up and head 963);
+        to 128 rows those three, which have tiles for every SM, while o and down are a weight stream that the decode GEMM's
+        smaller CTAs begin under the launch before (65 / 96 / 128 rows: none 1010 / 1077 / 1157, three 984 / 1042 / 1093, all
+        1016 / 1090 / 1144); above, where the decode GEMM reads x in slabs, all (129 / 160 / 192 / 256: the library's linears
+        with norms and silu * up of their own 1295 / 1294 / 1429 / 1543, all 1210 / 1255 / 1302 / 1398).  257 to 384 rows need a
+        third, partly filled row tile (257: 1741 / 1822) and stay with the library, as do larger batches (512: 2481 / 2322,
+        but at hidden 8192 768 rows 2711 / 3083).
+        Hidden 2048 the same (65 / 128 rows three 418 / 495 for 441 / 547, 144 / 208 all 542 / 584 for 572 / 636); hidden
+        8192 from 177 rows (two layers, 144 / 176 / 208 rows: 1001 / 1063 / 1084 for 937 / 1067 / 1147), three at 65 / 128
+        789 / 841 for 840 / 922.  Smaller layers were not timed."""
+        if cfg.hidden < 2048 or cfg.hidden % 128 or not 64 < batch <= 256:
+            return frozenset()
+        if batch <= 128:
+            return frozenset(("qkv", "gate_up", "head"))
+        return frozenset() if cfg.hidden >= 8192 and batch <= 176 else frozenset(("qkv", "o", "gate_up", "down", "head"))
 
     # ------------------------------------------------------------------ weights
     def _init_weights(self, seed: int, full_init: bool):
@@ -238,7 +261,7 @@ class LlamaTPDecoder:
             layer = dict(
                 wqkv=wqkv, wo=row_shard(H, cfg.heads * D, base + 3), wgu=wgu, wdown=row_shard(H, cfg.ffn, base + 6),
                 norm1=torch.ones(H, dtype=dt, device=self.dev), norm2=torch.ones(H, dtype=dt, device=self.dev))
-            if self.linears == "cublas":
+            if self.linears == "cublas" or "gate_up" in self.tiled:
                 layer["wgu_cat"] = torch.cat(self.split_gate_up(wgu)).contiguous()
             self.layers.append(layer)
 
@@ -314,23 +337,35 @@ class LlamaTPDecoder:
             ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, 0, push)
 
     def _layers_folded(self, tokens):
-        """One rank: five launches per layer.  x holds the residual stream times the next norm's weight, sumsq its
+        """One rank: five launches per layer, each linear on the tiled or on the decode GEMM (`tiled_linears`).  x holds the residual stream times the next norm's weight, sumsq its
         sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
         x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.stream, self.pdl
+        tiled, parts = self.tiled, self.sumsq[1]
+
+        def linear(name, x, w, out, silu=False, **fold):
+            """The rows of the sums of squares that it wrote, for a linear with a residual."""
+            if name not in tiled:
+                if "residual" in fold:
+                    fold["sumsq_out"] = parts[:w.shape[0] // 128]
+                ops.gemm_decode(x, w, out, silu, pdl=pdl, eps=eps, **fold)
+                return fold.get("sumsq_out")
+            if "residual" not in fold:
+                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, **fold)
+                return None
+            return parts[:ops.gemm_tile(x, w, out, 2, pdl=pdl, eps=eps, sumsq_out=parts, **fold)]
         ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
         for li, L in enumerate(self.layers):
-            ops.gemm_decode(x, L["wqkv"], self.qkv, pdl=pdl, sumsq=ss, eps=eps)
+            linear("qkv", x, L["wqkv"], self.qkv, sumsq=ss)
             ops.decode_attention_fused(self.qkv, self.kcache[li], self.vcache[li], self.positions, self.attn,
                                        self.workspace, self.Hq, self.Hkv, self.pieces, self.scale, self.cfg.rope_theta,
                                        pdl, balance=True)
-            ss = self.sumsq[1]
-            ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=res, norm_w=L["norm2"], sumsq_out=ss)
-            ops.gemm_decode(x, L["wgu"], self.act, True, pdl=pdl, sumsq=ss, eps=eps)
+            ss = linear("o", self.attn, L["wo"], x, residual=res, norm_w=L["norm2"])
+            linear("gate_up", x, L["wgu_cat" if "gate_up" in tiled else "wgu"], self.act, True, sumsq=ss)
             last = li + 1 == self.cfg.layers
-            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=res, sumsq_out=ss,
-                            norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
-                            stream_out=self.residual if last else None)
-        ops.gemm_decode(x, self.lm_head, self.logits, pdl=pdl, sumsq=ss, eps=eps)
+            ss = linear("down", self.act, L["wdown"], x, residual=res,
+                        norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
+                        stream_out=self.residual if last else None)
+        linear("head", x, self.lm_head, self.logits, sumsq=ss)
 
     def _layers(self, warm_up: bool):
         cfg = self.cfg
