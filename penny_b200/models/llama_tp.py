@@ -82,6 +82,7 @@ class LlamaTPDecoder:
         assert cfg.vocab % world == 0 and cfg.head_dim == 128 and (cfg.ffn // world) % 64 == 0
         assert backend in ("penny", "penny_unfused", "nccl") and linears in ("auto", "penny", "cublas")
         # One rank: the linears of the folded step that the tiled GEMM takes (see _layers_folded).
+        asked = linears
         self.tiled = self.tiled_linears(cfg, max_batch) if linears == "auto" and world == 1 else frozenset()
         if linears == "auto":
             # Several ranks, and what one rank's step does not have on the tiled GEMM: this library's decode GEMM is a
@@ -91,6 +92,11 @@ class LlamaTPDecoder:
             # against 34.3).  Up to 128 rows it is level by itself (91.9 against 93.7 us a layer at 64 rows, with silu * up)
             # and lets the norms ride in its epilogues.
             linears = "penny" if max_batch <= 128 else "cublas"
+        # One rank beside the library's linears: gate/up on the tiled GEMM, whose epilogue takes silu * up.  8 layers and the
+        # head: 129 / 144 / 160 / 176 rows level to 2 % slower, 192 / 224 / 256 rows 1801 / 1613 / 2797 -> 1732 / 1528 / 2728 us (kv
+        # 300 / 16 / 1024); alone 512 rows 88 us against 98 and 8 for the kernel behind it.  Layers under hidden 2048 were not
+        # timed.
+        self.tiled_gate_up = asked == "auto" and world == 1 and max_batch > 176 and cfg.hidden >= 2048
         self.linears, self.pdl = linears, pdl
         # LM head beside the library's linears (layers under hidden 2048, several ranks): on this library's tiles while one
         # row tile of a CTA pair holds the batch.  Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 / 217 / 222 us against the library's
@@ -202,18 +208,10 @@ class LlamaTPDecoder:
         8 Llama-3-8B-shaped layers and the head, kv 100, us.  Up to 64 rows none (64: 948, with q/k/v, gate/up and head 963);
         to 128 rows those three, which have tiles for every SM, while o and down are a weight stream that the decode GEMM's
         smaller CTAs begin under the launch before (65 / 96 / 128 rows: none 1010 / 1077 / 1157, three 984 / 1042 / 1093, all
-        1016 / 1090 / 1144); above, where the decode GEMM reads x in slabs, all (129 / 160 / 192 / 256: the library's linears
-        with norms and silu * up of their own 1295 / 1294 / 1429 / 1543, all 1210 / 1255 / 1302 / 1398).  257 to 384 rows need a
-        third, partly filled row tile (257: 1741 / 1822) and stay with the library, as do larger batches (512: 2481 / 2322,
-        but at hidden 8192 768 rows 2711 / 3083).
-        Hidden 2048 the same (65 / 128 rows three 418 / 495 for 441 / 547, 144 / 208 all 542 / 584 for 572 / 636); hidden
-        8192 from 177 rows (two layers, 144 / 176 / 208 rows: 1001 / 1063 / 1084 for 937 / 1067 / 1147), three at 65 / 128
-        789 / 841 for 840 / 922.  Smaller layers were not timed."""
-        if cfg.hidden < 2048 or cfg.hidden % 128 or not 64 < batch <= 256:
-            return frozenset()
-        if batch <= 128:
-            return frozenset(("qkv", "gate_up", "head"))
-        return frozenset() if cfg.hidden >= 8192 and batch <= 176 else frozenset(("qkv", "o", "gate_up", "down", "head"))
+        1016 / 1090 / 1144).  Hidden 2048: 65 / 128 rows three 418 / 495 for 441 / 547; hidden 8192, two layers, 789 / 841 for
+        840 / 922.  Smaller layers were not timed.  Larger batches are not folded: all five on tiles took 3 to 7 % longer at
+        129 to 176 rows than the library's linears.  (They took 5 to 10 % less from 192 rows on.)"""
+        return frozenset(("qkv", "gate_up", "head")) if cfg.hidden >= 2048 and cfg.hidden % 128 == 0 and 64 < batch <= 128 else frozenset()
 
     # ------------------------------------------------------------------ weights
     def _init_weights(self, seed: int, full_init: bool):
@@ -367,7 +365,7 @@ class LlamaTPDecoder:
                         stream_out=self.residual if last else None)
         linear("head", x, self.lm_head, self.logits, sumsq=ss)
 
-    def _layers(self, warm_up: bool):
+    def _layers(self, warm_up: bool, separate: bool):
         cfg = self.cfg
         torch.index_select(self.embed, 0, self.tokens, out=self.residual)
         ops.add_rmsnorm(self.residual, None, self.layers[0]["norm1"], self.x, None, cfg.eps)
@@ -387,6 +385,9 @@ class LlamaTPDecoder:
             if self.linears == "penny":
                 self._linear(self.x, L["wgu"], self.act, silu_pairs=True)
                 self._linear(self.act, L["wdown"], self.parts[1], push=self._push)
+            elif self.tiled_gate_up and not separate:
+                ops.gemm_tile(self.x, L["wgu_cat"], self.act, 1, pdl=self.pdl)
+                torch.matmul(self.act, L["wdown"].t(), out=self.parts[1])
             else:
                 torch.matmul(self.x, L["wgu_cat"].t(), out=self.gu)
                 ops.silu_mul(self.gu, self.act)
@@ -407,7 +408,7 @@ class LlamaTPDecoder:
         if self.fold and not separate:
             self._layers_folded(self._host_in if host else self.tokens)
         else:
-            self._layers(warm_up)
+            self._layers(warm_up, separate)
         # greedy sampling: per-row (value, index) of this rank's vocabulary shard (indices < 2^24, exact
         # in fp32), gathered over the ranks; one kernel then picks the best rank per sequence, feeds the
         # token back (step() overwrites self.tokens with the caller's tokens) and advances the positions
