@@ -232,10 +232,11 @@ void bind_decode(py::module_& m) {
   // A MoE layer of one rank: router, rows by expert, expert SwiGLU FFNs, gate-weighted sum.  Nothing comes
   // back to the host, and it is one call: as Python calls the launches took 113 us of host time, of which a
   // layer of a few tokens hid half.  w13: per expert [2 ffn, hidden] (gate rows, then up rows), w2: [hidden, ffn], each
-  // list one stack, else None is returned and nothing runs; block_n and down_cluster as in gemm_tile.  The router meets
+  // list one stack, else None is returned and nothing runs; block_n and down_cluster as in gemm_tile, up_rows and down_rows
+  // above 0: gate/up and down with the weight on the M side (gemm_tile's pair 2) and tiles of that many rows.  The router meets
   // the library's GEMM only and may have any strides.
   m.def("moe_layer", [](at::Tensor x, at::Tensor router, const std::vector<at::Tensor>& w13, const std::vector<at::Tensor>& w2,
-                        int64_t topk, int64_t block_n, int64_t down_cluster) -> c10::optional<at::Tensor> {
+                        int64_t topk, int64_t block_n, int64_t down_cluster, int64_t up_rows, int64_t down_rows) -> c10::optional<at::Tensor> {
     if (!stacked(w13) || !stacked(w2)) return c10::nullopt;
     need(bf16_cuda(x) && x.dim() == 2 && ((uintptr_t)x.data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 x");
     need(router.is_cuda() && router.scalar_type() == at::kBFloat16 && router.dim() == 2, "moe_layer: 2-D bf16 router");
@@ -266,7 +267,11 @@ void bind_decode(py::module_& m) {
     g.groups = E;
     g.ranges = borders;
     g.range_stride = 1;
-    g.block_n = (int)block_n;
+    auto tiles = [&](int64_t rows) {
+      g.pair = rows > 0 ? 2 : 0;
+      g.block_n = (int)(rows > 0 ? rows : block_n);
+    };
+    tiles(up_rows);
     g.pdl = true;
     ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "moe_layer: gate / up");
     g.a = act.data_ptr();
@@ -276,11 +281,13 @@ void bind_decode(py::module_& m) {
     g.K = g.lda = g.ldb = F;
     g.ldo = H;
     g.epi = sm100::TILE_EPI_PLAIN;
-    g.cluster = (int)down_cluster;
+    tiles(down_rows);
+    g.cluster = down_rows > 0 ? 0 : (int)down_cluster;
     ck(sm100::launch_gemm_tile(g, penny_gemm_error_word(), stream), "moe_layer: down");
     ck(launch_moe_sum(rows.data_ptr(), row_of_pair, gates.data_ptr<float>(), T, (int)topk, H, out.data_ptr(), stream), "moe_layer: sum");
     return out;
-  }, py::arg("x"), py::arg("router"), py::arg("w13"), py::arg("w2"), py::arg("topk"), py::arg("block_n"), py::arg("down_cluster"));
+  }, py::arg("x"), py::arg("router"), py::arg("w13"), py::arg("w2"), py::arg("topk"), py::arg("block_n"), py::arg("down_cluster"),
+     py::arg("up_rows") = 0, py::arg("down_rows") = 0);
   m.def("sample_finish", [](at::Tensor pairs, int64_t world, at::Tensor next_tokens, at::Tensor tokens,
                             at::Tensor positions) {
     const int64_t B = next_tokens.numel();

@@ -119,7 +119,8 @@ void bind_gemm(py::module_& m) {
   // b (a weight); everything else is waited for.  The residual may be fp32, stream_out then takes the sum in bf16 as
   // well.  sumsq_out [rows of b / 128, M]: a sum for every 128 columns; [rows of b / 16, M]: as many rows as the call returns
   // hold sums of some columns each, which leaves the width of the tiles free.  block_n, cluster: tile columns and CTAs (or
-  // pairs) that share a tile's K, 0: choose; pair 1 / -1: CTA pairs or single CTAs (0: pairs of 256 x 256 for block_n 512).
+  // pairs) that share a tile's K, 0: choose; pair 1 / -1: CTA pairs or single CTAs (0: pairs of 256 x 256 for block_n 512), 2: pairs with the weight on the M side and
+  // up to block_n rows of a (plain or silu).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,

@@ -1,5 +1,5 @@
 // Launchers of the tiled GEMM (kernel: gemm_tile_sm100.cuh).
-#include "gemm_tile_sm100.cuh"
+#include "gemm_swap_sm100.cuh"
 
 #include <algorithm>
 #include <array>
@@ -130,6 +130,44 @@ void choose_tile_once(TileGemm& g, int dev, int sms, int pairs) {
   kept[key] = Choice{g.block_n, g.pair, g.cluster};
 }
 
+template <bool SILU>
+cudaError_t launch_swap(const TileGemm& g, const TileArgs& t, uint32_t* error_word, cudaStream_t stream) {
+  const int width = g.block_n > 0 ? g.block_n : 256;
+  if (width % 16 != 0 || width < 16 || width > 256 || g.cluster > 1) return cudaErrorInvalidValue;
+  SwapArgs a = {};
+  a.out = t.out;
+  a.ldo = t.ldo;
+  a.M = t.M;
+  a.n_out = t.n_out;
+  a.num_kb = t.num_kb;
+  const int cols = SILU ? kBlockM : 2 * kBlockM;  // of out that a pair's rows of the weight are
+  a.m_tiles = (t.n_out + cols - 1) / cols;
+  a.groups = t.groups;
+  a.b_rows = t.b_rows;
+  a.width = width;
+  a.ranges = t.ranges;
+  a.range_stride = t.range_stride;
+  a.scale_sumsq = t.scale_sumsq;
+  a.scale_parts = t.scale_parts;
+  a.inv_width = t.inv_width;
+  a.eps = t.eps;
+  a.stage_bytes = kTileABytes + width / 2 * kBlockK * 2;
+  const int rest = 8 * kSwapWarpBytes + kSwapScaleBytes + 1024;
+  a.stages = std::min(kTileMaxStages, (kTileSmem - rest) / a.stage_bytes);
+  CUtensorMap mw, mx;
+  cudaError_t rc = make_tile_map(&mw, g.b, (uint64_t)std::max(1, g.groups) * g.b_rows, (uint64_t)g.K, (uint64_t)g.ldb,
+                                 (uint32_t)(SILU ? kBlockM / 2 : kBlockM));
+  if (rc != cudaSuccess) return rc;
+  rc = make_tile_map(&mx, g.a, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda, (uint32_t)(width / 2));
+  if (rc != cudaSuccess) return rc;
+  const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_swap_kernel<SILU>), kTileSmem, kTileThreads);
+  if (ks.rc != cudaSuccess) return ks.rc;
+  const long long tiles = (long long)((g.M + width - 1) / width) * a.m_tiles;  // grouped: counted on the device
+  const int workers = (int)(g.groups > 0 ? ks.pairs : std::min<long long>(ks.pairs, tiles));
+  return launch_kernel_ex(gemm_swap_kernel<SILU>, dim3((unsigned)(2 * workers)), dim3(kTileThreads),
+                          (size_t)(a.stages * a.stage_bytes + rest), stream, g.pdl, 2, mw, mx, a, error_word);
+}
+
 template <int EPI>
 cudaError_t launch_tile_epi(const TileGemm& g, TileArgs a, int sms, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows) {
   TileShape t;
@@ -191,6 +229,11 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   a.stream_out = reinterpret_cast<__nv_bfloat16*>(g.stream_out);
   a.norm_w = reinterpret_cast<const __nv_bfloat16*>(g.norm_w);
   a.sumsq_out = g.sumsq_out;
+  if (sumsq_rows != nullptr) *sumsq_rows = 0;
+  if (g.pair == 2) {
+    if (g.epi == TILE_EPI_PLAIN) return launch_swap<false>(g, a, error_word, stream);
+    return g.epi == TILE_EPI_SILU ? launch_swap<true>(g, a, error_word, stream) : cudaErrorInvalidValue;
+  }
   TileGemm c = g;
   if (g.block_n == 0) {
     const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_kernel<true, TILE_EPI_PLAIN, false, 1>), kTileSmem,

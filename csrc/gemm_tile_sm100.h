@@ -40,7 +40,9 @@ struct TileGemm {
                         // tile's columns evenly
   int block_n;          // 0: choose; else the columns of a tile: a multiple of 16 up to 256, or of 32 up to 512 (two
                         // accumulators).  pair = 0: 512 stands for CTA pairs, 256 x 256
-  int pair;             // 0: by block_n; 1: CTA pairs, tiles of 256 rows; -1: single CTAs
+  int pair;             // 0: by block_n; 1: CTA pairs, tiles of 256 rows; -1: single CTAs; 2: pairs with 256 rows of the
+                        // weight on the M side and tiles of up to block_n rows of a (a multiple of 16 up to 256, 0: 256),
+                        // plain or silu, no cluster
   int cluster;          // pairs or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
                         // groups only for M <= the tile's rows
   bool pdl;             // may start, and without groups load b, while the kernel before it on the stream still runs:

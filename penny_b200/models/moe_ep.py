@@ -136,6 +136,21 @@ def expert_tiles(rows: int, experts: int, hidden: int, ffn: int, sms: int):
     return (512 if rows > 640 * experts and ops.gemm_pair_enabled() else 256), (2 if shared else 0)
 
 
+def expert_rows(rows: int, experts: int):
+    """Rows per tile of gate/up and of down where one rank's grouped GEMMs have the weight on the M side, 0 where
+    `expert_tiles` holds.
+
+    There a group's rows are paid to the next 16 instead of 128 or 256, and few rows leave the shared memory to the
+    weights.  The whole layer (8 experts, hidden 4096, ffn 14336, four draws of the router each) against tiles of rows,
+    by rows per expert: 0.75 (3 tokens) 0.85 with 16 rows in both, 2 and 5 0.98 and 0.99; 15 and 40 0.975 and 0.979 with
+    128 in gate/up alone, 0.978 and 0.989 in both; 60 and 75 1.00 and 1.01; 88 0.99, 105 to 250 0.93, 0.87, 1.00 and 0.89 with
+    256 in both, 310 to 1024 0.89 to 0.96."""
+    per = rows / experts
+    if not ops.gemm_pair_enabled() or 52 < per < 88:
+        return 0, 0
+    return (256, 256) if per >= 88 else (128, 0) if per > 6 else (16, 16)
+
+
 class MoeEPLayer:
     def __init__(self, cfg: MoeConfig, comm, tokens: int, cap_factor: float = 2.0, backend: str = "penny",
                  seed: int = 0, use_own_gemm: bool = True):
@@ -233,7 +248,7 @@ class MoeEPLayer:
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
                 and cfg.topk <= 8 and cfg.experts <= 256):
             out = ops.moe_layer(x0, self.router[0], self.w13[0][:self.epr], self.w2[0][:self.epr], cfg.topk,
-                                *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms))
+                                *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms), *expert_rows(pairs, self.epr))
             if out is not None:
                 return [out] if comm.emulated else out
         ids, gates, tables = [], [], []

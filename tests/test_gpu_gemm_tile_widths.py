@@ -16,8 +16,8 @@ def _data(M, N, K):
 
 
 def _close(out, want):
-    # one rounding to bf16: at most 2^-9 of the value, 2^-9 / sqrt(3) of the 2-norm
-    assert ((out.float() - want).norm() / want.norm()).item() < 2 ** -9
+    # one rounding to bf16 (8 bits): at most 2^-8 of every value, and so of the 2-norm
+    assert ((out.float() - want).norm() / want.norm()).item() < 2 ** -8
     torch.testing.assert_close(out.float(), want, atol=1e-4 * want.std().item(), rtol=2 ** -8)
 
 
@@ -41,7 +41,7 @@ def test_plain_and_silu(M, bn, cl, pair):
     ops.gemm_tile(a, b, act, 1, sumsq=ss, block_n=bn, cluster=cl, pair=pair)
     assert ops.gemm_error() == 0
     want = torch.nn.functional.silu(y[:, :N // 2]) * y[:, N // 2:]
-    assert ((act.float() - want).norm() / want.norm()).item() < 2 ** -9
+    assert ((act.float() - want).norm() / want.norm()).item() < 2 ** -8
 
 
 @pytest.mark.parametrize("bn,cl,pair", SHAPES + [(0, 0, 0)])
