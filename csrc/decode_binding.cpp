@@ -126,13 +126,14 @@ void bind_decode(py::module_& m) {
     need(B >= 1 && Hkv >= 1, "decode_attn_balanced_splits: rows and KV heads");
     return (int64_t)decode_attn_balanced_splits((int)B, (int)Hkv);
   });
-  m.def("silu_mul", [](at::Tensor gate_up, at::Tensor out) {
+  // pairs: gate and up columns in turn, 64 of each (what a weight in gemm_decode's silu_pairs layout gives)
+  m.def("silu_mul", [](at::Tensor gate_up, at::Tensor out, bool pairs) {
     need(bf16_cuda(gate_up) && bf16_cuda(out) && gate_up.dim() == 2, "silu_mul expects [rows, 2F] bf16");
     const int64_t rows = gate_up.size(0), F = gate_up.size(1) / 2;
     need(out.numel() == rows * F, "silu_mul output must be [rows, F]");
     const at::cuda::OptionalCUDAGuard guard(gate_up.device());
-    ck(launch_silu_mul(gate_up.data_ptr(), out.data_ptr(), (int)rows, (int)F, cur()), "silu_mul");
-  });
+    ck(launch_silu_mul(gate_up.data_ptr(), out.data_ptr(), (int)rows, (int)F, cur(), pairs ? 64 : 0), "silu_mul");
+  }, py::arg("gate_up"), py::arg("out"), py::arg("pairs") = false);
   // dst (int64 in host memory) = src; returns whether every id lies in [0, rows).  One call from Python for both: a look at
   // the ids by numpy beside the copy was 1.3 us of a step, more on a cold first one.
   m.def("take_ids", [](at::Tensor src, at::Tensor dst, int64_t rows) {

@@ -390,16 +390,18 @@ __global__ void k_attn_merge(const float* __restrict__ part_o, const float* __re
   *reinterpret_cast<uint2*>(out + ((size_t)b * Hq + hq) * kD + lane * 4) = raw;
 }
 
-// out[b, j] = silu(gu[b, j]) * gu[b, F + j]; 8 elements per thread
+// out[b, j] = silu(gu[b, j]) * gu[b, F + j]; 8 elements per thread.  `block`: gate and up columns come in turn, that many
+// (a multiple of 8) of each; F: all gate columns before all up columns.
 __global__ void k_silu_mul(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
-                           int rows, int F) {
+                           int rows, int F, int block) {
   const size_t vec_per_row = (size_t)F / 8;
   const size_t total = (size_t)rows * vec_per_row;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / vec_per_row, c = (i % vec_per_row) * 8;
-    const uint4 g = *reinterpret_cast<const uint4*>(gu + r * 2 * F + c);
-    const uint4 u = *reinterpret_cast<const uint4*>(gu + r * 2 * F + F + c);
+    const __nv_bfloat16* gate = gu + r * 2 * F + c + (int)c / block * block;
+    const uint4 g = *reinterpret_cast<const uint4*>(gate);
+    const uint4 u = *reinterpret_cast<const uint4*>(gate + block);
     const __nv_bfloat162* gp = reinterpret_cast<const __nv_bfloat162*>(&g);
     const __nv_bfloat162* up = reinterpret_cast<const __nv_bfloat162*>(&u);
     uint4 o;
@@ -640,12 +642,13 @@ cudaError_t launch_decode_attention(const void* qkv, const void* kcache, const v
   return cudaGetLastError();
 }
 
-cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cudaStream_t stream) {
-  if (F % 8 != 0) return cudaErrorInvalidValue;
+cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cudaStream_t stream, int block) {
+  if (block <= 0) block = F;
+  if (F % 8 != 0 || block % 8 != 0 || (block > 0 && F % block != 0)) return cudaErrorInvalidValue;
   const size_t total = (size_t)rows * (F / 8);
   const int blocks = (int)((total + 255) / 256 > 148 * 8 ? 148 * 8 : (total + 255) / 256);
   k_silu_mul<<<blocks < 1 ? 1 : blocks, 256, 0, stream>>>((const __nv_bfloat16*)gate_up,
-                                                          (__nv_bfloat16*)out, rows, F);
+                                                          (__nv_bfloat16*)out, rows, F, block);
   return cudaGetLastError();
 }
 

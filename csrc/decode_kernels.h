@@ -47,7 +47,7 @@ cudaError_t launch_decode_attention_fused(const void* qkv, void* kcache, void* v
 int decode_attn_balanced_splits(int B, int Hkv);
 
 // gate_up: [rows, 2F] (gate | up) -> out [rows, F] = silu(gate) * up
-cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cudaStream_t stream);
+cudaError_t launch_silu_mul(const void* gate_up, void* out, int rows, int F, cudaStream_t stream, int block = 0);
 
 // logits: [rows, cols] bf16 -> per-row max value and index (+ index_base).  workspace: zeroed once,
 // argmax_workspace_bytes(rows) bytes (nullptr: one block per row); pair: optional [2 * rows] fp32

@@ -112,7 +112,7 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("stream_out") = py::none());
   // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
-  // rows before its up rows, out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
+  // rows before its up rows, or with silu_pairs, without ranges, as for gemm_decode; out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
   // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
   // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).  pdl: may start,
   // and without ranges load b, while the kernel before it on the stream still runs, so that kernel must not write
@@ -124,7 +124,7 @@ void bind_gemm(py::module_& m) {
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
-                        int64_t cluster, c10::optional<at::Tensor> stream_out, int64_t pair) {
+                        int64_t cluster, c10::optional<at::Tensor> stream_out, int64_t pair, bool silu_pairs) {
     auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
     TORCH_CHECK(bf16(a) && bf16(b) && bf16(out) && a.dim() == 2 && b.dim() == 2 && out.dim() == 2,
                 "gemm_tile: 2-D bf16 CUDA tensors with contiguous rows");
@@ -186,6 +186,7 @@ void bind_gemm(py::module_& m) {
     g.pdl = pdl;
     g.cluster = (int)cluster;
     g.pair = (int)pair;
+    g.silu_pairs = silu_pairs;
     TORCH_CHECK(epi == 2 || !stream_out.has_value(), "gemm_tile: stream_out beside a residual");
     const at::cuda::OptionalCUDAGuard guard(a.device());
     int sumsq_rows = 0;
@@ -196,7 +197,8 @@ void bind_gemm(py::module_& m) {
   }, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("epi") = 0, py::arg("ranges") = py::none(),
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
-     py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0);
+     py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0,
+     py::arg("silu_pairs") = false);
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K, bool folded) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K, folded);
   }, py::arg("B"), py::arg("N"), py::arg("K"), py::arg("folded") = false,

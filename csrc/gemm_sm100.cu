@@ -102,6 +102,23 @@ cudaError_t make_tile_map(CUtensorMap* map, const void* base, uint64_t rows, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t make_gate_up_map(CUtensorMap* map, const void* base, uint64_t blocks, uint64_t rows, uint64_t cols,
+                             uint64_t row_stride_elems, uint32_t box_blocks, uint32_t box_rows) {
+  EncodeFn fn = encode_fn();
+  if (fn == nullptr) return cudaErrorNotSupported;
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (row_stride_elems * 2) % 16 != 0 || box_rows == 0 || box_rows > 256 ||
+      box_blocks == 0 || box_blocks > 256)
+    return cudaErrorInvalidValue;
+  cuuint64_t dims[4] = {cols, rows, 2, blocks};
+  cuuint64_t strides[3] = {row_stride_elems * 2, rows * row_stride_elems * 2, 2 * rows * row_stride_elems * 2};
+  cuuint32_t box[4] = {(cuuint32_t)kBlockK, box_rows, 1, box_blocks};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 // Plain GEMM: C row-major in this GPU's memory, nothing to wait for.
 struct StoreLocal : PolicyBase {
   __nv_bfloat16* c;

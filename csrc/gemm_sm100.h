@@ -12,6 +12,10 @@ namespace sm100 {
 // aligned and the row stride a multiple of 8 elements.
 cudaError_t make_tile_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                           uint64_t row_stride_elems, uint32_t box_rows);
+// The same of gate and up rows, [blocks][gate, up][rows] of one matrix, as a tensor of four dimensions: a box is box_rows
+// gate or up rows of each of box_blocks blocks, one behind the other.
+cudaError_t make_gate_up_map(CUtensorMap* map, const void* base, uint64_t blocks, uint64_t rows, uint64_t cols,
+                             uint64_t row_stride_elems, uint32_t box_blocks, uint32_t box_rows);
 
 // C[M, N] = A[M, K] * B[N, K]^T, bf16, row-major with leading dimensions lda /
 // ldb / ldc (elements).  K, lda, ldb multiples of 8.  block_n: 0 (choose), 128, 192 or

@@ -16,18 +16,44 @@ namespace {
 
 constexpr int kTileSmem = 224 << 10;  // ring and staging of the one CTA of an SM
 
+// Gate and up rows in blocks: the tiles of `nsub` accumulators of `sub_out` features each, and log2 of the rows that an
+// accumulator takes of a block (the most, 8 to 64, that leave the fewest tiles).  -1 where no such strip fits.
+int strip_tiles(int n_out, int sub_out, int nsub, int* tiles_n) {
+  int best = -1;
+  for (int shift = 6; shift >= 3; --shift) {
+    if (sub_out % (1 << shift) != 0) continue;
+    const int per = kPairRows >> shift, blocks = nsub * (sub_out >> shift);
+    const int tiles = (n_out / kPairRows + blocks - 1) / blocks * per;
+    if (best < 0 || tiles < *tiles_n) best = shift, *tiles_n = tiles;
+  }
+  return best;
+}
+
 template <bool PAIR, int EPI, bool SPLIT, int NSUB>
 cudaError_t launch_tile(const TileGemm& g, TileArgs a, TileShape t, int sms, uint32_t* error_word, cudaStream_t stream) {
   constexpr bool kSilu = EPI == TILE_EPI_SILU;
   const int sub_out = kSilu ? t.sub / 2 : t.sub;
   a.sub = t.sub;
   a.tiles_n = (a.n_out + t.nsub * sub_out - 1) / (t.nsub * sub_out);
+  a.strip_shift = -1;
+  if (kSilu && g.silu_pairs) {
+    a.strip_shift = strip_tiles(a.n_out, sub_out, t.nsub, &a.tiles_n);
+    if (a.strip_shift < 0) return cudaErrorInvalidValue;
+  }
   a.band = std::max(1, 2048 / t.rows());
   CUtensorMap ma, mb;
   cudaError_t rc = make_tile_map(&ma, g.a, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda, kBlockM);
   if (rc != cudaSuccess) return rc;
-  rc = make_tile_map(&mb, g.b, (uint64_t)std::max(1, g.groups) * g.b_rows, (uint64_t)g.K, (uint64_t)g.ldb,
-                     (uint32_t)(PAIR || kSilu ? t.sub / 2 : t.sub));
+  if (kSilu) {
+    const int shift = a.strip_shift;
+    rc = shift < 0 ? make_gate_up_map(&mb, g.b, (uint64_t)std::max(1, g.groups), (uint64_t)g.b_rows / 2, (uint64_t)g.K, (uint64_t)g.ldb,
+                                      1, (uint32_t)sub_out)
+                   : make_gate_up_map(&mb, g.b, (uint64_t)a.n_out / kPairRows, kPairRows, (uint64_t)g.K, (uint64_t)g.ldb,
+                                      (uint32_t)(sub_out >> shift), 1u << shift);
+  } else {
+    rc = make_tile_map(&mb, g.b, (uint64_t)std::max(1, g.groups) * g.b_rows, (uint64_t)g.K, (uint64_t)g.ldb,
+                       (uint32_t)(PAIR ? t.sub / 2 : t.sub));
+  }
   if (rc != cudaSuccess) return rc;
   const auto kernel = gemm_tile_kernel<PAIR, EPI, SPLIT, NSUB>;
   const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(kernel), kTileSmem, PAIR ? kTileThreads : 0);
@@ -89,7 +115,8 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
         const int sub_out = silu ? t.sub / 2 : t.sub, out = t.nsub * sub_out;
         if (c > 1 && (sub_out % 16 != 0 || sub_out < 16 * c)) continue;
         const int n_out = silu ? g.b_rows / 2 : g.b_rows;
-        const int tiles_n = (n_out + out - 1) / out;
+        int tiles_n = (n_out + out - 1) / out;
+        if (silu && g.silu_pairs && strip_tiles(n_out, sub_out, t.nsub, &tiles_n) < 0) continue;
         if (g.sumsq_cap > 0 && tiles_n * c > g.sumsq_cap) continue;
         const long long tiles = (long long)((g.M + rows - 1) / rows) * tiles_n;
         if (c > 1 && tiles > room) continue;
@@ -112,8 +139,9 @@ void choose_tile_once(TileGemm& g, int dev, int sms, int pairs) {
     int block_n, pair, cluster;
   };
   static std::mutex mu;
-  static std::map<std::array<int, 9>, Choice> kept;
-  const std::array<int, 9> key = {dev, g.M, g.b_rows, g.K, g.epi, g.groups > 0, g.norm_w != nullptr, g.sumsq_cap, pair_kernel_enabled()};
+  static std::map<std::array<int, 10>, Choice> kept;
+  const std::array<int, 10> key = {dev, g.M, g.b_rows, g.K, g.epi, g.groups > 0, g.norm_w != nullptr, g.sumsq_cap,
+                                   pair_kernel_enabled(), g.silu_pairs};
   {
     std::lock_guard<std::mutex> lock(mu);
     const auto it = kept.find(key);
@@ -199,6 +227,8 @@ cudaError_t launch_tile_epi(const TileGemm& g, TileArgs a, int sms, uint32_t* er
 cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows) {
   if (g.M <= 0 || g.b_rows <= 0 || g.K <= 0 || g.K % 8 != 0 || g.lda % 8 != 0 || g.ldb % 8 != 0 || g.groups < 0 ||
       g.groups > kTileMaxGroups || (g.groups > 0 && (g.ranges == nullptr || g.scale_sumsq != nullptr)))
+    return cudaErrorInvalidValue;
+  if (g.silu_pairs && (g.epi != TILE_EPI_SILU || g.groups > 0 || g.pair == 2 || g.b_rows % (2 * kPairRows) != 0))
     return cudaErrorInvalidValue;
   if (g.epi == TILE_EPI_SILU && g.b_rows % 2 != 0) return cudaErrorInvalidValue;
   if (g.epi == TILE_EPI_RESIDUAL &&

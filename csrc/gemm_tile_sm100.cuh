@@ -18,7 +18,10 @@
 // shared memory, each finishing all rows of its share of the columns.
 // SILU: an accumulator is sub / 2 gate columns and the sub / 2 up columns of the same features, so
 // both halves of a product are in one thread and only the activation
-// is written.  RESIDUAL: the output is added to the residual stream, which is kept
+// is written.  The weight holds all gate rows before all up rows, or both in turn in blocks of 64 (what the decode GEMM
+// reads): an accumulator then takes a strip of the same 2^k rows of each of several blocks, which is one box of a tensor
+// map of four dimensions, so the features of a tile may still be any multiple of 8 (whole blocks alone would leave 112 tiles
+// to 148 SMs where 14336 features of up to 128 rows have 144).  RESIDUAL: the output is added to the residual stream, which is kept
 // in the reader's form too (times the next norm's weight) together with the sums
 // of squares; the consumer multiplies its accumulator rows by 1 / rms.  The norm
 // between two linears then costs no pass of its own.
@@ -37,6 +40,7 @@ constexpr int kTileMaxGroups = 256;
 constexpr int kTileMaxCluster = 4;  // pairs or single CTAs
 constexpr int kTileMaxStages = 8;
 constexpr int kTileABytes = kBlockM * kBlockK * 2;
+constexpr int kPairRows = 64;  // gate rows, and up rows, of a block of a weight that holds them in turn
 
 struct TileArgs {
   __nv_bfloat16* out;
@@ -44,6 +48,7 @@ struct TileArgs {
   int num_kb, tiles_n, band;
   int groups, b_rows;
   int sub;               // columns of an accumulator (NSUB of them are a tile)
+  int strip_shift;       // SILU: -1, or (blocks of gate and up rows) log2 of the rows of a block in an accumulator
   int stages, accs;      // ring; sets of accumulators
   int tmem_cols;
   int cl;                // pairs (or CTAs) per cluster; above 1 a cluster splits the K steps of its tile
@@ -197,6 +202,19 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     c.first = 0;
     if (active > 0) open_group(c);
   };
+  // SILU: where the first accumulator's features begin, row in the block and block (without strips: feature, group), and
+  // what a further accumulator adds to either
+  const bool strips = kSilu && a.strip_shift >= 0;
+  const int next_row = strips ? 0 : sub_out, next_block = strips ? sub_out >> a.strip_shift : 0;
+  auto features = [&](int n_blk, int group, int& row, int& block) {
+    row = n_blk * nsub * sub_out;
+    block = group;
+    if (strips) {
+      const int per = kPairRows >> a.strip_shift, g = n_blk / per;  // (the strips of a block are neighbours)
+      row = (n_blk - g * per) << a.strip_shift;
+      block = g * nsub * next_block;
+    }
+  };
   // first row of this CTA's share of the tile, column block
   auto locate = [&](TileCursor& c, int tile, int& row, int& n_blk) {
     while (tile - c.first >= c.mt * a.tiles_n) {
@@ -227,26 +245,35 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     int ahead = 0;
     TileCursor cur;
     start(cur);
-    auto b_row = [&](int n_blk) {  // of the tile's first accumulator; the second one's rows lie sub_out behind
-      const int b0 = s_group[cur.g] * a.b_rows + n_blk * nsub * sub_out;
-      if (!PAIR) return b0;
-      return b0 + (int)r * (kSilu ? a.b_rows / 2 : sub / 2);
+    // rows of b of the tile's first accumulator (the second one's lie sub_out behind), SILU: as `features`
+    auto b_rows_at = [&](int n_blk, int& by, int& bz) {
+      if (kSilu) features(n_blk, s_group[cur.g], by, bz);
+      else by = s_group[cur.g] * a.b_rows + n_blk * nsub * sub_out + (PAIR ? (int)r * (sub / 2) : 0), bz = 0;
     };
-    auto load_b = [&](int stage, int kb, int by) {
+    auto load_b = [&](int stage, int kb, int by, int bz) {
       unsigned char* sb = tiles + stage * stage_bytes + kTileABytes;
+      const int x = kb * kBlockK;
       if (PAIR) {
         if (r == 0) mbar_expect_tx(&full[stage], 2u * (uint32_t)stage_bytes);
         const uint32_t bar = map_to_cta(smem_u32(&full[stage]), lead);
-        tma_load_2d_pair(sb, &map_b, bar, kb * kBlockK, by);
-        if (nsub > 1) tma_load_2d_pair(sb + b_bytes, &map_b, bar, kb * kBlockK, by + sub_out);
+        if (kSilu) {  // one CTA has the gate rows, the other the up rows
+          tma_load_4d_pair(sb, &map_b, bar, x, by, (int)r, bz);
+          if (nsub > 1) tma_load_4d_pair(sb + b_bytes, &map_b, bar, x, by + next_row, (int)r, bz + next_block);
+        } else {
+          tma_load_2d_pair(sb, &map_b, bar, x, by);
+          if (nsub > 1) tma_load_2d_pair(sb + b_bytes, &map_b, bar, x, by + sub_out);
+        }
       } else {
         mbar_expect_tx(&full[stage], (uint32_t)stage_bytes);
 #pragma unroll
         for (int s = 0; s < nsub; ++s) {
-          tma_load_2d(sb, &map_b, &full[stage], kb * kBlockK, by);
-          if (kSilu) tma_load_2d(sb + b_bytes / 2, &map_b, &full[stage], kb * kBlockK, by + a.b_rows / 2);
+          if (kSilu) {
+            tma_load_4d(sb, &map_b, &full[stage], x, by + s * next_row, 0, bz + s * next_block);
+            tma_load_4d(sb + b_bytes / 2, &map_b, &full[stage], x, by + s * next_row, 1, bz + s * next_block);
+          } else {
+            tma_load_2d(sb, &map_b, &full[stage], x, by + s * sub_out);
+          }
           sb += b_bytes;
-          by += sub_out;
         }
       }
     };
@@ -254,9 +281,10 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       int row, n_blk;
       locate(cur, worker, row, n_blk);
       ahead = min(stages, kb1 - kb0);
-      const int by = b_row(n_blk);
+      int by, bz;
+      b_rows_at(n_blk, by, bz);
       for (int i = 0; i < ahead; ++i) {
-        if (elect_one()) load_b(i, kb0 + i, by);
+        if (elect_one()) load_b(i, kb0 + i, by, bz);
         __syncwarp();
       }
     }
@@ -264,13 +292,14 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
     for (int tile = worker; ok && tile < num_tiles; tile += workers) {
       int row, n_blk;
       locate(cur, tile, row, n_blk);
-      const int by = b_row(n_blk);
+      int by, bz;
+      b_rows_at(n_blk, by, bz);
       for (int kb = kb0; kb < kb1; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait_abortable(&empty[stage], phase ^ 1u, abort_flag));
         if (!ok) break;
         unsigned char* sa = tiles + stage * stage_bytes;
         if (elect_one()) {
-          if (ahead <= 0) load_b(stage, kb, by);
+          if (ahead <= 0) load_b(stage, kb, by, bz);
           if (PAIR) tma_load_2d_pair(sa, &map_a, map_to_cta(smem_u32(&full[stage]), lead), kb * kBlockK, row);
           else tma_load_2d(sa, &map_a, &full[stage], kb * kBlockK, row);
         }
@@ -386,7 +415,16 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
       // pass i: its accumulator, the columns in it, the first column of out
       auto sub_of = [&](int i) { return SPLIT || nsub == 1 || i < per_sub ? 0 : 1; };
       auto in_sub = [&](int i) { return SPLIT ? own0 + i * kChunk : (i - sub_of(i) * per_sub) * kChunk; };
-      auto out_col = [&](int i) { return (n_blk * nsub + sub_of(i)) * sub_out + in_sub(i); };
+      int f_row = 0, f_block = 0;
+      if (strips) features(n_blk, 0, f_row, f_block);
+      // strips: column of out of column `c` of accumulator s (eight columns, 16 bytes, never cross a strip)
+      auto strip_col = [&](int s, int c) {
+        const int in = c & ((1 << a.strip_shift) - 1);
+        return (f_block + s * next_block + (c >> a.strip_shift)) * kPairRows + f_row + in;
+      };
+      auto out_col = [&](int i) {
+        return strips ? strip_col(sub_of(i), in_sub(i)) : (n_blk * nsub + sub_of(i)) * sub_out + in_sub(i);
+      };
       // RESIDUAL (the launcher wants whole, aligned rows of 16 columns here): the stream and the norm's weight
       // travel two passes ahead, the first ones while the product is finished: 16 columns take a warp less time than their
       // loads (one pass ahead: 1152 x 4096 in one round of tiles 36.4 us instead of 32).  A thread has kResRows rows of
@@ -579,12 +617,15 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
             }
           } else {
             constexpr int kPer = 32 / kPieces;  // rows of a store instruction
-            const int col_end = min(a.n_out, col0 - in_sub(i) + sub_out);
+            // column of out of this lane's eight columns, and where they end (beyond the accumulator: nowhere)
+            const int pc = lane % kPieces, in = in_sub(i) + pc * 8;
+            const int col = strips ? strip_col(sub_of(i), in) : col0 + pc * 8;
+            const int col_end = strips ? (in < sub_out ? a.n_out : 0) : min(a.n_out, col0 - in_sub(i) + sub_out);
 #pragma unroll
             for (int j = 0; j < kPieces; ++j) {
-              const int rr = j * kPer + lane / kPieces, pc = lane % kPieces;
+              const int rr = j * kPer + lane / kPieces;
               const uint4 p = *reinterpret_cast<const uint4*>(piece(rr, pc));
-              store16_local(a.out, a.ldo, row + rr, col0 + pc * 8, p, row_end, col_end);
+              store16_local(a.out, a.ldo, row + rr, col, p, row_end, col_end);
             }
           }
           __syncwarp();

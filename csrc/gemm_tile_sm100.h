@@ -8,7 +8,7 @@ namespace sm100 {
 
 enum TileEpilogue : int {
   TILE_EPI_PLAIN = 0,     // out[m][n] = acc
-  TILE_EPI_SILU = 1,      // out[m][f] = silu(acc of gate row f) * (acc of up row f): b's rows are gate, then up
+  TILE_EPI_SILU = 1,      // out[m][f] = silu(acc of gate row f) * (acc of up row f): b's rows are gate, then up (or silu_pairs)
   TILE_EPI_RESIDUAL = 2,  // z = acc + residual; residual = z; out = z * norm_w; sumsq_out = sum z^2 per 128 columns
 };
 
@@ -20,6 +20,7 @@ struct TileGemm {
   int M, b_rows, K;
   int lda, ldb, ldo;
   int epi;
+  bool silu_pairs;  // TILE_EPI_SILU, without groups: b's rows are blocks of 64 gate rows and the 64 up rows of the same features
   // groups > 0: rows ranges[s g] .. ranges[s g + 1] of a and out (device memory, s = range_stride) meet b rows
   // g * b_rows ..  (what lies outside [0, M) is left out)
   int groups;

@@ -256,17 +256,14 @@ class LlamaTPDecoder:
             else:
                 wqkv = rnd((self.Hq + 2 * self.Hkv) * D, H, sub=base * 64 + r + 1)
                 wgu = rnd(2 * self.F, H, sub=(base + 4) * 64 + r + 1)  # random: already "interleaved"
-            layer = dict(
+            self.layers.append(dict(
                 wqkv=wqkv, wo=row_shard(H, cfg.heads * D, base + 3), wgu=wgu, wdown=row_shard(H, cfg.ffn, base + 6),
-                norm1=torch.ones(H, dtype=dt, device=self.dev), norm2=torch.ones(H, dtype=dt, device=self.dev))
-            if self.linears == "cublas" or "gate_up" in self.tiled:
-                layer["wgu_cat"] = torch.cat(self.split_gate_up(wgu)).contiguous()
-            self.layers.append(layer)
+                norm1=torch.ones(H, dtype=dt, device=self.dev), norm2=torch.ones(H, dtype=dt, device=self.dev)))
 
     @staticmethod
     def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
-        """[F, H] gate and up -> the layout the fused silu*mul epilogue reads: blocks of 64 gate rows
-        followed by the 64 up rows of the same features."""
+        """[F, H] gate and up -> the layout of a layer's "wgu", the one storage that every form of the step reads: blocks
+        of 64 gate rows followed by the 64 up rows of the same features."""
         F, H = gate.shape
         return torch.stack([gate.reshape(F // 64, 64, H), up.reshape(F // 64, 64, H)], 1).reshape(2 * F, H).contiguous()
 
@@ -295,7 +292,7 @@ class LlamaTPDecoder:
     def weight_bytes(self) -> int:
         n = self.embed.numel() + self.lm_head.numel()
         for l in self.layers:
-            n += sum(l[k].numel() for k in ("wqkv", "wo", "wgu", "wdown"))  # wgu_cat (cuBLAS mode) is a copy
+            n += sum(l[k].numel() for k in ("wqkv", "wo", "wgu", "wdown"))
         return n * 2
 
     # ------------------------------------------------------------------- state
@@ -348,7 +345,7 @@ class LlamaTPDecoder:
                 ops.gemm_decode(x, w, out, silu, pdl=pdl, eps=eps, **fold)
                 return fold.get("sumsq_out")
             if "residual" not in fold:
-                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, **fold)
+                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, silu_pairs=silu, **fold)
                 return None
             return parts[:ops.gemm_tile(x, w, out, 2, pdl=pdl, eps=eps, sumsq_out=parts, **fold)]
         ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
@@ -358,7 +355,7 @@ class LlamaTPDecoder:
                                        self.workspace, self.Hq, self.Hkv, self.pieces, self.scale, self.cfg.rope_theta,
                                        pdl, balance=True)
             ss = linear("o", self.attn, L["wo"], x, residual=res, norm_w=L["norm2"])
-            linear("gate_up", x, L["wgu_cat" if "gate_up" in tiled else "wgu"], self.act, True, sumsq=ss)
+            linear("gate_up", x, L["wgu"], self.act, True, sumsq=ss)
             last = li + 1 == self.cfg.layers
             ss = linear("down", self.act, L["wdown"], x, residual=res,
                         norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
@@ -386,11 +383,11 @@ class LlamaTPDecoder:
                 self._linear(self.x, L["wgu"], self.act, silu_pairs=True)
                 self._linear(self.act, L["wdown"], self.parts[1], push=self._push)
             elif self.tiled_gate_up and not separate:
-                ops.gemm_tile(self.x, L["wgu_cat"], self.act, 1, pdl=self.pdl)
+                ops.gemm_tile(self.x, L["wgu"], self.act, 1, pdl=self.pdl, silu_pairs=True)
                 torch.matmul(self.act, L["wdown"].t(), out=self.parts[1])
             else:
-                torch.matmul(self.x, L["wgu_cat"].t(), out=self.gu)
-                ops.silu_mul(self.gu, self.act)
+                torch.matmul(self.x, L["wgu"].t(), out=self.gu)
+                ops.silu_mul(self.gu, self.act, pairs=True)
                 torch.matmul(self.act, L["wdown"].t(), out=self.parts[1])
             nxt = self.layers[li + 1]["norm1"] if li + 1 < cfg.layers else self.final_norm
             self._reduce_norm(self.parts[1], nxt)
