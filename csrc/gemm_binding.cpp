@@ -120,11 +120,12 @@ void bind_gemm(py::module_& m) {
   // well.  sumsq_out [rows of b / 128, M]: a sum for every 128 columns; [rows of b / 16, M]: as many rows as the call returns
   // hold sums of some columns each, which leaves the width of the tiles free.  block_n, cluster: tile columns and CTAs (or
   // pairs) that share a tile's K, 0: choose; pair 1 / -1: CTA pairs or single CTAs (0: pairs of 256 x 256 for block_n 512), 2: pairs with the weight on the M side and
-  // up to block_n rows of a (plain or silu).
+  // up to block_n rows of a (plain or silu).  exact_silu: silu with a division that is no approximation, also for gates below -87.3
+  // (not with pair 2).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
-                        int64_t cluster, c10::optional<at::Tensor> stream_out, int64_t pair, bool silu_pairs) {
+                        int64_t cluster, c10::optional<at::Tensor> stream_out, int64_t pair, bool silu_pairs, bool exact_silu) {
     auto bf16 = [](const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.stride(-1) == 1; };
     TORCH_CHECK(bf16(a) && bf16(b) && bf16(out) && a.dim() == 2 && b.dim() == 2 && out.dim() == 2,
                 "gemm_tile: 2-D bf16 CUDA tensors with contiguous rows");
@@ -187,6 +188,7 @@ void bind_gemm(py::module_& m) {
     g.cluster = (int)cluster;
     g.pair = (int)pair;
     g.silu_pairs = silu_pairs;
+    g.exact_silu = exact_silu;
     TORCH_CHECK(epi == 2 || !stream_out.has_value(), "gemm_tile: stream_out beside a residual");
     const at::cuda::OptionalCUDAGuard guard(a.device());
     int sumsq_rows = 0;
@@ -198,7 +200,7 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
      py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0,
-     py::arg("silu_pairs") = false);
+     py::arg("silu_pairs") = false, py::arg("exact_silu") = false);
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K, bool folded) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K, folded);
   }, py::arg("B"), py::arg("N"), py::arg("K"), py::arg("folded") = false,

@@ -230,6 +230,7 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
     return cudaErrorInvalidValue;
   if (g.silu_pairs && (g.epi != TILE_EPI_SILU || g.groups > 0 || g.pair == 2 || g.b_rows % (2 * kPairRows) != 0))
     return cudaErrorInvalidValue;
+  if (g.exact_silu && (g.epi != TILE_EPI_SILU || g.pair == 2)) return cudaErrorInvalidValue;
   if (g.epi == TILE_EPI_SILU && g.b_rows % 2 != 0) return cudaErrorInvalidValue;
   if (g.epi == TILE_EPI_RESIDUAL &&
       (g.groups > 0 || g.b_rows % 128 != 0 || g.ldo % 8 != 0 || g.residual == nullptr ||
@@ -245,6 +246,7 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   a.ldo = g.ldo;
   a.M = g.M;
   a.n_out = g.epi == TILE_EPI_SILU ? g.b_rows / 2 : g.b_rows;
+  a.exact_silu = g.exact_silu;
   a.num_kb = (g.K + kBlockK - 1) / kBlockK;
   a.groups = g.groups;
   a.b_rows = g.b_rows;

@@ -48,6 +48,7 @@ struct TileArgs {
   int num_kb, tiles_n, band;
   int groups, b_rows;
   int sub;               // columns of an accumulator (NSUB of them are a tile)
+  bool exact_silu;       // SILU: a division rounded once
   int strip_shift;       // SILU: -1, or (blocks of gate and up rows) log2 of the rows of a block in an accumulator
   int stages, accs;      // ring; sets of accumulators
   int tmem_cols;
@@ -80,6 +81,16 @@ struct TileEpi {
   static constexpr int kRowBytes = kChunk * (EPI == TILE_EPI_RESIDUAL ? 4 : 2);
   static constexpr int kBytes = 8 * 32 * kRowBytes;
 };
+
+// silu(g) = g / (1 + exp(-g)) for |g| up to kNearGate by long division: an approximate quotient, and the remainder that it
+// leaves, which an fma gives exactly, divided once more.  (The divisor stays far below 2^126, where the fast division gives
+// up.)  Against the same quotient in 64 bits, all fp32 gates of 2^-40 to 40 on either side: 0.500000 units of fp32 at most, the
+// compiler's division 0.499999; two of 759 million differ between them.
+constexpr float kNearGate = 40.f;
+__device__ __forceinline__ float silu_near(float g) {
+  const float d = 1.f + __expf(-g), r = __fdividef(1.f, d), q = g * r;
+  return fmaf(fmaf(-q, d, g), r, q);
+}
 
 // Walks the tiles of all groups in order; `tile` only grows.
 struct TileCursor {
@@ -550,10 +561,32 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           if (kSilu) {
             float up[kChunk];
             load_acc(i, 1, up);
+            if (a.exact_silu) {
+              // The compiler's division branches for each quotient, and the zeros behind the last row take its slow side (8
+              // layers and the head of a decode step, us, without an exact quotient / with a division: 65 rows 1031 / 1137, 128
+              // 1197 / 1226, 192 1701 / 1804).  Gates in the ordinary range take silu_near (65 rows 1052 / 1066, 128 1207 / 1203,
+              // 192 1727 / 1729); one outside it brings its warp's pass to the division.
+              bool near = true;
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) {
-              const float gv = v[j] * scale, uv = up[j] * scale;
-              v[j] = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+              for (int j = 0; j < kChunk; ++j) near &= fabsf(v[j] * scale) <= kNearGate;
+              if (__all_sync(0xffffffffu, near)) {
+#pragma unroll
+                for (int j = 0; j < kChunk; ++j) v[j] = silu_near(v[j] * scale) * (up[j] * scale);
+              } else {
+#pragma unroll 1
+                for (int j = 0; j < kChunk; ++j) {
+                  const float gv = v[0] * scale, uv = up[0] * scale;
+#pragma unroll
+                  for (int k = 0; k + 1 < kChunk; ++k) v[k] = v[k + 1], up[k] = up[k + 1];
+                  v[kChunk - 1] = gv / (1.f + __expf(-gv)) * uv;
+                }
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < kChunk; ++j) {
+                const float gv = v[j] * scale, uv = up[j] * scale;
+                v[j] = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+              }
             }
           } else {
 #pragma unroll

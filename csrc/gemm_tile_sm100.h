@@ -21,6 +21,9 @@ struct TileGemm {
   int lda, ldb, ldo;
   int epi;
   bool silu_pairs;  // TILE_EPI_SILU, without groups: b's rows are blocks of 64 gate rows and the 64 up rows of the same features
+  // TILE_EPI_SILU, not with pair = 2: the quotient gate / (1 + exp(-gate)) is that of a division, as the decode GEMM's is;
+  // else it is off by up to 2 units of fp32 and zero for gates below -87.3 (their 1 + exp(-gate) is above 2^126)
+  bool exact_silu;
   // groups > 0: rows ranges[s g] .. ranges[s g + 1] of a and out (device memory, s = range_stride) meet b rows
   // g * b_rows ..  (what lies outside [0, M) is left out)
   int groups;

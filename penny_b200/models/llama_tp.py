@@ -345,7 +345,7 @@ class LlamaTPDecoder:
                 ops.gemm_decode(x, w, out, silu, pdl=pdl, eps=eps, **fold)
                 return fold.get("sumsq_out")
             if "residual" not in fold:
-                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, silu_pairs=silu, **fold)
+                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, silu_pairs=silu, exact_silu=silu, **fold)
                 return None
             return parts[:ops.gemm_tile(x, w, out, 2, pdl=pdl, eps=eps, sumsq_out=parts, **fold)]
         ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
@@ -383,7 +383,7 @@ class LlamaTPDecoder:
                 self._linear(self.x, L["wgu"], self.act, silu_pairs=True)
                 self._linear(self.act, L["wdown"], self.parts[1], push=self._push)
             elif self.tiled_gate_up and not separate:
-                ops.gemm_tile(self.x, L["wgu"], self.act, 1, pdl=self.pdl, silu_pairs=True)
+                ops.gemm_tile(self.x, L["wgu"], self.act, 1, pdl=self.pdl, silu_pairs=True, exact_silu=True)
                 torch.matmul(self.act, L["wdown"].t(), out=self.parts[1])
             else:
                 torch.matmul(self.x, L["wgu"].t(), out=self.gu)
