@@ -136,19 +136,35 @@ def expert_tiles(rows: int, experts: int, hidden: int, ffn: int, sms: int):
     return (512 if rows > 640 * experts and ops.gemm_pair_enabled() else 256), (2 if shared else 0)
 
 
-def expert_rows(rows: int, experts: int):
+def expert_rows(rows: int, experts: int, hidden: int = 4096, most: int | None = None):
     """Rows per tile of gate/up and of down where one rank's grouped GEMMs have the weight on the M side, 0 where
-    `expert_tiles` holds.
+    `expert_tiles` holds.  `most`: the rows that an expert can have at most (a token picks an expert once), None: as many as
+    a tile has.
 
     There a group's rows are paid to the next 16 instead of 128 or 256, and few rows leave the shared memory to the
-    weights.  The whole layer (8 experts, hidden 4096, ffn 14336, four draws of the router each) against tiles of rows,
-    by rows per expert: 0.75 (3 tokens) 0.85 with 16 rows in both, 2 and 5 0.98 and 0.99; 15 and 40 0.975 and 0.979 with
-    128 in gate/up alone, 0.978 and 0.989 in both; 60 and 75 1.00 and 1.01; 88 0.99, 105 to 250 0.93, 0.87, 1.00 and 0.89 with
-    256 in both, 310 to 1024 0.89 to 0.96."""
+    weights; but an expert with more rows than a tile has its weights staged again for each further one, so tiles are as
+    long as the longest expert can be, or 128 rows, as `expert_tiles` has them.  Whole layers against `expert_tiles`: 8 experts,
+    hidden 4096, ffn 14336 / 16, 6144, 10752 / 64, 2048, 1024 / 64, 2048, 1408 / 128, 2048, 768 / 8, 1024, 3584; in brackets the
+    range over them with nearly all rows at as many experts as a token picks.
+      up to 64 tokens, tiles that hold them      0.88 to 1.01 (0.77 to 0.99; 16 rows for 24 to 64 of them up to 1.17)
+      up to 6 rows per expert, 128 rows          0.97 to 1.00 (0.90 to 0.98; 16 rows 0.97 to 1.01 and up to 1.30)
+      15 / 30 rows per expert, 128 in gate/up    0.98 to 1.00 / 0.99 to 1.01 (0.95 to 1.04 / 0.97 to 1.04)
+      40 / 48 / 51 / 56                          0.96 to 1.00 / 0.99 to 1.00 / 0.98 to 1.01 / 0.98 to 1.02 (0.96 to 1.09)
+      64 / 75, 128 in gate/up; 256 in both       0.99 to 1.02 (0.99 to 1.11); 0.95 to 1.06 (0.89 to 1.05)
+      88 / 96 / 105 / 128, 256 in both           8 of 4096: 1.04 / 0.90 / 0.91 / 0.89 (0.86 to 0.97), 16 of 6144: 1.03 / 1.00 / 0.97 / 0.95
+                                                 (0.87 to 1.04), hidden 2048: 1.01 to 1.04 / 1.01 to 1.02 / 1.01 to 1.05 / 0.98 to 1.01
+      190 / 256 / 512 / 1024, 256 in both        0.84 to 0.99 (0.85 to 1.05), hidden 1024: 0.97 / 1.06 / 1.20 / 1.11 (1.10 to 1.20)
+    Layers under hidden 1024 were not timed."""
     per = rows / experts
-    if not ops.gemm_pair_enabled() or 52 < per < 88:
+    if not ops.gemm_pair_enabled() or hidden < 1024:
         return 0, 0
-    return (256, 256) if per >= 88 else (128, 0) if per > 6 else (16, 16)
+    if most is not None and most <= 64:
+        return ((most + 15) // 16 * 16,) * 2
+    if per <= 6:
+        return (16, 16) if most is None else (128, 128)
+    if per <= 52:
+        return 128, 0
+    return (256, 256) if hidden >= 2048 and per >= (88 if hidden >= 4096 else 128) else (0, 0)
 
 
 class MoeEPLayer:
@@ -248,7 +264,8 @@ class MoeEPLayer:
                 and x0.dtype == torch.bfloat16 and x0.is_contiguous() and x0.data_ptr() % 16 == 0
                 and cfg.topk <= 8 and cfg.experts <= 256):
             out = ops.moe_layer(x0, self.router[0], self.w13[0][:self.epr], self.w2[0][:self.epr], cfg.topk,
-                                *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms), *expert_rows(pairs, self.epr))
+                                *expert_tiles(pairs, self.epr, cfg.hidden, cfg.ffn, self.sms),
+                                *expert_rows(pairs, self.epr, cfg.hidden, x0.shape[0]))
             if out is not None:
                 return [out] if comm.emulated else out
         ids, gates, tables = [], [], []
