@@ -27,7 +27,8 @@ inline KernelSetup kernel_setup(const void* kernel, int smem_bytes, int threads_
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   auto it = done.find({dev, kernel});
-  if (it != done.end()) return it->second;
+  // (a call that did not ask for the pairs may have come first)
+  if (it != done.end() && (threads_for_pairs == 0 || it->second.pairs > 0)) return it->second;
   KernelSetup ks;
   ks.rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (ks.rc != cudaSuccess) {
