@@ -118,9 +118,10 @@ void bind_gemm(py::module_& m) {
   // and without ranges load b, while the kernel before it on the stream still runs, so that kernel must not write
   // b (a weight); everything else is waited for.  The residual may be fp32, stream_out then takes the sum in bf16 as
   // well.  sumsq_out [rows of b / 128, M]: a sum for every 128 columns; [rows of b / 16, M]: as many rows as the call returns
-  // hold sums of some columns each, which leaves the width of the tiles free.  block_n, cluster: tile columns and CTAs (or
-  // pairs) that share a tile's K, 0: choose; pair 1 / -1: CTA pairs or single CTAs (0: pairs of 256 x 256 for block_n 512), 2: pairs with the weight on the M side and
-  // up to block_n rows of a (plain or silu).  exact_silu: silu with a division that is no approximation, also for gates below -87.3
+  // hold sums of some columns each, which leaves the width of the tiles free.  block_n: columns of a tile; pair 1 / -1: CTA
+  // pairs or single CTAs (0: pairs of 256 x 256 for block_n 512); cluster: CTAs or pairs that share a tile's K.  With block_n
+  // 0 what is 0 of the three is chosen, a cluster taken where some width can be shared so.  pair 2: pairs with the weight on
+  // the M side and up to block_n rows of a (plain or silu).  exact_silu: silu with a division that is no approximation, also for gates below -87.3
   // (not with pair 2).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
@@ -201,6 +202,22 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
      py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0,
      py::arg("silu_pairs") = false, py::arg("exact_silu") = false);
+  m.def("gemm_tile_choice", [](int64_t M, int64_t N, int64_t K, int64_t epi, int64_t groups, int64_t pair, int64_t cluster, bool silu_pairs) {
+    penny::sm100::TileGemm g = {};
+    g.M = (int)M;
+    g.b_rows = (int)N;
+    g.K = (int)K;
+    g.epi = (int)epi;
+    g.groups = (int)groups;
+    g.pair = (int)pair;
+    g.cluster = (int)cluster;
+    g.silu_pairs = silu_pairs;
+    TORCH_CHECK(M > 0 && N > 0 && K > 0 && epi >= 0 && epi <= 2 && pair >= -1 && pair <= 1, "gemm_tile_choice: sizes, epi, pair");
+    const penny::sm100::TileGemm c = penny::sm100::gemm_tile_choice(g);
+    return std::make_tuple(c.block_n, c.pair, c.cluster);
+  }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("epi") = 0, py::arg("groups") = 0, py::arg("pair") = 0,
+     py::arg("cluster") = 0, py::arg("silu_pairs") = false,
+     "(block_n, pair, cluster) of gemm_tile(block_n=0) without norm_w; N: rows of b, per group");
   m.def("gemm_decode_splits", [](int64_t B, int64_t N, int64_t K, bool folded) {
     return penny::sm100::gemm_decode_splits((int)B, (int)N, (int)K, folded);
   }, py::arg("B"), py::arg("N"), py::arg("K"), py::arg("folded") = false,

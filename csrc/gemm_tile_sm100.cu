@@ -101,14 +101,20 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
     if (kernel_setup(fn, kTileSmem).rc != cudaSuccess) return 0;
     return max_clusters(fn, (pair ? 2 : 1) * c, kTileThreads, kTileSmem);
   };
+  // what the caller has settled: CTA pairs or single CTAs (pair), and how many of them share a tile (cluster)
+  const int want_pair = g.pair, want_cl = std::min({g.cluster, kTileMaxCluster, num_kb});
   double best = 0;
   g.block_n = 0;
-  for (int pair = 0; pair <= (pairs > 0 && pair_kernel_enabled() ? 1 : 0); ++pair) {
+  for (int pair = 0; pair <= 1; ++pair) {
+    if (pair != 0 && (pairs <= 0 || (want_pair == 0 && !pair_kernel_enabled()))) continue;
+    if (want_pair != 0 && (want_pair > 0) != (pair != 0)) continue;
     const int slots = pair ? pairs : sms, rows = pair ? 2 * kBlockM : kBlockM;
     const double fill = pair ? 71. : 83., step0 = pair ? 64. : 19.;
-    for (int c = 1; c <= (g.groups == 0 ? kTileMaxCluster : 1); ++c) {
-      if (c > 1 && num_kb < 4 * c) break;
+    for (int c = 1; c <= kTileMaxCluster; ++c) {
+      if (want_cl > 0 ? c != want_cl : c > 1 && (g.groups > 0 || num_kb < 4 * c)) continue;
+      if (c > 1 && g.groups > 0 && g.M > rows) continue;
       const int room = c > 1 ? clusters(pair != 0, c) : 0;
+      if (c > 1 && room <= 0) continue;
       for (int bn = blocks ? 128 : 64; bn <= (c > 1 ? 256 : 512); bn += blocks ? 128 : (bn < 256 ? 16 : 32)) {
         const TileShape t{pair != 0, bn > 256 ? bn / 2 : bn, bn > 256 ? 2 : 1};
         if (blocks && t.sub % 128 != 0) continue;
@@ -119,7 +125,7 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
         if (silu && g.silu_pairs && strip_tiles(n_out, sub_out, t.nsub, &tiles_n) < 0) continue;
         if (g.sumsq_cap > 0 && tiles_n * c > g.sumsq_cap) continue;
         const long long tiles = (long long)((g.M + rows - 1) / rows) * tiles_n;
-        if (c > 1 && tiles > room) continue;
+        if (want_cl <= 0 && c > 1 && tiles > room) continue;
         const double share = (double)tiles * c / slots;
         const double rounds = 0.75 * (double)((tiles * c + slots - 1) / slots) + 0.25 * std::max(1., share);
         const double step = std::max(2.1 * bn, t.stage_bytes() / fill + step0) / 1800.;
@@ -131,6 +137,10 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
       }
     }
   }
+  if (g.block_n == 0 && want_cl > 1) {  // no width that so many could share
+    g.cluster = 0;
+    choose_tile(g, sms, pairs);
+  }
 }
 
 // The choice depends on the shape and the device alone and takes some 10 us: kept per shape, up to a bound.
@@ -139,9 +149,9 @@ void choose_tile_once(TileGemm& g, int dev, int sms, int pairs) {
     int block_n, pair, cluster;
   };
   static std::mutex mu;
-  static std::map<std::array<int, 10>, Choice> kept;
-  const std::array<int, 10> key = {dev, g.M, g.b_rows, g.K, g.epi, g.groups > 0, g.norm_w != nullptr, g.sumsq_cap,
-                                   pair_kernel_enabled(), g.silu_pairs};
+  static std::map<std::array<int, 12>, Choice> kept;
+  const std::array<int, 12> key = {dev, g.M, g.b_rows, g.K, g.epi, g.groups > 0, g.norm_w != nullptr, g.sumsq_cap,
+                                   pair_kernel_enabled(), g.silu_pairs, g.pair, g.cluster};
   {
     std::lock_guard<std::mutex> lock(mu);
     const auto it = kept.find(key);
@@ -224,7 +234,20 @@ cudaError_t launch_tile_epi(const TileGemm& g, TileArgs a, int sms, uint32_t* er
 
 }  // namespace
 
+TileGemm gemm_tile_choice(const TileGemm& g) {
+  TileGemm c = g;
+  if (g.block_n != 0 || g.pair == 2) return c;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_kernel<true, TILE_EPI_PLAIN, false, 1>), kTileSmem,
+                                      kTileThreads);
+  choose_tile_once(c, dev, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
+  return c;
+}
+
 cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows) {
+  if (g.pair < -1 || g.pair > 2) return cudaErrorInvalidValue;
   if (g.M <= 0 || g.b_rows <= 0 || g.K <= 0 || g.K % 8 != 0 || g.lda % 8 != 0 || g.ldb % 8 != 0 || g.groups < 0 ||
       g.groups > kTileMaxGroups || (g.groups > 0 && (g.ranges == nullptr || g.scale_sumsq != nullptr)))
     return cudaErrorInvalidValue;
@@ -266,13 +289,8 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
     if (g.epi == TILE_EPI_PLAIN) return launch_swap<false>(g, a, error_word, stream);
     return g.epi == TILE_EPI_SILU ? launch_swap<true>(g, a, error_word, stream) : cudaErrorInvalidValue;
   }
-  TileGemm c = g;
-  if (g.block_n == 0) {
-    const KernelSetup ks = kernel_setup(reinterpret_cast<const void*>(gemm_tile_kernel<true, TILE_EPI_PLAIN, false, 1>), kTileSmem,
-                                        kTileThreads);
-    choose_tile_once(c, dev, sms, ks.rc == cudaSuccess ? ks.pairs : 0);
-    if (c.block_n == 0) return cudaErrorInvalidValue;
-  }
+  const TileGemm c = gemm_tile_choice(g);
+  if (c.block_n == 0) return cudaErrorInvalidValue;
   switch (g.epi) {
     case TILE_EPI_PLAIN: return launch_tile_epi<TILE_EPI_PLAIN>(c, a, sms, error_word, stream, sumsq_rows);
     case TILE_EPI_SILU: return launch_tile_epi<TILE_EPI_SILU>(c, a, sms, error_word, stream, sumsq_rows);

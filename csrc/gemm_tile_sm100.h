@@ -44,14 +44,17 @@ struct TileGemm {
                         // tile's columns evenly
   int block_n;          // 0: choose; else the columns of a tile: a multiple of 16 up to 256, or of 32 up to 512 (two
                         // accumulators).  pair = 0: 512 stands for CTA pairs, 256 x 256
-  int pair;             // 0: by block_n; 1: CTA pairs, tiles of 256 rows; -1: single CTAs; 2: pairs with 256 rows of the
+  int pair;             // 0: by block_n, or choose with it; 1: CTA pairs, tiles of 256 rows; -1: single CTAs; 2: pairs with 256 rows of the
                         // weight on the M side and tiles of up to block_n rows of a (a multiple of 16 up to 256, 0: 256),
                         // plain or silu, no cluster
-  int cluster;          // pairs or CTAs that split the K steps of a tile, up to 4; 0, 1: none.  With
-                        // groups only for M <= the tile's rows
+  int cluster;          // pairs or CTAs that split the K steps of a tile, up to 4; 1: none; 0: none, or with block_n = 0
+                        // choose.  (block_n = 0: where some width can be shared so.)  With groups only for M <= the tile's rows
   bool pdl;             // may start, and without groups load b, while the kernel before it on the stream still runs:
                         // that kernel must not write b
 };
+
+// block_n, pair and cluster that a launch with block_n = 0 takes on the current device (block_n 0: none).
+TileGemm gemm_tile_choice(const TileGemm& g);
 
 // sumsq_rows: null, or the rows of sumsq_out that the launch writes.
 cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream_t stream, int* sumsq_rows = nullptr);
