@@ -15,6 +15,9 @@ namespace sm100 {
 namespace {
 
 constexpr int kTileSmem = 224 << 10;  // ring and staging of the one CTA of an SM
+constexpr int kTileEpiBytes = 16 << 10;
+static_assert(TileEpi<TILE_EPI_PLAIN, false>::kBytes <= kTileEpiBytes && TileEpi<TILE_EPI_SILU, false>::kBytes <= kTileEpiBytes &&
+              TileEpi<TILE_EPI_RESIDUAL, false>::kBytes <= kTileEpiBytes, "staging of the epilogues");
 
 // Gate and up rows in blocks: the tiles of `nsub` accumulators of `sub_out` features each, and log2 of the rows that an
 // accumulator takes of a block (the most, 8 to 64, that leave the fewest tiles).  -1 where no such strip fits.
@@ -63,7 +66,8 @@ cudaError_t launch_tile(const TileGemm& g, TileArgs a, TileShape t, int sms, uin
   const int slots = PAIR ? ks.pairs : sms;
   // A cluster works on one tile, so with groups (whose tiles the device counts) no group may have two row tiles.
   if (SPLIT && g.groups > 0 && g.M > t.rows()) return cudaErrorInvalidValue;
-  long long workers = SPLIT ? (g.groups > 0 ? (long long)g.groups * a.tiles_n : tiles) : (g.groups > 0 ? slots : std::min<long long>(slots, tiles));
+  const long long workers = SPLIT ? (g.groups > 0 ? (long long)g.groups * a.tiles_n : tiles)
+                                  : (g.groups > 0 ? slots : std::min<long long>(slots, tiles));
   const int epi_bytes = TileEpi<EPI, SPLIT>::kBytes;
   const int kb_per = (a.num_kb + a.cl - 1) / a.cl;
   a.stages = std::min({kTileMaxStages, kb_per, (kTileSmem - epi_bytes - 1024) / t.stage_bytes()});
@@ -83,11 +87,13 @@ cudaError_t launch_tile(const TileGemm& g, TileArgs a, TileShape t, int sms, uin
                           (PAIR ? 2 : 1) * a.cl, ma, mb, a, error_word);
 }
 
-// Width of the tiles, CTAs or pairs, and cluster, by a time model that was fitted to 3000 launches on B200 (M 128 to
-// 4096, eight weights of a layer, the three epilogues, chains of launches with weights from HBM).  Its choice took 1.4 %
-// longer than the best of the candidates on average; the figures below are the fit's, in cycles at 1.8 GHz and us:
+// Width of the tiles, CTAs or pairs, and cluster, by a time model fitted to launches on B200 in chains with weights from HBM.
+// Against every width, pair and cluster of 272 shapes (65 to 3072 rows, the linears of layers of hidden 1024 to 8192, ffn 3.5
+// times that) its choice takes 1.6 % longer than the best on average; the worst are K of 1024 and 2048, 27 to 33 % longer at
+// 1152 to 2048 rows, where the epilogue counts more than below.  In cycles at 1.8 GHz and us:
 //   * a K step takes the MMAs' time (2 cycles a column) or that of filling its stage: 71 bytes a cycle and 64 cycles on
-//     pairs, 83 and 19 on single CTAs;
+//     pairs, 83 and 19 on single CTAs.  A ring of two stages (single CTAs from 448 columns on) does not keep up: 1.04 us a step of
+//     512 columns instead of 0.6 (640 x 12288 x 8192 137 us against 103 of 256 columns), so three are wanted;
 //   * a round that is partly empty costs three quarters of a whole one (the rest comes back as clock or as memory
 //     bandwidth for the others);
 //   * the last epilogue, and each one where a single set of accumulators has to be drained first (above 256 columns), 0.6 us
@@ -118,6 +124,7 @@ void choose_tile(TileGemm& g, int sms, int pairs) {
       for (int bn = blocks ? 128 : 64; bn <= (c > 1 ? 256 : 512); bn += blocks ? 128 : (bn < 256 ? 16 : 32)) {
         const TileShape t{pair != 0, bn > 256 ? bn / 2 : bn, bn > 256 ? 2 : 1};
         if (blocks && t.sub % 128 != 0) continue;
+        if (3 * t.stage_bytes() > kTileSmem - kTileEpiBytes - 1024) continue;
         const int sub_out = silu ? t.sub / 2 : t.sub, out = t.nsub * sub_out;
         if (c > 1 && (sub_out % 16 != 0 || sub_out < 16 * c)) continue;
         const int n_out = silu ? g.b_rows / 2 : g.b_rows;

@@ -21,6 +21,16 @@ def test_a_cluster_that_nothing_can_share_is_left():
     assert ops.gemm_tile_choice(700, 512, 256, groups=3, cluster=2)[2] == 1  # (a group may have two row tiles)
 
 
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_a_ring_has_three_stages(epi):
+    """Single CTAs from 448 columns on have room for two, which is slower than any narrower tile."""
+    from penny_b200._ext import ops
+    for M in (65, 128, 384, 640, 1152, 2048, 4096):
+        for N, K in [(12288, 8192), (8192, 28672), (28672, 4096), (4096, 14336), (6144, 4096)]:
+            block_n, pair, _ = ops.gemm_tile_choice(M, N, K, epi)
+            assert pair == 1 or block_n < 448
+
+
 @pytest.mark.parametrize("pair,cluster", [(1, 0), (-1, 0), (1, 2), (-1, 2), (-1, 4), (0, 3), (0, 1)])
 @pytest.mark.parametrize("M,groups", [(1, 0), (385, 0), (100, 2)])
 def test_products(M, groups, pair, cluster):
