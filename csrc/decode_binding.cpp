@@ -237,7 +237,8 @@ void bind_decode(py::module_& m) {
   // above 0: gate/up and down with the weight on the M side (gemm_tile's pair 2) and tiles of that many rows.  The router meets
   // the library's GEMM only and may have any strides.
   m.def("moe_layer", [](at::Tensor x, at::Tensor router, const std::vector<at::Tensor>& w13, const std::vector<at::Tensor>& w2,
-                        int64_t topk, int64_t block_n, int64_t down_cluster, int64_t up_rows, int64_t down_rows) -> c10::optional<at::Tensor> {
+                        int64_t topk, int64_t block_n, int64_t down_cluster, int64_t up_rows,
+                        int64_t down_rows) -> c10::optional<at::Tensor> {
     if (!stacked(w13) || !stacked(w2)) return c10::nullopt;
     need(bf16_cuda(x) && x.dim() == 2 && ((uintptr_t)x.data_ptr() & 15) == 0, "moe_layer: 2-D aligned contiguous bf16 x");
     need(router.is_cuda() && router.scalar_type() == at::kBFloat16 && router.dim() == 2, "moe_layer: 2-D bf16 router");

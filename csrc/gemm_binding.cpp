@@ -112,8 +112,9 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq") = py::none(), py::arg("eps") = 1e-5, py::arg("residual") = py::none(), py::arg("norm_w") = py::none(),
      py::arg("sumsq_out") = py::none(), py::arg("stream_out") = py::none());
   // Tiled GEMM with a fused epilogue (csrc/gemm_tile_sm100.cu).  epi: 0 plain, 1 silu(gate) * up (b's gate
-  // rows before its up rows, or with silu_pairs, without ranges, as for gemm_decode; out [M, rows / 2]), 2 residual add.  ranges: [groups, 2] starts and ends or
-  // [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
+  // rows before its up rows, or with silu_pairs, without ranges, as for gemm_decode; out [M, rows / 2]; exact_silu, not
+  // with pair 2: with a division that is no approximation, also for gates below -87.3), 2 residual add.  ranges:
+  // [groups, 2] starts and ends or [groups + 1] borders of the rows of a and out that meet each group of b [groups * rows, K].  sumsq
   // [parts, M]: rows of a before their norm weight; every output is scaled by rsqrt(sum / K + eps).  pdl: may start,
   // and without ranges load b, while the kernel before it on the stream still runs, so that kernel must not write
   // b (a weight); everything else is waited for.  The residual may be fp32, stream_out then takes the sum in bf16 as
@@ -121,8 +122,7 @@ void bind_gemm(py::module_& m) {
   // hold sums of some columns each, which leaves the width of the tiles free.  block_n: columns of a tile; pair 1 / -1: CTA
   // pairs or single CTAs (0: pairs of 256 x 256 for block_n 512); cluster: CTAs or pairs that share a tile's K.  With block_n
   // 0 what is 0 of the three is chosen, a cluster taken where some width can be shared so.  pair 2: pairs with the weight on
-  // the M side and up to block_n rows of a (plain or silu).  exact_silu: silu with a division that is no approximation, also for gates below -87.3
-  // (not with pair 2).
+  // the M side and up to block_n rows of a (plain or silu).
   m.def("gemm_tile", [](at::Tensor a, at::Tensor b, at::Tensor out, int64_t epi, c10::optional<at::Tensor> ranges,
                         c10::optional<at::Tensor> sumsq, double eps, c10::optional<at::Tensor> residual,
                         c10::optional<at::Tensor> norm_w, c10::optional<at::Tensor> sumsq_out, int64_t block_n, bool pdl,
@@ -202,7 +202,8 @@ void bind_gemm(py::module_& m) {
      py::arg("sumsq_out") = py::none(), py::arg("block_n") = 0, py::arg("pdl") = false,
      py::arg("cluster") = 0, py::arg("stream_out") = py::none(), py::arg("pair") = 0,
      py::arg("silu_pairs") = false, py::arg("exact_silu") = false);
-  m.def("gemm_tile_choice", [](int64_t M, int64_t N, int64_t K, int64_t epi, int64_t groups, int64_t pair, int64_t cluster, bool silu_pairs) {
+  m.def("gemm_tile_choice", [](int64_t M, int64_t N, int64_t K, int64_t epi, int64_t groups, int64_t pair, int64_t cluster,
+                               bool silu_pairs) {
     penny::sm100::TileGemm g = {};
     g.M = (int)M;
     g.b_rows = (int)N;

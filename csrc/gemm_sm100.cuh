@@ -7,7 +7,7 @@
 //   * operands are K-major bf16 tiles of [rows x 64] elements (128-byte rows) in
 //     the 128-byte swizzle that TMA writes and tcgen05.mma reads; 8-row groups
 //     are 1024 bytes apart, tiles are 1024-byte aligned;
-//   * one elected thread issues TMA, one issues MMA, four warps drain TMEM;
+//   * one warp issues TMA, one issues MMA (an elected lane, or one thread), the others drain TMEM;
 //   * every wait is bounded: after `kSpinLimit` polls (and a wall-clock check)
 //     it returns false, the caller sets an error word and unwinds, and TMEM is
 //     always freed before the kernel exits.

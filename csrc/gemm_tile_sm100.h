@@ -9,7 +9,7 @@ namespace sm100 {
 enum TileEpilogue : int {
   TILE_EPI_PLAIN = 0,     // out[m][n] = acc
   TILE_EPI_SILU = 1,      // out[m][f] = silu(acc of gate row f) * (acc of up row f): b's rows are gate, then up (or silu_pairs)
-  TILE_EPI_RESIDUAL = 2,  // z = acc + residual; residual = z; out = z * norm_w; sumsq_out = sum z^2 per 128 columns
+  TILE_EPI_RESIDUAL = 2,  // z = acc + residual; residual = z; out = z * norm_w; sumsq_out = sums of z^2
 };
 
 // out = a * b^T (bf16, fp32 accumulation), a [M, K], b [groups * b_rows, K].
@@ -35,18 +35,19 @@ struct TileGemm {
   int scale_parts;
   float eps;
   void* residual;       // [M, b_rows], ldo; bf16, or with residual_fp32 fp32
-  bool residual_fp32;
+  bool residual_fp32;   // (the models of this package pass bf16)
   void* stream_out;     // residual_fp32: null, or [M, b_rows], ldo: the sum once more in bf16
   const void* norm_w;   // [b_rows]; null: only the residual add (out unused)
-  float* sumsq_out;     // [b_rows / 128][M], or with sumsq_cap > 0 [sumsq_cap][M]
+  float* sumsq_out;     // [b_rows / 128][M]: a sum for every 128 columns (which wants tiles of whole 128s; kept for callers
+                        // of that form), or with sumsq_cap > 0 [sumsq_cap][M]
   int sumsq_cap;        // above 0: the first rows of sumsq_out take one sum per tile, or CTA of a cluster, of its columns
                         // (launch_gemm_tile says how many rows): any width of tile will do, and a cluster shares out a
                         // tile's columns evenly
   int block_n;          // 0: choose; else the columns of a tile: a multiple of 16 up to 256, or of 32 up to 512 (two
                         // accumulators).  pair = 0: 512 stands for CTA pairs, 256 x 256
-  int pair;             // 0: by block_n, or choose with it; 1: CTA pairs, tiles of 256 rows; -1: single CTAs; 2: pairs with 256 rows of the
-                        // weight on the M side and tiles of up to block_n rows of a (a multiple of 16 up to 256, 0: 256),
-                        // plain or silu, no cluster
+  int pair;             // 0: by block_n, or choose with it; 1: CTA pairs, tiles of 256 rows; -1: single CTAs; 2: pairs
+                        // with 256 rows of the weight on the M side and tiles of up to block_n rows of a (a multiple of
+                        // 16 up to 256, 0: 256), plain or silu, no cluster
   int cluster;          // pairs or CTAs that split the K steps of a tile, up to 4; 1: none; 0: none, or with block_n = 0
                         // choose.  (block_n = 0: where some width can be shared so.)  With groups only for M <= the tile's rows
   bool pdl;             // may start, and without groups load b, while the kernel before it on the stream still runs:

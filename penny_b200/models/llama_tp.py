@@ -98,10 +98,10 @@ class LlamaTPDecoder:
         # timed.
         self.tiled_gate_up = asked == "auto" and world == 1 and max_batch > 176 and cfg.hidden >= 2048
         self.linears, self.pdl = linears, pdl
-        # LM head beside the library's linears (layers under hidden 2048, several ranks): on this library's tiles while one
-        # row tile of a CTA pair holds the batch.  Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 / 217 / 222 us against the library's
-        # 224 / 293 / 238 / 328; vocabularies of 65536 to 151936 and hidden 2048 to 8192: 0.95 to 1.5 times as fast,
-        # 1.2 on average.  Level at 192.  A second row tile that is partly filled costs a whole one: 257 / 384 / 512
+        # LM head beside the library's linears (batches above 128 rows, one rank or several): on this library's tiles while
+        # one row tile of a CTA pair holds the batch.  Hidden 4096 x vocabulary 128256, rows 193 / 208 / 224 / 256: 207 / 205 /
+        # 217 / 222 us against the library's 224 / 293 / 238 / 328; vocabularies of 65536 to 151936 and hidden 2048 to 8192:
+        # 0.95 to 1.5 times as fast, 1.2 on average.  Level at 192.  A second row tile that is partly filled costs a whole one: 257 / 384 / 512
         # / 1024 rows 359 / 374 / 524 / 858 against 263 / 307 / 499 / 836.  Smaller vocabulary shards (32000: 0.84 to
         # 1.2 times as fast, by hidden and rows) stay with the library.
         self.own_head = linears == "cublas" and 192 < max_batch <= 256 and cfg.vocab // world >= 1 << 16
@@ -161,8 +161,7 @@ class LlamaTPDecoder:
         self.parts = [buf(B, H, heap=True), buf(B, H, heap=True)]
         self.part = self.parts[0]
         if self.fold:
-            # (the tiled GEMM says how many rows of the second one its tiles filled)
-            self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // (16 if self.tiled else 128))]
+            self.sumsq = [torch.empty(n, B, dtype=torch.float32, device=self.dev) for n in (1, H // 128)]
             # The folded step's stream stays fp32 from layer to layer (the residual buffer takes it in bf16 at the end), for
             # 0.3 us a layer.  Logits of 8 / 32 random Llama-3-8B-shaped layers, distance from 64 bits (2-norm): 0.0142 /
             # 0.0293, with norms of their own and a bf16 stream 0.0189 / 0.0417.
@@ -211,7 +210,8 @@ class LlamaTPDecoder:
         1016 / 1090 / 1144).  Hidden 2048: 65 / 128 rows three 418 / 495 for 441 / 547; hidden 8192, two layers, 789 / 841 for
         840 / 922.  Smaller layers were not timed.  Larger batches are not folded: all five on tiles took 3 to 7 % longer at
         129 to 176 rows than the library's linears.  (They took 5 to 10 % less from 192 rows on.)"""
-        return frozenset(("qkv", "gate_up", "head")) if cfg.hidden >= 2048 and cfg.hidden % 128 == 0 and 64 < batch <= 128 else frozenset()
+        takes = cfg.hidden >= 2048 and cfg.hidden % 128 == 0 and 64 < batch <= 128
+        return frozenset(("qkv", "gate_up", "head")) if takes else frozenset()
 
     # ------------------------------------------------------------------ weights
     def _init_weights(self, seed: int, full_init: bool):
@@ -332,35 +332,30 @@ class LlamaTPDecoder:
             ops.gemm_decode(x[r:r + 1024], w, out[r:r + 1024], silu_pairs, 0, self.pdl, -1, 0, push)
 
     def _layers_folded(self, tokens):
-        """One rank: five launches per layer, each linear on the tiled or on the decode GEMM (`tiled_linears`).  x holds the residual stream times the next norm's weight, sumsq its
-        sums of squares; the linear that reads x scales its outputs by 1 / rms, so a norm is no pass of its own."""
+        """One rank: five launches per layer, q/k/v, gate/up and head on the tiled or on the decode GEMM (`tiled_linears`).  x
+        holds the residual stream times the next norm's weight, sumsq its sums of squares; the linear that reads x scales its
+        outputs by 1 / rms, so a norm is no pass of its own."""
         x, ss, eps, res, pdl = self.x, self.sumsq[0], self.cfg.eps, self.stream, self.pdl
-        tiled, parts = self.tiled, self.sumsq[1]
 
-        def linear(name, x, w, out, silu=False, **fold):
-            """The rows of the sums of squares that it wrote, for a linear with a residual."""
-            if name not in tiled:
-                if "residual" in fold:
-                    fold["sumsq_out"] = parts[:w.shape[0] // 128]
-                ops.gemm_decode(x, w, out, silu, pdl=pdl, eps=eps, **fold)
-                return fold.get("sumsq_out")
-            if "residual" not in fold:
-                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, eps=eps, silu_pairs=silu, exact_silu=silu, **fold)
-                return None
-            return parts[:ops.gemm_tile(x, w, out, 2, pdl=pdl, eps=eps, sumsq_out=parts, **fold)]
+        def scaled(name, w, out, ss, silu=False):
+            if name in self.tiled:
+                ops.gemm_tile(x, w, out, int(silu), pdl=pdl, sumsq=ss, eps=eps, silu_pairs=silu, exact_silu=silu)
+            else:
+                ops.gemm_decode(x, w, out, silu, pdl=pdl, sumsq=ss, eps=eps)
         ops.norm_prep(self.embed, self.layers[0]["norm1"], res, x, ss, ids=tokens)
         for li, L in enumerate(self.layers):
-            linear("qkv", x, L["wqkv"], self.qkv, sumsq=ss)
+            scaled("qkv", L["wqkv"], self.qkv, ss)
             ops.decode_attention_fused(self.qkv, self.kcache[li], self.vcache[li], self.positions, self.attn,
                                        self.workspace, self.Hq, self.Hkv, self.pieces, self.scale, self.cfg.rope_theta,
                                        pdl, balance=True)
-            ss = linear("o", self.attn, L["wo"], x, residual=res, norm_w=L["norm2"])
-            linear("gate_up", x, L["wgu"], self.act, True, sumsq=ss)
+            ss = self.sumsq[1]
+            ops.gemm_decode(self.attn, L["wo"], x, pdl=pdl, residual=res, norm_w=L["norm2"], sumsq_out=ss)
+            scaled("gate_up", L["wgu"], self.act, ss, silu=True)
             last = li + 1 == self.cfg.layers
-            ss = linear("down", self.act, L["wdown"], x, residual=res,
-                        norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
-                        stream_out=self.residual if last else None)
-        linear("head", x, self.lm_head, self.logits, sumsq=ss)
+            ops.gemm_decode(self.act, L["wdown"], x, pdl=pdl, residual=res, sumsq_out=ss,
+                            norm_w=self.final_norm if last else self.layers[li + 1]["norm1"],
+                            stream_out=self.residual if last else None)
+        scaled("head", self.lm_head, self.logits, ss)
 
     def _layers(self, warm_up: bool, separate: bool):
         cfg = self.cfg
