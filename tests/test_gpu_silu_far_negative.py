@@ -66,3 +66,11 @@ def test_step(batch):
     m.step(torch.zeros(batch, dtype=torch.int64))
     assert ops.gemm_error() == 0
     _close(m.act[:, :64], gates, (1.0 + m.cfg.eps) ** -0.5 if m.fold else 1.0)  # (a norm of its own rounds to bf16: to one)
+
+
+def test_where_an_exact_silu_is_refused():
+    from penny_b200._ext import ops
+    x, w = torch.zeros(16, 64, device="cuda").bfloat16(), torch.zeros(128, 64, device="cuda").bfloat16()
+    for out, epi, kw in ((torch.empty_like(x), 1, dict(pair=2)), (torch.empty(16, 128, device="cuda").bfloat16(), 0, {})):
+        with pytest.raises(RuntimeError):
+            ops.gemm_tile(x, w, out, epi, exact_silu=True, **kw)
