@@ -93,9 +93,9 @@ class LlamaTPDecoder:
             # and lets the norms ride in its epilogues.
             linears = "penny" if max_batch <= 128 else "cublas"
         # One rank beside the library's linears: gate/up on the tiled GEMM, whose epilogue takes silu * up.  8 layers and the
-        # head: 129 / 144 / 160 / 176 rows level to 2 % slower, 192 / 224 / 256 rows 1801 / 1613 / 2797 -> 1732 / 1528 / 2728 us (kv
-        # 300 / 16 / 1024); alone 512 rows 88 us against 98 and 8 for the kernel behind it.  Layers under hidden 2048 were not
-        # timed.
+        # head: 129 / 144 / 160 / 176 rows level to 2 % slower, 177 / 192 / 224 / 256 rows 1401 / 1693 / 1471 / 2661 -> 1352 / 1601 /
+        # 1383 / 2551 us (kv 100 / 300 / 16 / 1000; hidden 2048, ffn 8192: 668 / 758 / 668 / 1273 -> 668 / 748 / 651 / 1249);
+        # alone 512 rows 88 us against 98 and 8 for the kernel behind it.  Layers under hidden 2048 were not timed.
         self.tiled_gate_up = asked == "auto" and world == 1 and max_batch > 176 and cfg.hidden >= 2048
         self.linears, self.pdl = linears, pdl
         # LM head beside the library's linears (batches above 128 rows, one rank or several): on this library's tiles while
@@ -206,9 +206,9 @@ class LlamaTPDecoder:
 
         8 Llama-3-8B-shaped layers and the head, kv 100, us.  Up to 64 rows none (64: 948, with q/k/v, gate/up and head 963);
         to 128 rows those three, which have tiles for every SM, while o and down are a weight stream that the decode GEMM's
-        smaller CTAs begin under the launch before (65 / 96 / 128 rows: none 1010 / 1077 / 1157, three 984 / 1042 / 1093, all
-        1016 / 1090 / 1144).  Hidden 2048: 65 / 128 rows three 418 / 495 for 441 / 547; hidden 8192, two layers, 789 / 841 for
-        840 / 922.  Smaller layers were not timed.  Larger batches are not folded: all five on tiles took 3 to 7 % longer at
+        smaller CTAs begin under the launch before (65 / 80 / 96 / 128 rows: none 1014 / 1075 / 1130 / 1202, three 993 / 1051 /
+        1093 / 1143; all five, on another box, 1016 / 1090 / 1144 at 65 / 96 / 128 for three's 984 / 1042 / 1093).  Hidden 2048, ffn 8192:
+        65 / 128 rows three 467 / 543 for 477 / 590; hidden 8192, two layers, 789 / 841 for 840 / 922.  Smaller layers were not timed.  Larger batches are not folded: all five on tiles took 3 to 7 % longer at
         129 to 176 rows than the library's linears.  (They took 5 to 10 % less from 192 rows on.)"""
         takes = cfg.hidden >= 2048 and cfg.hidden % 128 == 0 and 64 < batch <= 128
         return frozenset(("qkv", "gate_up", "head")) if takes else frozenset()
