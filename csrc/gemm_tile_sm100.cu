@@ -34,7 +34,7 @@ int strip_tiles(int n_out, int sub_out, int nsub, int* tiles_n) {
 
 template <bool PAIR, int EPI, bool SPLIT, int NSUB>
 cudaError_t launch_tile(const TileGemm& g, TileArgs a, TileShape t, int sms, uint32_t* error_word, cudaStream_t stream) {
-  constexpr bool kSilu = EPI == TILE_EPI_SILU;
+  constexpr bool kSilu = EPI == TILE_EPI_SILU || EPI == kTileEpiSiluExact;
   const int sub_out = kSilu ? t.sub / 2 : t.sub;
   a.sub = t.sub;
   a.tiles_n = (a.n_out + t.nsub * sub_out - 1) / (t.nsub * sub_out);
@@ -221,7 +221,7 @@ cudaError_t launch_tile_epi(const TileGemm& g, TileArgs a, int sms, uint32_t* er
   t.nsub = block_n > 256 ? 2 : 1;
   t.sub = block_n / t.nsub;
   if (block_n < 32 || block_n > 512 || block_n % (16 * t.nsub) != 0) return cudaErrorInvalidValue;
-  const int sub_out = EPI == TILE_EPI_SILU ? t.sub / 2 : t.sub;
+  const int sub_out = EPI == TILE_EPI_SILU || EPI == kTileEpiSiluExact ? t.sub / 2 : t.sub;
   a.cl = std::max(1, std::min({g.cluster, kTileMaxCluster, a.num_kb}));
   a.ss_cols = EPI == TILE_EPI_RESIDUAL && g.norm_w != nullptr && g.sumsq_cap <= 0 ? 128 : 0;
   if (a.ss_cols > 0 && t.sub % a.ss_cols != 0) return cudaErrorInvalidValue;
@@ -276,7 +276,6 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   a.ldo = g.ldo;
   a.M = g.M;
   a.n_out = g.epi == TILE_EPI_SILU ? g.b_rows / 2 : g.b_rows;
-  a.exact_silu = g.exact_silu;
   a.num_kb = (g.K + kBlockK - 1) / kBlockK;
   a.groups = g.groups;
   a.b_rows = g.b_rows;
@@ -300,7 +299,9 @@ cudaError_t launch_gemm_tile(const TileGemm& g, uint32_t* error_word, cudaStream
   if (c.block_n == 0) return cudaErrorInvalidValue;
   switch (g.epi) {
     case TILE_EPI_PLAIN: return launch_tile_epi<TILE_EPI_PLAIN>(c, a, sms, error_word, stream, sumsq_rows);
-    case TILE_EPI_SILU: return launch_tile_epi<TILE_EPI_SILU>(c, a, sms, error_word, stream, sumsq_rows);
+    case TILE_EPI_SILU:
+      return g.exact_silu ? launch_tile_epi<kTileEpiSiluExact>(c, a, sms, error_word, stream, sumsq_rows)
+                          : launch_tile_epi<TILE_EPI_SILU>(c, a, sms, error_word, stream, sumsq_rows);
     case TILE_EPI_RESIDUAL: return launch_tile_epi<TILE_EPI_RESIDUAL>(c, a, sms, error_word, stream, sumsq_rows);
     default: return cudaErrorInvalidValue;
   }

@@ -42,13 +42,14 @@ constexpr int kTileMaxStages = 8;
 constexpr int kTileABytes = kBlockM * kBlockK * 2;
 constexpr int kPairRows = 64;  // gate rows, and up rows, of a block of a weight that holds them in turn
 
+constexpr int kTileEpiSiluExact = 3;  // TILE_EPI_SILU with exact_silu: kernels of their own
+
 struct TileArgs {
   __nv_bfloat16* out;
   int ldo, M, n_out;     // n_out: columns of out
   int num_kb, tiles_n, band;
   int groups, b_rows;
   int sub;               // columns of an accumulator (NSUB of them are a tile)
-  bool exact_silu;       // SILU: a division rounded once
   int strip_shift;       // SILU: -1, or (blocks of gate and up rows) log2 of the rows of a block in an accumulator
   int stages, accs;      // ring; sets of accumulators
   int tmem_cols;
@@ -103,7 +104,7 @@ template <bool PAIR, int EPI, bool SPLIT, int NSUB>
 __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const CUtensorMap& map_b, const TileArgs& a,
                                                uint32_t* error_word) {
   using Epi = TileEpi<EPI, SPLIT>;
-  constexpr bool kSilu = EPI == TILE_EPI_SILU, kRes = EPI == TILE_EPI_RESIDUAL;
+  constexpr bool kExact = EPI == kTileEpiSiluExact, kSilu = EPI == TILE_EPI_SILU || kExact, kRes = EPI == TILE_EPI_RESIDUAL;
   constexpr int kRows = PAIR ? 2 * kBlockM : kBlockM;
   constexpr int kChunk = Epi::kChunk, kRowBytes = Epi::kRowBytes;
   extern __shared__ unsigned char smem_raw[];
@@ -561,7 +562,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
           if (kSilu) {
             float up[kChunk];
             load_acc(i, 1, up);
-            if (a.exact_silu) {
+            if constexpr (kExact) {
               // The compiler's division branches for each quotient, and the zeros behind the last row take its slow side (8
               // layers and the head of a decode step, us, without an exact quotient / with a division: 65 rows 1031 / 1137, 128
               // 1197 / 1226, 192 1701 / 1804).  Gates in the ordinary range take silu_near (65 rows 1052 / 1066, 128 1207 / 1203,
