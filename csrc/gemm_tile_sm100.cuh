@@ -565,8 +565,9 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap& map_a, const C
             if constexpr (kExact) {
               // The compiler's division branches for each quotient, and the zeros behind the last row take its slow side (8
               // layers and the head of a decode step, us, without an exact quotient / with a division: 65 rows 1031 / 1137, 128
-              // 1197 / 1226, 192 1701 / 1804).  Gates in the ordinary range take silu_near (65 rows 1052 / 1066, 128 1207 / 1203,
-              // 192 1727 / 1729); one outside it brings its warp's pass to the division.
+              // 1197 / 1226, 192 1701 / 1804).  Gates in the ordinary range take silu_near (65 rows 1045 / 1052, 128 1192 / 1194,
+              // 192 1710 / 1715); one outside it brings its warp's pass to the division.  (As a run-time branch this cost the
+              // launches without it 0.5 to 1 %: gate/up of one expert 52.7 -> 53.2 us.)
               bool near = true;
 #pragma unroll
               for (int j = 0; j < kChunk; ++j) near &= fabsf(v[j] * scale) <= kNearGate;
